@@ -3,12 +3,13 @@
 //   k_pyramid       every pyramid level as f32 rows of 16-byte pitch (level 0 =
 //                   u8 / 255, levels >= 1 one bilinear tap of LOD0): the
 //                   source of k_detect's tile loads
-//   k_detect   (K1) TMA-staged level tile + halo, FAST response + cull, blur
-//                   cache (or, in the cfg profile, FAST 9-of-16 at 20/255 +
-//                   3x3 NMS)
-//   k_blur_border   blur cache beyond the level edges (BRIEF points outside)
+//   k_detect   (K1) TMA-staged level tile + halo, FAST response + cull (or, in
+//                   the cfg profile, FAST 9-of-16 at 20/255 + 3x3 NMS)
 //   k_band_count, k_band_write
-//                   ordered keypoint compaction over 32-row bands, cap
+//                   ordered keypoint compaction over 32-row bands, cap; the
+//                   list of blur tiles that the kept keypoints' tests read
+//   k_blur          blur cache of the listed tiles, inside the level and
+//                   beyond its edges (BRIEF points outside)
 //   k_xsort         the matcher's lists: per horizontal band an x-sorted
 //                   candidate list, and the band-grouped query order
 //   k_describe (K2) orientation (one lane per keypoint of a warp's group) +
@@ -213,8 +214,8 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
     return false;
 }
 // 2D tiled TMA load of the map's box at element coordinates (x, y) into
-// shared memory, completing on the barrier (x * 4 bytes is 32-byte aligned
-// for every caller: x = tile origin - 8, tile widths multiples of 32).
+// shared memory, completing on the barrier (x * 4 bytes is 16-byte aligned
+// for every caller: x = tile origin - 8 or - 4, tile widths multiples of 32).
 __device__ __forceinline__ void tma_load_2d(void* dst, const void* tmap, int x, int y, uint64_t* bar) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::
@@ -329,13 +330,7 @@ k_pyramid(const FrameDev* __restrict__ frames, const TileItem* __restrict__ tile
 // ---------------------------------------------------------------- K1 ----
 // One TW x TH tile of one level: one TMA load stages the level pixels plus
 // halo (written by k_pyramid) in shared memory, then per pixel the FAST
-// response, the cull decision and the blur-cache value G(x, y).  The blur
-// taps' sampling coordinates depend only on the row or only on the column,
-// so they are computed once per tile row / column (same operations as the
-// per-pixel formula, hence the same bits).
-// Six CTAs per SM (40 registers, no spills): 0.700 against 0.718 ms at five
-// (48 registers) and 0.712 at four on the 64-frame step; seven spill.  The
-// cfg profile's form spills at 40 and keeps five.
+// response and the cull decision.
 template <int TW, int TH, bool CFG>
 __global__ void __launch_bounds__(K1_THREADS, CFG ? 5 : 6)
 k_detect(const FrameDev* __restrict__ frames, const TileItem* __restrict__ tiles, int shape, uint32_t* err) {
@@ -347,59 +342,23 @@ k_detect(const FrameDev* __restrict__ frames, const TileItem* __restrict__ tiles
     static_assert(K1_THREADS % TW == 0 && CX >= 0 && (BW * 4) % 16 == 0 && BW <= 256 && SH <= 256, "tile shape");
     __shared__ __align__(128) float sbox[SH][BW];
     __shared__ __align__(8) uint64_t s_bar;
-    __shared__ int s_by0[3][TH], s_by1[3][TH];   // blur taps: staged rows per output row
-    // blur taps, y weights per output row as pairs: rows j = 0, 1 side by
-    // side, and row j = 2 twice
-    __shared__ float2 s_b01[TH], s_nb01[TH], s_b22[TH], s_nb22[TH];
     __shared__ float s_score[CFG ? TH + 2 : 1][CFG ? TW + 2 : 1];  // cfg: FAST score, tile + 1 ring
     __shared__ uint8_t s_arc[CFG ? TH + 2 : 1][CFG ? TW + 2 : 1];
-    __shared__ uint8_t s_rowfast[TH];  // row taps at fixed offsets (no edge clamp)
     const TileItem it = tiles[blockIdx.x];
     const FrameDev& F = frames[it.frame];
     const int l = it.level;
     const int w = F.w[l], h = F.h[l];
     const int X0 = it.tx * TW, Y0 = it.ty * TH;
     const int t = threadIdx.x;
-    const float tex_x = 1.0f / (float)w;
-    const float tex_y = 1.0f / (float)h;
-    const float off[3] = {-1.2f, 0.0f, 1.2f};
 
-    // 0. one thread starts the tile load; the others build the tap tables
-    //    meanwhile.  Box cells outside the level arrive as 0 and are
-    //    replaced below.
+    // 0. one thread starts the tile load.  Box cells outside the level arrive
+    //    as 0 and are replaced below.
     if (t == 0) {
         const void* tmap = static_cast<const char*>(F.tmaps) +
                            (size_t)(l * USLAM_TMAPS_PER_LEVEL + shape) * USLAM_TMAP_BYTES;
         mbar_init(&s_bar, 1u);
         mbar_expect_tx(&s_bar, (uint32_t)(SH * BW * 4));
         tma_load_2d(&sbox[0][0], tmap, X0 - USLAM_TILE_XPAD, Y0 - HY, &s_bar);
-    }
-    for (int i = t; i < TH; i += K1_THREADS) s_rowfast[i] = 1;
-    __syncthreads();
-    for (int i = t; i < 3 * TH; i += K1_THREADS) {
-        // generate_features.wgsl:153-169, y part of the 9 taps
-        const int ty = i / 3, k = i % 3;
-        const float uvy = ((float)(Y0 + ty) + 0.5f) * tex_y;
-        const float offk = k == 0 ? -1.2f : (k == 1 ? 0.0f : 1.2f);
-        const float v = (uvy + offk * tex_y) * (float)h - 0.5f;
-        const float fj = floorf(v);
-        int r0 = edge_index(fj, h) - (Y0 - HY), r1 = edge_index(fj + 1.0f, h) - (Y0 - HY);
-        if (Y0 + ty < h && (r0 < 0 || r1 >= SH)) atomicOr(err, USLAM_ERR_SMEM_RANGE);
-        const float b = v - fj, nb = 1.0f - b;
-        if (k == 2) {
-            s_b22[ty] = make_float2(b, b);
-            s_nb22[ty] = make_float2(nb, nb);
-        } else {
-            reinterpret_cast<float*>(&s_b01[ty])[k] = b;
-            reinterpret_cast<float*>(&s_nb01[ty])[k] = nb;
-        }
-        s_by0[k][ty] = min(max(r0, 0), SH - 1);
-        s_by1[k][ty] = min(max(r1, 0), SH - 1);
-        // the row taps of an interior row sit at rows -2, -1 | d, d + 1 | 1, 2
-        // around the pixel (d = -1 or 0): no edge clamp
-        const int rr = ty + HY, e = k == 0 ? -2 : (k == 1 ? r0 - rr : 1);
-        const bool ok = r1 == r0 + 1 && r0 == rr + e && (k != 1 || e == -1 || e == 0);
-        if (!ok) s_rowfast[ty] = 0;
     }
     __syncthreads();  // the barrier is initialised before anyone polls it
     const uint32_t first_limit = F.detect_first_wait < 0 ? kTmaWaitLimit : (uint32_t)F.detect_first_wait;
@@ -457,45 +416,9 @@ k_detect(const FrameDev* __restrict__ frames, const TileItem* __restrict__ tiles
     const int tx = t % TW;
     const int x = X0 + tx;
     if (x >= w) return;
-    // blur taps, x part (this thread's column is fixed)
-    int ix0[3], ix1[3];
-    float ax[3];
-    {
-        const float uvx = ((float)x + 0.5f) * tex_x;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            const float u = (uvx + off[k] * tex_x) * (float)w - 0.5f;
-            const float fi = floorf(u);
-            ax[k] = u - fi;
-            int c0 = edge_index(fi, w) - (X0 - HX), c1 = edge_index(fi + 1.0f, w) - (X0 - HX);
-            if (c0 < 0 || c1 >= SW) atomicOr(err, USLAM_ERR_SMEM_RANGE);
-            ix0[k] = min(max(c0, 0), SW - 1);
-            ix1[k] = min(max(c1, 0), SW - 1);
-        }
-    }
-    // the column taps of an interior column sit at -2, -1 | d, d + 1 | 1, 2
-    // around the pixel (d = dcx = -1 or 0): no edge clamp (warp-uniform flag)
-    const int cc = tx + HX, dcx = ix0[1] - cc;
-    const bool colfast = __all_sync(__activemask(), ix0[0] == cc - 2 && ix1[0] == cc - 1 && (dcx == -1 || dcx == 0) &&
-                                                        ix1[1] == ix0[1] + 1 && ix0[2] == cc + 1 && ix1[2] == cc + 2);
     const uint32_t* mask = F.mask[l];
     uint8_t* const kpmap = F.kpmap[l];
-    float* const blur = F.blur[l];
-    const int kp_pitch = F.kp_pitch[l], bl_pitch = F.bl_pitch[l];
-    // x weights of the taps as pairs: (a_i, a_i) and (1 - a_i, 1 - a_i) for
-    // the pairs (i, j = 0 | 1), and (a_0, a_1), (1 - a_0, 1 - a_1) for the pair
-    // (i = 0 | 1, j = 2); tap weights 0.3125, 0.375, 0.3125
-    float2 pa[3], pna[3];
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        pa[i] = make_float2(ax[i], ax[i]);
-        pna[i] = make_float2(1.0f - ax[i], 1.0f - ax[i]);
-    }
-    const float2 pa01 = make_float2(ax[0], ax[1]);
-    const float2 pna01 = make_float2(1.0f - ax[0], 1.0f - ax[1]);
-    const float2 wt_same[3] = {make_float2(0.3125f, 0.3125f), make_float2(0.375f, 0.375f),
-                               make_float2(0.3125f, 0.3125f)};
-    const float2 wt01 = make_float2(0.3125f, 0.375f);
+    const int kp_pitch = F.kp_pitch[l];
     for (int ty = t / TW; ty < TH; ty += K1_THREADS / TW) {
         const int y = Y0 + ty;
         if (y >= h) break;
@@ -538,85 +461,328 @@ k_detect(const FrameDev* __restrict__ frames, const TileItem* __restrict__ tiles
             }
         }
         kpmap[(size_t)y * kp_pitch + x] = (uint8_t)keep;
+    }
+}
 
-        // 3. blur cache: G(x, y) of generate_features.wgsl:149-172.  Tap (i, j)
-        // is sv = (na nb) T00 + (a nb) T10 + (na b) T01 + (a b) T11 summed
-        // left to right, then q = (sv wt_i) wt_j, and G = the q summed j-major,
-        // i-minor from 0.  The products of two taps run as packed pairs
-        // ((i, 0) with (i, 1), and (0, 2) with (1, 2)); every lane is the scalar
-        // product, and the sums are scalar in the written order.
-        // texel(i, j, e, f): T of tap (i, j), e = row 0 / 1, f = column 0 / 1.
-        const auto blur_value = [&](auto texel) -> float {
-            float q[3][3];
-            {
-                const float2 b01 = s_b01[ty], nb01 = s_nb01[ty];
+// -------------------------------------------------------------- blur ----
+// The blur cache G(P) of generate_features.wgsl:149-172 at every integer
+// point a described keypoint's tests can read.  9 bilinear taps at offsets
+// -1.2, 0, 1.2: tap (i, j) is sv = (na nb) T00 + (a nb) T10 + (na b) T01 +
+// (a b) T11 summed left to right, q = (sv wt_i) wt_j, and G = the q summed
+// j-major, i-minor.  The sampling coordinates of a tap depend only on the
+// column or only on the row.
+//
+// The samples of a keypoint lie within R = margin - 1 of it, so a run needs
+// only the tiles that k_band_write listed: 71 % of the pixels on the 752x480
+// workload (the level caps keep the first features in (y, x) order, so the
+// lower part of most levels holds none), 55 % at 1920x1080 and a few per cent
+// where a frame cap of 20000 is used up by the first level of a 4K frame.
+// 64 frames of 752x480: 0.24 ms here and 0.31 in k_detect, where evaluating
+// every pixel in k_detect and the margins in a kernel of their own took 0.72
+// and 0.20; 8 frames of 3840x2160 with that cap: 0.16 and 0.59 against 1.77
+// and 0.13.
+constexpr int KBL_THREADS = 128;
+constexpr int KBL_TW = USLAM_BLUR_TW, KBL_TH = USLAM_BLUR_TH;
+constexpr int KBL_HY = USLAM_BLUR_HY, KBL_XPAD = USLAM_BLUR_XPAD;
+constexpr int KBL_SH = KBL_TH + 2 * KBL_HY;    // staged rows [Y0 - HY, Y0 + TH + HY)
+constexpr int KBL_BW = KBL_TW + 2 * KBL_XPAD;  // staged columns [X0 - XPAD, X0 + TW + XPAD)
+constexpr int KBL_CTAS_PER_SM = 6;
+static_assert(KBL_TW == 2 * 32 && KBL_THREADS % 32 == 0, "a warp covers a tile row, two columns a lane");
+
+// Tap k = 0, 1, 2 of coordinate c in a level of n pixels: the lower texel
+// (before the edge clamp) and the upper one's weight.
+__device__ __forceinline__ float blur_tap(uint32_t c, int k, int n, float* weight) {
+    const float tex = 1.0f / (float)n;
+    const float off = k == 0 ? -1.2f : (k == 1 ? 0.0f : 1.2f);
+    const float u = (((float)c + 0.5f) * tex + off * tex) * (float)n - 0.5f;
+    const float f = floorf(u);
+    *weight = u - f;
+    return f;
+}
+
+// G at (px, py), taps read from the level in global memory: the cells beyond
+// the level, where a coordinate of 0xffffffff stands for every negative one
+// (u32 wrap: the same f32 2^32 for all of them).
+__device__ __noinline__ float blur_cell(const float* lvl, int lp, int w, int h, uint32_t px, uint32_t py) {
+    float a[3], b[3];
+    int x0[3], x1[3];
+    const float *r0[3], *r1[3];
 #pragma unroll
-                for (int i = 0; i < 3; ++i) {
-                    const float2 t00 = make_float2(texel(i, 0, 0, 0), texel(i, 1, 0, 0));
-                    const float2 t10 = make_float2(texel(i, 0, 0, 1), texel(i, 1, 0, 1));
-                    const float2 t01 = make_float2(texel(i, 0, 1, 0), texel(i, 1, 1, 0));
-                    const float2 t11 = make_float2(texel(i, 0, 1, 1), texel(i, 1, 1, 1));
-                    const float2 sv = sum4(mul2_rn(mul2_rn(pna[i], nb01), t00), mul2_rn(mul2_rn(pa[i], nb01), t10),
-                                           mul2_rn(mul2_rn(pna[i], b01), t01), mul2_rn(mul2_rn(pa[i], b01), t11));
-                    const float2 qq = mul2_rn(mul2_rn(sv, wt_same[i]), wt01);
-                    q[0][i] = qq.x;
-                    q[1][i] = qq.y;
+    for (int k = 0; k < 3; ++k) {
+        const float fi = blur_tap(px, k, w, &a[k]), fj = blur_tap(py, k, h, &b[k]);
+        x0[k] = edge_index(fi, w);
+        x1[k] = edge_index(fi + 1.0f, w);
+        r0[k] = lvl + (size_t)edge_index(fj, h) * lp;
+        r1[k] = lvl + (size_t)edge_index(fj + 1.0f, h) * lp;
+    }
+    float sum = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const float na = 1.0f - a[i], nb = 1.0f - b[j];
+            float sv = (na * nb) * __ldg(r0[j] + x0[i]);
+            sv = sv + (a[i] * nb) * __ldg(r0[j] + x1[i]);
+            sv = sv + (na * b[j]) * __ldg(r1[j] + x0[i]);
+            sv = sv + (a[i] * b[j]) * __ldg(r1[j] + x1[i]);
+            sum = sum + (sv * (i == 1 ? 0.375f : 0.3125f)) * (j == 1 ? 0.375f : 0.3125f);
+        }
+    return sum;
+}
+
+// Two binary32 values side by side (sm_100 family f32x2 operands).
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+    f32x2 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
+    return d;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+    float2 d;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(v));
+    return d;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+// Packed sum: p * 1 + q with the 1 unknown to the compiler, so each lane is
+// rounded once, exactly as add.rn (p * 1 is exact), and the product that made
+// p keeps its own rounding (see mul2_rn).
+__device__ __forceinline__ f32x2 add2(f32x2 p, f32x2 q, f32x2 one) {
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(p), "l"(one), "l"(q));
+    return d;
+}
+
+// Persistent over the list: a CTA's first two items are fixed, the later ones
+// claimed (items cost different amounts), and the next tile's TMA load is
+// issued while this one is computed.
+//
+// A tile costs 36 weight products, 36 texel products, 18 tap weights and 35
+// sums a pixel on the FMA pipe, which bounds it (a packed operation holds the
+// pipe for two cycles, so packing saves issue slots only).  What is saved is
+// work on values that repeat, with every remaining operation as written:
+//  * the weights (b, 1 - b) of a row tap take about ten values in a whole
+//    level and equal the row above's in two rows of three, so the twelve
+//    products with the column weights are kept from row to row;
+//  * the middle row tap sits on the row itself (b = 0 exactly) in three rows
+//    of four: its products with 1 - b = 1 are the column weights and its lower
+//    row adds zeros;
+//  * a lane takes two adjacent columns as the halves of packed operations and
+//    four rows: the 6 columns its taps touch are three aligned 8-byte shared
+//    loads, and the rows of the outer taps are shared by consecutive rows.
+// The taps of a pixel sit at -2, -1 | d, d + 1 | 1, 2 around it, d = -1 or 0
+// per row and per column by rounding (a tile that holds another pixel takes
+// blur_cell throughout), and the staged cells beyond the level hold the edge
+// texel, so edge pixels take the same path.  one_f is 1.0f (see add2).
+__global__ void __launch_bounds__(KBL_THREADS, KBL_CTAS_PER_SM)
+k_blur(const FrameDev* __restrict__ frames, BlurList bl, uint32_t* err, float one_f) {
+    constexpr int ROWS = 4;  // rows of a warp at a time
+    __shared__ __align__(128) float sbox[2][KBL_SH][KBL_BW];
+    __shared__ __align__(8) uint64_t s_bar[2];
+    __shared__ __align__(16) float4 s_w[3][KBL_TH];  // (b, b, nb, nb) of the row taps
+    __shared__ __align__(8) float s_a[3][KBL_TW];    // upper weights of the column taps
+    __shared__ int s_dy[KBL_TH];                     // offset of the middle tap's rows
+    __shared__ __align__(2) int8_t s_dx[KBL_TW];     // offset of the middle tap's columns
+    __shared__ uint32_t s_claim[2];
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const uint32_t n = __ldcg(bl.count);
+    const f32x2 one = pack2(one_f, one_f);
+    auto fetch = [&](const TileItem& it, int buf) {  // one thread
+        if (it.pad != USLAM_BLUR_TILE) return;
+        const void* tmap = static_cast<const char*>(frames[it.frame].tmaps) +
+                           (size_t)(it.level * USLAM_TMAPS_PER_LEVEL + USLAM_TMAP_BLUR) * USLAM_TMAP_BYTES;
+        mbar_expect_tx(&s_bar[buf], (uint32_t)(KBL_SH * KBL_BW * 4));
+        tma_load_2d(&sbox[buf][0][0], tmap, it.tx * KBL_TW - KBL_XPAD, it.ty * KBL_TH - KBL_HY, &s_bar[buf]);
+    };
+    if (blockIdx.x >= n) return;
+    TileItem it = bl.items[blockIdx.x];
+    if (t == 0) {
+        mbar_init(&s_bar[0], 1u);
+        mbar_init(&s_bar[1], 1u);
+        fetch(it, 0);
+    }
+    __syncthreads();  // the barriers are initialised before anyone polls them
+    uint32_t phase = 0u;  // bit b: parity of buffer b's next load
+    int cur = 0;
+    uint32_t inext = blockIdx.x + gridDim.x;
+    while (true) {
+        const bool more = inext < n;
+        TileItem next{};
+        if (more) next = bl.items[inext];
+        uint32_t claimed = 0;
+        if (more && t == 0) {
+            fetch(next, cur ^ 1);  // that buffer was read before the last barrier
+            claimed = 2u * gridDim.x + atomicAdd(bl.count + 1, 1u);
+        }
+        const FrameDev& F = frames[it.frame];
+        const int l = it.level;
+        const int w = F.w[l], h = F.h[l], bp = F.bl_pitch[l];
+        float* const blur = F.blur[l];
+        const int X0 = it.tx * KBL_TW, Y0 = it.ty * KBL_TH;
+        bool regular = it.pad == USLAM_BLUR_TILE;
+        int c0 = X0, r0 = Y0, nc = min(KBL_TW, w - X0), nr = min(KBL_TH, h - Y0);  // the item's cells
+        if (regular) {
+            float a;
+            // taps of the tile's columns (threads 0 .. 63) and rows (64 .. 95)
+            if (t < KBL_TW + KBL_TH) {
+                const bool column = t < KBL_TW;
+                const int c = column ? t : t - KBL_TW, x = (column ? X0 : Y0) + c, size = column ? w : h;
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    const int d = (int)blur_tap((uint32_t)x, k, size, &a) - x;
+                    if (column) s_a[k][c] = a;
+                    else s_w[k][c] = make_float4(a, a, 1.0f - a, 1.0f - a);
+                    if (k == 1 && column) s_dx[c] = (int8_t)d;
+                    if (k == 1 && !column) s_dy[c] = d;
+                    regular = regular && (k == 0 ? d == -2 : (k == 1 ? d == -1 || d == 0 : d == 1));
                 }
             }
-            {
-                const float2 b22 = s_b22[ty], nb22 = s_nb22[ty];
-                const float2 t00 = make_float2(texel(0, 2, 0, 0), texel(1, 2, 0, 0));
-                const float2 t10 = make_float2(texel(0, 2, 0, 1), texel(1, 2, 0, 1));
-                const float2 t01 = make_float2(texel(0, 2, 1, 0), texel(1, 2, 1, 0));
-                const float2 t11 = make_float2(texel(0, 2, 1, 1), texel(1, 2, 1, 1));
-                const float2 sv = sum4(mul2_rn(mul2_rn(pna01, nb22), t00), mul2_rn(mul2_rn(pa01, nb22), t10),
-                                       mul2_rn(mul2_rn(pna01, b22), t01), mul2_rn(mul2_rn(pa01, b22), t11));
-                const float2 qq = mul2_rn(mul2_rn(sv, wt01), wt_same[2]);
-                q[2][0] = qq.x;
-                q[2][1] = qq.y;
-                const float a = ax[2], na = pna[2].x, b = b22.x, nb = nb22.x;
-                float s2 = (na * nb) * texel(2, 2, 0, 0);
-                s2 = s2 + (a * nb) * texel(2, 2, 0, 1);
-                s2 = s2 + (na * b) * texel(2, 2, 1, 0);
-                s2 = s2 + (a * b) * texel(2, 2, 1, 1);
-                q[2][2] = (s2 * 0.3125f) * 0.3125f;
+            const bool landed = mbar_wait(&s_bar[cur], (phase >> cur) & 1u, kTmaWaitLimit);
+            if (__syncthreads_or(!landed)) {
+                if (t == 0) atomicOr(err, USLAM_ERR_TMA_TIMEOUT);
+                // the copies in flight land before the CTA leaves
+                mbar_wait(&s_bar[cur], (phase >> cur) & 1u, kTmaWaitLimit);
+                if (more && next.pad == USLAM_BLUR_TILE) mbar_wait(&s_bar[cur ^ 1], (phase >> (cur ^ 1)) & 1u, kTmaWaitLimit);
+                return;
             }
-            float sum = 0.0f;
-#pragma unroll
-            for (int j = 0; j < 3; ++j)
-#pragma unroll
-                for (int i = 0; i < 3; ++i) sum = sum + q[j][i];
-            return sum;
-        };
-        float sum;
-        if (colfast && s_rowfast[ty]) {
-            // interior: the taps sit at rows / columns -2, -1 | d, d + 1 | 1, 2
-            // around the pixel (d = -1 or 0, per column dcx, per row dry), so
-            // every load is one of four base pointers plus a constant
-            const float* P = &sm[r][c];
-            const int dry = s_by0[1][ty] - r;
-            const float* Px = P + dcx;
-            const float* Py = P + dry * BW;
-            const float* Pxy = Py + dcx;
-            sum = blur_value([&](int i, int j, int e, int f) -> float {
-                const float* base = i == 1 ? (j == 1 ? Pxy : Px) : (j == 1 ? Py : P);
-                const int ro = (j == 0 ? -2 : (j == 1 ? 0 : 1)) + e;
-                const int co = (i == 0 ? -2 : (i == 1 ? 0 : 1)) + f;
-                return base[ro * BW + co];
-            });
+            phase ^= 1u << cur;
+            // cells up to two beyond the level take the edge texel
+            if (X0 == 0 || X0 + KBL_TW + 2 > w || Y0 == 0 || Y0 + KBL_TH + 2 > h) {
+                float(*sm)[KBL_BW] = sbox[cur];
+                const int x1 = min(X0 + KBL_TW, w), y1 = min(Y0 + KBL_TH, h);  // one past the tile's cells
+                auto edge = [&](int gy, int gx) {
+                    const int ey = min(max(gy, 0), h - 1), ex = min(max(gx, 0), w - 1);
+                    if (ey != gy || ex != gx)  // (the texel is inside the level, so no thread writes it, and in the box)
+                        sm[gy - Y0 + KBL_HY][gx - X0 + KBL_XPAD] = sm[ey - Y0 + KBL_HY][ex - X0 + KBL_XPAD];
+                };
+                // the two rows above and below over the tile's columns and two
+                // each side, the two columns left and right over its rows
+                for (int q = t; q < 4 * (x1 - X0 + 4); q += KBL_THREADS)
+                    edge((q & 2) ? y1 + (q & 1) : Y0 - 2 + (q & 1), X0 - 2 + (q >> 2));
+                for (int q = t; q < 4 * (y1 - Y0); q += KBL_THREADS)
+                    edge(Y0 + (q >> 2), (q & 2) ? x1 + (q & 1) : X0 - 2 + (q & 1));
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // a later load writes here again
+            }
+            regular = __syncthreads_and(regular);
+        } else if (it.pad == USLAM_BLUR_RIGHT) {
+            c0 = w;
+            nc = F.margin;
+        } else if (it.pad == USLAM_BLUR_BELOW) {
+            r0 = h;
+            nr = F.margin;
+            nc = min(KBL_TW, w + F.margin + 1 - c0);
+        } else if (it.pad == USLAM_BLUR_COL) {
+            c0 = w + F.margin;
+            nc = 1;
+            r0 = it.ty * USLAM_BLUR_RUN;
+            nr = min(USLAM_BLUR_RUN, h - r0);
         } else {
-            const float* row0[3];
-            const float* row1[3];
-#pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                row0[j] = sm[s_by0[j][ty]];
-                row1[j] = sm[s_by1[j][ty]];
-            }
-            sum = blur_value([&](int i, int j, int e, int f) -> float {
-                return (e ? row1[j] : row0[j])[f ? ix1[i] : ix0[i]];
-            });
+            r0 = h + F.margin;
+            nr = 1;
+            c0 = it.tx * USLAM_BLUR_RUN;
+            nc = min(USLAM_BLUR_RUN, w + F.margin + 1 - c0);
         }
-        blur[(size_t)y * bl_pitch + x] = sum;
+        if (regular) {
+            const int x = X0 + 2 * lane;
+            f32x2 pa[3], pna[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const float2 a = *reinterpret_cast<const float2*>(&s_a[k][2 * lane]);
+                pa[k] = pack2(a.x, a.y);
+                pna[k] = pack2(1.0f - a.x, 1.0f - a.y);
+            }
+            const char2 dx = *reinterpret_cast<const char2*>(&s_dx[2 * lane]);
+            const f32x2 w3 = pack2(0.3125f, 0.3125f), w4 = pack2(0.375f, 0.375f);
+            // the left and right texels of the three column taps in a staged row
+            auto texels = [&](const float* p, f32x2 (&lt)[3], f32x2 (&rt)[3]) {
+                lt[0] = *reinterpret_cast<const f32x2*>(p - 2);
+                const f32x2 mid = *reinterpret_cast<const f32x2*>(p);
+                rt[2] = *reinterpret_cast<const f32x2*>(p + 2);
+                const float2 f0 = unpack2(lt[0]), f1 = unpack2(mid), f2 = unpack2(rt[2]);
+                rt[0] = pack2(f0.y, f1.x);
+                lt[2] = pack2(f1.y, f2.x);
+                lt[1] = pack2(dx.x ? f0.y : f1.x, dx.y ? f1.x : f1.y);
+                rt[1] = pack2(dx.x ? f1.x : f1.y, dx.y ? f1.y : f2.x);
+            };
+            for (int ty0 = warp * ROWS; ty0 < nr; ty0 += KBL_THREADS / 32 * ROWS) {
+                const float* const col = &sbox[cur][KBL_HY + ty0][2 * lane + KBL_XPAD];
+                f32x2 sum[ROWS];
+#pragma unroll
+                for (int j = 0; j < 3; ++j) {
+                    const f32x2 wj = j == 1 ? w4 : w3;
+                    f32x2 w00[3], w10[3], w01[3], w11[3];  // the products of the column and row weights
+                    f32x2 lt[2][3], rt[2][3];
+                    ulonglong2 had = make_ulonglong2(0ull, 0ull);
+                    if (j != 1) texels(col + (j == 0 ? -2 : 1) * KBL_BW, lt[0], rt[0]);
+#pragma unroll
+                    for (int r = 0; r < ROWS; ++r) {
+                        const ulonglong2 wr = *reinterpret_cast<const ulonglong2*>(&s_w[j][ty0 + r]);
+                        if (j == 1 && wr.x == 0ull) {
+                            // b = 0: one row, weights 1 - a and a
+                            texels(col + (r + s_dy[ty0 + r]) * KBL_BW, lt[0], rt[0]);
+#pragma unroll
+                            for (int k = 0; k < 3; ++k) {
+                                const f32x2 sv = add2(mul2(pa[k], rt[0][k]), mul2(pna[k], lt[0][k]), one);
+                                sum[r] = add2(mul2(mul2(sv, k == 1 ? w4 : w3), wj), sum[r], one);
+                            }
+                            continue;
+                        }
+                        const int u = j == 1 ? 0 : r & 1, d = u ^ 1;  // the upper and the lower row's texels
+                        if (j == 1) {
+                            const float* p = col + (r + s_dy[ty0 + r]) * KBL_BW;
+                            texels(p, lt[0], rt[0]);
+                            texels(p + KBL_BW, lt[1], rt[1]);
+                        } else {
+                            texels(col + (r + (j == 0 ? -1 : 2)) * KBL_BW, lt[d], rt[d]);
+                        }
+                        if (j == 1 || r == 0 || wr.x != had.x) {  // (equal b, equal 1 - b)
+#pragma unroll
+                            for (int k = 0; k < 3; ++k) {
+                                w00[k] = mul2(pna[k], wr.y);
+                                w10[k] = mul2(pa[k], wr.y);
+                                w01[k] = mul2(pna[k], wr.x);
+                                w11[k] = mul2(pa[k], wr.x);
+                            }
+                            had = wr;
+                        }
+#pragma unroll
+                        for (int k = 0; k < 3; ++k) {
+                            f32x2 sv = mul2(w00[k], lt[u][k]);
+                            sv = add2(mul2(w10[k], rt[u][k]), sv, one);
+                            sv = add2(mul2(w01[k], lt[d][k]), sv, one);
+                            sv = add2(mul2(w11[k], rt[d][k]), sv, one);
+                            const f32x2 q = mul2(mul2(sv, k == 1 ? w4 : w3), wj);
+                            sum[r] = j == 0 && k == 0 ? q : add2(q, sum[r], one);  // 0 + q = q: no texel is negative
+                        }
+                    }
+                }
+                float* o = blur + (size_t)(Y0 + ty0) * bp + x;
+#pragma unroll
+                for (int r = 0; r < ROWS; ++r, o += bp) {
+                    const float2 s = unpack2(sum[r]);
+                    if (ty0 + r >= nr) break;
+                    if (x + 1 < w) *reinterpret_cast<float2*>(o) = s;  // bp and x are even
+                    else if (x < w) *o = s.x;
+                }
+            }
+        } else {
+            const int M = F.margin, lp = F.lvl_pitch[l];
+            const float* lvl = F.lvl[l];
+            for (int k = t; k < nc * nr; k += KBL_THREADS) {
+                const int r = k / nc, ey = r0 + r, ex = c0 + (k - r * nc);
+                blur[(size_t)ey * bp + ex] =
+                    blur_cell(lvl, lp, w, h, ex < w + M ? (uint32_t)ex : 0xffffffffu, ey < h + M ? (uint32_t)ey : 0xffffffffu);
+            }
+        }
+        if (!more) break;
+        if (t == 0) s_claim[cur] = claimed;
+        __syncthreads();  // the tables and this buffer are rewritten from here on
+        inext = s_claim[cur];
+        it = next;
+        cur ^= 1;
     }
 }
 
@@ -658,11 +824,10 @@ __device__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* s_warp, uint32_t*
     return res;
 }
 
+// (one 16-byte store; the orientation, its last word, is k_describe's)
 __device__ __forceinline__ void write_header(uint32_t* feats, uint32_t pos, int x, int y, uint32_t s) {
-    uint32_t* rec = feats + (size_t)pos * 12u;
-    rec[0] = __float_as_uint((float)x);
-    rec[1] = __float_as_uint((float)y);
-    rec[2] = s;
+    *reinterpret_cast<uint4*>(feats + (size_t)pos * 12u) =
+        make_uint4(__float_as_uint((float)x), __float_as_uint((float)y), s, 0u);
 }
 
 // One lane's 32-pixel row segment of a 32x32 cell (bytes at x >= w zeroed).
@@ -807,36 +972,57 @@ k_xsort(const FrameDev* __restrict__ frames, const SegDev* __restrict__ segs) {
 // order followed by the order inside each band; the level cap keeps the
 // first `cap` of it (generate_features.wgsl:67-70 appends in a racy order,
 // so this canonical order is the deterministic policy).
-constexpr int KBAND_THREADS = 256;
+// A CTA has one warp per row of its band: a lane reads 16 map bytes at a time
+// (a 752-pixel row is two loads a lane); four rows per warp, 4 bytes a lane at
+// a time, were 24 dependent scans (18 against 11 us on one 752x480 frame, with
+// the list of blur items on top here).
+// Cells mode: the warps take the band's cells in turn, a lane one cell row.
+constexpr int KBAND_THREADS = 1024;
 constexpr int KBAND_WARPS = KBAND_THREADS / 32;
+static_assert(KBAND_WARPS == USLAM_BLUR_TH, "a warp per row of a band, which is a blur tile row");
 
-// This warp's share of a band and its counts.  Rows mode: 4 rows per warp.
-// Cells mode: a contiguous run of the band's cells per warp.
+__device__ __forceinline__ uint32_t warp_sum_u32(uint32_t v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+__device__ __forceinline__ uint32_t warp_inclusive_scan(uint32_t v, int lane) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += t;
+    }
+    return v;
+}
+// Map bytes x .. x + 15 of a row (the map's padding beyond w is 0; x a multiple of 16).
+__device__ __forceinline__ uint4 map16(const uint8_t* row, int x, int w) {
+    return x < w ? *reinterpret_cast<const uint4*>(row + x) : make_uint4(0u, 0u, 0u, 0u);
+}
+__device__ __forceinline__ uint32_t nonzero_bytes16(const uint4& v) {
+    return (uint32_t)(nonzero_bytes(v.x) + nonzero_bytes(v.y) + nonzero_bytes(v.z) + nonzero_bytes(v.w));
+}
+
+// This warp's share of a band and its counts: one row (rows mode), or cells
+// warp, warp + KBAND_WARPS, ... (cells mode).
 __device__ __forceinline__ void band_warp_counts(const FrameDev& F, int l, int band, uint32_t* raw, uint32_t* kept) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int w = F.w[l], h = F.h[l], kpitch = F.kp_pitch[l];
     const uint8_t* kp = F.kpmap[l];
     uint32_t r = 0, k = 0;
     if (F.cell_cap <= 0) {
-        const int y0 = band * 32 + warp * (32 / KBAND_WARPS);
-        for (int y = y0; y < min(h, y0 + 32 / KBAND_WARPS); ++y) {
-            const uint32_t* row = reinterpret_cast<const uint32_t*>(kp + (size_t)y * kpitch);
-            for (int x4 = lane; x4 * 4 < w; x4 += 32) r += nonzero_bytes(row[x4]);
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
-        k = r;
+        const int y = band * 32 + warp;
+        if (y < h)
+            for (int x = 16 * lane; x < w; x += 512) r += nonzero_bytes16(map16(kp + (size_t)y * kpitch, x, w));
+        k = r = warp_sum_u32(r);
     } else {
         const uint32_t ccap = (uint32_t)F.cell_cap;
-        const int ncx = (w + 31) / 32, per = (ncx + KBAND_WARPS - 1) / KBAND_WARPS;
-        for (int cx = warp * per; cx < min(ncx, (warp + 1) * per); ++cx) {
+        for (int cx = warp; cx * 32 < w; cx += KBAND_WARPS) {
             uint32_t v[8];
             load_cell_row(kp, kpitch, w, h, cx * 32, band * 32 + lane, v);
             uint32_t n = 0;
 #pragma unroll
             for (int q = 0; q < 8; ++q) n += (uint32_t)nonzero_bytes(v[q]);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
+            n = warp_sum_u32(n);
             r += n;
             k += n < ccap ? n : ccap;
         }
@@ -845,32 +1031,77 @@ __device__ __forceinline__ void band_warp_counts(const FrameDev& F, int l, int b
     *kept = k;
 }
 
+// Also clears the band's blur marks and the run's list of blur items.
 __global__ void __launch_bounds__(KBAND_THREADS)
-k_band_count(const FrameDev* __restrict__ frames, const BandItem* __restrict__ items) {
+k_band_count(const FrameDev* __restrict__ frames, const BandItem* __restrict__ items, BlurList bl) {
     __shared__ uint32_t s_raw[KBAND_WARPS], s_kept[KBAND_WARPS];
     const BandItem it = items[blockIdx.x];
     const FrameDev& F = frames[it.frame];
+    {
+        const int l = it.level, w = F.w[l], h = F.h[l], nx = USLAM_BLUR_NX(w);
+        uint32_t* f = F.btile[l];
+        for (int i = threadIdx.x; i < nx; i += KBAND_THREADS) f[it.band * nx + i] = 0u;
+        if (threadIdx.x == 0) f[USLAM_BLUR_AT_RIGHT(w, h) + it.band] = 0u;
+        if (it.band == 0)
+            for (int i = USLAM_BLUR_AT_BELOW(w, h) + threadIdx.x; i < USLAM_BLUR_TILES(w, h, F.margin); i += KBAND_THREADS)
+                f[i] = 0u;
+        if (blockIdx.x == 0 && threadIdx.x < 2) bl.count[threadIdx.x] = 0u;
+    }
     uint32_t r, k;
     band_warp_counts(F, it.level, it.band, &r, &k);
-    if ((threadIdx.x & 31) == 0) {
+    const int lane = threadIdx.x & 31;
+    if (lane == 0) {
         s_raw[threadIdx.x >> 5] = r;
         s_kept[threadIdx.x >> 5] = k;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t R = 0, K = 0;
-        for (int q = 0; q < KBAND_WARPS; ++q) {
-            R += s_raw[q];
-            K += s_kept[q];
+    if (threadIdx.x < 32) {
+        const uint32_t R = warp_sum_u32(s_raw[lane]), K = warp_sum_u32(s_kept[lane]);
+        if (lane == 0) {
+            F.bands[it.level][2 * it.band] = R;
+            F.bands[it.level][2 * it.band + 1] = K;
         }
-        F.bands[it.level][2 * it.band] = R;
-        F.bands[it.level][2 * it.band + 1] = K;
     }
 }
 
-__global__ void __launch_bounds__(KBAND_THREADS)
-k_band_write(const FrameDev* __restrict__ frames, const BandItem* __restrict__ items) {
-    __shared__ uint32_t s_red[2][KBAND_WARPS];
+// The blur items that the tests of keypoints in columns x0 .. x1 and rows
+// y0 .. y1 can read: they reach R = margin - 1 cells each way, past the level
+// the margins, and for negative coordinates the last column / row.
+// visit(kind, index within the kind).
+template <typename Visit>
+__device__ __forceinline__ void for_blur_items(int w, int h, int M, int x0, int x1, int y0, int y1, Visit visit) {
+    const int R = M - 1, nx = USLAM_BLUR_NX(w);
+    const int xa = max(x0 - R, 0), ya = max(y0 - R, 0), xe = min(x1 + R, w + M - 1), ye = min(y1 + R, h - 1);
+    for (int ty = ya / USLAM_BLUR_TH; ty <= ye / USLAM_BLUR_TH; ++ty) {
+        for (int tx = xa / USLAM_BLUR_TW; tx <= min(xe, w - 1) / USLAM_BLUR_TW; ++tx) visit(USLAM_BLUR_TILE, ty * nx + tx);
+        if (x1 + R >= w) visit(USLAM_BLUR_RIGHT, ty);
+    }
+    if (x0 < R)
+        for (int ty = ya / USLAM_BLUR_RUN; ty <= ye / USLAM_BLUR_RUN; ++ty) visit(USLAM_BLUR_COL, ty);
+    if (y1 + R >= h) {
+        for (int tx = xa / USLAM_BLUR_TW; tx <= xe / USLAM_BLUR_TW; ++tx) visit(USLAM_BLUR_BELOW, tx);
+        if (x0 < R) visit(USLAM_BLUR_BELOW, (w + M) / USLAM_BLUR_TW);
+    }
+    if (y0 < R) {
+        for (int tx = xa / USLAM_BLUR_RUN; tx <= xe / USLAM_BLUR_RUN; ++tx) visit(USLAM_BLUR_ROW, tx);
+        if (x0 < R) visit(USLAM_BLUR_ROW, (w + M) / USLAM_BLUR_RUN);
+    }
+}
+
+// Kept keypoints are noted per 8 x 8 cells of the band in shared memory, the
+// items those cells need are gathered there too (where a band's reach is at
+// most the tile rows beside it), and each joins the run's list once.
+constexpr int KBAND_NOTES = 8192 / 8;                     // of the widest level
+constexpr int KBAND_REACH = 32;                           // of gathered marks
+constexpr int KBAND_NX = 8192 / USLAM_BLUR_TW;            // tile columns of the widest level
+constexpr int KBAND_NEX = KBAND_NX + 1;                   // with its margin
+constexpr int KBAND_MARKS = 3 * (KBAND_NX + 1) + 2 * KBAND_NEX + 2;
+
+__global__ void __launch_bounds__(KBAND_THREADS, 2)
+k_band_write(const FrameDev* __restrict__ frames, const BandItem* __restrict__ items, BlurList bl) {
+    __shared__ uint8_t s_note[4][KBAND_NOTES];
+    __shared__ uint8_t s_mark[KBAND_MARKS];
+    __shared__ uint32_t s_red[3][KBAND_WARPS];
     __shared__ uint32_t s_wbase[KBAND_WARPS];
     const BandItem it = items[blockIdx.x];
     const FrameDev& F = frames[it.frame];
@@ -878,7 +1109,7 @@ k_band_write(const FrameDev* __restrict__ frames, const BandItem* __restrict__ i
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int w = F.w[l], h = F.h[l], kpitch = F.kp_pitch[l];
     const uint8_t* kp = F.kpmap[l];
-    const int nb = (h + 31) / 32;
+    const int nb = (h + 31) / 32, notes = (w + 7) / 8;
     const uint32_t* bc = F.bands[l];
     uint32_t cap = (uint32_t)F.cap;
     if (F.frame_cap > 0) {
@@ -889,9 +1120,7 @@ k_band_write(const FrameDev* __restrict__ frames, const BandItem* __restrict__ i
             const int nbq = (F.h[q] + 31) / 32;
             uint32_t kq = 0;
             for (int b2 = lane; b2 < nbq; b2 += 32) kq += F.bands[q][2 * b2 + 1];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) kq += __shfl_xor_sync(0xffffffffu, kq, o);
-            kq = min(kq, (uint32_t)F.cap);
+            kq = min(warp_sum_u32(kq), (uint32_t)F.cap);
             left -= min(kq, left);
         }
         cap = min(cap, left);
@@ -904,89 +1133,149 @@ k_band_write(const FrameDev* __restrict__ frames, const BandItem* __restrict__ i
         tr += bc[2 * q];
         tk += kq;
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        pk += __shfl_xor_sync(0xffffffffu, pk, o);
-        tr += __shfl_xor_sync(0xffffffffu, tr, o);
-        tk += __shfl_xor_sync(0xffffffffu, tk, o);
-    }
+    pk = warp_sum_u32(pk);
+    tr = warp_sum_u32(tr);
+    tk = warp_sum_u32(tk);
+    uint32_t r, k;
+    band_warp_counts(F, l, band, &r, &k);
     if (lane == 0) {
         s_red[0][warp] = pk;
         s_red[1][warp] = tr;
+        s_red[2][warp] = tk;
+        s_wbase[warp] = k;
     }
-    __shared__ uint32_t s_tk[KBAND_WARPS];
-    if (lane == 0) s_tk[warp] = tk;
-    uint32_t r, k;
-    band_warp_counts(F, l, band, &r, &k);
-    if (lane == 0) s_wbase[warp] = k;
+    for (int i = threadIdx.x; i < 4 * notes; i += KBAND_THREADS) s_note[i & 3][i >> 2] = 0;
+    for (int i = threadIdx.x; i < KBAND_MARKS; i += KBAND_THREADS) s_mark[i] = 0;
     __syncthreads();
-    uint32_t prefix = 0;
-    for (int q = 0; q < KBAND_WARPS; ++q) prefix += s_red[0][q];
-    if (band == 0 && threadIdx.x == 0) {
-        uint32_t R = 0, K = 0;
-        for (int q = 0; q < KBAND_WARPS; ++q) {
-            R += s_red[1][q];
-            K += s_tk[q];
+    const uint32_t prefix = warp_sum_u32(s_red[0][lane]);
+    if (band == 0 && warp == 0) {
+        const uint32_t R = warp_sum_u32(s_red[1][lane]), K = warp_sum_u32(s_red[2][lane]);
+        if (lane == 0) {
+            F.raw[l] = R;
+            F.kept[l] = K < cap ? K : cap;
         }
-        F.raw[l] = R;
-        F.kept[l] = K < cap ? K : cap;
     }
-    uint32_t running = prefix;
-    for (int q = 0; q < warp; ++q) running += s_wbase[q];
     if (prefix >= cap) return;
     uint32_t* feats = F.feats[l];
     if (F.cell_cap <= 0) {
-        const int y0 = band * 32 + warp * (32 / KBAND_WARPS);
-        for (int y = y0; y < min(h, y0 + 32 / KBAND_WARPS); ++y) {
-            const uint32_t* row = reinterpret_cast<const uint32_t*>(kp + (size_t)y * kpitch);
-            for (int base = 0; base < w; base += 128) {
-                const int x4 = base / 4 + lane;
-                const uint32_t v = (x4 * 4 < w) ? row[x4] : 0u;
-                const uint32_t n = (uint32_t)nonzero_bytes(v);
-                uint32_t incl = n;
+        // (y, x) order: the band's earlier rows, then the row's earlier lanes
+        uint32_t running = prefix + warp_sum_u32(lane < warp ? s_wbase[lane] : 0u);
+        const int y = band * 32 + warp;
+        const uint8_t* row = kp + (size_t)y * kpitch;
+        for (int x0 = 0; y < h && x0 < w && running < cap; x0 += 512) {
+            const int x = x0 + 16 * lane;
+            const uint4 v = map16(row, x, w);
+            const uint32_t n = nonzero_bytes16(v);
+            const uint32_t incl = warp_inclusive_scan(n, lane);
+            uint32_t pos = running + incl - n;
+            const uint32_t words[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-                    if (lane >= o) incl += t;
-                }
-                uint32_t pos = running + incl - n;
+            for (int q = 0; q < 4; ++q) {
+                if (words[q] == 0u || pos >= cap) continue;
+                s_note[warp >> 3][(x >> 3) + (q >> 1)] = 1;
+#pragma unroll
                 for (int b = 0; b < 4; ++b) {
-                    const uint32_t sv = (v >> (8 * b)) & 0xffu;
+                    const uint32_t sv = (words[q] >> (8 * b)) & 0xffu;
                     if (sv == 0u) continue;
-                    if (pos < cap) write_header(feats, pos, x4 * 4 + b, y, sv);
+                    if (pos < cap) write_header(feats, pos, x + 4 * q + b, y, sv);
                     ++pos;
                 }
-                running += __shfl_sync(0xffffffffu, incl, 31);
             }
+            running += __shfl_sync(0xffffffffu, incl, 31);
         }
     } else {
+        // cell order: the band's earlier cells (all warps' shares are
+        // interleaved, so each cell's base comes from a pass over the counts)
         const uint32_t ccap = (uint32_t)F.cell_cap;
-        const int ncx = (w + 31) / 32, per = (ncx + KBAND_WARPS - 1) / KBAND_WARPS;
-        const int y = band * 32 + lane;
-        for (int cx = warp * per; cx < min(ncx, (warp + 1) * per); ++cx) {
+        const int ncx = (w + 31) / 32, y = band * 32 + lane;
+        __shared__ uint32_t s_cell[KBAND_WARPS];
+        uint32_t base = prefix;
+        for (int c0 = 0; c0 < ncx; c0 += KBAND_WARPS) {
+            const int cx = c0 + warp;
             uint32_t v[8];
-            load_cell_row(kp, kpitch, w, h, cx * 32, y, v);
             uint32_t n = 0;
+            if (cx < ncx) {
+                load_cell_row(kp, kpitch, w, h, cx * 32, y, v);
 #pragma unroll
-            for (int q = 0; q < 8; ++q) n += (uint32_t)nonzero_bytes(v[q]);
-            uint32_t incl = n;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += t;
+                for (int q = 0; q < 8; ++q) n += (uint32_t)nonzero_bytes(v[q]);
             }
+            const uint32_t incl = warp_inclusive_scan(n, lane);
             const uint32_t tot = __shfl_sync(0xffffffffu, incl, 31);
+            if (lane == 0) s_cell[warp] = min(tot, ccap);
+            __syncthreads();
+            const uint32_t mine = s_cell[lane];
+            const uint32_t running = base + warp_sum_u32(lane < warp ? mine : 0u);
+            base += warp_sum_u32(mine);
             uint32_t rank = incl - n;
-            for (int q = 0; q < 8 && rank < ccap; ++q) {
-                if (v[q] == 0u) continue;
-                for (int b = 0; b < 4; ++b) {
-                    const uint32_t sv = (v[q] >> (8 * b)) & 0xffu;
-                    if (sv == 0u) continue;
-                    if (rank < ccap && running + rank < cap) write_header(feats, running + rank, cx * 32 + 4 * q + b, y, sv);
-                    ++rank;
+            if (cx < ncx) {
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    if (v[q] == 0u || rank >= ccap || running + rank >= cap) continue;
+                    s_note[lane >> 3][4 * cx + (q >> 1)] = 1;
+#pragma unroll
+                    for (int b = 0; b < 4; ++b) {
+                        const uint32_t sv = (v[q] >> (8 * b)) & 0xffu;
+                        if (sv == 0u) continue;
+                        if (rank < ccap && running + rank < cap)
+                            write_header(feats, running + rank, cx * 32 + 4 * q + b, y, sv);
+                        ++rank;
+                    }
                 }
             }
-            running += tot < ccap ? tot : ccap;
+            __syncthreads();  // s_cell is rewritten
+        }
+    }
+    __syncthreads();
+    const int M = F.margin, nx = USLAM_BLUR_NX(w);
+    auto claim = [&](int kind, int k) {
+        uint32_t* m = F.btile[l] + k;
+        if (kind == USLAM_BLUR_RIGHT) m += USLAM_BLUR_AT_RIGHT(w, h);
+        else if (kind == USLAM_BLUR_BELOW) m += USLAM_BLUR_AT_BELOW(w, h);
+        else if (kind == USLAM_BLUR_COL) m += USLAM_BLUR_AT_COL(w, h, M);
+        else if (kind == USLAM_BLUR_ROW) m += USLAM_BLUR_AT_ROW(w, h, M);
+        if (atomicExch(m, 1u) != 0u) return;
+        const bool tile = kind == USLAM_BLUR_TILE, down = kind == USLAM_BLUR_RIGHT || kind == USLAM_BLUR_COL;
+        TileItem ti;
+        ti.frame = it.frame;
+        ti.level = it.level;
+        ti.pad = (uint8_t)kind;
+        ti.tx = (uint16_t)(tile ? k % nx : down ? 0 : k);
+        ti.ty = (uint16_t)(tile ? k / nx : down ? k : 0);
+        bl.items[atomicAdd(bl.count, 1u)] = ti;
+    };
+    // gathered marks: rows band - 1 .. band + 1 of tiles and their right
+    // margin runs, then the runs below, of the last column and of the last row
+    const bool gather = M - 1 <= KBAND_REACH;
+    const int ty0 = band - 1, cy0 = max(band * 32 - (M - 1), 0) / USLAM_BLUR_RUN;
+    const int g_below = 3 * (nx + 1), g_col = g_below + USLAM_BLUR_NX(w + M + 1), g_row = g_col + 2,
+              g_end = g_row + USLAM_BLUR_DIV(w + M + 1, USLAM_BLUR_RUN);
+    for (int i = threadIdx.x; i < 4 * notes; i += KBAND_THREADS) {
+        const int g = i & 3, c = i >> 2;
+        if (!s_note[g][c]) continue;
+        const int y0 = band * 32 + 8 * g;
+        for_blur_items(w, h, M, 8 * c, min(8 * c + 7, w - 1), y0, min(y0 + 7, h - 1), [&](int kind, int k) {
+            if (!gather) claim(kind, k);
+            else if (kind == USLAM_BLUR_TILE) s_mark[(k / nx - ty0) * (nx + 1) + k % nx] = 1;
+            else if (kind == USLAM_BLUR_RIGHT) s_mark[(k - ty0) * (nx + 1) + nx] = 1;
+            else if (kind == USLAM_BLUR_BELOW) s_mark[g_below + k] = 1;
+            else if (kind == USLAM_BLUR_COL) s_mark[g_col + k - cy0] = 1;
+            else s_mark[g_row + k] = 1;
+        });
+    }
+    if (!gather) return;
+    __syncthreads();
+    for (int i = threadIdx.x; i < g_end; i += KBAND_THREADS) {
+        if (!s_mark[i]) continue;
+        if (i < g_below) {
+            const int r = i / (nx + 1), c = i - r * (nx + 1);
+            if (c < nx) claim(USLAM_BLUR_TILE, (ty0 + r) * nx + c);
+            else claim(USLAM_BLUR_RIGHT, ty0 + r);
+        } else if (i < g_col) {
+            claim(USLAM_BLUR_BELOW, i - g_below);
+        } else if (i < g_row) {
+            claim(USLAM_BLUR_COL, cy0 + i - g_col);
+        } else {
+            claim(USLAM_BLUR_ROW, i - g_row);
         }
     }
 }
@@ -1026,116 +1315,6 @@ __device__ __forceinline__ int find_segment(const uint32_t* s_pref, int nseg, ui
     return lo;
 }
 
-
-// Blur-cache border of one level: columns [w, w + M) and the negative-x
-// sentinel column for rows [0, h), then rows [h, h + M) and the negative-y
-// sentinel row for all columns.  A sentinel stands for every negative
-// coordinate: u32(negative) converts to the same f32 2^32 for all offsets a
-// BRIEF test can reach, so G is identical for all of them.
-// Work units of one level's border: runs of 32 rows of the right margin
-// (columns w .. w + M) and runs of 32 columns of the bottom margin (rows
-// h .. h + M, all columns including the corner and the sentinel column).
-__device__ __forceinline__ uint32_t border_units(const FrameDev& F, int l) {
-    return (uint32_t)((F.h[l] + 31) / 32 + (F.w[l] + F.margin + 1 + 31) / 32);
-}
-
-// The blur cache beyond the level edges: G(P) of generate_features.wgsl:149-172
-// for every border cell, with the operation sequence of k_detect's blur
-// (canonical bilinear taps read from the level in global memory, coordinates
-// clamped to the edge) and the x part of the 9 taps computed once per lane (a
-// lane keeps one column and walks the rows of its unit).  Cells of the sentinel row / column use the
-// u32-wrapped coordinate 0xffffffff that every negative coordinate becomes.
-__global__ void __launch_bounds__(256)
-k_blur_border(const FrameDev* __restrict__ frames, const SegDev* __restrict__ segs, int nseg) {
-    __shared__ uint32_t s_pref[MAX_SEGS + 1];
-    __shared__ uint32_t s_warp[33];
-    __shared__ float s_lut[256];
-    s_lut[threadIdx.x] = (float)threadIdx.x / 255.0f;
-    const uint32_t total = segment_prefix(nseg, s_pref, s_warp, [&](int sg) {
-        return border_units(frames[segs[sg].frame], segs[sg].level);
-    });
-    const int lane = threadIdx.x & 31;
-    const int gw = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const int nw = gridDim.x * (blockDim.x >> 5);
-    const float off[3] = {-1.2f, 0.0f, 1.2f};
-    const float wt[3] = {0.3125f, 0.375f, 0.3125f};
-    for (uint32_t g = gw; g < total; g += nw) {
-        const int sidx = find_segment(s_pref, nseg, g);
-        const int unit = (int)(g - s_pref[sidx]);
-        const FrameDev& F = frames[segs[sidx].frame];
-        const int l = segs[sidx].level;
-        const int w = F.w[l], h = F.h[l], M = F.margin, bp = F.bl_pitch[l];
-        const int nr = (h + 31) / 32;
-        int ex, ey0, ey1;
-        bool active;
-        if (unit < nr) {
-            ex = w + lane;
-            active = lane <= M;
-            ey0 = unit * 32;
-            ey1 = min(h, ey0 + 32);
-        } else {
-            ex = (unit - nr) * 32 + lane;
-            active = ex <= w + M;
-            ey0 = h;
-            ey1 = h + M + 1;
-        }
-        if (!active) continue;
-        const uint8_t* img = F.img;
-        const int pitch = F.img_pitch;
-        const float* lvl = l > 0 ? F.lvl[l] : nullptr;
-        const int lp = F.lvl_pitch[l];
-        const float tex_x = 1.0f / (float)w;
-        const float tex_y = 1.0f / (float)h;
-        const uint32_t px = ex < w + M ? (uint32_t)ex : 0xffffffffu;
-        const float uvx = ((float)px + 0.5f) * tex_x;
-        float ax[3];
-        int ix0[3], ix1[3];
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            const float u = (uvx + off[i] * tex_x) * (float)w - 0.5f;
-            const float fi = floorf(u);
-            ax[i] = u - fi;
-            ix0[i] = edge_index(fi, w);
-            ix1[i] = edge_index(fi + 1.0f, w);
-        }
-        float* out = F.blur[l];
-        for (int ey = ey0; ey < ey1; ++ey) {
-            const uint32_t py = ey < h + M ? (uint32_t)ey : 0xffffffffu;
-            const float uvy = ((float)py + 0.5f) * tex_y;
-            float sum = 0.0f;
-#pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                const float v = (uvy + off[j] * tex_y) * (float)h - 0.5f;
-                const float fj = floorf(v);
-                const float b = v - fj;
-                const int j0 = edge_index(fj, h), j1 = edge_index(fj + 1.0f, h);
-#pragma unroll
-                for (int i = 0; i < 3; ++i) {
-                    float t00, t10, t01, t11;
-                    if (lvl) {
-                        t00 = __ldg(lvl + (size_t)j0 * lp + ix0[i]);
-                        t10 = __ldg(lvl + (size_t)j0 * lp + ix1[i]);
-                        t01 = __ldg(lvl + (size_t)j1 * lp + ix0[i]);
-                        t11 = __ldg(lvl + (size_t)j1 * lp + ix1[i]);
-                    } else {
-                        t00 = s_lut[__ldg(img + (size_t)j0 * pitch + ix0[i])];
-                        t10 = s_lut[__ldg(img + (size_t)j0 * pitch + ix1[i])];
-                        t01 = s_lut[__ldg(img + (size_t)j1 * pitch + ix0[i])];
-                        t11 = s_lut[__ldg(img + (size_t)j1 * pitch + ix1[i])];
-                    }
-                    const float a = ax[i];
-                    const float na = 1.0f - a, nb = 1.0f - b;
-                    float sv = (na * nb) * t00;
-                    sv = sv + (a * nb) * t10;
-                    sv = sv + (na * b) * t01;
-                    sv = sv + (a * b) * t11;
-                    sum = sum + (sv * wt[i]) * wt[j];
-                }
-            }
-            out[(size_t)ey * bp + ex] = sum;
-        }
-    }
-}
 
 // FP8 E4M3 code of an integer 0..16 (all exact: 2^k (1 + m / 8) with
 // k = floor(log2 v) <= 4 and m = (v - 2^k) 8 / 2^k an integer).
@@ -2362,15 +2541,14 @@ cudaError_t launch_detect(const FrameDev* frames, const TileItem* tiles, int nti
                          : launch_detect_profile<false>(frames, tiles, ntiles, shape, err, st);
 }
 
-cudaError_t launch_compact_banded(const FrameDev* frames, const BandItem* bands, int nbands, const SegDev* segs,
-                                  int nseg, int max_w, cudaStream_t st) {
-    if (nseg <= 0) return cudaSuccess;
-    k_band_count<<<nbands, KBAND_THREADS, 0, st>>>(frames, bands);
-    cudaError_t e = cudaGetLastError();
+// The ordered lists and the list of blur tiles they need.
+cudaError_t launch_compact_banded(const FrameDev* frames, const BandItem* bands, int nbands, BlurList bl,
+                                  cudaStream_t st) {
+    if (nbands <= 0) return cudaSuccess;
+    k_band_count<<<nbands, KBAND_THREADS, 0, st>>>(frames, bands, bl);
+    const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    k_band_write<<<nbands, KBAND_THREADS, 0, st>>>(frames, bands);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    k_xsort<<<nseg, KC_THREADS, (size_t)(max_w + 1) * sizeof(uint32_t), st>>>(frames, segs);
+    k_band_write<<<nbands, KBAND_THREADS, 0, st>>>(frames, bands, bl);
     return cudaGetLastError();
 }
 
@@ -2380,9 +2558,11 @@ cudaError_t launch_xsort(const FrameDev* frames, const SegDev* segs, int nseg, i
     return cudaGetLastError();
 }
 
-cudaError_t launch_blur_border(const FrameDev* frames, const SegDev* segs, int nseg, int grid, cudaStream_t st) {
-    if (nseg <= 0) return cudaSuccess;
-    k_blur_border<<<grid, 256, 0, st>>>(frames, segs, nseg);
+// max_tiles: the most items the list can hold.
+cudaError_t launch_blur(const FrameDev* frames, BlurList bl, int max_tiles, int num_sms, uint32_t* err,
+                        cudaStream_t st) {
+    if (max_tiles <= 0) return cudaSuccess;
+    k_blur<<<min(max_tiles, num_sms * KBL_CTAS_PER_SM), KBL_THREADS, 0, st>>>(frames, bl, err, 1.0f);
     return cudaGetLastError();
 }
 

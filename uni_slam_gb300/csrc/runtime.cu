@@ -8,9 +8,9 @@
 //   keypoint maps, band counts, the matcher's band lists, match directions,
 //   error word]
 // so one H2D copy feeds the whole batch and one D2H copy returns it.  The
-// batch's launch sequence (k_detect per tile shape; k_blur_border on a forked
-// branch beside k_band_count, k_band_write, k_xsort; k_describe; k_match or
-// k_bruteforce; k_mutual or the emit) is captured once into a CUDA graph.
+// batch's launch sequence (k_detect per tile shape; k_band_count,
+// k_band_write; k_xsort on a forked branch beside k_blur; k_describe; k_match
+// or k_bruteforce; k_mutual or the emit) is captured once into a CUDA graph.
 // A frontend (uslam_frontend) is a 2-slot batch driven frame by frame with
 // the reference's FeatureSet(0)/(1) rotation.
 #include <cuda.h>  // CUtensorMap and its encode enums (types only: the entry point comes through the runtime)
@@ -53,6 +53,9 @@ struct Program {
     SegDev* psegs = nullptr;  // one (pair, 0) entry per pair (brute-force matcher)
     void* units = nullptr;    // the windowed tensor-core matcher's unit slots (device scratch)
     size_t units_bytes = 0;
+    BlurList blur{};          // blur tiles of a run (device scratch: the count, then the items)
+    int nblur = 0;            // the most items it can hold
+    size_t blur_bytes = 0;
     std::vector<char> host;  // host image of the tables
     cudaGraphExec_t graph = nullptr;
 };
@@ -82,7 +85,7 @@ struct uslam_batch {
     size_t claim_stride = 0, claim_words = 0;
     cudaStream_t stream = nullptr;      // stream in use (own or caller's)
     cudaStream_t own_stream = nullptr;  // created with the batch
-    cudaStream_t aux_stream = nullptr;  // k_blur_border's branch beside the compaction
+    cudaStream_t aux_stream = nullptr;  // k_xsort's branch beside k_blur
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     // graph of a batch of >= kSplitFrames frames: kLanes parts of the frames on
     // as many lanes (streams), so that each part's kernels fill the others' tails
@@ -111,6 +114,7 @@ uslam_status build_program(uslam_batch* b, const std::vector<int>& fr, const std
     for (int f : fr) {
         const FrameDev& F = b->frames[f];
         append_tiles(&st.by_shape[b->ctx->shape_for(F.W0, F.H0)], f, F, b->ctx->shape_for(F.W0, F.H0));
+        P->nblur += blur_tiles_of(F);
         for (int l = 0; l < F.levels; ++l) {
             fsegs.push_back(SegDev{f, l});
             for (int q = 0; q < (F.h[l] + 31) / 32; ++q) {
@@ -196,11 +200,12 @@ uslam_status build_program(uslam_batch* b, const std::vector<int>& fr, const std
                 desc.size() * sizeof(BandItem));
     // unit slots of the windowed tensor-core matcher: written on the device
     P->units_bytes = b->win_tc ? round_up(msegs.size() * static_cast<size_t>(b->win_umax) * win_unit_bytes(), 256) : 0;
-    P->host.resize(P->host.size() + P->units_bytes, 0);
+    P->blur_bytes = 256 + round_up(static_cast<size_t>(P->nblur) * sizeof(TileItem), 256);
+    P->host.resize(P->host.size() + P->units_bytes + P->blur_bytes, 0);
     return USLAM_OK;
 }
 
-// A lane of launches: a stream, the stream k_blur_border forks to, their
+// A lane of launches: a stream, the stream k_xsort forks to, their
 // fork/join events, and the block k_match claims its query groups from (with
 // the group cost buckets its order is built from).
 struct Lane {
@@ -237,27 +242,24 @@ cudaError_t describe_stage(uslam_batch* b, const Program& P, cudaStream_t st) {
     return launch_describe(b->d_frames, P.fsegs, P.nfsegs, c->d_pattern, c->num_sms * 4, c->matcher == 2, b->win_tc, st);
 }
 
-// The frame stages of a program: pyramid, detect, blur border, compaction, describe.
+// The frame stages of a program: pyramid, detect, compaction, blur, describe.
 cudaError_t enqueue_frames(uslam_batch* b, const Program& P, const Lane& ln) {
     uslam_ctx* c = b->ctx;
     cudaError_t e = cudaSuccess;
     if (P.ntiles <= 0) return e;
     if ((e = launch_pyramid_shaped(b->d_frames, P.tiles, P.tile_begin, ln.st)) != cudaSuccess) return e;
-    const int grid = c->num_sms * 4;
-    // k_blur_border (the blur cache beyond the level edges) reads only the
-    // pyramid and the frame, and writes cells k_detect does not: it runs on a
-    // forked stream beside k_detect and the compaction and joins before
-    // k_describe, which needs both (in a captured graph this is a fork/join).
-    if ((e = cudaEventRecord(ln.fork, ln.st)) != cudaSuccess) return e;
-    if ((e = cudaStreamWaitEvent(ln.aux, ln.fork, 0)) != cudaSuccess) return e;
-    if ((e = launch_blur_border(b->d_frames, P.fsegs, P.nfsegs, grid, ln.aux)) != cudaSuccess) return e;
-    if ((e = cudaEventRecord(ln.join, ln.aux)) != cudaSuccess) return e;
     if ((e = launch_detect_only_shaped(b->d_frames, P.tiles, P.tile_begin, c->detector, b->d_err, ln.st)) !=
         cudaSuccess)
         return e;
-    if ((e = launch_compact_banded(b->d_frames, P.bands, P.nbands, P.fsegs, P.nfsegs, b->max_w, ln.st)) !=
-        cudaSuccess)
-        return e;
+    if ((e = launch_compact_banded(b->d_frames, P.bands, P.nbands, P.blur, ln.st)) != cudaSuccess) return e;
+    // k_blur (the blur cache where the kept keypoints' tests read it) needs
+    // the list of k_band_write, k_xsort the kept features: they run side by
+    // side, and k_describe needs both (in a captured graph a fork/join).
+    if ((e = cudaEventRecord(ln.fork, ln.st)) != cudaSuccess) return e;
+    if ((e = cudaStreamWaitEvent(ln.aux, ln.fork, 0)) != cudaSuccess) return e;
+    if ((e = launch_xsort(b->d_frames, P.fsegs, P.nfsegs, b->max_w, ln.aux)) != cudaSuccess) return e;
+    if ((e = cudaEventRecord(ln.join, ln.aux)) != cudaSuccess) return e;
+    if ((e = launch_blur(b->d_frames, P.blur, P.nblur, c->num_sms, b->d_err, ln.st)) != cudaSuccess) return e;
     if ((e = cudaStreamWaitEvent(ln.st, ln.join, 0)) != cudaSuccess) return e;
     return describe_stage(b, P, ln.st);
 }
@@ -396,7 +398,8 @@ uslam_status create_batch(uslam_ctx* ctx, int n_frames, const int* widths, const
     };
     struct FrameLayout {
         size_t lvl[USLAM_MAX_LEVELS], blur[USLAM_MAX_LEVELS], kpmap[USLAM_MAX_LEVELS], feats[USLAM_MAX_LEVELS],
-            xorder[USLAM_MAX_LEVELS], colstart[USLAM_MAX_LEVELS], qorder[USLAM_MAX_LEVELS], bands[USLAM_MAX_LEVELS], counts,
+            xorder[USLAM_MAX_LEVELS], colstart[USLAM_MAX_LEVELS], qorder[USLAM_MAX_LEVELS], bands[USLAM_MAX_LEVELS],
+            btile[USLAM_MAX_LEVELS], counts,
             tmaps, bf8, bfext, bfpop, bfid, wq8, wc8, wcext, wcy, wcid, winv[USLAM_MAX_LEVELS];
     };
     // the windowed tensor-core matcher (matcher 3, or matcher 0 in the
@@ -458,6 +461,7 @@ uslam_status create_batch(uslam_ctx* ctx, int n_frames, const int* widths, const
             Ly.colstart[l] = take(&scratch, (USLAM_MATCH_BANDS * (static_cast<size_t>(F.w[l]) + 1) + USLAM_MATCH_BANDS + 1) * 4);
             Ly.qorder[l] = take(&scratch, capa * 4);
             Ly.bands[l] = take(&scratch, static_cast<size_t>((F.h[l] + 31) / 32) * 8);
+            Ly.btile[l] = take(&scratch, sizeof(uint32_t) * USLAM_BLUR_TILES(F.w[l], F.h[l], F.margin));
         }
         Ly.tmaps = take(&scratch, static_cast<size_t>(L) * USLAM_TMAPS_PER_LEVEL * USLAM_TMAP_BYTES);
         if (ctx->matcher == 2) {
@@ -616,6 +620,7 @@ uslam_status create_batch(uslam_ctx* ctx, int n_frames, const int* widths, const
             F.colstart[l] = reinterpret_cast<uint32_t*>(sc_base + Ly.colstart[l]);
             F.qorder[l] = reinterpret_cast<uint32_t*>(sc_base + Ly.qorder[l]);
             F.bands[l] = reinterpret_cast<uint32_t*>(sc_base + Ly.bands[l]);
+            F.btile[l] = reinterpret_cast<uint32_t*>(sc_base + Ly.btile[l]);
             F.mask[l] = masks[l];
         }
         F.tmaps = sc_base + Ly.tmaps;
@@ -769,7 +774,9 @@ uslam_status create_batch(uslam_ctx* ctx, int n_frames, const int* widths, const
         P->bands = reinterpret_cast<BandItem*>(base + t_bytes + f_bytes + m_bytes + u_bytes + p_bytes);
         const size_t b_bytes = round_up(P->nbands * sizeof(BandItem), 256);
         P->desc = reinterpret_cast<BandItem*>(base + t_bytes + f_bytes + m_bytes + u_bytes + p_bytes + b_bytes);
-        P->units = P->units_bytes ? base + (P->host.size() - P->units_bytes) : nullptr;
+        P->units = P->units_bytes ? base + (P->host.size() - P->blur_bytes - P->units_bytes) : nullptr;
+        char* const bl = base + (P->host.size() - P->blur_bytes);
+        P->blur = BlurList{reinterpret_cast<TileItem*>(bl + 256), reinterpret_cast<uint32_t*>(bl)};
         P->tiles = reinterpret_cast<TileItem*>(base);
         P->fsegs = reinterpret_cast<SegDev*>(base + t_bytes);
         P->msegs = reinterpret_cast<MatchSegDev*>(base + t_bytes + f_bytes);
@@ -1056,7 +1063,36 @@ uslam_status uslam_batch_blur_level(uslam_batch* b, int frame, int level, float*
         return USLAM_INVALID_ARG;
     const FrameDev& F = b->frames[frame];
     const size_t cols = static_cast<size_t>(F.w[level] + F.margin + 1);
-    cudaError_t e = cudaMemcpy2D(out, sizeof(float) * cols, F.blur[level], sizeof(float) * F.bl_pitch[level],
+    // a run evaluates the cache where its tests read it: evaluate all of the level's
+    std::vector<TileItem> items;
+    auto add = [&](int kind, int tx, int ty) {
+        TileItem it{};
+        it.frame = static_cast<uint16_t>(frame);
+        it.level = static_cast<uint8_t>(level);
+        it.pad = static_cast<uint8_t>(kind);
+        it.tx = static_cast<uint16_t>(tx);
+        it.ty = static_cast<uint16_t>(ty);
+        items.push_back(it);
+    };
+    const int ew = F.w[level] + F.margin + 1;
+    for (int ty = 0; ty < USLAM_BLUR_NY(F.h[level]); ++ty) {
+        for (int tx = 0; tx < USLAM_BLUR_NX(F.w[level]); ++tx) add(USLAM_BLUR_TILE, tx, ty);
+        add(USLAM_BLUR_RIGHT, 0, ty);
+    }
+    for (int tx = 0; tx < USLAM_BLUR_NX(ew); ++tx) add(USLAM_BLUR_BELOW, tx, 0);
+    for (int ty = 0; ty < USLAM_BLUR_DIV(F.h[level], USLAM_BLUR_RUN); ++ty) add(USLAM_BLUR_COL, 0, ty);
+    for (int tx = 0; tx < USLAM_BLUR_DIV(ew, USLAM_BLUR_RUN); ++tx) add(USLAM_BLUR_ROW, tx, 0);
+    const uint32_t n = static_cast<uint32_t>(items.size()), head[2] = {n, 0u};
+    char* d = nullptr;
+    cudaError_t e = cudaMalloc(&d, 256 + n * sizeof(TileItem));
+    if (e == cudaSuccess) e = cudaMemcpy(d, head, sizeof(head), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(d + 256, items.data(), n * sizeof(TileItem), cudaMemcpyHostToDevice);
+    const BlurList bl{reinterpret_cast<TileItem*>(d + 256), reinterpret_cast<uint32_t*>(d)};
+    if (e == cudaSuccess) e = launch_blur(b->d_frames, bl, static_cast<int>(n), b->ctx->num_sms, b->d_err, b->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
+    if (d) cudaFree(d);
+    if (e != cudaSuccess) return b->ctx->cuda_fail(e, "blur cache");
+    e = cudaMemcpy2D(out, sizeof(float) * cols, F.blur[level], sizeof(float) * F.bl_pitch[level],
                                  sizeof(float) * cols, static_cast<size_t>(F.h[level] + F.margin + 1),
                                  cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return b->ctx->cuda_fail(e, "blur readback");
@@ -1110,10 +1146,10 @@ uslam_status uslam_batch_profile(uslam_batch* b, int iters, float* kernel_ms) {
             e = launch_detect(b->d_frames, P.tiles + P.tile_begin[sh], P.tile_begin[sh + 1] - P.tile_begin[sh], sh,
                               c->detector, b->d_err, b->stream);
         mark();
-        if (e == cudaSuccess) e = launch_blur_border(b->d_frames, P.fsegs, P.nfsegs, grid, b->stream);
+        if (e == cudaSuccess) e = launch_compact_banded(b->d_frames, P.bands, P.nbands, P.blur, b->stream);
+        if (e == cudaSuccess) e = launch_xsort(b->d_frames, P.fsegs, P.nfsegs, b->max_w, b->stream);
         mark();
-        if (e == cudaSuccess)
-            e = launch_compact_banded(b->d_frames, P.bands, P.nbands, P.fsegs, P.nfsegs, b->max_w, b->stream);
+        if (e == cudaSuccess) e = launch_blur(b->d_frames, P.blur, P.nblur, c->num_sms, b->d_err, b->stream);
         mark();
         if (e == cudaSuccess)
             e = describe_stage(b, P, b->stream);
@@ -1144,6 +1180,7 @@ uslam_status uslam_batch_profile(uslam_batch* b, int iters, float* kernel_ms) {
     for (auto& x : ev)
         if (x) cudaEventDestroy(x);
     if (e != cudaSuccess) return c->cuda_fail(e, "profile");
+    std::swap(acc[2], acc[3]);  // the blur cache is reported before the compaction, which it follows
     for (int q = 0; q < K; ++q) kernel_ms[q] = static_cast<float>(acc[q] / iters);
     return check_err_word(b);
 }
@@ -1698,6 +1735,22 @@ uslam_status encode_tile_maps(const FrameDev& F, int detector, void* out, ErrTex
                                "tensor map encode failed (level " + std::to_string(l) + ", shape " + std::to_string(sh) +
                                    ", code " + std::to_string(static_cast<int>(r)) + ")");
         }
+    // k_blur's tiles
+    for (int l = 0; l < F.levels; ++l) {
+        CUtensorMap* m = reinterpret_cast<CUtensorMap*>(
+            static_cast<char*>(out) + (static_cast<size_t>(l) * USLAM_TMAPS_PER_LEVEL + USLAM_TMAP_BLUR) * USLAM_TMAP_BYTES);
+        const cuuint64_t dims[2] = {static_cast<cuuint64_t>(F.w[l]), static_cast<cuuint64_t>(F.h[l])};
+        const cuuint64_t strides[1] = {static_cast<cuuint64_t>(F.lvl_pitch[l]) * 4u};
+        const cuuint32_t box[2] = {USLAM_BLUR_TW + 2 * USLAM_BLUR_XPAD, USLAM_BLUR_TH + 2 * USLAM_BLUR_HY};
+        const cuuint32_t estr[2] = {1u, 1u};
+        const CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, F.lvl[l], dims, strides, box, estr,
+                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                              CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (r != CUDA_SUCCESS)
+            return set_err(err, USLAM_CUDA_ERROR,
+                           "blur tile tensor map encode failed (level " + std::to_string(l) + ", code " +
+                               std::to_string(static_cast<int>(r)) + ")");
+    }
     // the blur caches, for k_describe_tiled: box = a describe item's chunk
     // (KDT_CW columns, 32 rows) widened by RX columns and R rows each side
     if (uslam::describe_tiled_smem(F.margin) == 0) return USLAM_OK;

@@ -26,8 +26,9 @@ struct MatchSegDev {
 cudaError_t init_constants();
 cudaError_t launch_detect(const FrameDev*, const TileItem*, int, int, int, uint32_t*, cudaStream_t);
 cudaError_t launch_pyramid(const FrameDev*, const TileItem*, int, int, cudaStream_t);
-cudaError_t launch_compact_banded(const FrameDev*, const BandItem*, int, const SegDev*, int, int, cudaStream_t);
-cudaError_t launch_blur_border(const FrameDev*, const SegDev*, int, int, cudaStream_t);
+cudaError_t launch_compact_banded(const FrameDev*, const BandItem*, int, BlurList, cudaStream_t);
+cudaError_t launch_xsort(const FrameDev*, const SegDev*, int, int, cudaStream_t);
+cudaError_t launch_blur(const FrameDev*, BlurList, int max_tiles, int num_sms, uint32_t* err, cudaStream_t);
 cudaError_t launch_describe(const FrameDev*, const SegDev*, int, const int32_t*, int, bool, bool, cudaStream_t);
 // k_describe_tiled over describe items (one per KDT_CW-column chunk of every
 // 32-row band); describe_tiled_smem(margin) = its dynamic shared memory, 0 if
@@ -232,6 +233,13 @@ inline cudaError_t launch_detect_shaped(const FrameDev* frames, const TileItem* 
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
+}
+
+// Blur tiles of every level of a frame (the most k_band_write can list).
+inline int blur_tiles_of(const FrameDev& F) {
+    int n = 0;
+    for (int l = 0; l < F.levels; ++l) n += USLAM_BLUR_TILES(F.w[l], F.h[l], F.margin);
+    return n;
 }
 
 // Row pitch (floats) of a pyramid level buffer: 16-byte rows for TMA.

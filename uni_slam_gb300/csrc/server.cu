@@ -38,6 +38,7 @@ struct SrvClass {
     int first_slot = 0, n_slots = 0;
     int tiles_per_frame = 0;
     int shape = 0;                // detect tile shape (index into kTileShapes)
+    int blur_tiles = 0;           // blur tiles of one frame
     std::vector<TileItem> tiles;  // one frame's tile list (frame field patched per launch)
     std::vector<BandItem> bands;  // one frame's compaction bands (frame field patched per launch)
     std::vector<BandItem> desc;   // one frame's describe items (chunks of the bands)
@@ -79,8 +80,8 @@ struct SrvLaunch {
 
 struct LaunchBuf {
     char* h = nullptr;  // pinned table image
-    char* d = nullptr;  // device tables
-    size_t bytes = 0;
+    char* d = nullptr;  // device tables, then the launch's blur tile list (its count, its items)
+    size_t bytes = 0;   // of the tables
     bool busy = false;
 };
 
@@ -225,6 +226,7 @@ cudaError_t launch_batch(uslam_server* s, const std::vector<uint64_t>& tickets, 
     std::vector<PairDev> pairs;
     std::vector<BandItem> bands, desc;
     std::vector<SrvEmitItem> emits;
+    int blur_tiles = 0;
     cudaError_t e = cudaSuccess;
     for (uint64_t tk : tickets) {
         SrvReq& r = s->reqs[tk];
@@ -239,6 +241,7 @@ cudaError_t launch_batch(uslam_server* s, const std::vector<uint64_t>& tickets, 
             em.match_count = sl.match_count;
         }
         emits.push_back(em);
+        blur_tiles += C.blur_tiles;
         for (TileItem t : C.tiles) {
             t.frame = static_cast<uint16_t>(r.slot);
             shaped.by_shape[C.shape].push_back(t);
@@ -316,13 +319,14 @@ cudaError_t launch_batch(uslam_server* s, const std::vector<uint64_t>& tickets, 
     const auto* d_bands = reinterpret_cast<const BandItem*>(B.d + t_b + f_b + m_b + u_b + p_b);
     const auto* d_emits = reinterpret_cast<const SrvEmitItem*>(B.d + t_b + f_b + m_b + u_b + p_b + b_b);
     const auto* d_desc = reinterpret_cast<const BandItem*>(B.d + t_b + f_b + m_b + u_b + p_b + b_b + x_b);
+    const BlurList bl{reinterpret_cast<TileItem*>(B.d + B.bytes + 256), reinterpret_cast<uint32_t*>(B.d + B.bytes)};
     const int grid = c->num_sms * 4;
     const int nf = static_cast<int>(fsegs.size());
     if ((e = launch_detect_shaped(s->d_frames, d_tiles, shaped.begin, c->detector, s->d_err, st)) != cudaSuccess) return e;
-    if ((e = launch_blur_border(s->d_frames, d_fsegs, nf, grid, st)) != cudaSuccess) return e;
-    if ((e = launch_compact_banded(s->d_frames, d_bands, static_cast<int>(bands.size()), d_fsegs, nf, s->max_w,
-                                   st)) != cudaSuccess)
+    if ((e = launch_compact_banded(s->d_frames, d_bands, static_cast<int>(bands.size()), bl, st)) != cudaSuccess)
         return e;
+    if ((e = launch_xsort(s->d_frames, d_fsegs, nf, s->max_w, st)) != cudaSuccess) return e;
+    if ((e = launch_blur(s->d_frames, bl, blur_tiles, c->num_sms, s->d_err, st)) != cudaSuccess) return e;
     e = c->describe_form == 1 && static_cast<int>(emits.size()) >= kTiledDescribeFrames &&
                 describe_tiled_smem(c->margin) > 0
             ? launch_describe_tiled(s->d_frames, d_desc, static_cast<int>(desc.size()), c->d_pattern, false, false,
@@ -472,12 +476,13 @@ uslam_status uslam_server_create(uslam_ctx* ctx, const uslam_server_params* p, u
     // slot bytes per class, then slots per class from an equal share of the budget
     struct SlotLayout {
         size_t bytes, in, counts, lvl[USLAM_MAX_LEVELS], blur[USLAM_MAX_LEVELS], kpmap[USLAM_MAX_LEVELS],
-            feats[USLAM_MAX_LEVELS], xorder[USLAM_MAX_LEVELS], colstart[USLAM_MAX_LEVELS], qorder[USLAM_MAX_LEVELS], bands[USLAM_MAX_LEVELS], a2b, bacc, matches, mcount,
+            feats[USLAM_MAX_LEVELS], xorder[USLAM_MAX_LEVELS], colstart[USLAM_MAX_LEVELS], qorder[USLAM_MAX_LEVELS], bands[USLAM_MAX_LEVELS],
+            btile[USLAM_MAX_LEVELS], a2b, bacc, matches, mcount,
             tmaps;
     };
     std::vector<SlotLayout> lay(p->n_sizes);
     std::vector<FrameDev> proto(p->n_sizes);
-    int max_tiles = 1, max_bands = 1, max_desc = 1;
+    int max_tiles = 1, max_bands = 1, max_desc = 1, max_blur = 1;
     for (int k = 0; k < p->n_sizes; ++k) {
         const int W0 = p->widths[k], H0 = p->heights[k];
         if (W0 < 1 || H0 < 1 || W0 > ctx->max_w || H0 > ctx->max_h) {
@@ -526,6 +531,7 @@ uslam_status uslam_server_create(uslam_ctx* ctx, const uslam_server_params* p, u
             Y.colstart[l] = take((USLAM_MATCH_BANDS * (static_cast<size_t>(F.w[l]) + 1) + USLAM_MATCH_BANDS + 1) * 4);
             Y.qorder[l] = take(capa * 4);
             Y.bands[l] = take(static_cast<size_t>((F.h[l] + 31) / 32) * 8);
+            Y.btile[l] = take(sizeof(uint32_t) * USLAM_BLUR_TILES(F.w[l], F.h[l], F.margin));
         }
         C.shape = ctx->shape_for(W0, H0);
         append_tiles(&C.tiles, 0, F, C.shape);
@@ -547,6 +553,8 @@ uslam_status uslam_server_create(uslam_ctx* ctx, const uslam_server_params* p, u
         Y.tmaps = take(static_cast<size_t>(L) * USLAM_TMAPS_PER_LEVEL * USLAM_TMAP_BYTES);
         Y.bytes = round_up(cur, 256);
         C.tiles_per_frame = static_cast<int>(C.tiles.size());
+        C.blur_tiles = blur_tiles_of(F);
+        max_blur = std::max(max_blur, C.blur_tiles);
         max_tiles = std::max(max_tiles, C.tiles_per_frame);
         max_bands = std::max(max_bands, static_cast<int>(C.bands.size()));
         max_desc = std::max(max_desc, static_cast<int>(C.desc.size()));
@@ -602,6 +610,7 @@ uslam_status uslam_server_create(uslam_ctx* ctx, const uslam_server_params* p, u
                 F.colstart[l] = reinterpret_cast<uint32_t*>(base + Y.colstart[l]);
                 F.qorder[l] = reinterpret_cast<uint32_t*>(base + Y.qorder[l]);
                 F.bands[l] = reinterpret_cast<uint32_t*>(base + Y.bands[l]);
+                F.btile[l] = reinterpret_cast<uint32_t*>(base + Y.btile[l]);
                 F.mask[l] = masks[l];
             }
             F.tmaps = base + Y.tmaps;
@@ -637,7 +646,8 @@ uslam_status uslam_server_create(uslam_ctx* ctx, const uslam_server_params* p, u
     for (int b = 0; b < 2 && e == cudaSuccess; ++b) {
         s->bufs[b].bytes = tables_bytes(s->max_batch, max_tiles, max_bands, max_desc, L);
         e = cudaHostAlloc(&s->bufs[b].h, s->bufs[b].bytes, cudaHostAllocDefault);
-        if (e == cudaSuccess) e = cudaMalloc(&s->bufs[b].d, s->bufs[b].bytes);
+        if (e == cudaSuccess)
+            e = cudaMalloc(&s->bufs[b].d, s->bufs[b].bytes + 256 + sizeof(TileItem) * static_cast<size_t>(s->max_batch) * max_blur);
         if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s->cs[b], cudaStreamNonBlocking);
     }
     if (e == cudaSuccess) e = set_compact_smem(s->max_w);

@@ -9,7 +9,7 @@
 //                                          loads, so lvl_pitch_l = w_l rounded up to 4
 //                                          floats (16-byte rows) and the base is 256-byte
 //                                          aligned
-//   tmaps    CUtensorMap [levels][USLAM_NUM_TILE_SHAPES]  2D tiled maps over lvl[l], one per tile
+//   tmaps    CUtensorMap [levels][USLAM_TMAPS_PER_LEVEL]  2D tiled maps over lvl[l], one per tile
 //                                          shape (box = tile + halo, widened to TW + 16
 //                                          columns), 128 bytes each
 //   blur[l]  f32  [h_l + M + 1][bl_pitch_l] 9-tap blurred sample G(P) of level l for
@@ -19,6 +19,9 @@
 //                                          negative u32-wrapped x convert to the same
 //                                          f32, 2^32); rows likewise.  M = pattern
 //                                          radius + 2, bl_pitch_l = w_l + M + 1.
+//                                          Evaluated per run in the blur tiles that a test
+//                                          of a kept keypoint can read (k_blur)
+//   btile[l] u32  [USLAM_BLUR_TILES]       1 where the run needs the blur item
 //   kpmap[l] u8   [h_l][kp_pitch_l]        culled FAST strength (0 = no keypoint)
 //   bands[l] u32  [ceil(h_l / 32)][2]      raw and kept keypoint counts per 32-row band
 //   feats[l] Feature[cap]                  gpumodels::Feature records, (y, x) order
@@ -58,8 +61,9 @@ struct FrameDev {
     // kernels' own limits); a test hook of uslam_batch_set_first_wait
     int detect_first_wait, match_first_wait;
     float* lvl[USLAM_MAX_LEVELS];
-    const void* tmaps;  // CUtensorMap [levels][USLAM_NUM_TILE_SHAPES] over lvl (device, 64-byte aligned)
+    const void* tmaps;  // CUtensorMap [levels][USLAM_TMAPS_PER_LEVEL] (device, 64-byte aligned)
     float* blur[USLAM_MAX_LEVELS];
+    uint32_t* btile[USLAM_MAX_LEVELS];       // blur tiles the run needs (k_band_write sets, k_band_count clears)
     uint8_t* kpmap[USLAM_MAX_LEVELS];
     uint32_t* bands[USLAM_MAX_LEVELS];       // per 32-row band: raw and kept keypoint counts
     const uint32_t* mask[USLAM_MAX_LEVELS];  // combined cull coverage bitmap
@@ -125,12 +129,41 @@ struct PairDev {
     float bf_ratio;
 };
 
-// K1 work item: one TW x TH tile of one level of one frame.
+// K1 work item: one TW x TH tile of one level of one frame.  As a blur item
+// (k_blur) pad is its kind (USLAM_BLUR_*).
 struct TileItem {
     uint16_t frame;
     uint8_t level;
     uint8_t pad;
     uint16_t tx, ty;
+};
+
+// Blur items of a w x h level with margin M (the cache is (w + M + 1) x
+// (h + M + 1) cells, the last column and row standing for negative
+// coordinates).  Tile rows are the compaction's 32-row bands, so a band's
+// keypoints reach at most a few of them.
+#define USLAM_BLUR_TILE 0   // 64 x 32 cells of the level: (tx, ty)
+#define USLAM_BLUR_RIGHT 1  // columns w .. w + M - 1 of tile row ty
+#define USLAM_BLUR_BELOW 2  // rows h .. h + M - 1 of columns 64 tx .. (to w + M)
+#define USLAM_BLUR_COL 3    // column w + M of rows 256 ty ..
+#define USLAM_BLUR_ROW 4    // row h + M of columns 256 tx .. (to w + M)
+#define USLAM_BLUR_TW 64
+#define USLAM_BLUR_TH 32
+#define USLAM_BLUR_RUN 256
+#define USLAM_BLUR_DIV(n, d) (((n) + (d) - 1) / (d))
+#define USLAM_BLUR_NX(w) USLAM_BLUR_DIV(w, USLAM_BLUR_TW)
+#define USLAM_BLUR_NY(h) USLAM_BLUR_DIV(h, USLAM_BLUR_TH)
+// first mark of each kind in btile (kinds in order)
+#define USLAM_BLUR_AT_RIGHT(w, h) (USLAM_BLUR_NX(w) * USLAM_BLUR_NY(h))
+#define USLAM_BLUR_AT_BELOW(w, h) (USLAM_BLUR_AT_RIGHT(w, h) + USLAM_BLUR_NY(h))
+#define USLAM_BLUR_AT_COL(w, h, M) (USLAM_BLUR_AT_BELOW(w, h) + USLAM_BLUR_NX((w) + (M) + 1))
+#define USLAM_BLUR_AT_ROW(w, h, M) (USLAM_BLUR_AT_COL(w, h, M) + USLAM_BLUR_DIV(h, USLAM_BLUR_RUN))
+#define USLAM_BLUR_TILES(w, h, M) (USLAM_BLUR_AT_ROW(w, h, M) + USLAM_BLUR_DIV((w) + (M) + 1, USLAM_BLUR_RUN))
+
+// The blur items of one run, in arrival order.
+struct BlurList {
+    TileItem* items;
+    uint32_t* count;  // [0] their number, [1] items claimed by k_blur's CTAs
 };
 
 // Segment tables for the persistent describe / match kernels.
@@ -165,8 +198,13 @@ struct BandItem {
 #define USLAM_TMAP_BYTES 128
 #define USLAM_NUM_TILE_SHAPES 5  // k_detect tile shapes (kTileShapes of the runtime)
 // Tensor maps per level of a frame: one per k_detect tile shape over the
-// level, then one over the level's blur cache (k_describe_tiled's box).
-#define USLAM_TMAPS_PER_LEVEL (USLAM_NUM_TILE_SHAPES + 1)
+// level, one over the level's blur cache (k_describe_tiled's box), then one
+// over the level for k_blur: box = a blur tile and its halo of two cells
+// (columns from 4 left of it, a 16-byte aligned x).
+#define USLAM_TMAPS_PER_LEVEL (USLAM_NUM_TILE_SHAPES + 2)
+#define USLAM_TMAP_BLUR (USLAM_NUM_TILE_SHAPES + 1)
+#define USLAM_BLUR_HY 2
+#define USLAM_BLUR_XPAD 4
 // k_describe_tiled: columns of a describe item (a chunk of a 32-row band).
 #define KDT_CW 128
 
