@@ -79,13 +79,25 @@ __device__ __forceinline__ int edge_index(float f, int n) {
     return (int)f;
 }
 
+__device__ __forceinline__ int nonzero_bytes(uint32_t v) {
+    return __popc(__vcmpne4(v, 0u)) >> 3;
+}
+
+__device__ __forceinline__ uint32_t nonzero_bytes16(const uint4& v) {
+    return (uint32_t)(nonzero_bytes(v.x) + nonzero_bytes(v.y) + nonzero_bytes(v.z) + nonzero_bytes(v.w));
+}
+
+__device__ __forceinline__ uint32_t warp_sum_u32(uint32_t v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
 // FAST response at smem cell (r, c): 1 + longest non-wrapping run of
 // |centre - p_i| > 0.15, kept iff > 9 (detect_corners.wgsl:58-81).
 template <int SW>
 __device__ __forceinline__ uint32_t fast_response(const float (*sm)[SW], int r, int c) {
     const float center = sm[r][c];
-    // every non-wrapping run of >= 9 of the 16 points contains points 7 and 8
-    if (!(fabsf(center - sm[r + 3][c + 1]) > 0.15f && fabsf(center - sm[r + 3][c]) > 0.15f)) return 0u;
     uint32_t m = 0;
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
@@ -97,13 +109,13 @@ __device__ __forceinline__ uint32_t fast_response(const float (*sm)[SW], int r, 
     t &= t >> 2;
     t &= t >> 4;
     t &= t >> 1;
-    if (t == 0u) return 0u;
-    uint32_t run = 0;
-    while (m) {
-        m &= m << 1;
+    // bit i of t starts a run of 9, so n + 1 adjacent bits of t are a run of 9 + n
+    uint32_t run = t ? 9u : 0u;
+    while (t) {
+        t &= t << 1;
         ++run;
     }
-    return run + 1u;
+    return run;
 }
 
 // Longest run of ones of a 16-bit circle mask, wrapping around (16 if all set).
@@ -168,6 +180,17 @@ __device__ __forceinline__ float2 mul2_rn(float2 a, float2 b) {
     return d;
 }
 
+// f32(u8) / 255, correctly rounded: u hi + u lo in one fused step with
+// hi + lo = 1/255 to 48 bits (multiplication by a constant held as two words,
+// Brisebarre and Muller 2008); equal to the quotient for all 256 bytes.  Four
+// arithmetic instructions; a 256-entry shared table cost a load with bank
+// conflicts each (k_pyramid on 32 frames of 752x480: 67 us with the table).
+__device__ __forceinline__ float unit_u8(uint32_t byte) {
+    constexpr float hi = 1.0f / 255.0f, lo = (float)(1.0 / 255.0 - (double)hi);
+    const float u = __uint_as_float(0x4B000000u | byte) - 8388608.0f;
+    return __fmaf_rn(u, hi, u * lo);
+}
+
 // Left-to-right sum of four packed products, lane by lane, in scalar adds.
 __device__ __forceinline__ float2 sum4(float2 p, float2 q, float2 r, float2 t) {
     float x = p.x, y = p.y;
@@ -178,10 +201,6 @@ __device__ __forceinline__ float2 sum4(float2 p, float2 q, float2 r, float2 t) {
     x = x + t.x;
     y = y + t.y;
     return make_float2(x, y);
-}
-
-__device__ __forceinline__ bool mask_bit(const uint32_t* mask, int p) {
-    return (__ldg(mask + (p >> 5)) >> (p & 31)) & 1u;
 }
 
 // ------------------------------------------------------ TMA + mbarrier ----
@@ -235,12 +254,11 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const void* tmap, int x, 
 // the sum is scalar in the written order.
 template <int TW, int TH>
 __global__ void __launch_bounds__(K1_THREADS)
-k_pyramid(const FrameDev* __restrict__ frames, const TileItem* __restrict__ tiles) {
+k_pyramid(const FrameDev* __restrict__ frames, const TileItem* __restrict__ tiles, uint32_t* blur_count) {
     static_assert(K1_THREADS % TW == 0 && TW % 8 == 0, "tile shape");
-    __shared__ float s_lut[256];  // f32(u8) / 255
-    __shared__ int2 s_fx[TW];     // LOD0 source columns (x0, x1) per tile column
-    __shared__ float2 s_fa[TW];   // (1 - a, a)
-    __shared__ int2 s_fy[TH];     // LOD0 source rows (y0, y1) per tile row
+    __shared__ int2 s_fx[TW];    // LOD0 source columns (x0, x1) per tile column
+    __shared__ float2 s_fa[TW];  // (1 - a, a)
+    __shared__ int2 s_fy[TH];    // offsets of the LOD0 source rows (y0, y1) per tile row
     __shared__ float2 s_fnb[TH], s_fb[TH];  // (1 - b, 1 - b), (b, b)
     const TileItem it = tiles[blockIdx.x];
     const FrameDev& F = frames[it.frame];
@@ -252,13 +270,25 @@ k_pyramid(const FrameDev* __restrict__ frames, const TileItem* __restrict__ tile
     const int lp = F.lvl_pitch[l];
     const uint8_t* img = F.img;
     const int pitch = F.img_pitch;
-    s_lut[t] = (float)t / 255.0f;
+    // the run's counts and blur marks start empty: the first tile of a row
+    // clears the bands it holds (a band is two rows of the 16-row shapes)
+    if (it.tx == 0 && Y0 % 32 == 0) {
+        const int nx = USLAM_BLUR_NX(w);
+        uint32_t* f = F.btile[l];
+        for (int band = Y0 / 32; band * 32 < min(Y0 + TH, h); ++band) {
+            if (t < 2) F.bands[l][2 * band + t] = 0u;
+            for (int i = t; i < nx; i += K1_THREADS) f[band * nx + i] = 0u;
+            if (t == 0) f[USLAM_BLUR_AT_RIGHT(w, h) + band] = 0u;
+        }
+        if (Y0 == 0)
+            for (int i = USLAM_BLUR_AT_BELOW(w, h) + t; i < USLAM_BLUR_TILES(w, h, F.margin); i += K1_THREADS) f[i] = 0u;
+    }
+    if (blockIdx.x == 0 && t < 2 && blur_count) blur_count[t] = 0u;
     if (l == 0) {
         // 8 pixels per thread (8-byte loads): a 64-wide tile of 32 rows is
         // 256 segments, one per thread.  16-byte loads left half the threads
         // without a segment and measured slower (0.151 against 0.144 ms on 64
         // frames of 752x480).
-        __syncthreads();
         constexpr int SEGS = TW / 8;
         for (int u = t; u < SEGS * TH; u += K1_THREADS) {
             const int r = u / SEGS;
@@ -269,8 +299,8 @@ k_pyramid(const FrameDev* __restrict__ frames, const TileItem* __restrict__ tile
             float v[8];
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                v[k] = s_lut[(q.x >> (8 * k)) & 255u];
-                v[4 + k] = s_lut[(q.y >> (8 * k)) & 255u];
+                v[k] = unit_u8((q.x >> (8 * k)) & 255u);
+                v[4 + k] = unit_u8((q.y >> (8 * k)) & 255u);
             }
             float* o = out + (size_t)y * lp + x;
             if (x + 8 <= lp) {
@@ -300,7 +330,7 @@ k_pyramid(const FrameDev* __restrict__ frames, const TileItem* __restrict__ tile
             const float b = v - fj, nb = 1.0f - b;
             s_fb[r] = make_float2(b, b);
             s_fnb[r] = make_float2(nb, nb);
-            s_fy[r] = make_int2(edge_index(fj, F.H0), edge_index(fj + 1.0f, F.H0));
+            s_fy[r] = make_int2(edge_index(fj, F.H0) * pitch, edge_index(fj + 1.0f, F.H0) * pitch);
         }
     }
     __syncthreads();
@@ -309,14 +339,13 @@ k_pyramid(const FrameDev* __restrict__ frames, const TileItem* __restrict__ tile
     if (x >= w) return;
     const float2 nab = s_fa[tx];
     const int2 fx = s_fx[tx];
+#pragma unroll 2
     for (int ty = t / TW; ty < TH; ty += K1_THREADS / TW) {
         const int y = Y0 + ty;
         if (y >= h) break;
         const int2 fy = s_fy[ty];
-        const uint8_t* r0 = img + (size_t)fy.x * pitch;
-        const uint8_t* r1 = img + (size_t)fy.y * pitch;
-        const float2 t0 = make_float2(s_lut[__ldg(r0 + fx.x)], s_lut[__ldg(r0 + fx.y)]);
-        const float2 t1 = make_float2(s_lut[__ldg(r1 + fx.x)], s_lut[__ldg(r1 + fx.y)]);
+        const float2 t0 = make_float2(unit_u8(__ldg(img + (uint32_t)(fy.x + fx.x))), unit_u8(__ldg(img + (uint32_t)(fy.x + fx.y))));
+        const float2 t1 = make_float2(unit_u8(__ldg(img + (uint32_t)(fy.y + fx.x))), unit_u8(__ldg(img + (uint32_t)(fy.y + fx.y))));
         const float2 p0 = mul2_rn(mul2_rn(nab, s_fnb[ty]), t0);
         const float2 p1 = mul2_rn(mul2_rn(nab, s_fb[ty]), t1);
         float val = p0.x;
@@ -329,27 +358,44 @@ k_pyramid(const FrameDev* __restrict__ frames, const TileItem* __restrict__ tile
 
 // ---------------------------------------------------------------- K1 ----
 // One TW x TH tile of one level: one TMA load stages the level pixels plus
-// halo (written by k_pyramid) in shared memory, then per pixel the FAST
-// response and the cull decision.
+// halo (written by k_pyramid) in shared memory, then the corner test in two
+// passes: a warp first rejects its cells on a few points (and, in the
+// reference's detector, on the cull mask) and lists the rest, then evaluates
+// the listed ones 32 at a time, so the full circle runs on full warps.  On
+// the 752x480 workload 5 % of the pixels are listed, while nearly every warp
+// ran the circle for one lane or another: 32 frames 0.155 -> 0.100 ms; the cfg
+// profile on 16 frames 0.29 -> 0.144.  Issue-bound still (71 %), 8 CTAs of 32
+// registers per SM.  A persistent form with the next tile's load in flight was
+// slower (0.140): the CTAs of a launch already hide each other's loads.
+// The strengths go through shared memory to 16-byte stores, whose nonzero
+// bytes are the band's keypoint counts (without per-cell caps).
 template <int TW, int TH, bool CFG>
-__global__ void __launch_bounds__(K1_THREADS, CFG ? 5 : 6)
+__global__ void __launch_bounds__(K1_THREADS, CFG ? 4 : 8)
 k_detect(const FrameDev* __restrict__ frames, const TileItem* __restrict__ tiles, int shape, uint32_t* err) {
     constexpr int HY = CFG ? HY_CFG : uslam::HY;
     constexpr int SW = TW + 2 * HX;                   // staged columns [X0 - HX, X0 + TW + HX)
     constexpr int SH = TH + 2 * HY;                   // staged rows [Y0 - HY, Y0 + TH + HY)
     constexpr int BW = TW + 2 * USLAM_TILE_XPAD;      // TMA box columns [X0 - XPAD, X0 + TW + XPAD)
     constexpr int CX = USLAM_TILE_XPAD - HX;          // box column of staged column 0
-    static_assert(K1_THREADS % TW == 0 && CX >= 0 && (BW * 4) % 16 == 0 && BW <= 256 && SH <= 256, "tile shape");
+    constexpr int WARPS = K1_THREADS / 32;
+    constexpr int ROWS = TH / WARPS;                  // tile rows of a warp
+    constexpr int CELLS = CFG ? (TW + 2) * (TH + 2) : TW * TH;  // tested cells (cfg: with a ring of one)
+    // listed cells of one warp (the widest cfg tiles in rounds of 128, for their shared memory)
+    constexpr int LIST = CFG && TW * TH > 2048 ? 128 : (CELLS + 32 * WARPS - 1) / (32 * WARPS) * 32;
+    constexpr int ARC0 = 15;  // s_arc's column of ring column 0: the tile's columns start on 16 bytes
+    static_assert(TH % WARPS == 0 && TW % 32 == 0 && CX >= 0 && (BW * 4) % 16 == 0 && BW <= 256 && SH <= 256, "tile shape");
     __shared__ __align__(128) float sbox[SH][BW];
     __shared__ __align__(8) uint64_t s_bar;
+    __shared__ __align__(16) uint8_t s_out[CFG ? 1 : TH][TW];      // strengths of the tile
+    __shared__ uint16_t s_list[WARPS][LIST];                       // cells that passed the quick test
     __shared__ float s_score[CFG ? TH + 2 : 1][CFG ? TW + 2 : 1];  // cfg: FAST score, tile + 1 ring
-    __shared__ uint8_t s_arc[CFG ? TH + 2 : 1][CFG ? TW + 2 : 1];
+    __shared__ __align__(16) uint8_t s_arc[CFG ? TH + 2 : 1][TW + 32];  // cfg: arc lengths, then strengths
     const TileItem it = tiles[blockIdx.x];
     const FrameDev& F = frames[it.frame];
     const int l = it.level;
     const int w = F.w[l], h = F.h[l];
     const int X0 = it.tx * TW, Y0 = it.ty * TH;
-    const int t = threadIdx.x;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
 
     // 0. one thread starts the tile load.  Box cells outside the level arrive
     //    as 0 and are replaced below.
@@ -360,6 +406,8 @@ k_detect(const FrameDev* __restrict__ frames, const TileItem* __restrict__ tiles
         mbar_expect_tx(&s_bar, (uint32_t)(SH * BW * 4));
         tma_load_2d(&sbox[0][0], tmap, X0 - USLAM_TILE_XPAD, Y0 - HY, &s_bar);
     }
+    if constexpr (!CFG)
+        for (int i = t; i < TW * TH / 16; i += K1_THREADS) reinterpret_cast<uint4*>(s_out)[i] = make_uint4(0u, 0u, 0u, 0u);
     __syncthreads();  // the barrier is initialised before anyone polls it
     const uint32_t first_limit = F.detect_first_wait < 0 ? kTmaWaitLimit : (uint32_t)F.detect_first_wait;
     const bool landed = mbar_wait(&s_bar, 0u, first_limit);
@@ -397,70 +445,130 @@ k_detect(const FrameDev* __restrict__ frames, const TileItem* __restrict__ tiles
     }
     // staged cell (r, c) = sm[r][c], c counted from X0 - HX
     const float(*sm)[BW] = reinterpret_cast<const float(*)[BW]>(&sbox[0][CX]);
-
+    uint16_t* const list = s_list[warp];
+    const uint32_t below = (1u << lane) - 1u;
+    uint32_t nlist = 0;
     if constexpr (CFG) {
-        // score of every pixel of the tile and its 1-pixel ring; pixels within
-        // 3 of the level edge (and outside the level) are never corners
-        for (int i = t; i < (TH + 2) * (TW + 2); i += K1_THREADS) {
-            const int sr = i / (TW + 2), sc = i - sr * (TW + 2);
-            const int y = Y0 - 1 + sr, x = X0 - 1 + sc;
-            uint32_t arc = 0u;
-            float score = 0.0f;
-            if (y >= 3 && y < h - 3 && x >= 3 && x < w - 3) score = cfg_corner(sm, sr - 1 + HY, sc - 1 + HX, &arc);
-            s_score[sr][sc] = score;
-            s_arc[sr][sc] = (uint8_t)arc;
-        }
-        __syncthreads();
-    }
-
-    const int tx = t % TW;
-    const int x = X0 + tx;
-    if (x >= w) return;
-    const uint32_t* mask = F.mask[l];
-    uint8_t* const kpmap = F.kpmap[l];
-    const int kp_pitch = F.kp_pitch[l];
-    for (int ty = t / TW; ty < TH; ty += K1_THREADS / TW) {
-        const int y = Y0 + ty;
-        if (y >= h) break;
-        const int r = ty + HY, c = tx + HX;
-        const size_t p = (size_t)y * (size_t)w + (size_t)x;
-
-        uint32_t keep = 0;
-        if constexpr (CFG) {
-            // 3x3 NMS on the score; a tie goes to the first pixel in raster order
-            const uint32_t A = s_arc[ty + 1][tx + 1];
-            if (A) {
-                const float Sc = s_score[ty + 1][tx + 1];
-                bool ok = true;
+        // 2. cells of the tile and its 1-pixel ring; pixels within 3 of the
+        //    level edge (and outside the level) are never corners.  An arc of 9
+        //    of the 16 points holds two of the points 0, 4, 8 and 12.
+        for (int i0 = 32 * warp; i0 < CELLS;) {
+            for (nlist = 0; i0 < CELLS && nlist + 32u <= (uint32_t)LIST; i0 += 32 * WARPS) {
+                const int i = i0 + lane, sr = i / (TW + 2), sc = i - sr * (TW + 2);
+                const int y = Y0 - 1 + sr, x = X0 - 1 + sc;
+                bool pass = false;
+                if (i < CELLS) {
+                    s_score[sr][sc] = 0.0f;
+                    s_arc[sr][ARC0 + sc] = 0;
+                    if (y >= 3 && y < h - 3 && x >= 3 && x < w - 3) {
+                        const int r = sr - 1 + HY, c = sc - 1 + HX;
+                        const float center = sm[r][c];
+                        int nb = 0, nd = 0;
 #pragma unroll
-                for (int dy = -1; dy <= 1; ++dy)
-#pragma unroll
-                    for (int dx = -1; dx <= 1; ++dx) {
-                        if (dy == 0 && dx == 0) continue;
-                        const float q = s_score[ty + 1 + dy][tx + 1 + dx];
-                        const bool earlier = dy < 0 || (dy == 0 && dx < 0);
-                        ok = ok && (earlier ? (Sc > q) : (Sc >= q));
-                    }
-                keep = ok ? A : 0u;
-            }
-        } else {
-            // 2. FAST response + cull (resources/cull_corners.wgsl; see mask_bit)
-            const uint32_t S = fast_response(sm, r, c);
-            if (S > 0u && mask_bit(mask, (int)p)) {
-                keep = S;
-                if (y == 0) {
-                    // row 0: first arg-max of the 1x3 region [9k, min(9k+3, w))
-                    const int start = x - x % 9;
-                    const int end = min(start + 3, w);
-                    for (int q = start; q < end; ++q) {
-                        if (q == x) continue;
-                        const uint32_t Sq = fast_response(sm, r, c + (q - x));
-                        if ((q < x && Sq >= S) || (q > x && Sq > S)) keep = 0;
+                        for (int k = 0; k < 16; k += 4) {
+                            const float p = sm[r + circle_y(k)][c + circle_x(k)];
+                            nb += p - center > kCfgThreshold ? 1 : 0;
+                            nd += center - p > kCfgThreshold ? 1 : 0;
+                        }
+                        pass = nb >= 2 || nd >= 2;
                     }
                 }
+                const uint32_t b = __ballot_sync(0xffffffffu, pass);
+                if (pass) list[nlist + __popc(b & below)] = (uint16_t)i;
+                nlist += __popc(b);
+            }
+            __syncwarp();
+            for (uint32_t q = lane; q < nlist; q += 32u) {
+                const int i = list[q], sr = i / (TW + 2), sc = i - sr * (TW + 2);
+                uint32_t arc;
+                s_score[sr][sc] = cfg_corner(sm, sr - 1 + HY, sc - 1 + HX, &arc);
+                s_arc[sr][ARC0 + sc] = (uint8_t)arc;
+            }
+            __syncwarp();
+        }
+        __syncthreads();
+        // 3. 3x3 NMS on the score; a tie goes to the first pixel in raster
+        //    order (a cell's arc is read and replaced by its own thread alone)
+        for (int i = lane; i < ROWS * TW; i += 32) {
+            const int sr = warp * ROWS + i / TW + 1, sc = i % TW + 1;
+            const uint32_t A = s_arc[sr][ARC0 + sc];
+            if (A == 0u) continue;
+            const float Sc = s_score[sr][sc];
+            bool ok = true;
+#pragma unroll
+            for (int dy = -1; dy <= 1; ++dy)
+#pragma unroll
+                for (int dx = -1; dx <= 1; ++dx) {
+                    if (dy == 0 && dx == 0) continue;
+                    const float v = s_score[sr + dy][sc + dx];
+                    const bool earlier = dy < 0 || (dy == 0 && dx < 0);
+                    ok = ok && (earlier ? (Sc > v) : (Sc >= v));
+                }
+            if (!ok) s_arc[sr][ARC0 + sc] = 0;
+        }
+        __syncwarp();
+    } else {
+        // 2. the warp's rows: the cull mask (resources/cull_corners.wgsl; 32
+        //    bits of it per segment), then points 7 and 8, which every
+        //    non-wrapping run of 9 holds, and 4 or 12, one of which it holds
+        const uint32_t* mask = F.mask[l];
+        const int last = (w * h - 1) >> 5;  // (a level holds fewer than 2^31 pixels)
+#pragma unroll
+        for (int rr = 0; rr < ROWS; ++rr) {
+            const int ty = warp * ROWS + rr, y = Y0 + ty;
+            if (y >= h) break;
+#pragma unroll
+            for (int s = 0; s < TW / 32; ++s) {
+                const int tx = 32 * s + lane, x = X0 + tx;
+                const int p0 = y * w + X0 + 32 * s, q0 = p0 >> 5;
+                const uint32_t m = __funnelshift_r(__ldg(mask + min(q0, last)), __ldg(mask + min(q0 + 1, last)), p0 & 31);
+                const int r = ty + HY, c = tx + HX;
+                const float center = sm[r][c];
+                const float d7 = fabsf(center - sm[r + 3][c + 1]), d8 = fabsf(center - sm[r + 3][c]);
+                const float d4 = fabsf(center - sm[r][c + 3]), d12 = fabsf(center - sm[r][c - 3]);
+                const bool pass = (x < w) & ((m >> lane) & 1u) & (fminf(fminf(d7, d8), fmaxf(d4, d12)) > 0.15f);
+                const uint32_t b = __ballot_sync(0xffffffffu, pass);
+                if (pass) list[nlist + __popc(b & below)] = (uint16_t)(ty * TW + tx);
+                nlist += __popc(b);
             }
         }
-        kpmap[(size_t)y * kp_pitch + x] = (uint8_t)keep;
+        __syncwarp();
+        // 3. the listed cells: FAST response (and the rest of the cull)
+        for (uint32_t q = lane; q < nlist; q += 32u) {
+            const int i = list[q], ty = i / TW, tx = i - ty * TW;
+            const int r = ty + HY, c = tx + HX;
+            const uint32_t S = fast_response(sm, r, c);
+            uint32_t keep = S;
+            if (S > 0u && Y0 + ty == 0) {
+                // row 0: first arg-max of the 1x3 region [9k, min(9k+3, w))
+                const int x = X0 + tx, start = x - x % 9, end = min(start + 3, w);
+                for (int u = start; u < end; ++u) {
+                    if (u == x) continue;
+                    const uint32_t Sq = fast_response(sm, r, c + (u - x));
+                    if ((u < x && Sq >= S) || (u > x && Sq > S)) keep = 0;
+                }
+            }
+            s_out[ty][tx] = (uint8_t)keep;
+        }
+        __syncwarp();
+    }
+    // 4. the warp's rows of the map, 16 bytes a lane (X0 + 16 k < w lies within the row's pitch)
+    uint8_t* const kpmap = F.kpmap[l];
+    const int kp_pitch = F.kp_pitch[l];
+    uint32_t found = 0;
+    for (int q = lane; q < ROWS * TW / 16; q += 32) {
+        const int ty = warp * ROWS + q / (TW / 16), tx = q % (TW / 16) * 16;
+        if (Y0 + ty >= h || X0 + tx >= w) continue;
+        const uint4 v = *reinterpret_cast<const uint4*>(CFG ? &s_arc[CFG ? ty + 1 : 0][ARC0 + 1 + tx] : &s_out[CFG ? 0 : ty][tx]);
+        *reinterpret_cast<uint4*>(kpmap + (size_t)(Y0 + ty) * kp_pitch + X0 + tx) = v;
+        found += nonzero_bytes16(v);
+    }
+    if (F.cell_cap <= 0) {
+        // raw and kept counts of the 32-row band (equal), as one 64-bit word
+        found = warp_sum_u32(found);
+        if (lane == 0 && found > 0u)
+            atomicAdd(reinterpret_cast<unsigned long long*>(F.bands[l] + 2 * ((Y0 + warp * ROWS) / 32)),
+                      (unsigned long long)found << 32 | found);
     }
 }
 
@@ -789,10 +897,6 @@ k_blur(const FrameDev* __restrict__ frames, BlurList bl, uint32_t* err, float on
 // ------------------------------------------------------------ compact ----
 constexpr int KC_THREADS = 1024;
 
-__device__ __forceinline__ int nonzero_bytes(uint32_t v) {
-    return __popc(__vcmpne4(v, 0u)) >> 3;
-}
-
 // Block-wide exclusive scan of one value per thread; returns the prefix and
 // writes the block total to *total.
 __device__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* s_warp, uint32_t* total) {
@@ -981,11 +1085,6 @@ constexpr int KBAND_THREADS = 1024;
 constexpr int KBAND_WARPS = KBAND_THREADS / 32;
 static_assert(KBAND_WARPS == USLAM_BLUR_TH, "a warp per row of a band, which is a blur tile row");
 
-__device__ __forceinline__ uint32_t warp_sum_u32(uint32_t v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
 __device__ __forceinline__ uint32_t warp_inclusive_scan(uint32_t v, int lane) {
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -998,68 +1097,49 @@ __device__ __forceinline__ uint32_t warp_inclusive_scan(uint32_t v, int lane) {
 __device__ __forceinline__ uint4 map16(const uint8_t* row, int x, int w) {
     return x < w ? *reinterpret_cast<const uint4*>(row + x) : make_uint4(0u, 0u, 0u, 0u);
 }
-__device__ __forceinline__ uint32_t nonzero_bytes16(const uint4& v) {
-    return (uint32_t)(nonzero_bytes(v.x) + nonzero_bytes(v.y) + nonzero_bytes(v.z) + nonzero_bytes(v.w));
-}
 
 // This warp's share of a band and its counts: one row (rows mode), or cells
 // warp, warp + KBAND_WARPS, ... (cells mode).
-__device__ __forceinline__ void band_warp_counts(const FrameDev& F, int l, int band, uint32_t* raw, uint32_t* kept) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int w = F.w[l], h = F.h[l], kpitch = F.kp_pitch[l];
-    const uint8_t* kp = F.kpmap[l];
-    uint32_t r = 0, k = 0;
-    if (F.cell_cap <= 0) {
-        const int y = band * 32 + warp;
-        if (y < h)
-            for (int x = 16 * lane; x < w; x += 512) r += nonzero_bytes16(map16(kp + (size_t)y * kpitch, x, w));
-        k = r = warp_sum_u32(r);
-    } else {
-        const uint32_t ccap = (uint32_t)F.cell_cap;
-        for (int cx = warp; cx * 32 < w; cx += KBAND_WARPS) {
-            uint32_t v[8];
-            load_cell_row(kp, kpitch, w, h, cx * 32, band * 32 + lane, v);
-            uint32_t n = 0;
-#pragma unroll
-            for (int q = 0; q < 8; ++q) n += (uint32_t)nonzero_bytes(v[q]);
-            n = warp_sum_u32(n);
-            r += n;
-            k += n < ccap ? n : ccap;
-        }
-    }
-    *raw = r;
-    *kept = k;
+__device__ __forceinline__ uint32_t band_row_count(const FrameDev& F, int l, int y) {
+    const int lane = threadIdx.x & 31, w = F.w[l];
+    const uint8_t* row = F.kpmap[l] + (size_t)y * F.kp_pitch[l];
+    uint32_t r = 0;
+    if (y < F.h[l])
+        for (int x = 16 * lane; x < w; x += 512) r += nonzero_bytes16(map16(row, x, w));
+    return warp_sum_u32(r);
 }
 
-// Also clears the band's blur marks and the run's list of blur items.
+// Raw and kept counts of a band with per-cell caps (without them k_detect
+// counts, and this kernel does not run).
 __global__ void __launch_bounds__(KBAND_THREADS)
-k_band_count(const FrameDev* __restrict__ frames, const BandItem* __restrict__ items, BlurList bl) {
+k_band_count(const FrameDev* __restrict__ frames, const BandItem* __restrict__ items) {
     __shared__ uint32_t s_raw[KBAND_WARPS], s_kept[KBAND_WARPS];
     const BandItem it = items[blockIdx.x];
     const FrameDev& F = frames[it.frame];
-    {
-        const int l = it.level, w = F.w[l], h = F.h[l], nx = USLAM_BLUR_NX(w);
-        uint32_t* f = F.btile[l];
-        for (int i = threadIdx.x; i < nx; i += KBAND_THREADS) f[it.band * nx + i] = 0u;
-        if (threadIdx.x == 0) f[USLAM_BLUR_AT_RIGHT(w, h) + it.band] = 0u;
-        if (it.band == 0)
-            for (int i = USLAM_BLUR_AT_BELOW(w, h) + threadIdx.x; i < USLAM_BLUR_TILES(w, h, F.margin); i += KBAND_THREADS)
-                f[i] = 0u;
-        if (blockIdx.x == 0 && threadIdx.x < 2) bl.count[threadIdx.x] = 0u;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int l = it.level, w = F.w[l], h = F.h[l];
+    const uint32_t ccap = (uint32_t)F.cell_cap;
+    uint32_t r = 0, k = 0;
+    for (int cx = warp; cx * 32 < w; cx += KBAND_WARPS) {
+        uint32_t v[8];
+        load_cell_row(F.kpmap[l], F.kp_pitch[l], w, h, cx * 32, it.band * 32 + lane, v);
+        uint32_t n = 0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) n += (uint32_t)nonzero_bytes(v[q]);
+        n = warp_sum_u32(n);
+        r += n;
+        k += n < ccap ? n : ccap;
     }
-    uint32_t r, k;
-    band_warp_counts(F, it.level, it.band, &r, &k);
-    const int lane = threadIdx.x & 31;
     if (lane == 0) {
-        s_raw[threadIdx.x >> 5] = r;
-        s_kept[threadIdx.x >> 5] = k;
+        s_raw[warp] = r;
+        s_kept[warp] = k;
     }
     __syncthreads();
-    if (threadIdx.x < 32) {
+    if (warp == 0) {
         const uint32_t R = warp_sum_u32(s_raw[lane]), K = warp_sum_u32(s_kept[lane]);
         if (lane == 0) {
-            F.bands[it.level][2 * it.band] = R;
-            F.bands[it.level][2 * it.band + 1] = K;
+            F.bands[l][2 * it.band] = R;
+            F.bands[l][2 * it.band + 1] = K;
         }
     }
 }
@@ -1136,13 +1216,12 @@ k_band_write(const FrameDev* __restrict__ frames, const BandItem* __restrict__ i
     pk = warp_sum_u32(pk);
     tr = warp_sum_u32(tr);
     tk = warp_sum_u32(tk);
-    uint32_t r, k;
-    band_warp_counts(F, l, band, &r, &k);
+    const uint32_t mine_in_row = F.cell_cap <= 0 ? band_row_count(F, l, band * 32 + warp) : 0u;
     if (lane == 0) {
         s_red[0][warp] = pk;
         s_red[1][warp] = tr;
         s_red[2][warp] = tk;
-        s_wbase[warp] = k;
+        s_wbase[warp] = mine_in_row;
     }
     for (int i = threadIdx.x; i < 4 * notes; i += KBAND_THREADS) s_note[i & 3][i >> 2] = 0;
     for (int i = threadIdx.x; i < KBAND_MARKS; i += KBAND_THREADS) s_mark[i] = 0;
@@ -2521,14 +2600,15 @@ cudaError_t launch_detect_profile(const FrameDev* frames, const TileItem* tiles,
     }
     return cudaGetLastError();
 }
-cudaError_t launch_pyramid(const FrameDev* frames, const TileItem* tiles, int ntiles, int shape, cudaStream_t st) {
+cudaError_t launch_pyramid(const FrameDev* frames, const TileItem* tiles, int ntiles, int shape, uint32_t* blur_count,
+                           cudaStream_t st) {
     if (ntiles <= 0) return cudaSuccess;
     switch (shape) {
-        case 0: k_pyramid<64, 32><<<ntiles, K1_THREADS, 0, st>>>(frames, tiles); break;
-        case 1: k_pyramid<128, 32><<<ntiles, K1_THREADS, 0, st>>>(frames, tiles); break;
-        case 2: k_pyramid<64, 16><<<ntiles, K1_THREADS, 0, st>>>(frames, tiles); break;
-        case 3: k_pyramid<32, 32><<<ntiles, K1_THREADS, 0, st>>>(frames, tiles); break;
-        case 4: k_pyramid<128, 16><<<ntiles, K1_THREADS, 0, st>>>(frames, tiles); break;
+        case 0: k_pyramid<64, 32><<<ntiles, K1_THREADS, 0, st>>>(frames, tiles, blur_count); break;
+        case 1: k_pyramid<128, 32><<<ntiles, K1_THREADS, 0, st>>>(frames, tiles, blur_count); break;
+        case 2: k_pyramid<64, 16><<<ntiles, K1_THREADS, 0, st>>>(frames, tiles, blur_count); break;
+        case 3: k_pyramid<32, 32><<<ntiles, K1_THREADS, 0, st>>>(frames, tiles, blur_count); break;
+        case 4: k_pyramid<128, 16><<<ntiles, K1_THREADS, 0, st>>>(frames, tiles, blur_count); break;
         default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
@@ -2542,12 +2622,14 @@ cudaError_t launch_detect(const FrameDev* frames, const TileItem* tiles, int nti
 }
 
 // The ordered lists and the list of blur tiles they need.
-cudaError_t launch_compact_banded(const FrameDev* frames, const BandItem* bands, int nbands, BlurList bl,
+cudaError_t launch_compact_banded(const FrameDev* frames, const BandItem* bands, int nbands, int cell_cap, BlurList bl,
                                   cudaStream_t st) {
     if (nbands <= 0) return cudaSuccess;
-    k_band_count<<<nbands, KBAND_THREADS, 0, st>>>(frames, bands, bl);
-    const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
+    if (cell_cap > 0) {
+        k_band_count<<<nbands, KBAND_THREADS, 0, st>>>(frames, bands);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
     k_band_write<<<nbands, KBAND_THREADS, 0, st>>>(frames, bands, bl);
     return cudaGetLastError();
 }

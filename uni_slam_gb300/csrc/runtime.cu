@@ -247,11 +247,11 @@ cudaError_t enqueue_frames(uslam_batch* b, const Program& P, const Lane& ln) {
     uslam_ctx* c = b->ctx;
     cudaError_t e = cudaSuccess;
     if (P.ntiles <= 0) return e;
-    if ((e = launch_pyramid_shaped(b->d_frames, P.tiles, P.tile_begin, ln.st)) != cudaSuccess) return e;
+    if ((e = launch_pyramid_shaped(b->d_frames, P.tiles, P.tile_begin, P.blur.count, ln.st)) != cudaSuccess) return e;
     if ((e = launch_detect_only_shaped(b->d_frames, P.tiles, P.tile_begin, c->detector, b->d_err, ln.st)) !=
         cudaSuccess)
         return e;
-    if ((e = launch_compact_banded(b->d_frames, P.bands, P.nbands, P.blur, ln.st)) != cudaSuccess) return e;
+    if ((e = launch_compact_banded(b->d_frames, P.bands, P.nbands, c->cell_cap, P.blur, ln.st)) != cudaSuccess) return e;
     // k_blur (the blur cache where the kept keypoints' tests read it) needs
     // the list of k_band_write, k_xsort the kept features: they run side by
     // side, and k_describe needs both (in a captured graph a fork/join).
@@ -1140,13 +1140,13 @@ uslam_status uslam_batch_profile(uslam_batch* b, int iters, float* kernel_ms) {
         mark();
         for (int sh = 0; sh < kNumTileShapes && e == cudaSuccess; ++sh)
             e = launch_pyramid(b->d_frames, P.tiles + P.tile_begin[sh], P.tile_begin[sh + 1] - P.tile_begin[sh], sh,
-                               b->stream);
+                               P.blur.count, b->stream);
         mark();
         for (int sh = 0; sh < kNumTileShapes && e == cudaSuccess; ++sh)
             e = launch_detect(b->d_frames, P.tiles + P.tile_begin[sh], P.tile_begin[sh + 1] - P.tile_begin[sh], sh,
                               c->detector, b->d_err, b->stream);
         mark();
-        if (e == cudaSuccess) e = launch_compact_banded(b->d_frames, P.bands, P.nbands, P.blur, b->stream);
+        if (e == cudaSuccess) e = launch_compact_banded(b->d_frames, P.bands, P.nbands, c->cell_cap, P.blur, b->stream);
         if (e == cudaSuccess) e = launch_xsort(b->d_frames, P.fsegs, P.nfsegs, b->max_w, b->stream);
         mark();
         if (e == cudaSuccess) e = launch_blur(b->d_frames, P.blur, P.nblur, c->num_sms, b->d_err, b->stream);
@@ -1245,7 +1245,7 @@ uslam_status uslam_autotune(uslam_ctx* ctx, int width, int height, const uint8_t
         std::vector<float> t;
         for (int r = -2; r < reps && e == cudaSuccess; ++r) {
             e = cudaEventRecord(e0, b->stream);
-            if (e == cudaSuccess) e = launch_pyramid(b->d_frames, d_tiles, n, s, b->stream);
+            if (e == cudaSuccess) e = launch_pyramid(b->d_frames, d_tiles, n, s, nullptr, b->stream);
             if (e == cudaSuccess) e = launch_detect(b->d_frames, d_tiles, n, s, ctx->detector, b->d_err, b->stream);
             if (e == cudaSuccess) e = cudaEventRecord(e1, b->stream);
             if (e == cudaSuccess) e = cudaEventSynchronize(e1);

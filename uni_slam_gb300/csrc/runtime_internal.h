@@ -25,8 +25,9 @@ struct MatchSegDev {
 };
 cudaError_t init_constants();
 cudaError_t launch_detect(const FrameDev*, const TileItem*, int, int, int, uint32_t*, cudaStream_t);
-cudaError_t launch_pyramid(const FrameDev*, const TileItem*, int, int, cudaStream_t);
-cudaError_t launch_compact_banded(const FrameDev*, const BandItem*, int, BlurList, cudaStream_t);
+// blur_count: the run's BlurList::count, cleared (null: none)
+cudaError_t launch_pyramid(const FrameDev*, const TileItem*, int, int, uint32_t* blur_count, cudaStream_t);
+cudaError_t launch_compact_banded(const FrameDev*, const BandItem*, int, int cell_cap, BlurList, cudaStream_t);
 cudaError_t launch_xsort(const FrameDev*, const SegDev*, int, int, cudaStream_t);
 cudaError_t launch_blur(const FrameDev*, BlurList, int max_tiles, int num_sms, uint32_t* err, cudaStream_t);
 cudaError_t launch_describe(const FrameDev*, const SegDev*, int, const int32_t*, int, bool, bool, cudaStream_t);
@@ -200,11 +201,11 @@ struct ShapedTiles {
 
 // One k_pyramid launch per tile shape present.
 inline cudaError_t launch_pyramid_shaped(const FrameDev* frames, const TileItem* d_tiles, const int* begin,
-                                         cudaStream_t st) {
+                                         uint32_t* blur_count, cudaStream_t st) {
     for (int s = 0; s < kNumTileShapes; ++s) {
         const int n = begin[s + 1] - begin[s];
         if (n <= 0) continue;
-        const cudaError_t e = launch_pyramid(frames, d_tiles + begin[s], n, s, st);
+        const cudaError_t e = launch_pyramid(frames, d_tiles + begin[s], n, s, blur_count, st);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -223,8 +224,8 @@ inline cudaError_t launch_detect_only_shaped(const FrameDev* frames, const TileI
 // One k_pyramid launch, then one k_detect launch, per tile shape present
 // (every pyramid level is written before any tile of that shape reads it).
 inline cudaError_t launch_detect_shaped(const FrameDev* frames, const TileItem* d_tiles, const int* begin,
-                                        int detector, uint32_t* err, cudaStream_t st) {
-    const cudaError_t e = launch_pyramid_shaped(frames, d_tiles, begin, st);
+                                        int detector, uint32_t* err, uint32_t* blur_count, cudaStream_t st) {
+    const cudaError_t e = launch_pyramid_shaped(frames, d_tiles, begin, blur_count, st);
     if (e != cudaSuccess) return e;
     for (int s = 0; s < kNumTileShapes; ++s) {
         const int n = begin[s + 1] - begin[s];

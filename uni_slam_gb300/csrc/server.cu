@@ -322,8 +322,8 @@ cudaError_t launch_batch(uslam_server* s, const std::vector<uint64_t>& tickets, 
     const BlurList bl{reinterpret_cast<TileItem*>(B.d + B.bytes + 256), reinterpret_cast<uint32_t*>(B.d + B.bytes)};
     const int grid = c->num_sms * 4;
     const int nf = static_cast<int>(fsegs.size());
-    if ((e = launch_detect_shaped(s->d_frames, d_tiles, shaped.begin, c->detector, s->d_err, st)) != cudaSuccess) return e;
-    if ((e = launch_compact_banded(s->d_frames, d_bands, static_cast<int>(bands.size()), bl, st)) != cudaSuccess)
+    if ((e = launch_detect_shaped(s->d_frames, d_tiles, shaped.begin, c->detector, s->d_err, bl.count, st)) != cudaSuccess) return e;
+    if ((e = launch_compact_banded(s->d_frames, d_bands, static_cast<int>(bands.size()), c->cell_cap, bl, st)) != cudaSuccess)
         return e;
     if ((e = launch_xsort(s->d_frames, d_fsegs, nf, s->max_w, st)) != cudaSuccess) return e;
     if ((e = launch_blur(s->d_frames, bl, blur_tiles, c->num_sms, s->d_err, st)) != cudaSuccess) return e;
