@@ -959,58 +959,9 @@ __device__ __forceinline__ void load_cell_row(const uint8_t* kp, int kpitch, int
     }
 }
 
-__device__ void xsort_level(const FrameDev& F, int l, uint32_t kept, uint32_t* s_hist, uint32_t* s_warp);
-
-// One counting-sort pass over a level's kept features (dynamic shared memory
-// s_hist of w + 1 counters): the indices of the features with pick(i) true,
-// sorted by x, go to order_out; colstart_out (if given) receives the first
-// slot of each column.  Returns the number of features picked.
-// inv_out (if given) receives for every picked feature i its position plus
-// inv_base, and with inv_miss set ~0 for the others.
-template <typename Pick>
-__device__ uint32_t xsort_pass(const uint32_t* feats, uint32_t kept, int w, Pick pick, uint32_t* order_out,
-                               uint32_t* colstart_out, uint32_t* s_hist, uint32_t* s_warp, uint32_t* inv_out = nullptr,
-                               uint32_t inv_base = 0u, bool inv_miss = false) {
-    for (int i = threadIdx.x; i <= w; i += blockDim.x) s_hist[i] = 0u;
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < kept; i += blockDim.x)
-        if (pick(i)) atomicAdd(&s_hist[(int)__uint_as_float(feats[(size_t)i * 12u])], 1u);
-    __syncthreads();
-    const int per = (w + (int)blockDim.x) / (int)blockDim.x;  // bins per thread over w + 1 bins
-    const int b0 = threadIdx.x * per;
-    uint32_t local = 0;
-    for (int k = 0; k < per; ++k) {
-        const int b = b0 + k;
-        if (b < w) local += s_hist[b];
-    }
-    uint32_t tot;
-    uint32_t run = block_exclusive_scan(local, s_warp, &tot);
-    for (int k = 0; k < per; ++k) {
-        const int b = b0 + k;
-        if (b <= w) {
-            const uint32_t c = b < w ? s_hist[b] : 0u;
-            if (colstart_out) colstart_out[b] = run;
-            s_hist[b] = run;  // becomes the fill cursor
-            run += c;
-        }
-    }
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < kept; i += blockDim.x) {
-        if (pick(i)) {
-            const uint32_t pos = atomicAdd(&s_hist[(int)__uint_as_float(feats[(size_t)i * 12u])], 1u);
-            order_out[pos] = i;
-            if (inv_out) inv_out[i] = inv_base + pos;
-        } else if (inv_out && inv_miss) {
-            inv_out[i] = 0xffffffffu;
-        }
-    }
-    __syncthreads();
-    return tot;
-}
-
 // LOD-0 y of a feature (match_features_cpu.cpp:58-64: f32 scale iterated).
-__device__ __forceinline__ float lod0_y(const uint32_t* feats, uint32_t i, float scale) {
-    return (float)(uint32_t)__uint_as_float(feats[(size_t)i * 12u + 1u]) * scale;
+__device__ __forceinline__ float lod0_y(uint32_t y_bits, float scale) {
+    return (float)(uint32_t)__uint_as_float(y_bits) * scale;
 }
 
 // The matcher's index of one level.  The frame height is cut into
@@ -1021,47 +972,103 @@ __device__ __forceinline__ float lod0_y(const uint32_t* feats, uint32_t i, float
 //    of band b is in list b;
 //  * query order = the features grouped by the band of their own LOD-0 y,
 //    sorted by x within a band, with the band offsets after the column tables.
-__device__ void xsort_level(const FrameDev& F, int l, uint32_t kept, uint32_t* s_hist, uint32_t* s_warp) {
+// One CTA per (frame, level, list): a counting sort by x in shared memory
+// (s_hist of w + 1 counters), the candidate lists and the bands of the query
+// order side by side (a CTA that made all six lists in turn took 51 us on the
+// largest level of a 1920x1080 frame).  XU features a thread are in flight at
+// a time.
+constexpr int XU = 4;
+__global__ void __launch_bounds__(KC_THREADS, 2)
+k_xsort(const FrameDev* __restrict__ frames, const SegDev* __restrict__ segs) {
     constexpr int NB = USLAM_MATCH_BANDS;
-    const int w = F.w[l];
+    extern __shared__ uint32_t s_hist[];  // [w + 1]
+    __shared__ uint32_t s_warp[33];
+    const SegDev sg = segs[blockIdx.x];
+    const FrameDev& F = frames[sg.frame];
+    const int l = sg.level, w = F.w[l];
+    const bool query = blockIdx.y >= NB;
+    const int b = (int)blockIdx.y - (query ? NB : 0);
+    const uint32_t kept = F.kept[l];
     const uint32_t* feats = F.feats[l];
     float scale = 1.0f;
     for (int i = 0; i < l; ++i) scale = scale * 1.2f;
     const float H = (float)(uint32_t)F.H0;
     const float margin = 0.1f * H + 2.0f;
+    const float lo = (float)b * H / (float)NB - margin, hi = (float)(b + 1) * H / (float)NB + margin;
     const size_t cap = (size_t)(F.cap > 0 ? F.cap : 1);
-    uint32_t* qband = F.colstart[l] + (size_t)NB * (size_t)(w + 1);
-    uint32_t* inv = F.winv[l];  // the tensor-core matcher's positions (null without it)
-    for (int b = 0; b < NB; ++b) {
-        const float lo = (float)b * H / (float)NB - margin, hi = (float)(b + 1) * H / (float)NB + margin;
-        xsort_pass(
-            feats, kept, w,
-            [&](uint32_t i) {
-                const float y = lod0_y(feats, i, scale);
-                return y >= lo && y <= hi;
-            },
-            F.xorder[l] + (size_t)b * cap, F.colstart[l] + (size_t)b * (size_t)(w + 1), s_hist, s_warp,
-            inv ? inv + cap * (size_t)(1 + b) : nullptr, 0u, true);
+    // -1: in an earlier band's list of the query order, 0: in this list, 1: in neither
+    auto place = [&](float y) {
+        if (!query) return y >= lo && y <= hi ? 0 : 1;
+        const int q = match_band(y, H);
+        return q < b ? -1 : (q == b ? 0 : 1);
+    };
+    for (int i = threadIdx.x; i <= w; i += KC_THREADS) s_hist[i] = 0u;
+    __syncthreads();
+    uint32_t earlier = 0;
+    for (uint32_t i0 = threadIdx.x; i0 < kept; i0 += XU * KC_THREADS) {
+        uint2 xy[XU];
+#pragma unroll
+        for (int u = 0; u < XU; ++u) {
+            const uint32_t i = i0 + u * KC_THREADS;
+            if (i < kept) xy[u] = *reinterpret_cast<const uint2*>(feats + (size_t)i * 12u);
+        }
+#pragma unroll
+        for (int u = 0; u < XU; ++u) {
+            if (i0 + u * KC_THREADS >= kept) break;
+            const int p = place(lod0_y(xy[u].y, scale));
+            if (p == 0) atomicAdd(&s_hist[(int)__uint_as_float(xy[u].x)], 1u);
+            earlier += p < 0 ? 1u : 0u;
+        }
     }
+    __syncthreads();
+    // this band's queries start after the earlier bands'
     uint32_t base = 0;
-    for (int b = 0; b < NB; ++b) {
-        const uint32_t n = xsort_pass(
-            feats, kept, w, [&](uint32_t i) { return match_band(lod0_y(feats, i, scale), H) == b; },
-            F.qorder[l] + base, nullptr, s_hist, s_warp, inv, base, false);
-        if (threadIdx.x == 0) qband[b] = base;
-        base += n;
+    if (query) block_exclusive_scan(earlier, s_warp, &base);
+    uint32_t* const qband = F.colstart[l] + (size_t)NB * (size_t)(w + 1);
+    uint32_t* const order = query ? F.qorder[l] + base : F.xorder[l] + (size_t)b * cap;
+    uint32_t* const colstart = F.colstart[l] + (size_t)b * (size_t)(w + 1);
+    // the tensor-core matcher's positions (null without it): of the query
+    // order, then of each list (~0: not in it)
+    uint32_t* const inv = F.winv[l] ? F.winv[l] + (query ? 0 : cap * (size_t)(1 + b)) : nullptr;
+    const int per = (w + KC_THREADS) / KC_THREADS;  // bins per thread over w + 1 bins
+    const int b0 = threadIdx.x * per;
+    uint32_t local = 0;
+    for (int k = 0; k < per; ++k)
+        if (b0 + k < w) local += s_hist[b0 + k];
+    uint32_t tot;
+    uint32_t run = block_exclusive_scan(local, s_warp, &tot);
+    for (int k = 0; k < per; ++k) {
+        if (b0 + k > w) break;
+        const uint32_t c = b0 + k < w ? s_hist[b0 + k] : 0u;
+        if (!query) colstart[b0 + k] = run;
+        s_hist[b0 + k] = run;  // becomes the fill cursor
+        run += c;
     }
-    if (threadIdx.x == 0) qband[NB] = base;
-}
-
-// Per (frame, level): the x counting sort after the banded compaction.
-__global__ void __launch_bounds__(KC_THREADS)
-k_xsort(const FrameDev* __restrict__ frames, const SegDev* __restrict__ segs) {
-    extern __shared__ uint32_t s_hist[];  // [w + 1]
-    __shared__ uint32_t s_warp[33];
-    const SegDev sg = segs[blockIdx.x];
-    const FrameDev& F = frames[sg.frame];
-    xsort_level(F, sg.level, F.kept[sg.level], s_hist, s_warp);
+    if (query && threadIdx.x == 0) {
+        qband[b] = base;
+        if (b == NB - 1) qband[NB] = base + tot;
+    }
+    __syncthreads();
+    for (uint32_t i0 = threadIdx.x; i0 < kept; i0 += XU * KC_THREADS) {
+        uint2 xy[XU];
+#pragma unroll
+        for (int u = 0; u < XU; ++u) {
+            const uint32_t i = i0 + u * KC_THREADS;
+            if (i < kept) xy[u] = *reinterpret_cast<const uint2*>(feats + (size_t)i * 12u);
+        }
+#pragma unroll
+        for (int u = 0; u < XU; ++u) {
+            const uint32_t i = i0 + u * KC_THREADS;
+            if (i >= kept) break;
+            if (place(lod0_y(xy[u].y, scale)) == 0) {
+                const uint32_t pos = atomicAdd(&s_hist[(int)__uint_as_float(xy[u].x)], 1u);
+                order[pos] = i;
+                if (inv) inv[i] = base + pos;
+            } else if (inv && !query) {
+                inv[i] = 0xffffffffu;
+            }
+        }
+    }
 }
 
 // --------------------------------------------------- banded compaction ----
@@ -2463,33 +2470,45 @@ k_bruteforce(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pa
 }
 
 // ---------------------------------------------------------- mutual ----
-constexpr int KU_THREADS = 256;
+constexpr int KU_THREADS = 1024;
+constexpr int KU_ITEMS = 8;  // features of a thread in one round
 
 // One CTA per (pair, level of a): keep (a, b) iff b2a[b] == a, in a order
 // (match_features_cpu.cpp:196-205).
 // MUTUAL = false: every a with a2b[a] >= 0 is emitted (brute-force mode,
 // which has no cross-check).
+// Latency bounds it: a round looks at 8192 features with all of a thread's
+// loads in flight and orders them by one scan of the warps' counts (rounds of
+// 256 took 53 us on the largest level of a 1920x1080 frame, 172 on a
+// 3840x2160 one).
 template <bool MUTUAL>
 __global__ void __launch_bounds__(KU_THREADS)
 k_mutual(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pairs, const SegDev* __restrict__ segs,
          uint32_t* err, uint32_t* reset_word) {
+    constexpr int WARPS = KU_THREADS / 32;
+    static_assert(WARPS == 32, "the scan takes a warp per item index and a lane per warp");
     // k_match's claim counters for its next launch on this stream (k_mutual
     // always follows k_match, which has finished with them)
     if (reset_word && blockIdx.x == 0)
         for (int i = threadIdx.x; i < KM_CLAIM_WORDS; i += blockDim.x) reset_word[i] = 0u;
-    __shared__ uint32_t s_warp[33];
+    __shared__ uint32_t s_cnt[KU_ITEMS][WARPS];  // matches per (item index, warp), then those before them in the row
+    __shared__ uint32_t s_row[KU_ITEMS];
     const int pi = segs[blockIdx.x].frame;  // pair index
     const int l = segs[blockIdx.x].level;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const PairDev& P = pairs[pi];
     const FrameDev& A = frames[P.prev];
     const FrameDev& B = frames[P.curr];
     const uint32_t n = A.kept[l];
+    int32_t* const a2b = P.a2b + (size_t)l * A.cap;
     uint32_t base = 0;
-    for (uint32_t c0 = 0; c0 < n; c0 += KU_THREADS) {
-        const uint32_t i = c0 + threadIdx.x;
-        int32_t m = -1;
-        bool ok = false;
-        if (i < n) {
+    for (uint32_t c0 = 0; c0 < n; c0 += KU_THREADS * KU_ITEMS) {
+        int32_t m[KU_ITEMS];
+#pragma unroll
+        for (int u = 0; u < KU_ITEMS; ++u) {
+            const uint32_t i = c0 + u * KU_THREADS + threadIdx.x;
+            m[u] = -1;
+            if (i >= n) continue;
             if (!MUTUAL && P.bf_splits > 1) {
                 // merge the brute-force splits: the two smallest distances of the
                 // union of the splits' (best, second) pairs; a tie on the best
@@ -2511,44 +2530,76 @@ k_mutual(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pairs,
                 }
                 uint32_t nt = 0;
                 for (int q = 0; q < B.levels; ++q) nt += B.kept[q];
-                m = (nt >= 2u && bi >= 0 && (float)bd < P.bf_ratio * (float)sd) ? bi : -1;
-                P.a2b[(size_t)l * A.cap + i] = m;
+                m[u] = (nt >= 2u && bi >= 0 && (float)bd < P.bf_ratio * (float)sd) ? bi : -1;
+                a2b[i] = m[u];
             } else {
-                m = P.a2b[(size_t)l * A.cap + i];
+                m[u] = a2b[i];
             }
-            if (m >= 0) {
-                const int bl = USLAM_PACK_LEVEL(m), bi = USLAM_PACK_INDEX(m);
-                if (!MUTUAL) {
-                    ok = true;
-                } else if (P.bacc) {
-                    // b's search from its accumulator (k_match): the pool rule
-                    // over a's levels bl - 1 .. bl + 1, the ratio test, and
-                    // its nearest a is this a
-                    const uint4 e = P.bacc[(size_t)bl * B.cap + bi];
-                    uint32_t pool = A.kept[bl];
-                    if (bl > 0) pool += A.kept[bl - 1];
-                    if (bl + 1 < A.levels) pool += A.kept[bl + 1];
-                    ok = pool >= 2u && e.y != 0xffffffffu && (float)e.y < 0.85f * (float)e.z &&
-                         e.x == (uint32_t)USLAM_PACK(l, i);
+        }
+        uint32_t ok = 0u;  // bit u: item u is a match
+        if (!MUTUAL) {
+#pragma unroll
+            for (int u = 0; u < KU_ITEMS; ++u) ok |= (m[u] >= 0 ? 1u : 0u) << u;
+        } else if (P.bacc) {
+            // b's search from its accumulator (k_match): the pool rule over a's
+            // levels bl - 1 .. bl + 1, the ratio test, and its nearest a is this a
+            uint4 e[KU_ITEMS];
+#pragma unroll
+            for (int u = 0; u < KU_ITEMS; ++u)
+                if (m[u] >= 0) e[u] = P.bacc[(size_t)USLAM_PACK_LEVEL(m[u]) * B.cap + USLAM_PACK_INDEX(m[u])];
+#pragma unroll
+            for (int u = 0; u < KU_ITEMS; ++u) {
+                if (m[u] < 0) continue;
+                const int bl = USLAM_PACK_LEVEL(m[u]);
+                uint32_t pool = A.kept[bl];
+                if (bl > 0) pool += A.kept[bl - 1];
+                if (bl + 1 < A.levels) pool += A.kept[bl + 1];
+                const uint32_t i = c0 + u * KU_THREADS + threadIdx.x;
+                if (pool >= 2u && e[u].y != 0xffffffffu && (float)e[u].y < 0.85f * (float)e[u].z &&
+                    e[u].x == (uint32_t)USLAM_PACK(l, i))
+                    ok |= 1u << u;
+            }
+        } else {
+            int32_t back[KU_ITEMS];
+#pragma unroll
+            for (int u = 0; u < KU_ITEMS; ++u)
+                if (m[u] >= 0) back[u] = P.b2a[(size_t)USLAM_PACK_LEVEL(m[u]) * B.cap + USLAM_PACK_INDEX(m[u])];
+#pragma unroll
+            for (int u = 0; u < KU_ITEMS; ++u)
+                if (m[u] >= 0 && back[u] == USLAM_PACK(l, c0 + u * KU_THREADS + threadIdx.x)) ok |= 1u << u;
+        }
+        uint32_t before[KU_ITEMS];  // matches of earlier lanes of the warp in the same item row
+#pragma unroll
+        for (int u = 0; u < KU_ITEMS; ++u) {
+            const uint32_t bal = __ballot_sync(0xffffffffu, (ok >> u) & 1u);
+            before[u] = (uint32_t)__popc(bal & ((1u << lane) - 1u));
+            if (lane == 0) s_cnt[u][warp] = (uint32_t)__popc(bal);
+        }
+        __syncthreads();
+        if (warp < KU_ITEMS) {
+            const uint32_t v = s_cnt[warp][lane], incl = warp_inclusive_scan(v, lane);
+            s_cnt[warp][lane] = incl - v;
+            if (lane == 31) s_row[warp] = incl;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < KU_ITEMS; ++u) {
+            if ((ok >> u) & 1u) {
+                const uint32_t pos = base + s_cnt[u][warp] + before[u];
+                if (pos < (uint32_t)P.max_matches_per_level) {
+                    // (four stores: a caller's match buffer may be aligned to 4 bytes only)
+                    int32_t* o = P.matches + ((size_t)l * P.max_matches_per_level + pos) * 4;
+                    o[0] = l;
+                    o[1] = (int32_t)(c0 + u * KU_THREADS + threadIdx.x);
+                    o[2] = USLAM_PACK_LEVEL(m[u]);
+                    o[3] = USLAM_PACK_INDEX(m[u]);
                 } else {
-                    ok = P.b2a[(size_t)bl * B.cap + bi] == USLAM_PACK(l, i);
+                    atomicOr(err, USLAM_ERR_MATCH_OVERFLOW);
                 }
             }
+            base += s_row[u];
         }
-        uint32_t tot;
-        const uint32_t pos = base + block_exclusive_scan(ok ? 1u : 0u, s_warp, &tot);
-        if (ok) {
-            if (pos < (uint32_t)P.max_matches_per_level) {
-                int32_t* o = P.matches + ((size_t)l * P.max_matches_per_level + pos) * 4;
-                o[0] = l;
-                o[1] = (int32_t)i;
-                o[2] = USLAM_PACK_LEVEL(m);
-                o[3] = USLAM_PACK_INDEX(m);
-            } else {
-                atomicOr(err, USLAM_ERR_MATCH_OVERFLOW);
-            }
-        }
-        base += tot;
+        __syncthreads();  // s_cnt and s_row are rewritten
     }
     if (threadIdx.x == 0) P.match_count[l] = base;
 }
@@ -2636,7 +2687,7 @@ cudaError_t launch_compact_banded(const FrameDev* frames, const BandItem* bands,
 
 cudaError_t launch_xsort(const FrameDev* frames, const SegDev* segs, int nseg, int max_w, cudaStream_t st) {
     if (nseg <= 0) return cudaSuccess;
-    k_xsort<<<nseg, KC_THREADS, (size_t)(max_w + 1) * sizeof(uint32_t), st>>>(frames, segs);
+    k_xsort<<<dim3(nseg, 2 * USLAM_MATCH_BANDS), KC_THREADS, (size_t)(max_w + 1) * sizeof(uint32_t), st>>>(frames, segs);
     return cudaGetLastError();
 }
 

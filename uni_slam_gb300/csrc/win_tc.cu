@@ -600,6 +600,20 @@ k_win_mma(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pairs
                 const uint32_t buf = tk % WN_BUFS, use = tk / WN_BUFS;
                 bad = bad || *fail != 0 || !bar_wait(&acc_full[buf], use & 1u) || !bar_wait(&y_full[buf], use & 1u);
                 fence_after();
+                // this range's window of the row, and the list position of this
+                // warp's first column
+                const int c0k = pick3(k, u.c0[0], u.c0[1], u.c0[2]);
+                const int plk = pick3(k, u.pl[0], u.pl[1], u.pl[2]);
+                const int M0 = pick3(k, m0[0], m0[1], m0[2]), M1 = pick3(k, m1[0], m1[1], m1[2]);
+                const int cb = c0k + i * WN_N + 32 * cq;
+                // the tiles cover the windows of 128 queries, of which this warp
+                // holds a quarter, x-consecutive: a column group outside all of
+                // its windows is released unread
+                if (!__any_sync(0xffffffffu, bad || (M0 < cb + 32 && cb < M1))) {
+                    fence_before();
+                    if (lane == 0) bar_arrive(&acc_empty[buf]);
+                    continue;
+                }
                 // tcgen05.ld is warp-wide: a warp reads the accumulator only if
                 // every lane saw it complete
                 const bool go = __all_sync(0xffffffffu, !bad);
@@ -619,13 +633,7 @@ k_win_mma(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pairs
                     bad = true;
                     continue;
                 }
-                // this range's window of the row, and the list position of this
-                // warp's first column
-                const int c0k = pick3(k, u.c0[0], u.c0[1], u.c0[2]);
-                const int plk = pick3(k, u.pl[0], u.pl[1], u.pl[2]);
-                const int M0 = pick3(k, m0[0], m0[1], m0[2]), M1 = pick3(k, m1[0], m1[1], m1[2]);
                 const uint32_t YL = pick3(k, ylo2[0], ylo2[1], ylo2[2]), YH = pick3(k, yhi2[0], yhi2[1], yhi2[2]);
-                const int cb = c0k + i * WN_N + 32 * cq;
                 uint32_t cbk[4] = {0u, 0u, 0u, 0u}, csk[4] = {0u, 0u, 0u, 0u};
                 // every column of the group inside this row's x range?
                 const bool inside = M0 <= cb && cb + 32 <= M1;
