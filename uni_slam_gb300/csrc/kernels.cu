@@ -29,6 +29,7 @@
 // Arithmetic contract: binary32, round-to-nearest-even, no FMA contraction
 // (the library is compiled with --fmad=false), evaluation order as in the
 // reference shaders.  Every kernel is bit-exact against the CPU oracle.
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -50,10 +51,11 @@ constexpr uint32_t kTmaWaitLimit = 1u << 20;
 // cfg detection profile threshold: 20 grey levels on the u8/255 scale.
 constexpr float kCfgThreshold = 20.0f / 255.0f;
 
-// Matcher band of a LOD-0 y in a frame of height H (rows [b H / B, (b + 1) H / B)).
-__device__ __forceinline__ int match_band(float y, float H) {
-    const int b = (int)floorf(y * (float)USLAM_MATCH_BANDS / H);
-    return b < 0 ? 0 : (b >= USLAM_MATCH_BANDS ? USLAM_MATCH_BANDS - 1 : b);
+// Matcher band of a LOD-0 y in a frame of height H cut into n bands (rows
+// [b H / n, (b + 1) H / n)).
+__device__ __forceinline__ int match_band(float y, float H, int n) {
+    const int b = (int)floorf(y * (float)n / H);
+    return b < 0 ? 0 : (b >= n ? n - 1 : b);
 }
 
 // Bresenham circle of radius 3 (resources/detect_corners.wgsl:31-32) as
@@ -965,7 +967,7 @@ __device__ __forceinline__ float lod0_y(uint32_t y_bits, float scale) {
 }
 
 // The matcher's index of one level.  The frame height is cut into
-// USLAM_MATCH_BANDS bands (LOD-0 rows [b H0 / B, (b + 1) H0 / B)):
+// B = F.nbands bands (LOD-0 rows [b H0 / B, (b + 1) H0 / B)):
 //  * candidate list b = the features whose LOD-0 y lies in band b widened by
 //    0.1 H0 + 2 (the window half-height plus slack), sorted by x, with the
 //    first slot of each column; every feature inside the window of a query
@@ -980,13 +982,14 @@ __device__ __forceinline__ float lod0_y(uint32_t y_bits, float scale) {
 constexpr int XU = 4;
 __global__ void __launch_bounds__(KC_THREADS, 2)
 k_xsort(const FrameDev* __restrict__ frames, const SegDev* __restrict__ segs) {
-    constexpr int NB = USLAM_MATCH_BANDS;
     extern __shared__ uint32_t s_hist[];  // [w + 1]
     __shared__ uint32_t s_warp[33];
     const SegDev sg = segs[blockIdx.x];
     const FrameDev& F = frames[sg.frame];
+    const int NB = F.nbands;
+    if ((int)blockIdx.y >= 2 * NB) return;  // a batch with frames of more bands
     const int l = sg.level, w = F.w[l];
-    const bool query = blockIdx.y >= NB;
+    const bool query = (int)blockIdx.y >= NB;
     const int b = (int)blockIdx.y - (query ? NB : 0);
     const uint32_t kept = F.kept[l];
     const uint32_t* feats = F.feats[l];
@@ -999,7 +1002,7 @@ k_xsort(const FrameDev* __restrict__ frames, const SegDev* __restrict__ segs) {
     // -1: in an earlier band's list of the query order, 0: in this list, 1: in neither
     auto place = [&](float y) {
         if (!query) return y >= lo && y <= hi ? 0 : 1;
-        const int q = match_band(y, H);
+        const int q = match_band(y, H, NB);
         return q < b ? -1 : (q == b ? 0 : 1);
     };
     for (int i = threadIdx.x; i <= w; i += KC_THREADS) s_hist[i] = 0u;
@@ -1367,7 +1370,7 @@ k_band_write(const FrameDev* __restrict__ frames, const BandItem* __restrict__ i
 }
 
 // ------------------------------------------------------------- K2 ----
-constexpr int KD_THREADS = 256;
+constexpr int KD_THREADS = 1024;
 constexpr int MAX_SEGS = 4096;
 
 // Prefix over per-segment counts, shared by the persistent kernels.
@@ -1444,9 +1447,9 @@ __device__ __forceinline__ void write_ext_row(uint8_t* base, uint32_t R, uint32_
 }
 // Query-order position k of level l -> its operand row (each band's queries
 // from a multiple of 128 rows).
-__device__ __forceinline__ uint32_t win_query_row(const uint32_t* qband, int l, int wq_rows, uint32_t k) {
+__device__ __forceinline__ uint32_t win_query_row(const uint32_t* qband, int nb, int l, int wq_rows, uint32_t k) {
     uint32_t off = (uint32_t)l * (uint32_t)wq_rows, b = 0;
-    while (b + 1 < (uint32_t)USLAM_MATCH_BANDS && k >= qband[b + 1]) {
+    while (b + 1 < (uint32_t)nb && k >= qband[b + 1]) {
         off += (qband[b + 1] - qband[b] + 127u) / 128u * 128u;
         ++b;
     }
@@ -1458,7 +1461,7 @@ __device__ __forceinline__ uint32_t win_query_row(const uint32_t* qband, int l, 
 // (generate_features.wgsl:170-172), plus the tensor-core operand rows (PACK,
 // WIN) of the matchers that take them.
 template <bool PACK, bool WIN>
-__device__ __forceinline__ void emit_feature(const FrameDev& F, int l, uint32_t i, int w, int y, float theta,
+__device__ __forceinline__ void emit_feature(const FrameDev& F, int l, uint32_t i, int y, float theta,
                                              const uint32_t (&words)[8], int lane) {
     uint32_t* rec = F.feats[l] + (size_t)i * 12u;
     uint32_t out = __float_as_uint(theta);
@@ -1476,13 +1479,13 @@ __device__ __forceinline__ void emit_feature(const FrameDev& F, int l, uint32_t 
         }
         const uint32_t* inv = F.winv[l];
         const size_t cap = (size_t)(F.cap > 0 ? F.cap : 1);
-        const uint32_t* qband = F.colstart[l] + (size_t)USLAM_MATCH_BANDS * (size_t)(w + 1);
-        write_fp8_row(F.wq8, win_query_row(qband, l, F.wq_rows, __ldg(inv + i)), wj, lane);
-#pragma unroll
-        for (int b = 0; b < USLAM_MATCH_BANDS; ++b) {
+        const int nb = F.nbands;
+        const uint32_t* qband = F.colstart[l] + (size_t)nb * (size_t)(F.w[l] + 1);
+        write_fp8_row(F.wq8, win_query_row(qband, nb, l, F.wq_rows, __ldg(inv + i)), wj, lane);
+        for (int b = 0; b < nb; ++b) {
             const uint32_t pos = __ldg(inv + cap * (size_t)(1 + b) + i);
             if (pos == 0xffffffffu) continue;
-            const uint32_t R = (uint32_t)(USLAM_MATCH_BANDS * l + b) * (uint32_t)F.wc_rows + pos;
+            const uint32_t R = (uint32_t)(nb * l + b) * (uint32_t)F.wc_rows + pos;
             write_fp8_row(F.wc8, R, wj, lane);
             if (lane < 4) write_ext_row(F.wcext, R, pc, (int)(pos & 31u), lane);
             else if (lane == 4) F.wcy[R] = (uint16_t)y;
@@ -1543,54 +1546,70 @@ __device__ __forceinline__ void emit_feature(const FrameDev& F, int l, uint32_t 
 // tensor-core matcher's rows: the feature's query row (wq8) and its row in
 // every candidate list that holds it (wc8, wcext, wcy, wcid), at the
 // positions k_xsort recorded (winv).
+//
+// One CTA of 32 warps per SM over runs of consecutive keypoints, so that the
+// blur-cache strip its warps gather from stays in L1 (97 % sector hits against
+// 86 % with four CTAs of 8 warps over runs far apart: 32 frames of 752x480
+// 186 -> 155 us).  The gathers are then bound by the cache lines that a warp
+// load touches: in test order 22 of 32 lanes' points lie in lines of their
+// own, in compact clusters of the pattern under 9 (DescTable), and the values
+// reach their tests through shared memory (155 -> 145 us; 3840x2160 frames of
+// the mixed batch 700 -> 553 in all).  The L1 data pipe bounds it now, three
+// quarters busy.
+constexpr size_t kDescSmem = 512 * sizeof(__half2) + KD_THREADS / 32 * 512 * sizeof(float);
+
 template <bool PACK, bool WIN>
 __global__ void __launch_bounds__(KD_THREADS)
 k_describe(const FrameDev* __restrict__ frames, const SegDev* __restrict__ segs, int nseg,
-           const int32_t* __restrict__ pattern) {
-    // the test pattern as f32 (each coordinate converted once per CTA, exactly)
-    __shared__ float4 s_pat[256];
+           const DescTable* __restrict__ table) {
+    extern __shared__ __align__(16) uint8_t kd_smem[];  // the table's points, then each warp's gathered values
     __shared__ uint32_t s_pref[MAX_SEGS + 1];
     __shared__ uint32_t s_warp[33];
-    __shared__ float s_lut[256];
     // the r = 3 disc in (dy outer, dx inner) order as compile-time constants, so
     // the unrolled moment sum multiplies by immediates (same f32 operations)
     constexpr int8_t kdx[29] = {0, -2, -1, 0, 1, 2, -2, -1, 0, 1, 2, -3, -2, -1, 0, 1, 2, 3, -2, -1, 0, 1, 2, -2, -1, 0, 1, 2, 0};
     constexpr int8_t kdy[29] = {-3, -2, -2, -2, -2, -2, -1, -1, -1, -1, -1, 0, 0, 0, 0, 0, 0, 0, 1, 1, 1, 1, 1, 2, 2, 2, 2, 2, 3};
-    for (int i = threadIdx.x; i < 256; i += KD_THREADS) {
-        s_pat[i] = make_float4((float)pattern[4 * i], (float)pattern[4 * i + 1], (float)pattern[4 * i + 2],
-                               (float)pattern[4 * i + 3]);
-        s_lut[i] = (float)i / 255.0f;
-    }
+    constexpr uint32_t WARPS = KD_THREADS / 32;
+    const int lane = threadIdx.x & 31;
+    const uint32_t warp = threadIdx.x >> 5;
+    // (a point's coordinates are integers below 1024, exact in 16 bits: half the shared-memory reads)
+    __half2* const s_pts = reinterpret_cast<__half2*>(kd_smem);
+    float* const vals = reinterpret_cast<float*>(kd_smem + 512 * sizeof(__half2)) + warp * 512u;
+    for (int i = threadIdx.x; i < 512; i += KD_THREADS)
+        s_pts[i] = __floats2half2_rn(table->pts[i >> 5][i & 31][0], table->pts[i >> 5][i & 31][1]);
+    uint32_t pair[8];  // this lane's tests
+#pragma unroll
+    for (int k = 0; k < 8; ++k) pair[k] = table->pair[k][lane];
     const uint32_t total = segment_prefix(nseg, s_pref, s_warp, [&](int s) {
         return frames[segs[s].frame].kept[segs[s].level];
     });
-    const int lane = threadIdx.x & 31;
-    const int gw = blockIdx.x * (KD_THREADS / 32) + (threadIdx.x >> 5);
-    const int nw = gridDim.x * (KD_THREADS / 32);
-    // A warp takes G consecutive keypoints: lane j < G first computes the
-    // orientation of keypoint j, then the warp runs the 256 tests of each in
-    // turn with its position and angle broadcast from that lane.  Warps take
-    // every nw-th group; k = the groups per warp at 32 keypoints each, and G
-    // (<= 32) the group size that spreads the keypoints evenly over k groups
-    // per warp, so that no warp runs a group more than the others.
-    const uint32_t per_round = 32u * (uint32_t)nw;
-    const uint32_t kq = (total + per_round - 1u) / per_round;
-    const uint32_t G = kq ? (total + kq * (uint32_t)nw - 1u) / (kq * (uint32_t)nw) : 1u;
-    for (uint32_t g0 = (uint32_t)gw * G; g0 < total; g0 += (uint32_t)nw * G) {
+    // A CTA takes an equal share of consecutive keypoints in runs of WARPS * G
+    // (G <= 32), of which warp q takes every WARPS-th from the q-th on: lane
+    // j < G first computes the orientation of the warp's keypoint j, then the
+    // warp runs the 256 tests of each in turn with its position and angle
+    // broadcast from that lane.
+    const uint32_t share = (total + gridDim.x - 1u) / gridDim.x;
+    const uint32_t end = min(total, (blockIdx.x + 1u) * share);
+    const uint32_t kq = max((share + 32u * WARPS - 1u) / (32u * WARPS), 1u);
+    const uint32_t G = (share + kq * WARPS - 1u) / (kq * WARPS);
+    for (uint32_t c0 = blockIdx.x * share; c0 < end; c0 += WARPS * G) {
+        const uint32_t g0 = c0 + warp;
+        if (g0 >= end) break;
         // orientation (generate_features.wgsl:80-99): intensity moments over
         // the r = 3 disc, summed in the reference's order, then atan2
         int my_seg = 0;
-        uint32_t my_idx = 0;
+        uint32_t my_idx = 0, my_xy = 0;
         float my_theta = 0.0f, my_s = 0.0f, my_c = 0.0f;
-        if ((uint32_t)lane < G && g0 + lane < total) {
-            my_seg = find_segment(s_pref, nseg, g0 + lane);
-            my_idx = g0 + lane - s_pref[my_seg];
+        if ((uint32_t)lane < G && g0 + lane * WARPS < end) {
+            my_seg = find_segment(s_pref, nseg, g0 + lane * WARPS);
+            my_idx = g0 + lane * WARPS - s_pref[my_seg];
             const FrameDev& F = frames[segs[my_seg].frame];
             const int l = segs[my_seg].level;
             const int w = F.w[l], h = F.h[l];
             const uint32_t* rec = F.feats[l] + (size_t)my_idx * 12u;
             const int x = (int)__uint_as_float(rec[0]);
             const int y = (int)__uint_as_float(rec[1]);
+            my_xy = (uint32_t)y << 16 | (uint32_t)x;
             const float* lvl = F.lvl[l];
             const int lp = F.lvl_pitch[l];
             float m10 = 0.0f, m01 = 0.0f;
@@ -1598,53 +1617,77 @@ k_describe(const FrameDev* __restrict__ frames, const SegDev* __restrict__ segs,
             for (int k = 0; k < 29; ++k) {
                 const int cx = tint_clamp(x + kdx[k], w);
                 const int cy = tint_clamp(y + kdy[k], h);
-                const float v = l == 0 ? s_lut[__ldg(F.img + (size_t)cy * F.img_pitch + cx)]
-                                       : __ldg(lvl + (size_t)cy * (size_t)lp + cx);
+                const float v = __ldg(lvl + (size_t)cy * (size_t)lp + cx);
                 m10 = m10 + (float)kdx[k] * v;
                 m01 = m01 + (float)kdy[k] * v;
             }
             my_theta = uslam_atan2f(m01, m10);
             uslam_sincosf(my_theta, &my_s, &my_c);
         }
-        const int nk = (int)min(G, total - g0);
+        int seg = -1, l = 0, reach = 0;
+        const FrameDev* F = frames;
+        const float* blur = nullptr;
+        uint32_t bp = 0;
+        const int nk = (int)min(G, (end - g0 + WARPS - 1u) / WARPS);
         for (int kp = 0; kp < nk; ++kp) {
             const int sidx = __shfl_sync(0xffffffffu, my_seg, kp);
             const uint32_t i = __shfl_sync(0xffffffffu, my_idx, kp);
             const float theta = __shfl_sync(0xffffffffu, my_theta, kp);
             const float s = __shfl_sync(0xffffffffu, my_s, kp);
             const float c = __shfl_sync(0xffffffffu, my_c, kp);
-            const FrameDev& F = frames[segs[sidx].frame];
-            const int l = segs[sidx].level;
-            const int w = F.w[l], h = F.h[l];
-            uint32_t* rec = F.feats[l] + (size_t)i * 12u;
-            const int x = (int)__uint_as_float(rec[0]);
-            const int y = (int)__uint_as_float(rec[1]);
-
-            // 256 tests, lane j owns tests j, j + 32, ..., j + 224: 16 independent
-            // gathers from the blur cache (negative coordinates -> sentinel).
-            const float* blur = F.blur[l];
-            const int bp = F.bl_pitch[l];
-            const int sx = w + F.margin, sy = h + F.margin;
-            float ga[8], gb[8];
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const float4 t = s_pat[lane + 32 * k];
-                const float fax = t.x, fay = t.y, fbx = t.z, fby = t.w;
-                int xa = x + (int)rintf(fax * c - fay * s);
-                int ya = y + (int)rintf(fax * s + fay * c);
-                int xb = x + (int)rintf(fbx * c - fby * s);
-                int yb = y + (int)rintf(fbx * s + fby * c);
-                xa = xa < 0 ? sx : xa;
-                ya = ya < 0 ? sy : ya;
-                xb = xb < 0 ? sx : xb;
-                yb = yb < 0 ? sy : yb;
-                ga[k] = __ldg(blur + (size_t)ya * bp + xa);
-                gb[k] = __ldg(blur + (size_t)yb * bp + xb);
+            const uint32_t xy = __shfl_sync(0xffffffffu, my_xy, kp);
+            const int x = (int)(xy & 0xffffu), y = (int)(xy >> 16);
+            if (sidx != seg) {
+                // the level's addresses are kept from keypoint to keypoint
+                seg = sidx;
+                F = frames + segs[sidx].frame;
+                l = segs[sidx].level;
+                blur = F->blur[l];
+                bp = (uint32_t)F->bl_pitch[l];
+                reach = F->margin - 1;
             }
+            // The 512 points' samples.  Adding 1.5 2^23 rounds a rotated
+            // coordinate to the nearest integer, ties to even, into the low
+            // bits of the sum (|coordinate| < 2^22), so the cache index is two
+            // integer operations on the sums' bits, modulo 2^32, where the
+            // constants cancel.  Keypoints within the pattern's reach of the
+            // left or top edge (the same for the whole warp) also replace
+            // negative coordinates by the sentinel column / row.
+            constexpr float kRound = 12582912.0f;
+            constexpr uint32_t kRoundBits = 0x4B400000u;
+            const uint32_t cx = (uint32_t)x - kRoundBits, cy = (uint32_t)y - kRoundBits;
+            // at(rounded x bits, rounded y bits): the sample
+            auto gather = [&](auto at) {
+#pragma unroll
+                for (int q0 = 0; q0 < USLAM_DESC_CLUSTERS; q0 += 8) {
+                    float v[8];
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                        const float2 p = __half22float2(s_pts[(q0 + q) * 32 + lane]);
+                        v[q] = at(__float_as_uint((p.x * c - p.y * s) + kRound), __float_as_uint((p.x * s + p.y * c) + kRound));
+                    }
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) vals[(q0 + q) * 32 + lane] = v[q];
+                }
+            };
+            if (x >= reach && y >= reach) {
+                const uint32_t origin = cy * bp + cx;
+                gather([&](uint32_t xr, uint32_t yr) { return __ldg(blur + (yr * bp + (xr + origin))); });
+            } else {
+                const int sx = F->w[l] + F->margin, sy = F->h[l] + F->margin;
+                gather([&](uint32_t xr, uint32_t yr) {
+                    const int px = (int)(xr + cx), py = (int)(yr + cy);
+                    return __ldg(blur + (size_t)(py < 0 ? sy : py) * bp + (px < 0 ? sx : px));
+                });
+            }
+            __syncwarp();
+            // lane j runs tests j, j + 32, ..., j + 224
             uint32_t words[8];
 #pragma unroll
-            for (int k = 0; k < 8; ++k) words[k] = __ballot_sync(0xffffffffu, ga[k] > gb[k]);
-            emit_feature<PACK, WIN>(F, l, i, w, y, theta, words, lane);
+            for (int k = 0; k < 8; ++k)
+                words[k] = __ballot_sync(0xffffffffu, vals[pair[k] & 0xffffu] > vals[pair[k] >> 16]);
+            emit_feature<PACK, WIN>(*F, l, i, y, theta, words, lane);
+            __syncwarp();  // the values are rewritten for the next keypoint
         }
     }
 }
@@ -1822,7 +1865,7 @@ k_describe_tiled(const FrameDev* __restrict__ frames, const BandItem* __restrict
             uint32_t words[8];
 #pragma unroll
             for (int k = 0; k < 8; ++k) words[k] = __ballot_sync(0xffffffffu, ga[k] > gb[k]);
-            emit_feature<PACK, WIN>(F, l, i2, w, y, theta, words, lane);
+            emit_feature<PACK, WIN>(F, l, i2, y, theta, words, lane);
         }
         __syncthreads();  // s_list / s_wcount reused by the next pass
     }
@@ -1965,16 +2008,17 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 __device__ __forceinline__ uint32_t match_groups(const FrameDev* frames, const PairDev* pairs, const MatchSegDev& sg) {
     const FrameDev& Qf = frames[pairs[sg.pair].prev];
     const int ql = sg.level;
-    const uint32_t* qb = Qf.colstart[ql] + (size_t)USLAM_MATCH_BANDS * (size_t)(Qf.w[ql] + 1);
+    const int nb = Qf.nbands;
+    const uint32_t* qb = Qf.colstart[ql] + (size_t)nb * (size_t)(Qf.w[ql] + 1);
     uint32_t n = 0;
-    for (int b = 0; b < USLAM_MATCH_BANDS; ++b) n += (qb[b + 1] - qb[b] + 31u) / 32u;
+    for (int b = 0; b < nb; ++b) n += (qb[b + 1] - qb[b] + 31u) / 32u;
     return n;
 }
 
 // Band of group grp of a segment (grp becomes the group within the band).
-__device__ __forceinline__ int match_group_band(const uint32_t* qband, uint32_t* grp) {
+__device__ __forceinline__ int match_group_band(const uint32_t* qband, int nb, uint32_t* grp) {
     int band = 0;
-    while (band + 1 < USLAM_MATCH_BANDS && *grp >= (qband[band + 1] - qband[band] + 31u) / 32u) {
+    while (band + 1 < nb && *grp >= (qband[band + 1] - qband[band] + 31u) / 32u) {
         *grp -= (qband[band + 1] - qband[band] + 31u) / 32u;
         ++band;
     }
@@ -1998,8 +2042,8 @@ __device__ uint32_t match_group_cost(const FrameDev* frames, const PairDev* pair
     const FrameDev& Q = frames[P.prev];
     const FrameDev& B = frames[P.curr];
     const int l = sg.level;
-    const uint32_t* qband = Q.colstart[l] + (size_t)USLAM_MATCH_BANDS * (size_t)(Q.w[l] + 1);
-    const int band = match_group_band(qband, &grp);
+    const uint32_t* qband = Q.colstart[l] + (size_t)Q.nbands * (size_t)(Q.w[l] + 1);
+    const int band = match_group_band(qband, Q.nbands, &grp);
     const uint32_t k0 = qband[band] + grp * 32u, k1 = min(k0 + 31u, qband[band + 1] - 1u);
     const float ql = lod_scale(l);
     const float x0 = (float)(uint32_t)__uint_as_float(Q.feats[l][(size_t)__ldg(Q.qorder[l] + k0) * 12u]) * ql;
@@ -2126,8 +2170,8 @@ k_match(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pairs,
         const FrameDev& Q = frames[P.prev];
         const FrameDev& B = frames[P.curr];
         const int l = sg.level;
-        const uint32_t* qband = Q.colstart[l] + (size_t)USLAM_MATCH_BANDS * (size_t)(Q.w[l] + 1);
-        const int band = match_group_band(qband, &grp);
+        const uint32_t* qband = Q.colstart[l] + (size_t)Q.nbands * (size_t)(Q.w[l] + 1);
+        const int band = match_group_band(qband, Q.nbands, &grp);
         const uint32_t qk = qband[band] + grp * 32u + (uint32_t)lane;
         const bool valid = qk < qband[band + 1];
         const uint32_t qi = valid ? __ldg(Q.qorder[l] + qk) : 0u;
@@ -2685,9 +2729,10 @@ cudaError_t launch_compact_banded(const FrameDev* frames, const BandItem* bands,
     return cudaGetLastError();
 }
 
-cudaError_t launch_xsort(const FrameDev* frames, const SegDev* segs, int nseg, int max_w, cudaStream_t st) {
+// max_bands: the largest FrameDev::nbands of the segments' frames.
+cudaError_t launch_xsort(const FrameDev* frames, const SegDev* segs, int nseg, int max_w, int max_bands, cudaStream_t st) {
     if (nseg <= 0) return cudaSuccess;
-    k_xsort<<<dim3(nseg, 2 * USLAM_MATCH_BANDS), KC_THREADS, (size_t)(max_w + 1) * sizeof(uint32_t), st>>>(frames, segs);
+    k_xsort<<<dim3(nseg, 2 * max_bands), KC_THREADS, (size_t)(max_w + 1) * sizeof(uint32_t), st>>>(frames, segs);
     return cudaGetLastError();
 }
 
@@ -2699,13 +2744,21 @@ cudaError_t launch_blur(const FrameDev* frames, BlurList bl, int max_tiles, int 
     return cudaGetLastError();
 }
 
-cudaError_t launch_describe(const FrameDev* frames, const SegDev* segs, int nseg, const int32_t* pattern,
-                            int grid, bool pack, bool win, cudaStream_t st) {
+cudaError_t launch_describe(const FrameDev* frames, const SegDev* segs, int nseg, const DescTable* table,
+                            int num_sms, bool pack, bool win, cudaStream_t st) {
     if (nseg <= 0) return cudaSuccess;
-    if (pack) k_describe<true, false><<<grid, KD_THREADS, 0, st>>>(frames, segs, nseg, pattern);
-    else if (win) k_describe<false, true><<<grid, KD_THREADS, 0, st>>>(frames, segs, nseg, pattern);
-    else k_describe<false, false><<<grid, KD_THREADS, 0, st>>>(frames, segs, nseg, pattern);
+    if (pack) k_describe<true, false><<<num_sms, KD_THREADS, kDescSmem, st>>>(frames, segs, nseg, table);
+    else if (win) k_describe<false, true><<<num_sms, KD_THREADS, kDescSmem, st>>>(frames, segs, nseg, table);
+    else k_describe<false, false><<<num_sms, KD_THREADS, kDescSmem, st>>>(frames, segs, nseg, table);
     return cudaGetLastError();
+}
+cudaError_t set_describe_smem() {
+    cudaError_t e = cudaFuncSetAttribute(k_describe<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDescSmem);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_describe<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDescSmem);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_describe<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDescSmem);
+    return e;
 }
 
 cudaError_t launch_describe_tiled(const FrameDev* frames, const BandItem* items, int nitems, const int32_t* pattern,

@@ -29,7 +29,7 @@ struct MatchSegDev {
 cudaError_t launch_match(const FrameDev*, const PairDev*, const void*, int, int, cudaStream_t);
 cudaError_t launch_mutual(const FrameDev*, const PairDev*, const SegDev*, int, uint32_t*, cudaStream_t);
 cudaError_t launch_bacc_init(const FrameDev*, const PairDev*, const SegDev*, int, cudaStream_t);
-cudaError_t launch_xsort(const FrameDev*, const SegDev*, int, int, cudaStream_t);
+cudaError_t launch_xsort(const FrameDev*, const SegDev*, int, int, int, cudaStream_t);
 cudaError_t set_compact_smem(int max_w);
 }  // namespace uslam
 
@@ -39,6 +39,7 @@ namespace {
 
 constexpr size_t kNoallocScratchBytes = size_t(4) << 20;  // 4 MiB per device
 constexpr int kMaxDevices = 64;
+constexpr int kBands = 3;  // of the lists (more take more of the fixed scratch)
 
 // The no-alloc matcher's scratch.  Host code must not use this name as an
 // address: it is a host-side stand-in.  The device address comes from
@@ -205,18 +206,18 @@ extern "C" uslam_status uslam_match_noalloc(int device, int width, int height, i
 
     // scratch layout: [tables][xorder, qorder f0][xorder, qorder f1][colstart f0][colstart f1][a2b][b -> a
     // accumulators][error]
-    // (per level: USLAM_MATCH_BANDS candidate lists of cap entries, the query order, and per band
+    // (per level: kBands candidate lists of cap entries, the query order, and per band
     // the column table, then the band offsets)
     size_t cur = align256(sizeof(NoallocTables));
     size_t xorder_off[2], qorder_off[2], colstart_off[2];
     for (int f = 0; f < 2; ++f) {
         xorder_off[f] = cur;
-        cur = align256(cur + sizeof(uint32_t) * USLAM_MATCH_BANDS * static_cast<size_t>(levels) * cap[f]);
+        cur = align256(cur + sizeof(uint32_t) * kBands * static_cast<size_t>(levels) * cap[f]);
         qorder_off[f] = cur;
         cur = align256(cur + sizeof(uint32_t) * static_cast<size_t>(levels) * cap[f]);
     }
     size_t colsum = 0;
-    for (int l = 0; l < levels; ++l) colsum += USLAM_MATCH_BANDS * (static_cast<size_t>(wl[l]) + 1) + USLAM_MATCH_BANDS + 1;
+    for (int l = 0; l < levels; ++l) colsum += kBands * (static_cast<size_t>(wl[l]) + 1) + kBands + 1;
     for (int f = 0; f < 2; ++f) {
         colstart_off[f] = cur;
         cur = align256(cur + sizeof(uint32_t) * colsum);
@@ -249,6 +250,7 @@ extern "C" uslam_status uslam_match_noalloc(int device, int width, int height, i
         F.W0 = width;
         F.H0 = height;
         F.levels = levels;
+        F.nbands = kBands;
         F.cap = cap[f];
         F.kept = reinterpret_cast<uint32_t*>(base + offsetof(NoallocTables, counts)) + f * 2 * USLAM_MAX_LEVELS;
         F.raw = F.kept + levels;
@@ -258,13 +260,13 @@ extern "C" uslam_status uslam_match_noalloc(int device, int width, int height, i
             F.h[l] = hl[l];
             F.feats[l] = reinterpret_cast<uint32_t*>(const_cast<uslam_feature*>(feats[f]) + foff);
             F.xorder[l] = reinterpret_cast<uint32_t*>(base + xorder_off[f]) +
-                          static_cast<size_t>(l) * USLAM_MATCH_BANDS * cap[f];
+                          static_cast<size_t>(l) * kBands * cap[f];
             F.qorder[l] = reinterpret_cast<uint32_t*>(base + qorder_off[f]) + static_cast<size_t>(l) * cap[f];
             F.colstart[l] = reinterpret_cast<uint32_t*>(base + colstart_off[f]) + coff;
             t.counts[f][l] = static_cast<uint32_t>(kept[f][l]);
             t.counts[f][levels + l] = static_cast<uint32_t>(kept[f][l]);
             foff += static_cast<size_t>(kept[f][l]);
-            coff += USLAM_MATCH_BANDS * (static_cast<size_t>(wl[l]) + 1) + USLAM_MATCH_BANDS + 1;
+            coff += kBands * (static_cast<size_t>(wl[l]) + 1) + kBands + 1;
             t.xsegs[f * levels + l] = SegDev{f, l};
         }
     }
@@ -301,7 +303,7 @@ extern "C" uslam_status uslam_match_noalloc(int device, int width, int height, i
     }
     if (e == cudaSuccess) {
         e = set_compact_smem(max_w);  // a function attribute, not an allocation
-        if (e == cudaSuccess) e = launch_xsort(dtab->frames, dtab->xsegs, 2 * levels, max_w, st);
+        if (e == cudaSuccess) e = launch_xsort(dtab->frames, dtab->xsegs, 2 * levels, max_w, kBands, st);
     }
     if (e == cudaSuccess) e = launch_bacc_init(dtab->frames, &dtab->pair, dtab->usegs, levels, st);
     if (e == cudaSuccess) e = launch_match(dtab->frames, &dtab->pair, dtab->msegs, levels, ds.num_sms, st);

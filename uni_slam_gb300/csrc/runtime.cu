@@ -20,6 +20,7 @@
 #include <chrono>
 #include <cmath>
 #include <cstring>
+#include <functional>
 #include <map>
 #include <mutex>
 #include <string>
@@ -65,7 +66,7 @@ struct Program {
 struct uslam_batch {
     uslam_ctx* ctx = nullptr;
     int levels = 0;
-    int max_w = 0;
+    int max_w = 0, max_bands = 1;
     std::vector<FrameDev> frames;
     std::vector<PairDev> pairs;
     std::vector<size_t> in_off;    // per frame, offset of the input in the inputs region
@@ -239,7 +240,7 @@ cudaError_t describe_stage(uslam_batch* b, const Program& P, cudaStream_t st) {
     if (tiled_describe(c, static_cast<int>(b->frames.size())))
         return launch_describe_tiled(b->d_frames, P.desc, P.ndesc, c->d_pattern, c->matcher == 2, b->win_tc, c->margin,
                                      b->d_err, st);
-    return launch_describe(b->d_frames, P.fsegs, P.nfsegs, c->d_pattern, c->num_sms * 4, c->matcher == 2, b->win_tc, st);
+    return launch_describe(b->d_frames, P.fsegs, P.nfsegs, c->d_desc, c->num_sms, c->matcher == 2, b->win_tc, st);
 }
 
 // The frame stages of a program: pyramid, detect, compaction, blur, describe.
@@ -257,7 +258,7 @@ cudaError_t enqueue_frames(uslam_batch* b, const Program& P, const Lane& ln) {
     // side, and k_describe needs both (in a captured graph a fork/join).
     if ((e = cudaEventRecord(ln.fork, ln.st)) != cudaSuccess) return e;
     if ((e = cudaStreamWaitEvent(ln.aux, ln.fork, 0)) != cudaSuccess) return e;
-    if ((e = launch_xsort(b->d_frames, P.fsegs, P.nfsegs, b->max_w, ln.aux)) != cudaSuccess) return e;
+    if ((e = launch_xsort(b->d_frames, P.fsegs, P.nfsegs, b->max_w, b->max_bands, ln.aux)) != cudaSuccess) return e;
     if ((e = cudaEventRecord(ln.join, ln.aux)) != cudaSuccess) return e;
     if ((e = launch_blur(b->d_frames, P.blur, P.nblur, c->num_sms, b->d_err, ln.st)) != cudaSuccess) return e;
     if ((e = cudaStreamWaitEvent(ln.st, ln.join, 0)) != cudaSuccess) return e;
@@ -411,7 +412,6 @@ uslam_status create_batch(uslam_ctx* ctx, int n_frames, const int* widths, const
         max_cap = static_cast<int>(std::max<long long>(max_cap, c));
     }
     b->win_tc = (ctx->win_tc || (ctx->matcher == 0 && per_frame_form)) && max_cap <= kWinMaxCap && ctx->max_h < 65535;
-    b->win_umax = b->win_tc ? win_units_per_seg(max_cap) : 0;
     std::vector<FrameLayout> fl(n_frames);
     for (int f = 0; f < n_frames; ++f) {
         const int W0 = widths[f], H0 = heights[f];
@@ -444,6 +444,9 @@ uslam_status create_batch(uslam_ctx* ctx, int n_frames, const int* widths, const
         const long long cap_ll = ctx->cap_override > 0 ? ctx->cap_override
                                                        : static_cast<long long>(W0) * H0 / 250;
         F.cap = static_cast<int>(cap_ll);
+        F.nbands = match_bands_for(F.cap, b->win_tc);
+        b->max_bands = std::max(b->max_bands, F.nbands);
+        if (b->win_tc) b->win_umax = std::max(b->win_umax, win_units_per_seg(F.cap, F.nbands));
         const size_t capa = static_cast<size_t>(F.cap > 0 ? F.cap : 1);
         b->in_off[f] = take(&in_bytes, static_cast<size_t>(H0) * F.img_pitch);
         b->feat_off[f] = take(&out_bytes, 2 * sizeof(uint32_t) * L);
@@ -457,8 +460,8 @@ uslam_status create_batch(uslam_ctx* ctx, int n_frames, const int* widths, const
             F.bl_pitch[l] = lvl_pitch_of(F.w[l] + ctx->margin + 1);  // 16-byte rows (TMA)
             Ly.blur[l] = take(&scratch, static_cast<size_t>(F.h[l] + ctx->margin + 1) * F.bl_pitch[l] * 4);
             Ly.kpmap[l] = take(&scratch, static_cast<size_t>(F.h[l]) * F.kp_pitch[l]);
-            Ly.xorder[l] = take(&scratch, USLAM_MATCH_BANDS * capa * 4);
-            Ly.colstart[l] = take(&scratch, (USLAM_MATCH_BANDS * (static_cast<size_t>(F.w[l]) + 1) + USLAM_MATCH_BANDS + 1) * 4);
+            Ly.xorder[l] = take(&scratch, F.nbands * capa * 4);
+            Ly.colstart[l] = take(&scratch, (F.nbands * (static_cast<size_t>(F.w[l]) + 1) + F.nbands + 1) * 4);
             Ly.qorder[l] = take(&scratch, capa * 4);
             Ly.bands[l] = take(&scratch, static_cast<size_t>((F.h[l] + 31) / 32) * 8);
             Ly.btile[l] = take(&scratch, sizeof(uint32_t) * USLAM_BLUR_TILES(F.w[l], F.h[l], F.margin));
@@ -474,16 +477,16 @@ uslam_status create_batch(uslam_ctx* ctx, int n_frames, const int* widths, const
         if (b->win_tc) {
             // queries: each band from a multiple of 128 rows; lists: room for a
             // last 128-row tile that starts below the list's end
-            F.wq_rows = static_cast<int>(round_up(capa, 128) + USLAM_MATCH_BANDS * 128);
+            F.wq_rows = static_cast<int>(round_up(capa, 128) + F.nbands * 128);
             F.wc_rows = static_cast<int>(round_up(capa, 32) + 128);
             const size_t qrows = static_cast<size_t>(L) * F.wq_rows;
-            const size_t crows = static_cast<size_t>(L) * USLAM_MATCH_BANDS * F.wc_rows;
+            const size_t crows = static_cast<size_t>(L) * F.nbands * F.wc_rows;
             Ly.wq8 = take(&scratch, qrows * 256);
             Ly.wc8 = take(&scratch, crows * 256);
             Ly.wcext = take(&scratch, crows * 32);
             Ly.wcy = take(&scratch, crows * 2);
             Ly.wcid = take(&scratch, crows * 4);
-            for (int l = 0; l < L; ++l) Ly.winv[l] = take(&scratch, (1 + USLAM_MATCH_BANDS) * capa * 4);
+            for (int l = 0; l < L; ++l) Ly.winv[l] = take(&scratch, (1 + F.nbands) * capa * 4);
         }
         b->max_w = std::max(b->max_w, F.w[0]);
     }
@@ -743,7 +746,7 @@ uslam_status create_batch(uslam_ctx* ctx, int n_frames, const int* widths, const
         size_t max_groups = 0;
         for (int p = 0; p < n_pairs; ++p)
             max_groups += static_cast<size_t>(L) *
-                          (static_cast<size_t>(std::max(b->frames[pair_prev[p]].cap, 1)) / 32 + USLAM_MATCH_BANDS + 1);
+                          (static_cast<size_t>(std::max(b->frames[pair_prev[p]].cap, 1)) / 32 + b->max_bands + 1);
         b->claim_words = match_claim_words(max_groups);
         b->claim_stride = round_up(b->claim_words * sizeof(uint32_t), 256) + round_up(std::max<size_t>(max_groups, 1), 256);
         e = cudaMalloc(&b->d_claim, b->claim_stride * kLanes);
@@ -796,6 +799,60 @@ uslam_status create_batch(uslam_ctx* ctx, int n_frames, const int* widths, const
     }
     *out = b;
     return USLAM_OK;
+}
+
+// Clusters: the points halved along the wider axis of their extent, four
+// times.  Lanes: the points are the edges between their clusters and their
+// (k, point) groups of tests, every node of degree 32, so the graph splits
+// into 32 perfect matchings (Koenig), each found by augmenting paths and given
+// a lane.
+void build_desc_table(const int32_t* pattern, DescTable* out) {
+    constexpr int N = USLAM_DESC_CLUSTERS, P = 512;
+    int px[P], py[P], order[P], cluster[P];
+    for (int i = 0; i < P; ++i) {
+        px[i] = pattern[2 * i];
+        py[i] = pattern[2 * i + 1];
+        order[i] = i;
+    }
+    for (int size = P; size > P / N; size /= 2)
+        for (int* a = order; a < order + P; a += size) {
+            const auto by_x = [&](int i, int j) { return px[i] != px[j] ? px[i] < px[j] : i < j; };
+            const auto by_y = [&](int i, int j) { return py[i] != py[j] ? py[i] < py[j] : i < j; };
+            const auto mx = std::minmax_element(a, a + size, by_x), my = std::minmax_element(a, a + size, by_y);
+            if (px[*mx.second] - px[*mx.first] >= py[*my.second] - py[*my.first]) std::sort(a, a + size, by_x);
+            else std::sort(a, a + size, by_y);
+        }
+    std::vector<int> edges[N][N];  // [cluster][group]: points left
+    for (int i = 0; i < P; ++i) cluster[order[i]] = i / (P / N);
+    for (int i = 0; i < P; ++i) edges[cluster[i]][i / 64 * 2 + (i & 1)].push_back(i);  // point i: test i / 2
+    for (int lane = 0; lane < P / N; ++lane) {
+        int of_group[N];
+        std::fill(of_group, of_group + N, -1);
+        for (int c = 0; c < N; ++c) {
+            bool seen[N] = {false};
+            std::function<bool(int)> augment = [&](int u) {
+                for (int g = 0; g < N; ++g) {
+                    if (seen[g] || edges[u][g].empty()) continue;
+                    seen[g] = true;
+                    if (of_group[g] < 0 || augment(of_group[g])) {
+                        of_group[g] = u;
+                        return true;
+                    }
+                }
+                return false;
+            };
+            augment(c);
+        }
+        for (int g = 0; g < N; ++g) {
+            const int c = of_group[g], i = edges[c][g].back();
+            edges[c][g].pop_back();
+            out->pts[c][lane][0] = static_cast<float>(px[i]);
+            out->pts[c][lane][1] = static_cast<float>(py[i]);
+            const int test = i / 2, shift = (i & 1) * 16;
+            uint32_t& w = out->pair[test / 32][test % 32];
+            w = (w & ~(0xffffu << shift)) | (static_cast<uint32_t>(c * 32 + lane) << shift);
+        }
+    }
 }
 
 uslam_status check_err_word(uslam_batch* b) {
@@ -949,9 +1006,17 @@ uslam_status uslam_create(const uslam_params* params, uslam_ctx** out) {
     if (e == cudaSuccess) e = cudaMalloc(&c->d_pattern, 1024 * sizeof(int32_t));
     if (e == cudaSuccess)
         e = cudaMemcpy(c->d_pattern, params->brief_pattern, 1024 * sizeof(int32_t), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMalloc(&c->d_desc, sizeof(DescTable));
+    if (e == cudaSuccess) {
+        DescTable table;
+        build_desc_table(params->brief_pattern, &table);
+        e = cudaMemcpy(c->d_desc, &table, sizeof(table), cudaMemcpyHostToDevice);
+    }
+    if (e == cudaSuccess) e = set_describe_smem();
     if (e != cudaSuccess) {
         cudaGetLastError();
         if (c->d_pattern) cudaFree(c->d_pattern);
+        if (c->d_desc) cudaFree(c->d_desc);
         delete c;
         return e == cudaErrorMemoryAllocation ? USLAM_OOM : USLAM_CUDA_ERROR;
     }
@@ -968,6 +1033,7 @@ void uslam_destroy(uslam_ctx* c) {
     if (c->ransac_buf) cudaFree(c->ransac_buf);
     if (c->tri_buf) cudaFree(c->tri_buf);
     if (c->d_pattern) cudaFree(c->d_pattern);
+    if (c->d_desc) cudaFree(c->d_desc);
     delete c;
 }
 
@@ -1147,7 +1213,7 @@ uslam_status uslam_batch_profile(uslam_batch* b, int iters, float* kernel_ms) {
                               c->detector, b->d_err, b->stream);
         mark();
         if (e == cudaSuccess) e = launch_compact_banded(b->d_frames, P.bands, P.nbands, c->cell_cap, P.blur, b->stream);
-        if (e == cudaSuccess) e = launch_xsort(b->d_frames, P.fsegs, P.nfsegs, b->max_w, b->stream);
+        if (e == cudaSuccess) e = launch_xsort(b->d_frames, P.fsegs, P.nfsegs, b->max_w, b->max_bands, b->stream);
         mark();
         if (e == cudaSuccess) e = launch_blur(b->d_frames, P.blur, P.nblur, c->num_sms, b->d_err, b->stream);
         mark();
@@ -1559,10 +1625,10 @@ cudaError_t copy_frame_state(const uslam_batch* src, uslam_batch* dst, int slot,
     const size_t capa = static_cast<size_t>(std::max(A.cap, 1));
     cudaError_t e = cudaMemcpyAsync(B.kept, A.kept, 2 * sizeof(uint32_t) * A.levels, cudaMemcpyDeviceToDevice, st);
     for (int l = 0; l < A.levels && e == cudaSuccess; ++l) {
-        const size_t cols = USLAM_MATCH_BANDS * (static_cast<size_t>(A.w[l]) + 1) + USLAM_MATCH_BANDS + 1;
+        const size_t cols = A.nbands * (static_cast<size_t>(A.w[l]) + 1) + A.nbands + 1;
         e = cudaMemcpyAsync(B.feats[l], A.feats[l], capa * 48, cudaMemcpyDeviceToDevice, st);
         if (e == cudaSuccess)
-            e = cudaMemcpyAsync(B.xorder[l], A.xorder[l], USLAM_MATCH_BANDS * capa * 4, cudaMemcpyDeviceToDevice, st);
+            e = cudaMemcpyAsync(B.xorder[l], A.xorder[l], A.nbands * capa * 4, cudaMemcpyDeviceToDevice, st);
         if (e == cudaSuccess) e = cudaMemcpyAsync(B.colstart[l], A.colstart[l], cols * 4, cudaMemcpyDeviceToDevice, st);
         if (e == cudaSuccess) e = cudaMemcpyAsync(B.qorder[l], A.qorder[l], capa * 4, cudaMemcpyDeviceToDevice, st);
     }
@@ -1577,7 +1643,7 @@ cudaError_t copy_frame_state(const uslam_batch* src, uslam_batch* dst, int slot,
         // the windowed tensor-core matcher's operand rows (same frame size,
         // so the same row strides)
         const size_t qrows = static_cast<size_t>(A.levels) * A.wq_rows;
-        const size_t crows = static_cast<size_t>(A.levels) * USLAM_MATCH_BANDS * A.wc_rows;
+        const size_t crows = static_cast<size_t>(A.levels) * A.nbands * A.wc_rows;
         e = cudaMemcpyAsync(B.wq8, A.wq8, qrows * 256, cudaMemcpyDeviceToDevice, st);
         if (e == cudaSuccess) e = cudaMemcpyAsync(B.wc8, A.wc8, crows * 256, cudaMemcpyDeviceToDevice, st);
         if (e == cudaSuccess) e = cudaMemcpyAsync(B.wcext, A.wcext, crows * 32, cudaMemcpyDeviceToDevice, st);

@@ -28,9 +28,11 @@ cudaError_t launch_detect(const FrameDev*, const TileItem*, int, int, int, uint3
 // blur_count: the run's BlurList::count, cleared (null: none)
 cudaError_t launch_pyramid(const FrameDev*, const TileItem*, int, int, uint32_t* blur_count, cudaStream_t);
 cudaError_t launch_compact_banded(const FrameDev*, const BandItem*, int, int cell_cap, BlurList, cudaStream_t);
-cudaError_t launch_xsort(const FrameDev*, const SegDev*, int, int, cudaStream_t);
+cudaError_t launch_xsort(const FrameDev*, const SegDev*, int, int max_w, int max_bands, cudaStream_t);
 cudaError_t launch_blur(const FrameDev*, BlurList, int max_tiles, int num_sms, uint32_t* err, cudaStream_t);
-cudaError_t launch_describe(const FrameDev*, const SegDev*, int, const int32_t*, int, bool, bool, cudaStream_t);
+cudaError_t launch_describe(const FrameDev*, const SegDev*, int, const DescTable*, int num_sms, bool pack, bool win,
+                            cudaStream_t);
+cudaError_t set_describe_smem();
 // k_describe_tiled over describe items (one per KDT_CW-column chunk of every
 // 32-row band); describe_tiled_smem(margin) = its dynamic shared memory, 0 if
 // the box does not fit a TMA box (then k_describe runs instead).
@@ -58,7 +60,7 @@ cudaError_t set_bf_mma_smem();
 cudaError_t launch_frame_from_f32(const float* src, int W, int H, uint8_t* dst, int dpitch, cudaStream_t st);
 // the windowed matcher on the tensor cores (win_tc.cu)
 cudaError_t set_win_mma_smem();
-int win_units_per_seg(int cap);
+int win_units_per_seg(int cap, int nbands);
 size_t win_unit_bytes();
 cudaError_t launch_win_match(const FrameDev*, const PairDev*, const void*, int, int, void*, int, uint32_t*,
                              cudaStream_t);
@@ -236,6 +238,20 @@ inline cudaError_t launch_detect_shaped(const FrameDev* frames, const TileItem* 
     return cudaSuccess;
 }
 
+// Horizontal bands of the matcher's lists for levels of up to cap features.
+// A band's lists hold the rows of its queries and 0.1 H each side, so more
+// bands leave fewer candidates outside the windows, but a group of 32 queries
+// (128 with the tensor cores) then reaches further in x.  Measured with 2, 3,
+// 4, 6, 8, 12, 16 and 24 bands: 64 frames of 752x480 (cap 1443) 1.59, 1.60,
+// 1.61, 1.62, 1.68 ... ms a step; the mixed batch up to 3840x2160 (cap 33177)
+// 6.13, 5.67, 5.54, 5.42, 5.38, 5.42, 5.52, 5.76 ms; one 1920x1080 frame on the
+// tensor cores 790, 767, 753, 769, 765, 841 ... us, one 752x480 frame 307, 305,
+// 310, 316 ... us.
+inline int match_bands_for(int cap, bool win_tc) {
+    if (win_tc) return cap > 5000 ? 4 : 3;
+    return cap > 16000 ? 10 : cap > 5000 ? 6 : cap > 2500 ? 4 : 3;
+}
+
 // Blur tiles of every level of a frame (the most k_band_write can list).
 inline int blur_tiles_of(const FrameDev& F) {
     int n = 0;
@@ -288,6 +304,7 @@ struct uslam_ctx {
         return it == tile_shape.end() ? 0 : it->second;
     }
     int32_t* d_pattern = nullptr;
+    DescTable* d_desc = nullptr;  // the same points as k_describe takes them
     ErrText err;
     std::map<std::pair<int, int>, ResClass> classes;
 

@@ -157,7 +157,7 @@ struct uslam_server {
     char* arena = nullptr;
     uint32_t* d_err = nullptr;
     uint32_t* h_err = nullptr;  // pinned: the error word as of the end of each table buffer's last launch
-    int max_w = 0;
+    int max_w = 0, max_bands = 1;
     cudaStream_t cs[2] = {nullptr, nullptr};
     LaunchBuf bufs[2];
     std::vector<SrvStream> streams;
@@ -320,18 +320,17 @@ cudaError_t launch_batch(uslam_server* s, const std::vector<uint64_t>& tickets, 
     const auto* d_emits = reinterpret_cast<const SrvEmitItem*>(B.d + t_b + f_b + m_b + u_b + p_b + b_b);
     const auto* d_desc = reinterpret_cast<const BandItem*>(B.d + t_b + f_b + m_b + u_b + p_b + b_b + x_b);
     const BlurList bl{reinterpret_cast<TileItem*>(B.d + B.bytes + 256), reinterpret_cast<uint32_t*>(B.d + B.bytes)};
-    const int grid = c->num_sms * 4;
     const int nf = static_cast<int>(fsegs.size());
     if ((e = launch_detect_shaped(s->d_frames, d_tiles, shaped.begin, c->detector, s->d_err, bl.count, st)) != cudaSuccess) return e;
     if ((e = launch_compact_banded(s->d_frames, d_bands, static_cast<int>(bands.size()), c->cell_cap, bl, st)) != cudaSuccess)
         return e;
-    if ((e = launch_xsort(s->d_frames, d_fsegs, nf, s->max_w, st)) != cudaSuccess) return e;
+    if ((e = launch_xsort(s->d_frames, d_fsegs, nf, s->max_w, s->max_bands, st)) != cudaSuccess) return e;
     if ((e = launch_blur(s->d_frames, bl, blur_tiles, c->num_sms, s->d_err, st)) != cudaSuccess) return e;
     e = c->describe_form == 1 && static_cast<int>(emits.size()) >= kTiledDescribeFrames &&
                 describe_tiled_smem(c->margin) > 0
             ? launch_describe_tiled(s->d_frames, d_desc, static_cast<int>(desc.size()), c->d_pattern, false, false,
                                     c->margin, s->d_err, st)
-            : launch_describe(s->d_frames, d_fsegs, nf, c->d_pattern, grid, false, false, st);
+            : launch_describe(s->d_frames, d_fsegs, nf, c->d_desc, c->num_sms, false, false, st);
     if (e != cudaSuccess) return e;
     if (!pairs.empty()) {
         if ((e = launch_bacc_init(s->d_frames, d_pairs, d_usegs, static_cast<int>(usegs.size()), st)) != cudaSuccess)
@@ -506,6 +505,8 @@ uslam_status uslam_server_create(uslam_ctx* ctx, const uslam_server_params* p, u
                 return set_err(&ctx->err, USLAM_INVALID_ARG, "server_create: empty pyramid level");
             }
         F.cap = ctx->cap_override > 0 ? ctx->cap_override : static_cast<int>(static_cast<long long>(W0) * H0 / 250);
+        F.nbands = match_bands_for(F.cap, false);
+        s->max_bands = std::max(s->max_bands, F.nbands);
         const size_t capa = static_cast<size_t>(std::max(F.cap, 1));
         SlotLayout& Y = lay[k];
         size_t cur = 0;
@@ -527,8 +528,8 @@ uslam_status uslam_server_create(uslam_ctx* ctx, const uslam_server_params* p, u
             Y.lvl[l] = take(static_cast<size_t>(F.h[l]) * F.lvl_pitch[l] * 4);
             Y.blur[l] = take(static_cast<size_t>(F.h[l] + ctx->margin + 1) * F.bl_pitch[l] * 4);
             Y.kpmap[l] = take(static_cast<size_t>(F.h[l]) * F.kp_pitch[l]);
-            Y.xorder[l] = take(USLAM_MATCH_BANDS * capa * 4);
-            Y.colstart[l] = take((USLAM_MATCH_BANDS * (static_cast<size_t>(F.w[l]) + 1) + USLAM_MATCH_BANDS + 1) * 4);
+            Y.xorder[l] = take(F.nbands * capa * 4);
+            Y.colstart[l] = take((F.nbands * (static_cast<size_t>(F.w[l]) + 1) + F.nbands + 1) * 4);
             Y.qorder[l] = take(capa * 4);
             Y.bands[l] = take(static_cast<size_t>((F.h[l] + 31) / 32) * 8);
             Y.btile[l] = take(sizeof(uint32_t) * USLAM_BLUR_TILES(F.w[l], F.h[l], F.margin));

@@ -26,7 +26,7 @@
 //   bands[l] u32  [ceil(h_l / 32)][2]      raw and kept keypoint counts per 32-row band
 //   feats[l] Feature[cap]                  gpumodels::Feature records, (y, x) order
 //   xorder[l] u32 [B][cap]                 per band b of the frame height (B =
-//                                          USLAM_MATCH_BANDS): indices of the features
+//                                          FrameDev::nbands): indices of the features
 //                                          whose LOD-0 y lies in the band widened by the
 //                                          window half-height + 2, sorted by x (the
 //                                          matcher's candidate lists)
@@ -41,7 +41,7 @@
 #include <vector_types.h>
 
 #define USLAM_MAX_LEVELS 12
-#define USLAM_MATCH_BANDS 3  // horizontal bands of the frame for the matcher's lists
+#define USLAM_MAX_BANDS 24  // most horizontal bands of a frame for the matcher's lists (FrameDev::nbands)
 #define USLAM_MAX_MATCH_SEGS 2048  // (pair, level) segments of one k_match launch
 
 // Device copy of one frame's geometry and buffer addresses.
@@ -54,6 +54,7 @@ struct FrameDev {
     int bl_pitch[USLAM_MAX_LEVELS];  // blur cache row pitch (floats): w + margin + 1
     int lvl_pitch[USLAM_MAX_LEVELS]; // pyramid level row pitch (floats): w rounded up to 4
     int margin;                      // blur cache margin M beyond the level
+    int nbands;                      // horizontal bands of the matcher's lists (1 .. USLAM_MAX_BANDS)
     int cell_cap;                    // > 0: keypoints kept per 32x32 cell (cell order); 0: (y, x) order
     int frame_cap;                   // > 0: features kept per frame, levels filled in order; 0: none
     // polls of the first mbarrier wait of k_detect's tile load and of the
@@ -91,7 +92,7 @@ struct FrameDev {
     // otherwise): the frame's descriptors as operand rows in the bf8 layout.
     // wq8: the query order of each level (level l from row l * wq_rows), each
     // band's queries starting at a multiple of 128 rows; wc8 / wcext: the
-    // candidate lists (list b of level l from row (USLAM_MATCH_BANDS l + b) *
+    // candidate lists (list b of level l from row (nbands l + b) *
     // wc_rows), with the extension rows of the bfext layout (row index within
     // its 32-row group = list position % 32); wcy: the candidate's y in its
     // level; wcid: packed (level, index).
@@ -181,6 +182,18 @@ struct BandItem {
     uint8_t pad;
     uint16_t band;
     uint16_t pad2;
+};
+
+// The BRIEF table as k_describe gathers it: the 512 test points in 16 compact
+// clusters of 32, pts[cluster][lane], and for test j + 32 k the words of its
+// two points in a warp's 512 gathered values (cluster * 32 + lane; point a in
+// the low half).  In every cluster and in every (k, point) group of 32 the
+// lanes are distinct, so neither the gathers' stores nor the tests' reads
+// meet in a bank.
+#define USLAM_DESC_CLUSTERS 16
+struct DescTable {
+    float pts[USLAM_DESC_CLUSTERS][32][2];
+    uint32_t pair[8][32];
 };
 
 #define USLAM_ERR_SMEM_RANGE 1u

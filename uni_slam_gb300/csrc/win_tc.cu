@@ -65,7 +65,6 @@ static_assert(sizeof(WinUnit) == 80, "unit record");
 
 namespace {
 
-constexpr int NB = USLAM_MATCH_BANDS;
 constexpr int WN_CONSUMERS = 16;                     // 4 lane quarters x 4 column quarters
 constexpr int WN_THREADS = 32 * (WN_CONSUMERS + 1);  // plus one producer warp
 constexpr int WN_M = 128;                            // queries per unit (TMEM lanes)
@@ -273,12 +272,11 @@ __global__ void __launch_bounds__(64) k_win_plan(const FrameDev* __restrict__ fr
     const FrameDev& Q = frames[sg.dir == 0 ? P.curr : P.prev];
     const FrameDev& B = frames[sg.dir == 0 ? P.prev : P.curr];
     const int l = sg.level;
+    const int NB = Q.nbands;
     const uint32_t* qband = Q.colstart[l] + (size_t)NB * (size_t)(Q.w[l] + 1);
-    uint32_t nt[NB], tot = 0;
-    for (int b = 0; b < NB; ++b) {
-        nt[b] = (qband[b + 1] - qband[b] + 127u) / 128u;
-        tot += nt[b];
-    }
+    auto nt = [&](int b) { return (qband[b + 1] - qband[b] + 127u) / 128u; };  // query tiles of band b
+    uint32_t tot = 0;
+    for (int b = 0; b < NB; ++b) tot += nt(b);
     const int L = B.levels;
     uint32_t pool = B.kept[l];
     if (l > 0) pool += B.kept[l - 1];
@@ -303,10 +301,9 @@ __global__ void __launch_bounds__(64) k_win_plan(const FrameDev* __restrict__ fr
         if ((uint32_t)j < tot) {
             uint32_t t = (uint32_t)j, qoff = 0;
             int b = 0;
-            while (t >= nt[b]) {
-                t -= nt[b];
-                qoff += nt[b] * 128u;
-                ++b;
+            for (uint32_t m = nt(0); t >= m; m = nt(++b)) {
+                t -= m;
+                qoff += m * 128u;
             }
             u.band = b;
             u.qpos = (int)(qband[b] + 128u * t);
@@ -465,7 +462,7 @@ k_win_mma(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pairs
                     const uint32_t st = kk_ld % WN_STAGES;
                     ok = bar_wait(&b_empty[st], ((kk_ld / WN_STAGES) + 1u) & 1u);
                     if (!ok) break;
-                    const uint32_t row = (uint32_t)(NB * ld.u.pl[ld.k] + ld.u.band) * (uint32_t)Bf.wc_rows +
+                    const uint32_t row = (uint32_t)(Bf.nbands * ld.u.pl[ld.k] + ld.u.band) * (uint32_t)Bf.wc_rows +
                                          (uint32_t)ld.u.c0[ld.k] + (uint32_t)ld.i * WN_N;
                     bar_expect(&b_full[st], WN_B_BYTES + WN_BX_BYTES);
                     bulk_load(sB + st * WN_B_BYTES, Bf.wc8 + (size_t)(row >> 3) * 2048u, WN_B_BYTES, &b_full[st]);
@@ -489,7 +486,7 @@ k_win_mma(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pairs
                 ok = ok && bar_wait(&b_full[st], (kk_mm / WN_STAGES) & 1u) && bar_wait(&acc_empty[buf], (use + 1u) & 1u);
                 if (!ok) break;
                 // the candidates' y of this tile, for the consumers of accumulator buf
-                const uint32_t row = (uint32_t)(NB * mm.u.pl[mm.k] + mm.u.band) * (uint32_t)Bm.wc_rows +
+                const uint32_t row = (uint32_t)(Bm.nbands * mm.u.pl[mm.k] + mm.u.band) * (uint32_t)Bm.wc_rows +
                                      (uint32_t)mm.u.c0[mm.k] + (uint32_t)mm.i * WN_N;
                 bar_expect(&y_full[buf], WN_Y_BYTES);
                 bulk_load(sY + buf * WN_N, Bm.wcy + row, WN_Y_BYTES, &y_full[buf]);
@@ -662,7 +659,7 @@ k_win_mma(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pairs
                 uint32_t tb = widen(cbk[0] & 0xffffu, gb), ts = widen(csk[0] & 0xffffu, gb);
                 top2_merge(tb, ts, widen(cbk[0] >> 16, gb), widen(csk[0] >> 16, gb));
                 if (tb > best) {
-                    const uint32_t lrow = (uint32_t)(NB * plk + u.band) * (uint32_t)B.wc_rows +
+                    const uint32_t lrow = (uint32_t)(B.nbands * plk + u.band) * (uint32_t)B.wc_rows +
                                           (uint32_t)(c0k + i * WN_N) + (tb & 255u);
                     bidx = __ldg(B.wcid + lrow);
                 }
@@ -711,7 +708,7 @@ cudaError_t set_win_mma_smem() {
 }
 
 // Unit slots per (pair, direction, level) for levels of at most `cap` features.
-int win_units_per_seg(int cap) { return (cap + WN_M - 1) / WN_M + NB; }
+int win_units_per_seg(int cap, int nbands) { return (cap + WN_M - 1) / WN_M + nbands; }
 
 cudaError_t launch_win_match(const FrameDev* frames, const PairDev* pairs, const void* msegs, int nmsegs, int umax,
                              void* units, int num_sms, uint32_t* err, cudaStream_t st) {
