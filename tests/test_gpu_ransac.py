@@ -53,3 +53,25 @@ def test_ransac_score_on_matched_frames(brief_pattern):
     ec, _ = oracle.sampson_counts(Fs, p, q, 3.84)
     assert np.array_equal(counts, ec)
     assert counts.max() > len(m) // 4
+
+
+@pytest.mark.parametrize("n_hyp,n", [(1, 1), (7, 31), (8, 32), (9, 257), (17, 256), (3, 5000)])
+def test_binary32_decision_equals_binary64(n_hyp, n):
+    """The scoring decides in binary32 where that is certain.  Hypotheses of
+    every scale (also beyond binary32), points at the threshold, far outside
+    the frame, infinite and not numbers: counts and masks equal the oracle's."""
+    rs = np.random.RandomState(n_hyp * 1000 + n)
+    pat = np.clip(np.rint(rs.normal(0, 6, (256, 4))), -13, 13).astype(np.int32)
+    F, p, q = two_view(rs, n=n, outliers=n // 4)
+    Fs = np.concatenate([F[None], _hypotheses(rs, p, q, n_hyp - 1)])[:n_hyp] if n >= 8 else rs.normal(size=(n_hyp, 3, 3))
+    q = q.copy()
+    q[::5] += rs.normal(0, 1.4, q[::5].shape)  # near the threshold
+    p[-1:] = [[1e9, -3e7]]
+    if n > 100:
+        p[3], q[4], p[5] = [np.inf, 1.0], [np.nan, 2.0], [0.0, 0.0]
+    with Context(pat, levels=6, max_width=752, max_height=480) as c:
+        for scale in (1.0, 1e-4, 1e-9, 1e30, 1e-60, 1e150):
+            for thr in (3.84, 1e-7, 1e9):
+                counts, masks = c.ransac_score(Fs * scale, p, q, thr, masks=True)
+                ec, em = oracle.sampson_counts(Fs * scale, p, q, thr)
+                assert np.array_equal(counts, ec) and np.array_equal(masks, em), (scale, thr)

@@ -1032,6 +1032,8 @@ void uslam_destroy(uslam_ctx* c) {
     for (auto& kv : c->match_batches) free_batch(kv.second);
     if (c->ransac_buf) cudaFree(c->ransac_buf);
     if (c->tri_buf) cudaFree(c->tri_buf);
+    c->ransac_pin.release();
+    c->tri_pin.release();
     if (c->d_pattern) cudaFree(c->d_pattern);
     if (c->d_desc) cudaFree(c->d_desc);
     delete c;

@@ -268,6 +268,28 @@ inline int lvl_pitch_of(int w) { return static_cast<int>(round_up(static_cast<si
 // the detector.  out holds levels * kNumTileShapes maps of USLAM_TMAP_BYTES.
 uslam_status encode_tile_maps(const FrameDev& F, int detector, void* out, ErrText* err);
 
+// Pinned staging of a call that takes and returns host buffers, grown on
+// demand up to kMax and kept (its owner's lock guards it); a call that needs
+// more copies from and to the caller's memory.
+struct PinnedBuf {
+    static constexpr size_t kMax = size_t(32) << 20;
+    char* p = nullptr;
+    size_t bytes = 0;
+    cudaError_t reserve(size_t need) {
+        if (need <= bytes) return cudaSuccess;
+        release();
+        const cudaError_t e = cudaHostAlloc(&p, need, cudaHostAllocDefault);
+        if (e == cudaSuccess) bytes = need;
+        else p = nullptr;
+        return e;
+    }
+    void release() {
+        if (p) cudaFreeHost(p);
+        p = nullptr;
+        bytes = 0;
+    }
+};
+
 struct ResClass {
     int W0 = 0, H0 = 0;
     std::vector<uint32_t*> d_mask;
@@ -295,9 +317,11 @@ struct uslam_ctx {
     std::map<std::pair<int, int>, uslam_batch*> match_batches;  // uslam_match: a 2-frame batch per frame size
     void* ransac_buf = nullptr;  // uslam_ransac_score scratch, grown on demand
     size_t ransac_bytes = 0;
+    PinnedBuf ransac_pin;
     std::mutex ransac_mu;
     void* tri_buf = nullptr;  // uslam_triangulate scratch, grown on demand
     size_t tri_bytes = 0;
+    PinnedBuf tri_pin;
     std::mutex tri_mu;
     int shape_for(int W0, int H0) const {
         auto it = tile_shape.find(std::make_pair(W0, H0));
