@@ -93,3 +93,44 @@ def test_edge_calls(ctx):
     with pytest.raises(USlamError):
         ctx.triangulate(np.zeros((10, 4)), cam, {"min_inliers": 4})
     assert ctx.pixel_to_normalised(np.zeros((0, 2)), cam).shape == (0, 2)
+
+
+@pytest.fixture(scope="module")
+def own_ctx():
+    pat = np.clip(np.rint(np.random.RandomState(5).normal(0, 6, (256, 4))), -13, 13).astype(np.int32)
+    with Context(pat, max_width=752, max_height=480) as c:
+        yield c
+
+
+@pytest.mark.parametrize("n", [16, 31, 32, 33, 63, 64, 65, 1023, 1025, 2500])
+@pytest.mark.parametrize("noise", [0.0, 0.3])
+def test_edges_of_chunks_and_methods(own_ctx, n, noise):
+    """Row counts beside a chunk (32 rows), the 9-vector's two methods (64
+    rows) and 32 chunks, with and without a gap below the smallest singular
+    value, alone and as one of three pairs, against the oracle."""
+    px = synth.two_view_scene(seed=900 + n, n=n, noise_px=noise)[0][:, 1:5].astype(np.float64)
+    want = T.triangulate(px, synth.SCENE_CAMERA)
+    pose = np.concatenate([want["rotation"].ravel(), want["translation"]])
+    stats = [want["input_matches"], want["landmark_count"], want["cheirality_passes"],
+             want["mean_reprojection_error_px"], want["pose_recovered"], want["rotation_angle_rad"]]
+    one = own_ctx.triangulate(px, synth.SCENE_CAMERA)
+    for r in [one] + own_ctx.triangulate([px[:9], px, px[:8]], synth.SCENE_CAMERA)[1:2]:
+        check_against_reference(r, pose, stats, want["keep"], want["landmarks"], f"n={n} noise={noise}")
+
+
+@pytest.mark.parametrize("seed", [6, 12, 37])
+def test_tied_candidates(own_ctx, seed):
+    """Unrelated pixels, several candidates with the most points: one of them
+    is the result, the same one alone and among other pairs."""
+    px = np.random.RandomState(seed).uniform([20, 20, 20, 20], [700, 440, 700, 440], (12, 4))
+    want = T.triangulate(px, synth.SCENE_CAMERA)
+    top = np.flatnonzero(want["in_front"] == want["in_front"].max())
+    assert len(top) > 1
+    rays = [T.pixel_to_normalised(v, synth.SCENE_CAMERA, 20, 1e-9) for v in (px[:, :2], px[:, 2:])]
+    cands = T.decompose_essential(T.fit_essential(*rays))
+    one = own_ctx.triangulate(px, synth.SCENE_CAMERA)
+    two = own_ctx.triangulate([px[::-1].copy(), px], synth.SCENE_CAMERA)[1]
+    assert one["cheirality_passes"] == want["in_front"].max()
+    assert min(np.abs(one["rotation"] - cands[k][0]).max() + np.abs(one["translation"] - cands[k][1]).max()
+               for k in top) <= 1e-9
+    assert np.array_equal(one["rotation"], two["rotation"]) and np.array_equal(one["translation"], two["translation"])
