@@ -188,3 +188,35 @@ def test_tensor_core_matcher_pair_limit(brief_pattern):
                 with pytest.raises(USlamError) as ei:
                     Batch(c, sizes, pairs)
                 assert ei.value.status == capi.CAPACITY
+
+
+def _own_pattern():
+    return np.clip(np.rint(np.random.RandomState(5).normal(0, 6, (256, 4))), -13, 13).astype(np.int32)
+
+
+@pytest.mark.parametrize("matcher", [1, 2])
+@pytest.mark.parametrize("n,copies", [(2, 1), (127, 1), (128, 3), (129, 1), (255, 1), (256, 1), (257, 2), (1025, 1),
+                                      (129, 620)])
+def test_shares_cut_blocks_anywhere(matcher, n, copies):
+    """n features a frame beside the tiles (128) and query blocks (256): few
+    pairs, whose blocks are cut into parts, and so many that they stay whole
+    (matcher 2), an uneven pair and one with an empty frame among them."""
+    pat = _own_pattern()
+    f0, f1 = synth.warped_pair(41, 640, 480)
+    empty = np.full((480, 640), 90, np.uint8)
+    small = empty.copy()
+    small[100:220, 200:360] = synth.scene_frame(9, 160, 120)
+    frames = [f0, f1, small, empty]
+    distinct = [(0, 1), (1, 0), (0, 2), (2, 1), (0, 3), (3, 1)]
+    pairs = distinct * copies if copies < 100 else (distinct * copies)[:copies]
+    exp = [oracle.frame(f, pat, levels=1, cap=n) for f in frames]
+    assert exp[0][1].sum() == n and exp[1][1].sum() == n and exp[3][1].sum() == 0
+    want = [oracle.match_bruteforce(exp[p][0], exp[p][1], exp[q][0], exp[q][1], 0.9) for p, q in distinct]
+    with Context(pat, levels=1, max_width=640, max_height=480, cap_per_level=n, matcher=matcher, ratio=0.9) as c:
+        b = Batch(c, [(f.shape[1], f.shape[0]) for f in frames], pairs)
+        try:
+            b.process(frames)
+            for k in range(len(pairs)):
+                assert np.array_equal(_mm(b.matches(k)), want[k % len(distinct)]), k
+        finally:
+            b.close()

@@ -22,8 +22,8 @@
 //
 // One persistent CTA per SM holds 512 TMEM columns: two buffers of two
 // 128 x 128 f32 accumulators.  A work unit is 256 queries of one pair (one
-// accumulator per 128) against the pair's train set, or a share of it when
-// the train set is split.  A producer warp stages the query tile (64 KB) and
+// accumulator per 128) against the pair's train set, or the part of it that
+// the CTA's share of the work holds (bf_line.h).  A producer warp stages the query tile (64 KB) and
 // the train tiles (128 rows: 32 KB + 4 KB extension, four stages) by bulk
 // copies and issues, per train tile, nine tcgen05.mma (K = 32) into each
 // accumulator of one buffer; sixteen consumer warps (four per TMEM lane
@@ -45,6 +45,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "bf_line.h"
 #include "uslam_internal.h"
 
 namespace uslam {
@@ -185,55 +186,13 @@ __device__ __forceinline__ void top2_merge(uint32_t& b, uint32_t& s, uint32_t b2
     b = max(b, b2);
 }
 
-__device__ __forceinline__ uint32_t total_kept(const FrameDev& F) {
-    uint32_t n = 0;
-    for (int l = 0; l < F.levels; ++l) n += F.kept[l];
-    return n;
-}
-
 }  // namespace
 
-// Work units: 256 queries of one pair (two 128-row accumulators) against
-// the pair's train set, or a share of it when the train set is split.  Both
-// roles walk the same unit sequence and count the train tiles they pass
-// (kk, across units): tile kk uses stage kk % 3 and accumulator buffer
-// kk % 2, and the parity of the barrier phase it waits for follows from kk.
-struct TcUnit {
-    const PairDev* P;
-    const FrameDev* A;
-    const FrameDev* B;
-    uint32_t nq, nt, qbase, tb, split, nsplit;
-    int NT;
-};
+// Both roles walk the same units of the CTA's share (bf_line.h) and count
+// the train tiles they pass (kk, across units): tile kk uses stage
+// kk % TC_STAGES and accumulator buffer kk % 2, and the parity of the barrier
+// phase it waits for follows from kk.
 
-__device__ __forceinline__ TcUnit tc_unit(const FrameDev* frames, const PairDev* pairs, const SegDev* psegs,
-                                          const uint32_t* pref, int npairs, uint32_t g) {
-    int lo = 0, hi = npairs - 1;  // pair with pref[p] <= g < pref[p + 1]
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (pref[mid] <= g) lo = mid;
-        else hi = mid - 1;
-    }
-    TcUnit u;
-    u.P = &pairs[psegs[lo].frame];
-    u.A = &frames[u.P->prev];
-    u.B = &frames[u.P->curr];
-    u.nsplit = (uint32_t)max(u.P->bf_splits, 1);
-    const uint32_t unit = g - pref[lo];
-    const uint32_t qt = unit / u.nsplit;
-    u.split = unit - qt * u.nsplit;
-    u.qbase = qt * (uint32_t)TC_Q;
-    u.nq = total_kept(*u.A);
-    u.nt = total_kept(*u.B);
-    const uint32_t ntiles = (u.nt + TC_N - 1) / TC_N;
-    u.tb = u.split * ntiles / u.nsplit;
-    u.NT = (int)((u.split + 1u) * ntiles / u.nsplit - u.tb);
-    return u;
-}
-
-// Result per query a in a2b (packed (level, index) of its match in curr, or
-// -1), or, when the pair's train set is split, one partial record per split
-// ((distance << 8) of best and second, best id) merged by the emit kernel.
 __global__ void __launch_bounds__(TC_THREADS, 1)
 k_bf_mma(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pairs, const SegDev* __restrict__ psegs,
          int npairs, float ratio, uint32_t* err) {
@@ -241,7 +200,7 @@ k_bf_mma(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pairs,
     __shared__ __align__(8) uint64_t bar_a, b_full[TC_STAGES], b_empty[TC_STAGES], acc_full[2], acc_empty[2];
     __shared__ uint32_t s_tmem;
     __shared__ int s_fail;
-    __shared__ uint32_t s_pref[kMaxPairs + 1];
+    __shared__ unsigned long long s_pref[kMaxPairs + 1], s_warp[TC_THREADS / 32];
     __shared__ uint32_t s_hb[TC_Q], s_hs[TC_Q];  // second column group's top-2 per query row
     __shared__ int32_t s_hi[TC_Q];
     uint8_t* sA = tc_smem;
@@ -251,12 +210,6 @@ k_bf_mma(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pairs,
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     volatile int* fail = &s_fail;
 
-    // work units per pair: query blocks x train splits
-    for (int p = t; p < npairs; p += TC_THREADS) {
-        const PairDev& P = pairs[psegs[p].frame];
-        const uint32_t nq = total_kept(frames[P.prev]);
-        s_pref[p + 1] = (nq + TC_Q - 1) / TC_Q * (uint32_t)max(P.bf_splits, 1);
-    }
     // query-side extension, the same for every row: 16 x -32 (0xE0), 32 (0x60),
     // 1, 1 (0x38), 32, zeros
     for (int i = t; i < (int)TC_AX_BYTES; i += TC_THREADS) {
@@ -284,16 +237,12 @@ k_bf_mma(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pairs,
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    __syncthreads();
-    if (t == 0) {
-        s_pref[0] = 0;
-        for (int p = 0; p < npairs; ++p) s_pref[p + 1] += s_pref[p];
-    }
+    BfLine line = bf_line<TC_Q, TC_N>(frames, pairs, psegs, npairs, s_pref, s_warp);
+    BfUnit u;
     fence_before();
     __syncthreads();
     fence_after();
     const uint32_t tmem = s_tmem;
-    const uint32_t total = s_pref[npairs];
 
     if (warp == TC_CONSUMERS) {
         // ------------------------------------------------ producer (one lane)
@@ -307,34 +256,33 @@ k_bf_mma(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pairs,
             bool a_pending = false;  // a query tile in flight whose wait gave up
             int64_t last_mma = -1;  // tile index of the last MMA group committed
             int64_t loaded_to = 0;  // tiles [.., loaded_to) have had their loads issued
-            auto load_b = [&](const TcUnit& u, uint32_t tile_kk, uint32_t n) -> bool {
+            auto load_b = [&](const FrameDev& B, uint32_t tile, uint32_t tile_kk) -> bool {
                 const uint32_t st = tile_kk % TC_STAGES;
                 // the stage's previous tile (tile_kk - 3) must have been read by its MMAs
                 if (!bar_wait(&b_empty[st], ((tile_kk / TC_STAGES) + 1u) & 1u)) return false;
                 bar_expect(&b_full[st], TC_B_BYTES + TC_BX_BYTES);
-                const uint32_t tile = u.tb + n;
-                bulk_load(sB + st * TC_B_BYTES, u.B->bf8 + (size_t)tile * TC_B_BYTES, TC_B_BYTES, &b_full[st]);
-                bulk_load(sBx + st * TC_BX_BYTES, u.B->bfext + (size_t)tile * TC_BX_BYTES, TC_BX_BYTES, &b_full[st]);
+                bulk_load(sB + st * TC_B_BYTES, B.bf8 + (size_t)tile * TC_B_BYTES, TC_B_BYTES, &b_full[st]);
+                bulk_load(sBx + st * TC_BX_BYTES, B.bfext + (size_t)tile * TC_BX_BYTES, TC_BX_BYTES, &b_full[st]);
                 loaded_to = (int64_t)tile_kk + 1;
                 return true;
             };
-            for (uint32_t g = blockIdx.x; g < total && !*fail; g += gridDim.x) {
-                const TcUnit u = tc_unit(frames, pairs, psegs, s_pref, npairs, g);
-                if (u.NT <= 0) continue;
+            while (!*fail && bf_next<TC_Q, TC_N>(frames, pairs, psegs, npairs, s_pref, line, u)) {
+                const FrameDev &A = frames[u.P->prev], &B = frames[u.P->curr];
                 bool ok = true;
                 // the query tiles are rewritten: the previous unit's MMAs must be done
                 if (last_mma >= 0) ok = bar_wait(&acc_full[last_mma & 1], (uint32_t)(last_mma >> 1) & 1u);
                 if (ok) {
                     bar_expect(&bar_a, TC_A_BYTES);
-                    bulk_load(sA, u.A->bf8 + (size_t)u.qbase * TC_ROW_BYTES, TC_A_BYTES, &bar_a);
+                    bulk_load(sA, A.bf8 + (size_t)u.blk * (TC_Q * TC_ROW_BYTES), TC_A_BYTES, &bar_a);
                     // the launch's first query-tile wait may be shortened (a test hook)
-                    const int fw = u.A->match_first_wait;
+                    const int fw = A.match_first_wait;
                     ok = bar_wait(&bar_a, units_loaded & 1u, units_loaded == 0 && fw >= 0 ? (uint32_t)fw : kWaitLimit);
                     a_pending = !ok;
                     ++units_loaded;
                 }
-                for (int n = 0; n < TC_STAGES - 1 && n < u.NT && ok; ++n) ok = load_b(u, kk + (uint32_t)n, (uint32_t)n);
-                for (int n = 0; n < u.NT && ok; ++n) {
+                const int NT = (int)u.ntiles;
+                for (int n = 0; n < TC_STAGES - 1 && n < NT && ok; ++n) ok = load_b(B, u.tile + (uint32_t)n, kk + (uint32_t)n);
+                for (int n = 0; n < NT && ok; ++n) {
                     const uint32_t tk = kk + (uint32_t)n, st = tk % TC_STAGES, buf = tk & 1u;
                     ok = bar_wait(&b_full[st], (tk / TC_STAGES) & 1u) &&
                          bar_wait(&acc_empty[buf], ((tk >> 1) + 1u) & 1u);
@@ -355,10 +303,10 @@ k_bf_mma(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pairs,
                     mma_commit(&b_empty[st]);
                     last_mma = (int64_t)tk;
                     // the stage of tile tk - 1 takes tile tk + TC_STAGES - 1
-                    if (n + TC_STAGES - 1 < u.NT)
-                        ok = load_b(u, tk + (uint32_t)(TC_STAGES - 1), (uint32_t)(n + TC_STAGES - 1));
+                    if (n + TC_STAGES - 1 < NT)
+                        ok = load_b(B, u.tile + (uint32_t)(n + TC_STAGES - 1), tk + (uint32_t)(TC_STAGES - 1));
                 }
-                kk += (uint32_t)u.NT;
+                kk += u.ntiles;
                 if (!ok) *fail = 1;
             }
             if (*fail) {
@@ -380,12 +328,13 @@ k_bf_mma(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pairs,
         const int row = 32 * quarter + lane;
         const uint32_t s0 = (uint32_t)(64 * cgrp);  // this warp's first column in a tile
         uint32_t kk = 0;
-        for (uint32_t g = blockIdx.x; g < total; g += gridDim.x) {
-            const TcUnit u = tc_unit(frames, pairs, psegs, s_pref, npairs, g);
+        while (bf_next<TC_Q, TC_N>(frames, pairs, psegs, npairs, s_pref, line, u)) {
+            const FrameDev &A = frames[u.P->prev], &B = frames[u.P->curr];
+            const int NT = (int)u.ntiles;
             uint32_t best = 0u, second = 0u;  // widened keys; 0 = no candidate
             int32_t bidx = -1;
             bool bad = false;
-            for (int n = 0; n < u.NT; ++n) {
+            for (int n = 0; n < NT; ++n) {
                 const uint32_t tk = kk + (uint32_t)n, buf = tk & 1u;
                 bad = bad || *fail != 0 || !bar_wait(&acc_full[buf], (tk >> 1) & 1u);
                 fence_after();
@@ -406,7 +355,7 @@ k_bf_mma(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pairs,
                 __syncwarp();
                 if (lane == 0) bar_arrive(&acc_empty[buf]);
                 if (go) {
-                    const uint32_t base = (u.tb + (uint32_t)n) * (uint32_t)TC_N;
+                    const uint32_t base = (u.tile + (uint32_t)n) * (uint32_t)TC_N;
                     const uint32_t valid = u.nt - base < (uint32_t)TC_N ? u.nt - base : (uint32_t)TC_N;
                     uint32_t cb[4] = {0u, 0u, 0u, 0u}, cs[4] = {0u, 0u, 0u, 0u};
                     if (valid == (uint32_t)TC_N) {
@@ -427,13 +376,13 @@ k_bf_mma(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pairs,
                     top2x2_merge(cb[0], cs[0], cb[2], cs[2]);
                     uint32_t tb = widen(cb[0] & 0xffffu, s0), ts = widen(cs[0] & 0xffffu, s0);
                     top2_merge(tb, ts, widen(cb[0] >> 16, s0 + 32u), widen(cs[0] >> 16, s0 + 32u));
-                    if (tb > best) bidx = __ldg(u.B->bfid + base + (tb & 255u));
+                    if (tb > best) bidx = __ldg(B.bfid + base + (tb & 255u));
                     top2_merge(best, second, tb, ts);
                 } else {
                     bad = true;
                 }
             }
-            kk += (uint32_t)max(u.NT, 0);
+            kk += u.ntiles;
             if (bad) *fail = 1;
             // merge the two column groups of each query row (named barrier 1:
             // the consumer warps only)
@@ -444,25 +393,21 @@ k_bf_mma(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pairs,
                 s_hi[slot_row] = bidx;
             }
             asm volatile("bar.sync 1, %0;" ::"r"(32 * TC_CONSUMERS) : "memory");
-            const uint32_t q = u.qbase + (uint32_t)slot_row;
+            const uint32_t q = u.blk * (uint32_t)TC_Q + (uint32_t)slot_row;
             if (cgrp == 0 && !bad && q < u.nq) {
                 const uint32_t ob = s_hb[slot_row];
                 if (ob > best) bidx = s_hi[slot_row];
                 top2_merge(best, second, ob, s_hs[slot_row]);
-                const FrameDev& A = *u.A;
                 const int32_t qid = __ldg(A.bfid + q);
                 const size_t slot = (size_t)USLAM_PACK_LEVEL(qid) * A.cap + (size_t)USLAM_PACK_INDEX(qid);
                 // distance = popc(a) + 257 - (key >> 5), key >> 5 = widened key >> 8
                 const uint32_t pq = __ldg(A.bfpop + q);
                 const uint32_t db = best == 0u ? 0xffffffu : pq + 257u - (best >> 8);
                 const uint32_t ds = second == 0u ? 0xffffffu : pq + 257u - (second >> 8);
-                if (u.nsplit == 1u) {
+                if (u.P->bf_part == nullptr)
                     u.P->a2b[slot] = (u.nt >= 2u && bidx >= 0 && (float)db < ratio * (float)ds) ? bidx : -1;
-                } else {
-                    const size_t stride = (size_t)A.levels * A.cap;
-                    *reinterpret_cast<uint4*>(u.P->bf_part + (u.split * stride + slot) * 4u) =
-                        make_uint4(db << 8, ds << 8, (uint32_t)bidx, 0u);
-                }
+                else
+                    bf_record(u, (size_t)A.levels * A.cap, slot, db, ds, bidx);
             }
             asm volatile("bar.sync 1, %0;" ::"r"(32 * TC_CONSUMERS) : "memory");  // s_h* reused by the next unit
             if (*fail) break;

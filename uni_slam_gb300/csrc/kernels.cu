@@ -34,6 +34,7 @@
 #include <stdint.h>
 
 #include "../../include/uslam_canon.h"
+#include "bf_line.h"
 #include "uslam_internal.h"
 
 namespace uslam {
@@ -1881,6 +1882,16 @@ size_t describe_tiled_smem(int margin) {
     return (size_t)BW * (size_t)BH * 4u;
 }
 
+// One three-input logic operation; LUT: its value where the inputs are the
+// bits of 0xf0, 0xcc, 0xaa.  Written out: with shared terms such as x ^ y in a
+// sum and its carry the compiler keeps the term and needs an operation more.
+template <int LUT>
+__device__ __forceinline__ uint32_t lop3(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t d;
+    asm("lop3.b32 %0, %1, %2, %3, %4;" : "=r"(d) : "r"(a), "r"(b), "r"(c), "n"(LUT));
+    return d;
+}
+
 // ------------------------------------------------- Hamming distance ----
 // popcount(a ^ b) over 256 bits with 4 POPC instead of 8: three carry-save
 // adders fold x0..x6 into ones (o3) and twos (t1, t2, t3), a fourth folds
@@ -1892,11 +1903,33 @@ size_t describe_tiled_smem(int margin) {
 __device__ __forceinline__ uint32_t hamming256(const uint4& a0, const uint4& a1, const uint4& b0, const uint4& b1) {
     const uint32_t x0 = a0.x ^ b0.x, x1 = a0.y ^ b0.y, x2 = a0.z ^ b0.z, x3 = a0.w ^ b0.w;
     const uint32_t x4 = a1.x ^ b1.x, x5 = a1.y ^ b1.y, x6 = a1.z ^ b1.z, x7 = a1.w ^ b1.w;
-    const uint32_t o1 = x0 ^ x1 ^ x2, t1 = (x0 & x1) | (x2 & (x0 ^ x1));
-    const uint32_t o2 = o1 ^ x3 ^ x4, t2 = (o1 & x3) | (x4 & (o1 ^ x3));
-    const uint32_t o3 = o2 ^ x5 ^ x6, t3 = (o2 & x5) | (x6 & (o2 ^ x5));
-    const uint32_t tw = t1 ^ t2 ^ t3, f = (t1 & t2) | (t3 & (t1 ^ t2));
+    const uint32_t o1 = lop3<0x96>(x0, x1, x2), t1 = lop3<0xe8>(x0, x1, x2);
+    const uint32_t o2 = lop3<0x96>(o1, x3, x4), t2 = lop3<0xe8>(o1, x3, x4);
+    const uint32_t o3 = lop3<0x96>(o2, x5, x6), t3 = lop3<0xe8>(o2, x5, x6);
+    const uint32_t tw = lop3<0x96>(t1, t2, t3), f = lop3<0xe8>(t1, t2, t3);
     return (uint32_t)__popc(o3) + (uint32_t)__popc(x7) + 2u * (uint32_t)__popc(tw) + 4u * (uint32_t)__popc(f);
+}
+
+// The same between descriptors in the form of parity_words, 13 logic operations
+// instead of 16: a full adder's third input is not needed beside its sum
+// (carry = x y | (x ^ y) ~sum), and the sums of words of a ^ b are the
+// differences of the descriptors' own, kept in the third inputs' place.  The
+// weighted sum runs on the multiply-add pipe: two is 2 in a register the
+// compiler does not see through (of a constant it makes shifted adds, which
+// run on the ALU pipe beside the logic).
+__device__ __forceinline__ void parity_words(uint4& d0, uint4& d1) {
+    d0.z = d0.x ^ d0.y ^ d0.z;
+    d1.x = d0.z ^ d0.w ^ d1.x;
+    d1.z = d1.x ^ d1.y ^ d1.z;
+}
+__device__ __forceinline__ uint32_t hamming256_parity(const uint4& a0, const uint4& a1, const uint4& b0, const uint4& b1,
+                                                      uint32_t two, uint32_t one) {
+    const uint32_t x0 = a0.x ^ b0.x, x1 = a0.y ^ b0.y, o1 = a0.z ^ b0.z, x3 = a0.w ^ b0.w;
+    const uint32_t o2 = a1.x ^ b1.x, x5 = a1.y ^ b1.y, o3 = a1.z ^ b1.z, x7 = a1.w ^ b1.w;
+    const uint32_t t1 = lop3<0xd4>(x0, x1, o1), t2 = lop3<0xd4>(o1, x3, o2), t3 = lop3<0xd4>(o2, x5, o3);
+    const uint32_t tw = lop3<0x96>(t1, t2, t3), f = lop3<0xe8>(t1, t2, t3);
+    const uint32_t hi = (uint32_t)__popc(f) * two + (uint32_t)__popc(tw);
+    return (uint32_t)__popc(x7) * one + (hi * two + (uint32_t)__popc(o3));
 }
 
 // ------------------------------------------------------------- K3 ----
@@ -2385,9 +2418,12 @@ k_bacc_init(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pai
 }
 
 // ----------------------------------------------------- brute force ----
-constexpr int KB_THREADS = 128;  // two queries per thread: 256 queries per CTA
-constexpr int KB_TILE = 256;     // train descriptors per shared-memory tile
-static_assert(KB_TILE <= 256, "tile slots are packed into 8 bits of the top-2 keys");
+constexpr int KB_THREADS = 64;
+constexpr int KB_CTAS = 512 / KB_THREADS;  // per SM
+constexpr int KB_PAIRS = 2;      // pairs of queries per thread: 512 queries per CTA
+constexpr int KB_Q = 2 * KB_PAIRS;
+constexpr int KB_TILE = 128;     // train descriptors per shared-memory tile
+static_assert(256 * KB_TILE + KB_TILE - 1 < 0xffff, "distance and tile slot share 16 bits");
 
 // Level of flat index f given the per-level prefix pre[0..L] (pre[L] = total).
 __device__ __forceinline__ int flat_level(const uint32_t* pre, int L, uint32_t f) {
@@ -2399,33 +2435,35 @@ __device__ __forceinline__ int flat_level(const uint32_t* pre, int L, uint32_t f
 // Brute-force top-2 matching (the benchmark's `cfg` matcher): every feature
 // of frame prev (all levels) against every feature of frame curr, Lowe test
 // best < ratio * second in f32, no window and no cross-check.  One CTA holds
-// 256 queries in registers and streams the train set through shared memory
-// in tiles of 256 descriptors.  A tied best fails the ratio test, so the
-// result does not depend on the scan order; a train set of fewer than two
-// features gives no match (the pool rule of match_features_cpu.cpp:80-82).
-// Result per query a in a2b: packed (level, index) of its match in curr, or -1.
-__global__ void __launch_bounds__(KB_THREADS, 8)
+// 256 queries in registers, four a thread, and streams the train set through
+// shared memory in tiles of 128 descriptors.  A tied best fails the ratio
+// test, so the result does not depend on the scan order; a train set of fewer
+// than two features gives no match (the pool rule of
+// match_features_cpu.cpp:80-82).
+// Result per query a in a2b: packed (level, index) of its match in curr, or
+// -1; or one record per part of a cut block (bf_line.h).
+//
+// The ALU and popcount pipes bound it (71 and 76 % busy).  So: descriptors as
+// parity_words (13 logic operations and 4 popcounts a distance), weighted sums
+// by multiply-add, and two queries' keys of 16 bits in a word, which min and
+// max take together.  15 pairs of 8200 x 8200: 1.59 ms before, 1.05 now, 0.97 T
+// distances/s; four queries a thread measured 8 % faster than two, tiles of 64
+// or CTAs of 32 or 128 threads 1 to 3 % slower.
+__global__ void __launch_bounds__(KB_THREADS, KB_CTAS)
 k_bruteforce(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pairs, const SegDev* __restrict__ psegs,
-             int npairs, float ratio) {
-    __shared__ uint32_t s_pref[MAX_SEGS + 1];
-    __shared__ uint32_t s_warp[33];
+             int npairs, float ratio, uint32_t two) {
+    extern __shared__ unsigned long long s_pref[];  // npairs + 1
+    __shared__ unsigned long long s_warp[KB_THREADS / 32];
     __shared__ uint4 s_d[2 * KB_TILE];
     __shared__ int32_t s_id[KB_TILE];
     __shared__ uint32_t s_qpre[USLAM_MAX_LEVELS + 1], s_tpre[USLAM_MAX_LEVELS + 1];
-    const uint32_t total = segment_prefix(npairs, s_pref, s_warp, [&](int s) {
-        const PairDev& P = pairs[psegs[s].frame];
-        const FrameDev& A = frames[P.prev];
-        uint32_t n = 0;
-        for (int l = 0; l < A.levels; ++l) n += A.kept[l];
-        return (n + 2u * KB_THREADS - 1u) / (2u * KB_THREADS) * (uint32_t)max(P.bf_splits, 1);
-    });
     const int tid = threadIdx.x;
-    for (uint32_t g = blockIdx.x; g < total; g += gridDim.x) {
-        const int sidx = find_segment(s_pref, npairs, g);
-        const PairDev& P = pairs[psegs[sidx].frame];
-        const uint32_t nsplit = (uint32_t)max(P.bf_splits, 1);
-        const uint32_t unit = g - s_pref[sidx];
-        const uint32_t blk = unit / nsplit, split = unit - blk * nsplit;
+    const uint32_t one = two >> 1, two16 = two << 15, tile = two * (uint32_t)(KB_TILE / 2);
+    BfLine line = bf_line<KB_Q * KB_THREADS, KB_TILE>(frames, pairs, psegs, npairs, s_pref, s_warp);
+    BfUnit u;
+    while (bf_next<KB_Q * KB_THREADS, KB_TILE>(frames, pairs, psegs, npairs, s_pref, line, u)) {
+        const PairDev& P = *u.P;
+        const uint32_t blk = u.blk;
         const FrameDev& A = frames[P.prev];
         const FrameDev& B = frames[P.curr];
         const int LA = A.levels, LB = B.levels;
@@ -2439,30 +2477,30 @@ k_bruteforce(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pa
             }
         }
         __syncthreads();
-        const uint32_t nq = s_qpre[LA], nt = s_tpre[LB];
-        uint4 q0[2], q1[2];
-        uint32_t best[2], second[2];
-        int32_t bidx[2];
-        int ql[2];
-        uint32_t qi[2];
-        bool qv[2];
+        const uint32_t nq = u.nq, nt = u.nt;
+        const bool busy = blk * (uint32_t)(KB_Q * KB_THREADS) + (uint32_t)(KB_Q * (tid & ~31)) < nq;  // the warp has queries
+        uint4 q0[KB_Q], q1[KB_Q];
+        uint32_t best[KB_PAIRS], second[KB_PAIRS];  // two queries' keys of 16 bits each: distance * KB_TILE + tile slot
+        int32_t bidx[KB_Q];
+        int ql[KB_Q];
+        uint32_t qi[KB_Q];
+        bool qv[KB_Q];
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            const uint32_t f = blk * 2u * KB_THREADS + 2u * tid + k;
+        for (int k = 0; k < KB_Q; ++k) {
+            const uint32_t f = blk * (uint32_t)(KB_Q * KB_THREADS) + (uint32_t)(KB_Q * tid + k);
             qv[k] = f < nq;
             ql[k] = qv[k] ? flat_level(s_qpre, LA, f) : 0;
             qi[k] = qv[k] ? f - s_qpre[ql[k]] : 0u;
             const uint32_t* rec = A.feats[ql[k]] + (size_t)qi[k] * 12u;
             q0[k] = qv[k] ? *reinterpret_cast<const uint4*>(rec + 4) : make_uint4(0, 0, 0, 0);
             q1[k] = qv[k] ? *reinterpret_cast<const uint4*>(rec + 8) : make_uint4(0, 0, 0, 0);
-            best[k] = second[k] = 0xffffffffu;  // keys: distance << 8 | tile slot
+            parity_words(q0[k], q1[k]);
             bidx[k] = -1;
         }
-        // this unit's share of the train set: tiles [split T / S, (split + 1) T / S)
-        const uint32_t ntiles = (nt + KB_TILE - 1) / KB_TILE;
-        const uint32_t tb = split * ntiles / nsplit, te = (split + 1u) * ntiles / nsplit;
-        const uint32_t t_end = min(nt, te * (uint32_t)KB_TILE);
-        for (uint32_t t0 = tb * (uint32_t)KB_TILE; t0 < t_end; t0 += KB_TILE) {
+#pragma unroll
+        for (int k = 0; k < KB_PAIRS; ++k) best[k] = second[k] = 0xffffffffu;
+        const uint32_t t_end = min(nt, (u.tile + u.ntiles) * (uint32_t)KB_TILE);
+        for (uint32_t t0 = u.tile * (uint32_t)KB_TILE; t0 < t_end; t0 += KB_TILE) {
             __syncthreads();
             for (int j = tid; j < KB_TILE; j += KB_THREADS) {
                 const uint32_t f = t0 + (uint32_t)j;
@@ -2470,43 +2508,54 @@ k_bruteforce(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pa
                     const int l = flat_level(s_tpre, LB, f);
                     const uint32_t i = f - s_tpre[l];
                     const uint32_t* rec = B.feats[l] + (size_t)i * 12u;
-                    s_d[2 * j] = __ldg(reinterpret_cast<const uint4*>(rec + 4));
-                    s_d[2 * j + 1] = __ldg(reinterpret_cast<const uint4*>(rec + 8));
+                    uint4 d0 = __ldg(reinterpret_cast<const uint4*>(rec + 4)), d1 = __ldg(reinterpret_cast<const uint4*>(rec + 8));
+                    parity_words(d0, d1);
+                    s_d[2 * j] = d0;
+                    s_d[2 * j + 1] = d1;
                     s_id[j] = USLAM_PACK(l, i);
                 }
             }
             __syncthreads();
+            if (!busy) continue;
             const int n = (int)min((uint32_t)KB_TILE, t_end - t0);
-            const uint32_t prev0 = best[0], prev1 = best[1];
-            for (int j = 0; j < n; ++j) {
+            uint32_t prev[KB_PAIRS];
+#pragma unroll
+            for (int k = 0; k < KB_PAIRS; ++k) prev[k] = best[k];
+            uint32_t slot = 0u;  // j in both halves
+#pragma unroll 4
+            for (int j = 0; j < n; ++j, slot += 0x10001u) {
                 const uint4 d0 = s_d[2 * j], d1 = s_d[2 * j + 1];
 #pragma unroll
-                for (int k = 0; k < 2; ++k) {
-                    // min/max on (distance << 8 | slot) keep the two smallest
-                    // distances; a tie leaves second >> 8 == best >> 8
-                    const uint32_t key = (hamming256(q0[k], q1[k], d0, d1) << 8) | (uint32_t)j;
-                    second[k] = min(second[k], max(best[k], key));
-                    best[k] = min(best[k], key);
+                for (int k = 0; k < KB_PAIRS; ++k) {
+                    const uint32_t lo = hamming256_parity(q0[2 * k], q1[2 * k], d0, d1, two, one);
+                    const uint32_t hi = hamming256_parity(q0[2 * k + 1], q1[2 * k + 1], d0, d1, two, one);
+                    // min/max keep the two smallest distances; a tie leaves
+                    // equal distances in best and second
+                    const uint32_t key = (hi * two16 + lo) * tile + slot;
+                    second[k] = min_u16x2(second[k], max_u16x2(best[k], key));
+                    best[k] = min_u16x2(best[k], key);
                 }
             }
             // resolve this tile's winners to packed ids before the tile is overwritten
-            if (best[0] != prev0) bidx[0] = s_id[best[0] & 255u];
-            if (best[1] != prev1) bidx[1] = s_id[best[1] & 255u];
+#pragma unroll
+            for (int k = 0; k < KB_PAIRS; ++k) {
+                const uint32_t diff = best[k] ^ prev[k];
+                if (diff & 0xffffu) bidx[2 * k] = s_id[best[k] & (uint32_t)(KB_TILE - 1)];
+                if (diff >> 16) bidx[2 * k + 1] = s_id[(best[k] >> 16) & (uint32_t)(KB_TILE - 1)];
+            }
         }
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
+        for (int k = 0; k < KB_Q; ++k) {
             if (!qv[k]) continue;
             const size_t q = (size_t)ql[k] * A.cap + qi[k];
-            if (nsplit == 1u) {
-                const int32_t res =
-                    (nt >= 2u && bidx[k] >= 0 && (float)(best[k] >> 8) < ratio * (float)(second[k] >> 8)) ? bidx[k]
-                                                                                                          : -1;
+            // distances; all ones: none
+            const uint32_t bk = (best[k / 2] >> (16 * (k & 1))) & 0xffffu, sk = (second[k / 2] >> (16 * (k & 1))) & 0xffffu;
+            const uint32_t bd = bk == 0xffffu ? 0xffffffu : bk / KB_TILE, sd = sk == 0xffffu ? 0xffffffu : sk / KB_TILE;
+            if (u.parts == 1u && P.bf_part == nullptr) {
+                const int32_t res = (nt >= 2u && bidx[k] >= 0 && (float)bd < ratio * (float)sd) ? bidx[k] : -1;
                 P.a2b[q] = res;
             } else {
-                // partial record of this split; the emit kernel merges the splits
-                const size_t stride = (size_t)A.levels * A.cap;
-                *reinterpret_cast<uint4*>(P.bf_part + (split * stride + q) * 4u) =
-                    make_uint4(best[k], second[k], (uint32_t)bidx[k], 0u);
+                bf_record(u, (size_t)A.levels * A.cap, q, bd, sd, bidx[k]);
             }
         }
         __syncthreads();  // s_qpre / s_tpre are rewritten by the next work unit
@@ -2546,38 +2595,66 @@ k_mutual(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pairs,
     const uint32_t n = A.kept[l];
     int32_t* const a2b = P.a2b + (size_t)l * A.cap;
     uint32_t base = 0;
+    uint32_t nt = 0;  // the train set of the brute-force matchers
+    if (!MUTUAL)
+        for (int q = 0; q < B.levels; ++q) nt += B.kept[q];
     for (uint32_t c0 = 0; c0 < n; c0 += KU_THREADS * KU_ITEMS) {
         int32_t m[KU_ITEMS];
+        if (MUTUAL || P.bf_part == nullptr) {
 #pragma unroll
-        for (int u = 0; u < KU_ITEMS; ++u) {
-            const uint32_t i = c0 + u * KU_THREADS + threadIdx.x;
-            m[u] = -1;
-            if (i >= n) continue;
-            if (!MUTUAL && P.bf_splits > 1) {
-                // merge the brute-force splits: the two smallest distances of the
-                // union of the splits' (best, second) pairs; a tie on the best
-                // leaves second == best, which fails the ratio test
-                uint32_t bd = 0xffffffffu, sd = 0xffffffffu;
-                int32_t bi = -1;
-                const size_t stride = (size_t)A.levels * A.cap;
-                for (int sp = 0; sp < P.bf_splits; ++sp) {
-                    const uint4 e = *reinterpret_cast<const uint4*>(P.bf_part +
-                                                                    (sp * stride + (size_t)l * A.cap + i) * 4u);
-                    const uint32_t b = e.x >> 8, c = e.y >> 8;
-                    if (b < bd) {
-                        sd = min(bd, c);
-                        bd = b;
-                        bi = (int32_t)e.z;
-                    } else {
-                        sd = min(sd, b);
+            for (int u = 0; u < KU_ITEMS; ++u) {
+                const uint32_t i = c0 + u * KU_THREADS + threadIdx.x;
+                m[u] = i < n && (MUTUAL || nt >= 2u) ? a2b[i] : -1;  // nt: the pool rule
+            }
+        } else {
+            // merge the parts of each query's block: the two smallest distances
+            // of the union of their (best, second) pairs; a tie on the best
+            // leaves second == best, which fails the ratio test.  The records
+            // of four items are in flight together.
+            const size_t stride = (size_t)A.levels * A.cap;
+#pragma unroll
+            for (int h = 0; h < KU_ITEMS; h += 4) {
+                const uint4* rec[4];
+                uint4 e[4];
+                uint32_t bd[4], sd[4];
+                int32_t bi[4], parts[4], most = 1;
+#pragma unroll
+                for (int v = 0; v < 4; ++v) {
+                    const uint32_t i = c0 + (h + v) * KU_THREADS + threadIdx.x;
+                    const bool any = i < n && nt >= 2u;  // the pool rule; such a pair may have no records
+                    rec[v] = reinterpret_cast<const uint4*>(P.bf_part) + (size_t)l * A.cap + (any ? i : 0u);
+                    e[v] = any ? *rec[v] : make_uint4(~0u, ~0u, ~0u, 0u);
+                }
+#pragma unroll
+                for (int v = 0; v < 4; ++v) {
+                    bd[v] = e[v].x >> 8;
+                    sd[v] = e[v].y >> 8;
+                    bi[v] = (int32_t)e[v].z;
+                    parts[v] = min((int)e[v].w, P.bf_splits);
+                    most = max(most, parts[v]);
+                }
+                for (int sp = 1; sp < most; ++sp) {
+#pragma unroll
+                    for (int v = 0; v < 4; ++v)
+                        e[v] = sp < parts[v] ? rec[v][sp * stride] : make_uint4(~0u, ~0u, ~0u, 0u);
+#pragma unroll
+                    for (int v = 0; v < 4; ++v) {
+                        const uint32_t b = e[v].x >> 8, c = e[v].y >> 8;
+                        if (b < bd[v]) {
+                            sd[v] = min(bd[v], c);
+                            bd[v] = b;
+                            bi[v] = (int32_t)e[v].z;
+                        } else {
+                            sd[v] = min(sd[v], b);
+                        }
                     }
                 }
-                uint32_t nt = 0;
-                for (int q = 0; q < B.levels; ++q) nt += B.kept[q];
-                m[u] = (nt >= 2u && bi >= 0 && (float)bd < P.bf_ratio * (float)sd) ? bi : -1;
-                a2b[i] = m[u];
-            } else {
-                m[u] = a2b[i];
+#pragma unroll
+                for (int v = 0; v < 4; ++v) {
+                    const uint32_t i = c0 + (h + v) * KU_THREADS + threadIdx.x;
+                    m[h + v] = bi[v] >= 0 && (float)bd[v] < P.bf_ratio * (float)sd[v] ? bi[v] : -1;
+                    if (i < n) a2b[i] = m[h + v];
+                }
             }
         }
         uint32_t ok = 0u;  // bit u: item u is a match
@@ -2835,9 +2912,10 @@ cudaError_t launch_emit(const FrameDev* frames, const PairDev* pairs, const SegD
 }
 
 cudaError_t launch_bruteforce(const FrameDev* frames, const PairDev* pairs, const SegDev* psegs, int npairs,
-                              float ratio, int grid, cudaStream_t st) {
+                              float ratio, int sms, cudaStream_t st) {
     if (npairs <= 0) return cudaSuccess;
-    k_bruteforce<<<grid, KB_THREADS, 0, st>>>(frames, pairs, psegs, npairs, ratio);
+    static_assert((MAX_SEGS + 1) * 8 <= 40 * 1024, "the pairs' table fits the default limit beside the tile");
+    k_bruteforce<<<sms * KB_CTAS, KB_THREADS, (npairs + 1) * sizeof(unsigned long long), st>>>(frames, pairs, psegs, npairs, ratio, 2u);
     return cudaGetLastError();
 }
 

@@ -270,10 +270,9 @@ cudaError_t enqueue_pairs(uslam_batch* b, const Program& P, const Lane& ln) {
     uslam_ctx* c = b->ctx;
     cudaError_t e = cudaSuccess;
     if (P.nmsegs <= 0) return e;
-    const int grid = c->num_sms * 4;
     if (c->matcher != 0) {
         if (c->matcher == 1)
-            e = launch_bruteforce(b->d_frames, b->d_pairs, P.psegs, P.npsegs, c->ratio, grid, ln.st);
+            e = launch_bruteforce(b->d_frames, b->d_pairs, P.psegs, P.npsegs, c->ratio, c->num_sms, ln.st);
         else
             e = launch_bf_mma(b->d_frames, b->d_pairs, P.psegs, P.npsegs, c->ratio, c->num_sms, b->d_err, ln.st);
         if (e != cudaSuccess) return e;
@@ -523,36 +522,25 @@ uslam_status create_batch(uslam_ctx* ctx, int n_frames, const int* widths, const
         P.bf_splits = 1;
         P.bf_ratio = ctx->ratio;
     }
-    // Both brute-force matchers take 256 queries per work unit.  Matcher 1
-    // runs about 8 CTAs per SM: split each train set until the launch has
-    // that many units.  Matcher 2 runs one CTA per SM: pick the smallest
-    // split (<= 8) whose units fill at least 95 % of whole waves over the SMs.
+    // The brute-force matchers share their work out in equal parts, which cut
+    // query blocks (bf_line.h): records for as many parts of a block as
+    // equal shares make at least one block a pair, up to a limit (a single
+    // pair's blocks are cut into 32 parts by matcher 1, whose launch has 8
+    // CTAs per SM, and 16 by matcher 2), in at most 1 GiB; with more pairs
+    // than that a launch has blocks enough, and they stay whole.
     std::vector<size_t> bf_off(n_pairs, 0);
     if (ctx->matcher == 2 && n_pairs > 1024) {
         free_batch(b);
         return set_err(&ctx->err, USLAM_CAPACITY, "batch_create: the tensor-core matcher takes at most 1024 pairs per batch");
     }
     if (ctx->matcher != 0 && n_pairs > 0) {
-        size_t units = 0;
-        for (int p = 0; p < n_pairs; ++p)
-            units += (static_cast<size_t>(L) * std::max(b->frames[pair_prev[p]].cap, 1) + 255) / 256;
-        const size_t sms = static_cast<size_t>(std::max(ctx->num_sms, 1));
-        int splits = 1;
-        if (ctx->matcher == 1) {
-            const size_t target = sms * 8;
-            splits = static_cast<int>(std::min<size_t>(16, std::max<size_t>(1, (target + units - 1) / units)));
-        } else {
-            double best_eff = 0.0;
-            for (int sp = 1; sp <= 8; ++sp) {
-                const size_t u = units * static_cast<size_t>(sp);
-                const double eff = static_cast<double>(u) / static_cast<double>((u + sms - 1) / sms * sms);
-                if (eff > best_eff + 1e-9) {
-                    best_eff = eff;
-                    splits = sp;
-                }
-                if (eff >= 0.95) break;
-            }
-        }
+        size_t queries = 0;  // of one part's records
+        for (int p = 0; p < n_pairs; ++p) queries += static_cast<size_t>(L) * std::max(b->frames[pair_prev[p]].cap, 1);
+        const size_t ctas = static_cast<size_t>(std::max(ctx->num_sms, 1)) * (ctx->matcher == 1 ? 8 : 1);
+        const size_t pairs = static_cast<size_t>(n_pairs);
+        size_t parts = pairs > 4 * ctas ? 1 : std::min<size_t>(ctas / pairs + 2, ctx->matcher == 1 ? 32 : 16);
+        while (parts > 1 && parts * queries * 16 > (size_t{1} << 30)) --parts;
+        const int splits = static_cast<int>(parts);
         if (splits > 1)
             for (int p = 0; p < n_pairs; ++p) {
                 b->pairs[p].bf_splits = splits;
@@ -1199,7 +1187,6 @@ uslam_status uslam_batch_profile(uslam_batch* b, int iters, float* kernel_ms) {
     cudaError_t e = cudaSuccess;
     for (int i = 0; i <= K && e == cudaSuccess; ++i) e = cudaEventCreate(&ev[i]);
     double acc[K] = {0, 0, 0, 0, 0, 0, 0};
-    const int grid = c->num_sms * 4;
     for (int it = 0; it < iters && e == cudaSuccess; ++it) {
         int k = 0;
         auto mark = [&]() {
@@ -1225,7 +1212,7 @@ uslam_status uslam_batch_profile(uslam_batch* b, int iters, float* kernel_ms) {
         if (e == cudaSuccess && c->matcher == 0 && !b->win_tc)
             e = launch_bacc_init(b->d_frames, b->d_pairs, P.usegs, P.nusegs, b->stream);
         if (e == cudaSuccess)
-            e = c->matcher == 1 ? launch_bruteforce(b->d_frames, b->d_pairs, P.psegs, P.npsegs, c->ratio, grid, b->stream)
+            e = c->matcher == 1 ? launch_bruteforce(b->d_frames, b->d_pairs, P.psegs, P.npsegs, c->ratio, c->num_sms, b->stream)
                 : c->matcher == 2
                     ? launch_bf_mma(b->d_frames, b->d_pairs, P.psegs, P.npsegs, c->ratio, c->num_sms, b->d_err, b->stream)
                 : b->win_tc ? launch_win_match(b->d_frames, b->d_pairs, P.msegs, P.nmsegs, b->win_umax, P.units,

@@ -121,10 +121,10 @@ struct PairDev {
     uint32_t* match_count;  // [levels] matches whose a lies in that level
     int max_matches_per_level;
     float max_dx, max_dy;   // 0.1f * W0, 0.1f * H0 of the frame size
-    // brute-force matcher split over the train set: bf_splits partial top-2
-    // records (best key, second key, best id, unused) per query, at
-    // bf_part[(split * levels * cap_prev + level * cap_prev + index) * 4];
-    // unused (nullptr, 1) when the train set is not split
+    // brute-force matchers: records of the parts of a query block's train set,
+    // (best distance << 8, second << 8, best id, number of parts) per query at
+    // bf_part[(part * levels * cap_prev + level * cap_prev + index) * 4], for
+    // up to bf_splits parts; (nullptr, 1) where blocks are not cut
     uint32_t* bf_part;
     int bf_splits;
     float bf_ratio;
