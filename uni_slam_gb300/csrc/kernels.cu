@@ -1893,30 +1893,17 @@ __device__ __forceinline__ uint32_t lop3(uint32_t a, uint32_t b, uint32_t c) {
 }
 
 // ------------------------------------------------- Hamming distance ----
-// popcount(a ^ b) over 256 bits with 4 POPC instead of 8: three carry-save
-// adders fold x0..x6 into ones (o3) and twos (t1, t2, t3), a fourth folds
-// the twos into twos (tw) and fours (f); x7 is added as ones.  Per bit
+// popcount(a ^ b) over 256 bits with 4 POPC instead of 8: with x = a ^ b, three
+// carry-save adders fold x0..x6 into ones (o3) and twos (t1, t2, t3), a fourth
+// folds the twos into twos (tw) and fours (f); x7 is added as ones.  Per bit
 // position x0 + .. + x7 = o3 + x7 + 2 tw + 4 f, so the sum of the weighted
 // popcounts is the exact distance (integer arithmetic, no rounding).
-// POPC issues at a quarter of the ALU rate, so this trades 4 POPC for
-// 8 LOP3.
-__device__ __forceinline__ uint32_t hamming256(const uint4& a0, const uint4& a1, const uint4& b0, const uint4& b1) {
-    const uint32_t x0 = a0.x ^ b0.x, x1 = a0.y ^ b0.y, x2 = a0.z ^ b0.z, x3 = a0.w ^ b0.w;
-    const uint32_t x4 = a1.x ^ b1.x, x5 = a1.y ^ b1.y, x6 = a1.z ^ b1.z, x7 = a1.w ^ b1.w;
-    const uint32_t o1 = lop3<0x96>(x0, x1, x2), t1 = lop3<0xe8>(x0, x1, x2);
-    const uint32_t o2 = lop3<0x96>(o1, x3, x4), t2 = lop3<0xe8>(o1, x3, x4);
-    const uint32_t o3 = lop3<0x96>(o2, x5, x6), t3 = lop3<0xe8>(o2, x5, x6);
-    const uint32_t tw = lop3<0x96>(t1, t2, t3), f = lop3<0xe8>(t1, t2, t3);
-    return (uint32_t)__popc(o3) + (uint32_t)__popc(x7) + 2u * (uint32_t)__popc(tw) + 4u * (uint32_t)__popc(f);
-}
-
-// The same between descriptors in the form of parity_words, 13 logic operations
-// instead of 16: a full adder's third input is not needed beside its sum
-// (carry = x y | (x ^ y) ~sum), and the sums of words of a ^ b are the
-// differences of the descriptors' own, kept in the third inputs' place.  The
-// weighted sum runs on the multiply-add pipe: two is 2 in a register the
-// compiler does not see through (of a constant it makes shifted adds, which
-// run on the ALU pipe beside the logic).
+// 13 logic operations: both descriptors are in the form of parity_words, whose
+// third inputs are replaced by the sums of words, so that the adders' sums o1,
+// o2, o3 are differences of words, and a carry is taken from two inputs and
+// the sum (x y | (x ^ y) ~o).  The weighted sum runs on the multiply-add pipe:
+// two is 2 in a register the compiler does not see through (of a constant it
+// makes shifted adds, which run on the ALU pipe beside the logic).
 __device__ __forceinline__ void parity_words(uint4& d0, uint4& d1) {
     d0.z = d0.x ^ d0.y ^ d0.z;
     d1.x = d0.z ^ d0.w ^ d1.x;
@@ -1992,25 +1979,26 @@ __device__ __forceinline__ uint32_t min_u16x2(uint32_t a, uint32_t b) {
     asm("min.u16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
     return r;
 }
+// Byte i = eight copies of the sign bit of byte (SEL >> 4 i) & 7 (the
+// selector's upper bit asks for the sign; the __byte_perm function drops it).
+template <int SEL>
+__device__ __forceinline__ uint32_t byte_signs(uint32_t v) {
+    static_assert((SEL & 0x8888) == 0x8888, "signs");
+    uint32_t r;
+    asm("prmt.b32 %0, %1, 0, %2;" : "=r"(r) : "r"(v), "n"(SEL));
+    return r;
+}
 __device__ __forceinline__ uint32_t max_u16x2(uint32_t a, uint32_t b) {
     uint32_t r;
     asm("max.u16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
     return r;
 }
 
-// Bits [lo, hi) of a staged batch that starts at list position base.
-__device__ __forceinline__ uint32_t range_bits(uint32_t lo, uint32_t hi, uint32_t base) {
-    const int a = (int)(max(lo, base) - base);
-    const int b = (int)(min(hi, base + 32u) > base ? min(hi, base + 32u) - base : 0u);
-    const uint32_t lo_mask = a >= 32 ? 0u : (0xffffffffu << a);
-    const uint32_t hi_mask = b >= 32 ? 0xffffffffu : ((1u << b) - 1u);
-    return lo_mask & hi_mask;
-}
-
 // One warp's staging area: 32 candidates (LOD-0 y, packed (level, index),
 // descriptor halves), the packed (level, index) of each lane's query, and the
-// batch's column keys: col[t * 32 + lane] = distance << 5 | lane for a hit of
-// slot t by lane, all ones otherwise.
+// batch's column keys, two candidates in a word: halves 2 p and 2 p + 1 of
+// col[p * 32 + lane] = distance << 5 | lane where lane's query meets candidate
+// 2 p (2 p + 1), all ones otherwise.
 struct CandBuf {
     float py[32];
     int32_t idx[32];
@@ -2019,7 +2007,7 @@ struct CandBuf {
 struct CandStage {
     CandBuf buf[2];
     uint32_t qid[32];
-    uint16_t col[32 * 32];
+    uint32_t col[16 * 32];
 };
 constexpr int KM_MAX_SEGS = USLAM_MAX_MATCH_SEGS;
 
@@ -2147,20 +2135,25 @@ __global__ void __launch_bounds__(256) k_match_order(uint32_t* claim, const uint
 //    inside a's window, and [n0, n1), the b whose window holds a (the same
 //    features except where f32 rounding at the window's x edge differs);
 //    the y test |ya - yb| <= 0.1 H0 is the same both ways;
-//  * a lane keeps a's two smallest keys (distance << 5 | slot) in registers,
-//    and writes the key distance << 5 | lane of each hit into the column of
-//    its slot; after the batch lane t folds column t into b's two smallest
-//    and merges them into b's accumulator in HBM (atomic minimum of
+//  * a lane takes the distances to all candidates of the batch (about half of
+//    them are hits: picking those out, each lane its own, took more
+//    instructions and the shared memory's time in bank conflicts), two to a
+//    word with all ones in place of the others; it keeps a's two smallest keys
+//    (distance << 5 | slot) in registers and writes the keys distance << 5 |
+//    lane to the candidate's column; after the batch lane t folds column t
+//    into b's two smallest and merges them into b's accumulator in HBM (atomic minimum of
 //    (distance, packed a), then of the second distance), where the batches
 //    of every query group that meets b meet;
 //  * a2b is written per query group; k_mutual reads b's accumulator.
+// The logic and popcount pipes bound it (ALU 68 %, XU 47 %, shared memory 43 %
+// busy); 32 pairs of 752x480 frames: 318 us picking hits, 283 us so.
 // A tied best leaves the second distance equal to the best, which fails the
 // ratio test, so no result depends on the order of the candidates or of the
 // merges.  The pool rule (fewer than two candidates: no match) is applied to
 // a here and to b in k_mutual.
 __global__ void __launch_bounds__(KM_THREADS, KM_CTAS_PER_SM)
 k_match(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pairs,
-        const MatchSegDev* __restrict__ segs, int nseg, uint32_t* claim_block) {
+        const MatchSegDev* __restrict__ segs, int nseg, uint32_t* claim_block, uint32_t two) {
     __shared__ uint32_t s_pref[KM_MAX_SEGS + 1];
     __shared__ uint32_t s_warp[33];
     __shared__ __align__(16) CandStage s_stage[KM_THREADS / 32];
@@ -2175,12 +2168,17 @@ k_match(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pairs,
     const int gw = blockIdx.x * (KM_THREADS / 32) + warp;
     const int nw = gridDim.x * (KM_THREADS / 32);
     CandStage& S = s_stage[warp];
-    {
-        // the column keys start empty; each column pass empties its column again
-        uint4* c = reinterpret_cast<uint4*>(S.col);
-        for (int k = lane; k < (int)(sizeof(S.col) / 16); k += 32) c[k] = make_uint4(~0u, ~0u, ~0u, ~0u);
-        __syncwarp();
+    const uint32_t one = two >> 1, n32 = two << 4, n64k = two << 15;
+    // s_first[n]: the bits of the first n candidates of a batch.  Candidate i has
+    // bit 8 (i % 4) + 7 - i / 4, so that after q shifts to the left candidates
+    // 4 q .. 4 q + 3 have the bytes' signs, which a byte permute spreads.
+    __shared__ uint32_t s_first[33];
+    if (threadIdx.x < 33) {
+        uint32_t m = 0u;
+        for (int i = 0; i < (int)threadIdx.x; ++i) m |= 1u << (8 * (i & 3) + 7 - (i >> 2));
+        s_first[threadIdx.x] = m;
     }
+    __syncthreads();
     // Query groups cost very different amounts (the hits in their windows).
     // With a claim block (its counter zeroed before the launch, its order
     // written by k_match_rank / k_match_order) a warp claims the next group of
@@ -2212,21 +2210,23 @@ k_match(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pairs,
         const float ql = lod_scale(l);
         const float cx = (float)(uint32_t)__uint_as_float(qrec[0]) * ql;
         const float cy = (float)(uint32_t)__uint_as_float(qrec[1]) * ql;
-        const uint4 qd0 = *reinterpret_cast<const uint4*>(qrec + 4);
-        const uint4 qd1 = *reinterpret_cast<const uint4*>(qrec + 8);
+        uint4 qd0 = *reinterpret_cast<const uint4*>(qrec + 4);
+        uint4 qd1 = *reinterpret_cast<const uint4*>(qrec + 8);
+        parity_words(qd0, qd1);
         const float dx = P.max_dx, dy = P.max_dy;
         const float lo = cx - dx, hi = cx + dx;
         S.qid[lane] = (uint32_t)USLAM_PACK(l, qi);
         __syncwarp();
 
-        // a's best / second-best as keys (distance << 5 | slot); a tie on the
+        // a's best / second-best as 16-bit keys (distance << 5 | slot); a tie on the
         // best distance leaves second >> 5 == best >> 5, which fails the test
-        uint32_t bestk = 0xffffffffu, secondk = 0xffffffffu;
+        uint32_t bestk = 0xffffu, secondk = 0xffffu;
         int32_t bidx = -1;
         const int L = B.levels;
         uint4* const bacc = P.bacc;
         const size_t capb = (size_t)(B.cap > 0 ? B.cap : 1);
-        uint16_t* const colq = S.col + lane;  // this lane's key of slot t at colq[32 t]
+        uint32_t* const colq = S.col + lane;
+        const uint32_t lanes = (uint32_t)lane * 0x10001u;
         for (int k = 0; k < 3; ++k) {
             const int pl = k == 0 ? l : (k == 1 ? l - 1 : l + 1);
             if (pl < 0 || pl >= L) continue;
@@ -2298,74 +2298,72 @@ k_match(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pairs,
                     cp_async_wait<1>();
                     // the staged word is the record's f32 y; the LOD-0 y as in
                     // match_features_cpu.cpp:58-64
-                    if (kk < c1) SB.py[lane] = (float)(uint32_t)SB.py[lane] * ps;
+                    if (kk < c1) {
+                        SB.py[lane] = (float)(uint32_t)SB.py[lane] * ps;
+                        uint4 d0 = SB.d0[lane], d1 = SB.d1[lane];
+                        parity_words(d0, d1);
+                        SB.d0[lane] = d0;
+                        SB.d1[lane] = d1;
+                    }
                 }
                 __syncwarp();
-                // y test of all 32 staged candidates (unrolled, float4 loads);
-                // slots past the list's end lie outside both ranges
-                uint32_t ymask = 0u;
+                // |ya - yb| > dy of all 32 staged candidates, as the sign of
+                // dy - |ya - yb| (exact) shifted in: one ALU operation each.
+                // Candidates past the list's end lie outside both ranges.
+                uint32_t f0 = 0u, f1 = 0u, f2 = 0u, f3 = 0u;
                 const float4* py4 = reinterpret_cast<const float4*>(SB.py);
 #pragma unroll
                 for (int q = 0; q < 8; ++q) {
                     const float4 v = py4[q];
-                    ymask |= (!(fabsf(cy - v.x) > dy) ? 1u : 0u) << (4 * q);
-                    ymask |= (!(fabsf(cy - v.y) > dy) ? 1u : 0u) << (4 * q + 1);
-                    ymask |= (!(fabsf(cy - v.z) > dy) ? 1u : 0u) << (4 * q + 2);
-                    ymask |= (!(fabsf(cy - v.w) > dy) ? 1u : 0u) << (4 * q + 3);
+                    f0 = __funnelshift_l(__float_as_uint(dy - fabsf(cy - v.x)), f0, 1);
+                    f1 = __funnelshift_l(__float_as_uint(dy - fabsf(cy - v.y)), f1, 1);
+                    f2 = __funnelshift_l(__float_as_uint(dy - fabsf(cy - v.z)), f2, 1);
+                    f3 = __funnelshift_l(__float_as_uint(dy - fabsf(cy - v.w)), f3, 1);
                 }
-                const uint32_t h1 = ymask & range_bits(m0, m1, base);  // b in a's window
-                const uint32_t h0 = ymask & range_bits(n0, n1, base);  // a in b's window
-                const uint32_t prev = bestk;
-                uint32_t hb = h1 & h0;
-                if (hb) {
-                    // the next hit's descriptor is read while this one's
-                    // distance is computed
-                    int t = 31 - __clz(hb);
-                    hb ^= 1u << t;
-                    uint4 c0d = SB.d0[t], c1d = SB.d1[t];
-                    while (true) {
-                        const int tn = hb ? 31 - __clz(hb) : t;
-                        const uint4 n0d = SB.d0[tn], n1d = SB.d1[tn];
-                        const uint32_t d = hamming256(c0d, c1d, qd0, qd1);
-                        const uint32_t key = (d << 5) | (uint32_t)t;
-                        secondk = min(secondk, max(bestk, key));
-                        bestk = min(bestk, key);
-                        colq[32 * t] = (uint16_t)((d << 5) | (uint32_t)lane);
-                        if (!hb) break;
-                        hb ^= 1u << tn;
-                        t = tn;
-                        c0d = n0d;
-                        c1d = n1d;
+                const uint32_t far = __byte_perm(__byte_perm(f0, f1, 0x0040), __byte_perm(f2, f3, 0x0040), 0x5410);
+                auto first = [&](uint32_t upto) { return s_first[min(max(upto, base) - base, 32u)]; };
+                // candidates that are no hit: b outside a's window, a outside b's
+                uint32_t no1 = ~first(m1) | first(m0) | far, no0 = ~first(n1) | first(n0) | far;
+                uint32_t b2 = 0xffffffffu, s2 = 0xffffffffu, slots = 0x10000u;
+                const int quads = (int)(min(c1 - base, 32u) + 3u) >> 2;
+#pragma unroll 1
+                for (int q = 0; q < quads; ++q) {
+                    const uint4 *p0 = SB.d0 + 4 * q, *p1 = SB.d1 + 4 * q;
+                    const uint32_t dA = hamming256_parity(p0[1], p1[1], qd0, qd1, two, one) * n64k +
+                                        hamming256_parity(p0[0], p1[0], qd0, qd1, two, one);
+                    const uint32_t dB = hamming256_parity(p0[3], p1[3], qd0, qd1, two, one) * n64k +
+                                        hamming256_parity(p0[2], p1[2], qd0, qd1, two, one);
+                    const uint32_t rA = (dA * n32 + slots) | byte_signs<0x9988>(no1);
+                    const uint32_t rB = (dB * n32 + (slots + 0x20002u)) | byte_signs<0xbbaa>(no1);
+                    s2 = min_u16x2(s2, max_u16x2(b2, rA));
+                    b2 = min_u16x2(b2, rA);
+                    s2 = min_u16x2(s2, max_u16x2(b2, rB));
+                    b2 = min_u16x2(b2, rB);
+                    colq[64 * q] = (dA * n32 + lanes) | byte_signs<0x9988>(no0);
+                    colq[64 * q + 32] = (dB * n32 + lanes) | byte_signs<0xbbaa>(no0);
+                    no1 += no1;
+                    no0 += no0;
+                    slots += 0x40004u;
+                }
+                {
+                    const uint32_t bl = b2 & 0xffffu, bh = b2 >> 16, bb = min(bl, bh);
+                    const uint32_t ss = min(max(bl, bh), min(s2 & 0xffffu, s2 >> 16));
+                    secondk = min(min(secondk, ss), max(bestk, bb));
+                    if (bb < bestk) {
+                        bestk = bb;
+                        bidx = SB.idx[bb & 31u];
                     }
                 }
-                // pairs inside one direction's window only (rare)
-                uint32_t o1 = h1 & ~h0, o0 = h0 & ~h1;
-                if (__any_sync(0xffffffffu, (o1 | o0) != 0u)) {
-                    while (o1) {
-                        const int t = 31 - __clz(o1);
-                        o1 ^= 1u << t;
-                        const uint32_t key = (hamming256(SB.d0[t], SB.d1[t], qd0, qd1) << 5) | (uint32_t)t;
-                        secondk = min(secondk, max(bestk, key));
-                        bestk = min(bestk, key);
-                    }
-                    while (o0) {
-                        const int t = 31 - __clz(o0);
-                        o0 ^= 1u << t;
-                        colq[32 * t] = (uint16_t)((hamming256(SB.d0[t], SB.d1[t], qd0, qd1) << 5) | (uint32_t)lane);
-                    }
-                }
-                if (bestk != prev) bidx = SB.idx[bestk & 31u];
                 __syncwarp();
-                // column pass: lane t folds the keys of slot t into the two
-                // smallest (two 16-bit lanes at a time), empties the column
-                // and merges the pair into b's accumulator
-                if (kk < c1) {
-                    uint4* colt = reinterpret_cast<uint4*>(S.col + 32 * lane);
-                    uint32_t b2 = 0xffffffffu, s2 = 0xffffffffu;
+                // column pass: lanes 2 p and 2 p + 1 fold a half of the queries' keys of
+                // candidates 2 p and 2 p + 1 into the two smallest each, and
+                // lane t merges candidate t's into b's accumulator
+                {
+                    const uint4* colt = reinterpret_cast<const uint4*>(S.col + 16 * lane);
+                    b2 = s2 = 0xffffffffu;
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
-                        const uint4 v = colt[q];
-                        colt[q] = make_uint4(~0u, ~0u, ~0u, ~0u);
+                        const uint4 v = colt[(q + (lane >> 1)) & 3];  // no two lanes of a quarter warp in one bank
                         s2 = min_u16x2(s2, max_u16x2(b2, v.x));
                         b2 = min_u16x2(b2, v.x);
                         s2 = min_u16x2(s2, max_u16x2(b2, v.y));
@@ -2375,10 +2373,11 @@ k_match(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pairs,
                         s2 = min_u16x2(s2, max_u16x2(b2, v.w));
                         b2 = min_u16x2(b2, v.w);
                     }
-                    const uint32_t bl = b2 & 0xffffu, bh = b2 >> 16;
-                    const uint32_t cb = min(bl, bh);
-                    const uint32_t cs = min(max(bl, bh), min(s2 & 0xffffu, s2 >> 16));
-                    if (cb != 0xffffu) {
+                    const uint32_t ob = __shfl_xor_sync(0xffffffffu, b2, 1), os = __shfl_xor_sync(0xffffffffu, s2, 1);
+                    s2 = min_u16x2(min_u16x2(s2, os), max_u16x2(b2, ob));
+                    b2 = min_u16x2(b2, ob);
+                    const uint32_t cb = lane & 1 ? b2 >> 16 : b2 & 0xffffu, cs = lane & 1 ? s2 >> 16 : s2 & 0xffffu;
+                    if (kk < c1 && cb != 0xffffu) {
                         const unsigned long long key =
                             ((unsigned long long)(cb >> 5) << 32) | (unsigned long long)S.qid[cb & 31u];
                         const int32_t id = SB.idx[lane];
@@ -2863,7 +2862,7 @@ cudaError_t launch_match(const FrameDev* frames, const PairDev* pairs, const voi
                          cudaStream_t st) {
     if (nseg <= 0) return cudaSuccess;
     k_match<<<num_sms * KM_CTAS_PER_SM, KM_THREADS, 0, st>>>(frames, pairs, static_cast<const MatchSegDev*>(segs), nseg,
-                                                              nullptr);
+                                                              nullptr, 2u);
     return cudaGetLastError();
 }
 // The claim order (k_match_rank, k_match_order), then k_match claiming from
@@ -2880,7 +2879,7 @@ cudaError_t launch_match_dyn(const FrameDev* frames, const PairDev* pairs, const
     if (e != cudaSuccess) return e;
     k_match_order<<<num_sms, 256, 0, st>>>(claim, gbucket);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    k_match<<<num_sms * KM_CTAS_PER_SM, KM_THREADS, 0, st>>>(frames, pairs, ms, nseg, claim);
+    k_match<<<num_sms * KM_CTAS_PER_SM, KM_THREADS, 0, st>>>(frames, pairs, ms, nseg, claim, 2u);
     return cudaGetLastError();
 }
 

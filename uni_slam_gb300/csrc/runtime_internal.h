@@ -241,15 +241,15 @@ inline cudaError_t launch_detect_shaped(const FrameDev* frames, const TileItem* 
 // Horizontal bands of the matcher's lists for levels of up to cap features.
 // A band's lists hold the rows of its queries and 0.1 H each side, so more
 // bands leave fewer candidates outside the windows, but a group of 32 queries
-// (128 with the tensor cores) then reaches further in x.  Measured with 2, 3,
-// 4, 6, 8, 12, 16 and 24 bands: 64 frames of 752x480 (cap 1443) 1.59, 1.60,
-// 1.61, 1.62, 1.68 ... ms a step; the mixed batch up to 3840x2160 (cap 33177)
-// 6.13, 5.67, 5.54, 5.42, 5.38, 5.42, 5.52, 5.76 ms; one 1920x1080 frame on the
-// tensor cores 790, 767, 753, 769, 765, 841 ... us, one 752x480 frame 307, 305,
-// 310, 316 ... us.
+// (128 with the tensor cores) then reaches further in x.  Measured with k_match:
+// 64 frames of 752x480 (cap 1443) with 3, 4, 5, 6 and 8 bands 1455, 1427, 1443,
+// 1460, 1519 us a step; the mixed batch (caps 1228, 1443, 3686, 8294, 33177) with
+// 3/4/6/10 bands 4757, 3/4/8/14 4703, 3/6/10/14 4688, 3/6/10/20 4698 us.  On the
+// tensor cores: one 1920x1080 frame with 2, 3, 4, 6, 8, 12 bands 790, 767, 753, 769,
+// 765, 841 us, one 752x480 frame 307, 305, 310, 316 ... us.
 inline int match_bands_for(int cap, bool win_tc) {
     if (win_tc) return cap > 5000 ? 4 : 3;
-    return cap > 16000 ? 10 : cap > 5000 ? 6 : cap > 2500 ? 4 : 3;
+    return cap > 16000 ? 14 : cap > 5000 ? 10 : cap > 2500 ? 6 : 4;
 }
 
 // Blur tiles of every level of a frame (the most k_band_write can list).
