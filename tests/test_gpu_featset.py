@@ -83,3 +83,33 @@ def test_last_error_from_many_threads(brief_pattern):
             fs.close()
         assert set(statuses) == {capi.NOT_READY}
         assert set(msgs) == {b"featset_features: nothing detected yet"}
+
+
+@pytest.mark.parametrize("matcher", [0, 1, 2])
+def test_sets_matched_in_place(matcher):
+    """The match reads the sets where they are: a set with itself, sets that
+    are detected again or destroyed between matches, and an empty one."""
+    pat = np.clip(np.rint(np.random.RandomState(5).normal(0, 6, (256, 4))), -13, 13).astype(np.int32)
+    frames = list(synth.warped_pair(23, 320, 240)) + [synth.scene_frame(4, 320, 240), np.full((240, 320), 60, np.uint8)]
+    exp = [oracle.frame(f, pat) for f in frames]
+
+    def want(i, j):
+        a, b = exp[i], exp[j]
+        return oracle.match_bruteforce(a[0], a[1], b[0], b[1], 0.8) if matcher else oracle.match(a[0], a[1], b[0], b[1], 320, 240)
+
+    with Context(pat, levels=6, max_width=320, max_height=240, matcher=matcher, ratio=0.8) as c:
+        a, b = FeatureSet(c, 320, 240), FeatureSet(c, 320, 240)
+        a.detect(frames[0])
+        b.detect(frames[1])
+        assert np.array_equal(_mm(c.match(a, b)), want(0, 1)) and len(want(0, 1)) > 50
+        assert np.array_equal(_mm(c.match(b, b)), want(1, 1))
+        a.detect(frames[2])
+        assert np.array_equal(_mm(c.match(b, a)), want(1, 2))
+        b.close()
+        b = FeatureSet(c, 320, 240)
+        b.detect(frames[3])
+        assert np.array_equal(_mm(c.match(a, b)), want(2, 3)) and len(want(2, 3)) == 0
+        b.detect(frames[0])
+        assert np.array_equal(_mm(c.match(b, a)), want(0, 2))
+        a.close()
+        b.close()

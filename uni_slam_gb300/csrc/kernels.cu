@@ -2561,6 +2561,17 @@ k_bruteforce(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pa
     }
 }
 
+// A pair of frames to match where they are: entries 0 and 1 of a frame table
+// become a and b, and the run's error word 0.
+__global__ void __launch_bounds__(256)
+k_take_frames(FrameDev* __restrict__ dst, const FrameDev* __restrict__ a, const FrameDev* __restrict__ b, uint32_t* err) {
+    static_assert(sizeof(FrameDev) % 8 == 0, "copied by 8-byte words");
+    constexpr int N = (int)(sizeof(FrameDev) / 8);
+    for (int i = threadIdx.x; i < 2 * N; i += blockDim.x)
+        reinterpret_cast<unsigned long long*>(dst)[i] = reinterpret_cast<const unsigned long long*>(i < N ? a : b)[i < N ? i : i - N];
+    if (threadIdx.x == 0) *err = 0u;
+}
+
 // ---------------------------------------------------------- mutual ----
 constexpr int KU_THREADS = 1024;
 constexpr int KU_ITEMS = 8;  // features of a thread in one round
@@ -2915,6 +2926,11 @@ cudaError_t launch_bruteforce(const FrameDev* frames, const PairDev* pairs, cons
     if (npairs <= 0) return cudaSuccess;
     static_assert((MAX_SEGS + 1) * 8 <= 40 * 1024, "the pairs' table fits the default limit beside the tile");
     k_bruteforce<<<sms * KB_CTAS, KB_THREADS, (npairs + 1) * sizeof(unsigned long long), st>>>(frames, pairs, psegs, npairs, ratio, 2u);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_take_frames(FrameDev* dst, const FrameDev* a, const FrameDev* b, uint32_t* err, cudaStream_t st) {
+    k_take_frames<<<1, 256, 0, st>>>(dst, a, b, err);
     return cudaGetLastError();
 }
 

@@ -76,6 +76,7 @@ struct uslam_batch {
     size_t in_bytes = 0, out_bytes = 0, arena_bytes = 0;
     char* h_in = nullptr;   // pinned
     char* h_out = nullptr;  // pinned
+    uint32_t* h_err = nullptr;  // pinned, behind h_out: the error word as of the last synchronisation
     FrameDev* d_frames = nullptr;
     PairDev* d_pairs = nullptr;
     uint32_t* d_err = nullptr;
@@ -323,22 +324,28 @@ cudaError_t enqueue_split(uslam_batch* b) {
     return e;
 }
 
-uslam_status capture_graph(uslam_batch* b, Program* P) {
+// Capture what enqueue puts on the batch stream, behind the error word's reset.
+template <typename Enqueue>
+uslam_status capture(uslam_batch* b, cudaGraphExec_t* out, Enqueue enqueue) {
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return b->ctx->cuda_fail(e, "begin capture");
     e = cudaMemsetAsync(b->d_err, 0, sizeof(uint32_t), b->stream);
-    cudaError_t e2 = e == cudaSuccess ? (b->nparts > 1 && P == &b->full ? enqueue_split(b) : enqueue_program(b, *P)) : e;
+    cudaError_t e2 = e == cudaSuccess ? enqueue() : e;
     e = cudaStreamEndCapture(b->stream, &g);
     if (e2 != cudaSuccess) {
         if (g) cudaGraphDestroy(g);
         return b->ctx->cuda_fail(e2, "capture launches");
     }
     if (e != cudaSuccess) return b->ctx->cuda_fail(e, "end capture");
-    e = cudaGraphInstantiate(&P->graph, g, 0);
+    e = cudaGraphInstantiate(out, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) return b->ctx->cuda_fail(e, "graph instantiate");
     return USLAM_OK;
+}
+
+uslam_status capture_graph(uslam_batch* b, Program* P) {
+    return capture(b, &P->graph, [&] { return b->nparts > 1 && P == &b->full ? enqueue_split(b) : enqueue_program(b, *P); });
 }
 
 void free_batch(uslam_batch* b) {
@@ -565,14 +572,15 @@ uslam_status create_batch(uslam_ctx* ctx, int n_frames, const int* widths, const
         return set_err(&ctx->err, USLAM_OOM, m);
     }
     e = cudaHostAlloc(&b->h_in, in_bytes, cudaHostAllocDefault);
-    if (e == cudaSuccess) e = cudaHostAlloc(&b->h_out, out_bytes, cudaHostAllocDefault);
+    if (e == cudaSuccess) e = cudaHostAlloc(&b->h_out, round_up(out_bytes, 64) + 64, cudaHostAllocDefault);
     if (e != cudaSuccess) {
         free_batch(b);
         cudaGetLastError();
         return set_err(&ctx->err, USLAM_OOM, "pinned staging allocation refused");
     }
     std::memset(b->h_in, 0, in_bytes);
-    std::memset(b->h_out, 0, out_bytes);
+    std::memset(b->h_out, 0, round_up(out_bytes, 64) + 64);
+    b->h_err = reinterpret_cast<uint32_t*>(b->h_out + round_up(out_bytes, 64));
     e = cudaMemset(b->arena, 0, b->arena_bytes);
     if (e != cudaSuccess) {
         free_batch(b);
@@ -843,10 +851,7 @@ void build_desc_table(const int32_t* pattern, DescTable* out) {
     }
 }
 
-uslam_status check_err_word(uslam_batch* b) {
-    uint32_t word = 0;
-    cudaError_t e = cudaMemcpy(&word, b->d_err, sizeof(word), cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) return b->ctx->cuda_fail(e, "error word readback");
+uslam_status report_err_word(uslam_batch* b, uint32_t word) {
     if (word != 0u) {
         std::string m = "kernel bounds check tripped:";
         if (word & USLAM_ERR_SMEM_RANGE) m += " blur tap outside the staged tile;";
@@ -857,8 +862,18 @@ uslam_status check_err_word(uslam_batch* b) {
     return USLAM_OK;
 }
 
+uslam_status check_err_word(uslam_batch* b) {
+    uint32_t word = 0;
+    cudaError_t e = cudaMemcpy(&word, b->d_err, sizeof(word), cudaMemcpyDeviceToHost);
+    if (e != cudaSuccess) return b->ctx->cuda_fail(e, "error word readback");
+    return report_err_word(b, word);
+}
+
+// The error word is copied behind the work, so that one wait covers both (a
+// copy of its own after the wait took 8 us).
 uslam_status sync_stream(uslam_batch* b, int timeout_ms) {
-    cudaError_t e;
+    cudaError_t e = cudaMemcpyAsync(b->h_err, b->d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost, b->stream);
+    if (e != cudaSuccess) return b->ctx->cuda_fail(e, "error word readback");
     if (timeout_ms <= 0) {
         e = cudaStreamSynchronize(b->stream);
     } else {
@@ -871,7 +886,7 @@ uslam_status sync_stream(uslam_batch* b, int timeout_ms) {
         }
     }
     if (e != cudaSuccess) return b->ctx->cuda_fail(e, "stream synchronize");
-    return check_err_word(b);
+    return report_err_word(b, *static_cast<volatile uint32_t*>(b->h_err));
 }
 
 uslam_status copy_features(uslam_batch* b, const char* out_base, int frame, uslam_feature* out, int max_out, int* kept,
@@ -1359,6 +1374,9 @@ struct uslam_frontend {
     uint8_t* h_stage = nullptr;   // pinned u8 staging of the next host frame (H0 rows of img_pitch)
     float* h_stage_f32 = nullptr; // pinned f32 staging of the next f32 host frame (H0 rows of W0)
     float* d_f32 = nullptr;       // its device copy
+    // graph of a frame in slot i and its match against the other slot (launch
+    // by launch a 320x240 frame took 153 us instead of 119)
+    cudaGraphExec_t step[2] = {nullptr, nullptr};
     int cur = -1;                 // slot holding FeatureSet(0)
     int ref = -1;                 // slot holding FeatureSet(1)
     bool matched = false;
@@ -1434,16 +1452,18 @@ uslam_status frontend_enqueue(uslam_frontend* fe, const uint8_t* src_host, const
     } else {
         e = cudaMemcpyAsync(dst, fe->incoming, frame_bytes, cudaMemcpyDeviceToDevice, b->stream);
     }
-    if (e == cudaSuccess) e = cudaMemsetAsync(b->d_err, 0, sizeof(uint32_t), b->stream);
-    if (e == cudaSuccess) e = enqueue_program(b, b->frame_prog[slot]);
     fe->cur = slot;
     fe->matched = false;
     fe->host_frame[slot] = false;
     const int pair = slot == 0 ? 0 : 1;  // pair 0 = slot1 -> slot0, pair 1 = slot0 -> slot1
     if (e == cudaSuccess && fe->ref >= 0) {
         fe->host_pair[pair] = false;
-        e = enqueue_program(b, b->pair_prog[pair]);
+        e = cudaGraphLaunch(fe->step[slot], b->stream);
         fe->matched = true;
+    } else if (e == cudaSuccess) {
+        // the first frame: no pair yet
+        e = cudaMemsetAsync(b->d_err, 0, sizeof(uint32_t), b->stream);
+        if (e == cudaSuccess) e = enqueue_program(b, b->frame_prog[slot]);
     }
     if (e == cudaSuccess && download) {
         const auto fr = frame_out_range(b, slot);
@@ -1474,13 +1494,14 @@ uslam_status frontend_process_host(uslam_frontend* fe, const uint8_t* img, const
     return matched ? USLAM_OK : USLAM_NOT_READY;
 }
 
-// Bring the whole outputs region to the pinned staging (after asynchronous
-// enqueues, whose outputs were not downloaded).
-uslam_status frontend_refresh(uslam_frontend* fe) {
+// Bring a slot's feature set, or a pair's matches, to the pinned staging (after
+// asynchronous enqueues, whose outputs were not downloaded; the caller has
+// waited for them).
+uslam_status frontend_refresh(uslam_frontend* fe, std::pair<size_t, size_t> range, bool* fresh) {
     uslam_batch* b = fe->b;
-    cudaError_t e = cudaMemcpy(b->h_out, b->arena + b->in_bytes, b->out_bytes, cudaMemcpyDeviceToHost);
+    cudaError_t e = cudaMemcpy(b->h_out + range.first, b->arena + b->in_bytes + range.first, range.second, cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return b->ctx->cuda_fail(e, "outputs readback");
-    fe->host_frame[0] = fe->host_frame[1] = fe->host_pair[0] = fe->host_pair[1] = true;
+    *fresh = true;
     return USLAM_OK;
 }
 
@@ -1514,6 +1535,16 @@ uslam_status uslam_frontend_create(uslam_ctx* ctx, int width, int height, uslam_
         return set_err(&ctx->err, USLAM_OOM, "frontend input buffer allocation refused");
     }
     std::memset(fe->h_stage, 0, frame_bytes);
+    for (int slot = 0; slot < 2; ++slot) {
+        s = capture(b, &fe->step[slot], [&] {
+            const cudaError_t f = enqueue_program(b, b->frame_prog[slot]);
+            return f == cudaSuccess ? enqueue_program(b, b->pair_prog[slot]) : f;
+        });
+        if (s != USLAM_OK) {
+            uslam_frontend_destroy(fe);
+            return s;
+        }
+    }
     *out = fe;
     return USLAM_OK;
 }
@@ -1525,6 +1556,8 @@ void uslam_frontend_destroy(uslam_frontend* fe) {
     if (fe->h_stage) cudaFreeHost(fe->h_stage);
     if (fe->h_stage_f32) cudaFreeHost(fe->h_stage_f32);
     if (fe->d_f32) cudaFree(fe->d_f32);
+    for (cudaGraphExec_t g : fe->step)
+        if (g) cudaGraphExecDestroy(g);
     uslam_batch_destroy(fe->b);
     delete fe;
 }
@@ -1574,7 +1607,7 @@ uslam_status uslam_frontend_features(uslam_frontend* fe, int which, uslam_featur
     const int slot = which == 0 ? fe->cur : fe->ref;
     if (slot < 0) return set_err(fe->b->err(), USLAM_NOT_READY, "features: that feature set does not exist yet");
     if (!fe->host_frame[slot]) {
-        const uslam_status s = frontend_refresh(fe);
+        const uslam_status s = frontend_refresh(fe, frame_out_range(fe->b, slot), &fe->host_frame[slot]);
         if (s != USLAM_OK) return s;
     }
     return copy_features(fe->b, fe->b->h_out, slot, out, max_out, kept, raw);
@@ -1585,7 +1618,7 @@ uslam_status uslam_frontend_matches(uslam_frontend* fe, uslam_match* out, int ma
     if (!fe->matched) return set_err(fe->b->err(), USLAM_NOT_READY, "matches: no reference feature set yet");
     const int pair = fe->cur == 0 ? 0 : 1;
     if (!fe->host_pair[pair]) {
-        const uslam_status s = frontend_refresh(fe);
+        const uslam_status s = frontend_refresh(fe, pair_out_range(fe->b, pair), &fe->host_pair[pair]);
         if (s != USLAM_OK) return s;
     }
     return copy_matches(fe->b, fe->b->h_out, pair, out, max_out, n_out);
@@ -1603,46 +1636,6 @@ struct uslam_featset {
     int W = 0, H = 0;
     bool valid = false;
 };
-
-namespace {
-
-// Copy frame 0 of a one-frame batch (feature blocks, counts and the matcher's
-// lists) into frame `slot` of a batch of the same frame size.
-cudaError_t copy_frame_state(const uslam_batch* src, uslam_batch* dst, int slot, cudaStream_t st) {
-    const FrameDev& A = src->frames[0];
-    const FrameDev& B = dst->frames[slot];
-    const size_t capa = static_cast<size_t>(std::max(A.cap, 1));
-    cudaError_t e = cudaMemcpyAsync(B.kept, A.kept, 2 * sizeof(uint32_t) * A.levels, cudaMemcpyDeviceToDevice, st);
-    for (int l = 0; l < A.levels && e == cudaSuccess; ++l) {
-        const size_t cols = A.nbands * (static_cast<size_t>(A.w[l]) + 1) + A.nbands + 1;
-        e = cudaMemcpyAsync(B.feats[l], A.feats[l], capa * 48, cudaMemcpyDeviceToDevice, st);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(B.xorder[l], A.xorder[l], A.nbands * capa * 4, cudaMemcpyDeviceToDevice, st);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(B.colstart[l], A.colstart[l], cols * 4, cudaMemcpyDeviceToDevice, st);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(B.qorder[l], A.qorder[l], capa * 4, cudaMemcpyDeviceToDevice, st);
-    }
-    if (A.bf8 && B.bf8 && e == cudaSuccess) {
-        const size_t rows = tc_rows(A);
-        e = cudaMemcpyAsync(B.bf8, A.bf8, rows * 256, cudaMemcpyDeviceToDevice, st);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(B.bfext, A.bfext, rows * 32, cudaMemcpyDeviceToDevice, st);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(B.bfpop, A.bfpop, rows * 4, cudaMemcpyDeviceToDevice, st);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(B.bfid, A.bfid, rows * 4, cudaMemcpyDeviceToDevice, st);
-    }
-    if (A.wq8 && B.wq8 && e == cudaSuccess) {
-        // the windowed tensor-core matcher's operand rows (same frame size,
-        // so the same row strides)
-        const size_t qrows = static_cast<size_t>(A.levels) * A.wq_rows;
-        const size_t crows = static_cast<size_t>(A.levels) * A.nbands * A.wc_rows;
-        e = cudaMemcpyAsync(B.wq8, A.wq8, qrows * 256, cudaMemcpyDeviceToDevice, st);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(B.wc8, A.wc8, crows * 256, cudaMemcpyDeviceToDevice, st);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(B.wcext, A.wcext, crows * 32, cudaMemcpyDeviceToDevice, st);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(B.wcy, A.wcy, crows * 2, cudaMemcpyDeviceToDevice, st);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(B.wcid, A.wcid, crows * 4, cudaMemcpyDeviceToDevice, st);
-    }
-    return e;
-}
-
-}  // namespace
 
 extern "C" {
 
@@ -1729,15 +1722,20 @@ uslam_status uslam_match_sets(uslam_ctx* ctx, const uslam_featset* prev, const u
         it = ctx->match_batches.emplace(key, mb).first;
     }
     uslam_batch* mb = it->second;
-    // the sets' last work is complete (detect_describe synchronises); the
-    // copies and the match run on the match batch's stream
-    cudaError_t e = copy_frame_state(prev->b, mb, 0, mb->stream);
-    if (e == cudaSuccess) e = copy_frame_state(curr->b, mb, 1, mb->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(mb->d_err, 0, sizeof(uint32_t), mb->stream);
+    // The sets' last work is complete (detect_describe synchronises).  The
+    // match batch's frame table takes the sets' own entries, so the match
+    // reads their feature blocks and lists where they are, and the pair's
+    // matches alone come back (60 copies into the match batch and all of its
+    // outputs back made it 671 instead of 386 us for two 637x479 frames
+    // detected, read and matched).
+    cudaError_t e = launch_take_frames(mb->d_frames, prev->b->d_frames, curr->b->d_frames, mb->d_err, mb->stream);
     if (e == cudaSuccess) e = enqueue_program(mb, mb->pair_prog[0]);
+    const auto range = pair_out_range(mb, 0);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(mb->h_out + range.first, mb->arena + mb->in_bytes + range.first, range.second,
+                            cudaMemcpyDeviceToHost, mb->stream);
     if (e != cudaSuccess) return ctx->cuda_fail(e, "match");
-    uslam_status s = uslam_batch_download(mb);
-    if (s == USLAM_OK) s = uslam_batch_sync(mb, 0);
+    uslam_status s = uslam_batch_sync(mb, 0);
     if (s == USLAM_OK) s = uslam_batch_matches(mb, 0, out, max_out, n_out);
     return s;
 }

@@ -53,6 +53,7 @@ cudaError_t launch_bacc_init(const FrameDev*, const PairDev*, const SegDev*, int
 cudaError_t launch_mutual_reset(const FrameDev*, const PairDev*, const SegDev*, int, uint32_t*, uint32_t*,
                                 cudaStream_t);
 cudaError_t launch_emit(const FrameDev*, const PairDev*, const SegDev*, int, uint32_t*, cudaStream_t);
+cudaError_t launch_take_frames(FrameDev*, const FrameDev*, const FrameDev*, uint32_t*, cudaStream_t);
 cudaError_t launch_bruteforce(const FrameDev*, const PairDev*, const SegDev*, int, float, int, cudaStream_t);
 cudaError_t launch_bf_mma(const FrameDev*, const PairDev*, const SegDev*, int, float, int, uint32_t*, cudaStream_t);
 cudaError_t set_compact_smem(int max_w);
