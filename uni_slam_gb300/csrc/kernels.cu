@@ -14,13 +14,13 @@
 //                   candidate list, and the band-grouped query order
 //   k_describe (K2) orientation (one lane per keypoint of a warp's group) +
 //                   256-bit rotated BRIEF (the warp's lanes take 8 tests each)
-//   k_bacc_init     empties the b -> a accumulators before each k_match
-//   k_match_rank, k_match_order
-//                   k_match's claim order: query groups by estimated cost
+//   k_bacc_init     empties the accumulators before a k_match (the caller-
+//                   owned and served forms; batches reset all of theirs at once)
 //   k_match    (K3) windowed top-2 Hamming search of both directions, one
-//                   distance per pair; a warp claims groups of 32 x-adjacent
-//                   queries of the previous set in one band
-//   k_mutual        mutual cross-check (b's search read from its accumulator)
+//                   distance per pair; a warp claims units: 32 x-adjacent
+//                   queries of the previous set in one band against a part of
+//                   one pool level
+//   k_mutual        mutual cross-check (searches read from their accumulators)
 //                   and ordered match output
 //   k_bruteforce    brute-force top-2 matching (no window, no cross-check) on
 //                   the integer pipes; the tensor-core form is k_bf_mma
@@ -1925,6 +1925,7 @@ constexpr int KM_THREADS = 256;
 // measured faster than 4 CTAs at 64 registers (0.584 against 0.633 ms on
 // the 64-frame step) and than 2 at 128.
 constexpr int KM_CTAS_PER_SM = 3;
+constexpr uint32_t KM_UNITS_PER_WARP = 4, KM_MAX_CHUNKS = 8;
 
 struct MatchSegDev {
     int pair;
@@ -2046,81 +2047,6 @@ __device__ __forceinline__ int match_group_band(const uint32_t* qband, int nb, u
     return band;
 }
 
-// The claim order of k_match: query groups by estimated cost, costliest
-// first, so that the launch does not end on a few long groups.  A group's
-// cost follows the candidates it stages: the union of its x-windows in the
-// band lists of its pool levels, bounded by its first and last query (the
-// group is x-sorted).  KM_BUCKETS cost buckets of 64 candidates.  The claim
-// block of a launch: [0] the claim counter, [1, 1 + KM_BUCKETS) the groups
-// per bucket, then the buckets' write cursors, then the order; k_mutual
-// zeroes the first KM_CLAIM_WORDS words after the launch.
-constexpr int KM_BUCKETS = 64;
-constexpr int KM_CLAIM_WORDS = 1 + 2 * KM_BUCKETS;
-
-__device__ uint32_t match_group_cost(const FrameDev* frames, const PairDev* pairs, const MatchSegDev& sg,
-                                     uint32_t grp) {
-    const PairDev& P = pairs[sg.pair];
-    const FrameDev& Q = frames[P.prev];
-    const FrameDev& B = frames[P.curr];
-    const int l = sg.level;
-    const uint32_t* qband = Q.colstart[l] + (size_t)Q.nbands * (size_t)(Q.w[l] + 1);
-    const int band = match_group_band(qband, Q.nbands, &grp);
-    const uint32_t k0 = qband[band] + grp * 32u, k1 = min(k0 + 31u, qband[band + 1] - 1u);
-    const float ql = lod_scale(l);
-    const float x0 = (float)(uint32_t)__uint_as_float(Q.feats[l][(size_t)__ldg(Q.qorder[l] + k0) * 12u]) * ql;
-    const float x1 = (float)(uint32_t)__uint_as_float(Q.feats[l][(size_t)__ldg(Q.qorder[l] + k1) * 12u]) * ql;
-    const float lo = x0 - P.max_dx, hi = x1 + P.max_dx;
-    uint32_t n = 0;
-    for (int k = 0; k < 3; ++k) {
-        const int pl = k == 0 ? l : (k == 1 ? l - 1 : l + 1);
-        if (pl < 0 || pl >= B.levels) continue;
-        const float ps = lod_scale(pl);
-        const int wpl = B.w[pl];
-        const uint32_t* colstart = B.colstart[pl] + (size_t)band * (size_t)(wpl + 1);
-        const int xlo = first_col_ge(lo, ps, wpl), xhi = last_col_le(hi, ps, wpl);
-        if (xlo <= xhi) n += __ldg(colstart + xhi + 1) - __ldg(colstart + xlo);
-    }
-    return n;
-}
-
-// Pass 1: every group's cost bucket and the bucket sizes.
-__global__ void __launch_bounds__(256)
-k_match_rank(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pairs,
-             const MatchSegDev* __restrict__ segs, int nseg, uint32_t* claim, uint8_t* gbucket) {
-    __shared__ uint32_t s_pref[KM_MAX_SEGS + 1];
-    __shared__ uint32_t s_warp[33];
-    const uint32_t total =
-        segment_prefix(nseg, s_pref, s_warp, [&](int s) { return match_groups(frames, pairs, segs[s]); });
-    for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x) {
-        const int sidx = find_segment(s_pref, nseg, g);
-        const uint32_t c = match_group_cost(frames, pairs, segs[sidx], g - s_pref[sidx]);
-        const int b = KM_BUCKETS - 1 - (int)min(c >> 6, (uint32_t)(KM_BUCKETS - 1));
-        gbucket[g] = (uint8_t)b;
-        atomicAdd(claim + 1 + b, 1u);
-    }
-}
-
-// Pass 2: the order, bucket by bucket (within a bucket in arrival order).
-__global__ void __launch_bounds__(256) k_match_order(uint32_t* claim, const uint8_t* __restrict__ gbucket) {
-    __shared__ uint32_t s_start[KM_BUCKETS + 1];
-    if (threadIdx.x == 0) {
-        uint32_t run = 0;
-        for (int b = 0; b < KM_BUCKETS; ++b) {
-            s_start[b] = run;
-            run += claim[1 + b];
-        }
-        s_start[KM_BUCKETS] = run;
-    }
-    __syncthreads();
-    const uint32_t total = s_start[KM_BUCKETS];
-    uint32_t* cursor = claim + 1 + KM_BUCKETS;
-    uint32_t* order = claim + KM_CLAIM_WORDS;
-    for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x) {
-        const int b = gbucket[g];
-        order[s_start[b] + atomicAdd(cursor + b, 1u)] = g;
-    }
-}
-
 // The windowed mutual matcher (match_features_cpu.cpp:66-207), one Hamming
 // distance per pair of features.  Both directions of FindMatches compare the
 // same pairs: b in the window of a (a -> b, pool = the levels l - 1 .. l + 1
@@ -2144,16 +2070,18 @@ __global__ void __launch_bounds__(256) k_match_order(uint32_t* claim, const uint
 //    into b's two smallest and merges them into b's accumulator in HBM (atomic minimum of
 //    (distance, packed a), then of the second distance), where the batches
 //    of every query group that meets b meet;
-//  * a2b is written per query group; k_mutual reads b's accumulator.
+//  * a's search is merged into its own accumulator the same way when its
+//    units end; k_mutual reads both accumulators.
 // The logic and popcount pipes bound it (ALU 68 %, XU 47 %, shared memory 43 %
 // busy); 32 pairs of 752x480 frames: 318 us picking hits, 283 us so.
 // A tied best leaves the second distance equal to the best, which fails the
 // ratio test, so no result depends on the order of the candidates or of the
-// merges.  The pool rule (fewer than two candidates: no match) is applied to
-// a here and to b in k_mutual.
+// merges.  The pool rule (fewer than two candidates: no match) is applied in
+// k_mutual (to a here where a2b is written).
+template <bool PARTS>
 __global__ void __launch_bounds__(KM_THREADS, KM_CTAS_PER_SM)
 k_match(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pairs,
-        const MatchSegDev* __restrict__ segs, int nseg, uint32_t* claim_block, uint32_t two) {
+        const MatchSegDev* __restrict__ segs, int nseg, uint32_t* next_unit, uint32_t two) {
     __shared__ uint32_t s_pref[KM_MAX_SEGS + 1];
     __shared__ uint32_t s_warp[33];
     __shared__ __align__(16) CandStage s_stage[KM_THREADS / 32];
@@ -2161,8 +2089,6 @@ k_match(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pairs,
     // query level's column tables)
     const uint32_t total =
         segment_prefix(nseg, s_pref, s_warp, [&](int s) { return match_groups(frames, pairs, segs[s]); });
-    uint32_t* const next_group = claim_block;
-    const uint32_t* const order = claim_block ? claim_block + KM_CLAIM_WORDS : nullptr;
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const int gw = blockIdx.x * (KM_THREADS / 32) + warp;
@@ -2179,21 +2105,29 @@ k_match(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pairs,
         s_first[threadIdx.x] = m;
     }
     __syncthreads();
-    // Query groups cost very different amounts (the hits in their windows).
-    // With a claim block (its counter zeroed before the launch, its order
-    // written by k_match_rank / k_match_order) a warp claims the next group of
-    // the order, costliest first, when it finishes one; without it warps take
-    // every nw-th group.  Each group writes only its own queries' a2b entries and merges
-    // into b's accumulators by atomic minima, so the order does not change
-    // the result.
-    auto claim = [&](uint32_t g) -> uint32_t {
-        if (!next_group) return g + (uint32_t)nw;
+    // PARTS: a group's search is cut by pool level and then into chunks of its
+    // batches, for KM_UNITS_PER_WARP units a warp: a group in one piece takes 20
+    // batches on a 752x480 frame, 70 on a 1920x1080 one, 5 to 7 us each, and the
+    // groups cost very different amounts.  A warp's first unit is its own,
+    // then it claims the next from *next_unit (zero before the launch; without
+    // it warps take every nw-th unit).  The units of a group meet in aacc; else
+    // a warp has all of a group and writes a2b.  All merging is by atomic
+    // minima, so the order does not change the result.
+    // One 752x480 / 1920x1080 frame with 1, 2, 4, 6, 8, 16 units a warp: 246, 245,
+    // 240, 244, 246, 248 / 600, 620, 554, 544, 554, 572 us.  Whole groups in an
+    // order of their cost (two kernels before) took 1438 us for 64 frames, units
+    // 1431, the mixed batch 4689 and 4656.
+    auto claim = [&](uint32_t c) -> uint32_t {
+        if (!next_unit) return c + (uint32_t)nw;
         uint32_t n = 0;
-        if (lane == 0) n = atomicAdd(next_group, 1u);
-        return __shfl_sync(0xffffffffu, n, 0);
+        if (lane == 0) n = atomicAdd(next_unit, 1u);
+        return __shfl_sync(0xffffffffu, n, 0) + (uint32_t)nw;
     };
-    for (uint32_t c = next_group ? claim(0u) : (uint32_t)gw; c < total; c = claim(c)) {
-        const uint32_t g = order ? __ldg(order + c) : c;
+    const uint32_t chunks = PARTS ? min(max((KM_UNITS_PER_WARP * (uint32_t)nw) / max(3u * total, 1u), 1u), KM_MAX_CHUNKS) : 1u;
+    const uint32_t units = PARTS ? 3u * chunks * total : total;
+    for (uint32_t c = (uint32_t)gw; c < units; c = claim(c)) {
+        const uint32_t g = PARTS ? c / (3u * chunks) : c;
+        const uint32_t part = PARTS ? c - g * (3u * chunks) : 0u;
         const int sidx = find_segment(s_pref, nseg, g);
         uint32_t grp = g - s_pref[sidx];
         const MatchSegDev sg = segs[sidx];
@@ -2227,7 +2161,7 @@ k_match(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pairs,
         const size_t capb = (size_t)(B.cap > 0 ? B.cap : 1);
         uint32_t* const colq = S.col + lane;
         const uint32_t lanes = (uint32_t)lane * 0x10001u;
-        for (int k = 0; k < 3; ++k) {
+        for (int k = PARTS ? (int)(part / chunks) : 0; k < 3; k = PARTS ? 3 : k + 1) {
             const int pl = k == 0 ? l : (k == 1 ? l - 1 : l + 1);
             if (pl < 0 || pl >= L) continue;
             const float ps = lod_scale(pl);
@@ -2257,6 +2191,13 @@ k_match(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pairs,
                 c1 = max(c1, __shfl_xor_sync(0xffffffffu, c1, o));
             }
             if (c0 >= c1) continue;
+            if (PARTS) {
+                const uint32_t nb = (c1 - c0 + 31u) / 32u, ch = part % chunks;
+                const uint32_t from = c0 + 32u * (ch * nb / chunks), to = c0 + 32u * ((ch + 1u) * nb / chunks);
+                c1 = min(c1, to);
+                c0 = from;
+                if (c0 >= c1) continue;
+            }
             const uint32_t* xorder = B.xorder[pl] + (size_t)band * (size_t)(B.cap > 0 ? B.cap : 1);
             const uint32_t* feats = B.feats[pl];
             // Candidates are staged by asynchronous copies one batch ahead,
@@ -2392,7 +2333,13 @@ k_match(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pairs,
                 __syncwarp();
             }
         }
-        if (valid) {
+        if (PARTS && bidx >= 0) {
+            uint4* acc = P.aacc + (size_t)l * Q.cap + qi;
+            const unsigned long long key = ((unsigned long long)(bestk >> 5) << 32) | (unsigned long long)(uint32_t)bidx;
+            const unsigned long long old = atomicMin(reinterpret_cast<unsigned long long*>(acc), key);
+            atomicMin(&acc->z, min((uint32_t)((old > key ? old : key) >> 32), secondk == 0xffffu ? 0xffffffffu : secondk >> 5));
+        }
+        if (!PARTS && valid) {
             uint32_t pool = B.kept[l];
             if (l > 0) pool += B.kept[l - 1];
             if (l + 1 < L) pool += B.kept[l + 1];
@@ -2403,17 +2350,19 @@ k_match(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pairs,
     }
 }
 
-// b's accumulators start empty (all ones) before every k_match launch: one
-// CTA per (pair, level of b).
+// The accumulators start empty (all ones) before every k_match launch: one
+// CTA per (pair, level).
 __global__ void __launch_bounds__(256)
 k_bacc_init(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pairs, const SegDev* __restrict__ segs) {
     const int pi = segs[blockIdx.x].frame;  // pair index
     const int l = segs[blockIdx.x].level;
     const PairDev& P = pairs[pi];
-    const FrameDev& B = frames[P.curr];
-    const uint32_t n = B.kept[l];
-    uint4* acc = P.bacc + (size_t)l * (size_t)(B.cap > 0 ? B.cap : 1);
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) acc[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
+    auto empty = [&](uint4* all, const FrameDev& F) {
+        uint4* acc = all + (size_t)l * (size_t)(F.cap > 0 ? F.cap : 1);
+        for (uint32_t i = threadIdx.x; i < F.kept[l]; i += blockDim.x) acc[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
+    };
+    empty(P.bacc, frames[P.curr]);
+    if (P.aacc) empty(P.aacc, frames[P.prev]);
 }
 
 // ----------------------------------------------------- brute force ----
@@ -2590,10 +2539,9 @@ k_mutual(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pairs,
          uint32_t* err, uint32_t* reset_word) {
     constexpr int WARPS = KU_THREADS / 32;
     static_assert(WARPS == 32, "the scan takes a warp per item index and a lane per warp");
-    // k_match's claim counters for its next launch on this stream (k_mutual
-    // always follows k_match, which has finished with them)
-    if (reset_word && blockIdx.x == 0)
-        for (int i = threadIdx.x; i < KM_CLAIM_WORDS; i += blockDim.x) reset_word[i] = 0u;
+    // k_match's unit counter for its next launch on this stream (k_mutual
+    // always follows k_match, which has finished with it)
+    if (reset_word && blockIdx.x == 0 && threadIdx.x == 0) *reset_word = 0u;
     __shared__ uint32_t s_cnt[KU_ITEMS][WARPS];  // matches per (item index, warp), then those before them in the row
     __shared__ uint32_t s_row[KU_ITEMS];
     const int pi = segs[blockIdx.x].frame;  // pair index
@@ -2610,7 +2558,22 @@ k_mutual(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pairs,
         for (int q = 0; q < B.levels; ++q) nt += B.kept[q];
     for (uint32_t c0 = 0; c0 < n; c0 += KU_THREADS * KU_ITEMS) {
         int32_t m[KU_ITEMS];
-        if (MUTUAL || P.bf_part == nullptr) {
+        if (MUTUAL && P.aacc) {
+            // a's search from its accumulator: the pool rule and the ratio test
+            uint32_t pool = B.kept[l];
+            if (l > 0) pool += B.kept[l - 1];
+            if (l + 1 < B.levels) pool += B.kept[l + 1];
+            const uint4* acc = P.aacc + (size_t)l * A.cap;
+            uint4 e[KU_ITEMS];
+#pragma unroll
+            for (int u = 0; u < KU_ITEMS; ++u) {
+                const uint32_t i = c0 + u * KU_THREADS + threadIdx.x;
+                e[u] = i < n ? acc[i] : make_uint4(~0u, ~0u, ~0u, ~0u);
+            }
+#pragma unroll
+            for (int u = 0; u < KU_ITEMS; ++u)
+                m[u] = pool >= 2u && e[u].y != 0xffffffffu && (float)e[u].y < 0.85f * (float)e[u].z ? (int32_t)e[u].x : -1;
+        } else if (MUTUAL || P.bf_part == nullptr) {
 #pragma unroll
             for (int u = 0; u < KU_ITEMS; ++u) {
                 const uint32_t i = c0 + u * KU_THREADS + threadIdx.x;
@@ -2872,28 +2835,21 @@ cudaError_t set_describe_tiled_smem(int margin) {
 cudaError_t launch_match(const FrameDev* frames, const PairDev* pairs, const void* segs, int nseg, int num_sms,
                          cudaStream_t st) {
     if (nseg <= 0) return cudaSuccess;
-    k_match<<<num_sms * KM_CTAS_PER_SM, KM_THREADS, 0, st>>>(frames, pairs, static_cast<const MatchSegDev*>(segs), nseg,
-                                                              nullptr, 2u);
-    return cudaGetLastError();
-}
-// The claim order (k_match_rank, k_match_order), then k_match claiming from
-// it.  claim: a block of match_claim_words(max groups) words, its first
-// KM_CLAIM_WORDS zero (k_mutual_reset zeroes them again after each launch);
-// gbucket: max groups bytes.
-size_t match_claim_words(size_t max_groups) { return KM_CLAIM_WORDS + max_groups; }
-cudaError_t launch_match_dyn(const FrameDev* frames, const PairDev* pairs, const void* segs, int nseg, int num_sms,
-                             uint32_t* claim, uint8_t* gbucket, cudaStream_t st) {
-    if (nseg <= 0) return cudaSuccess;
-    const MatchSegDev* ms = static_cast<const MatchSegDev*>(segs);
-    k_match_rank<<<num_sms * 4, 256, 0, st>>>(frames, pairs, ms, nseg, claim, gbucket);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    k_match_order<<<num_sms, 256, 0, st>>>(claim, gbucket);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    k_match<<<num_sms * KM_CTAS_PER_SM, KM_THREADS, 0, st>>>(frames, pairs, ms, nseg, claim, 2u);
+    k_match<false><<<num_sms * KM_CTAS_PER_SM, KM_THREADS, 0, st>>>(frames, pairs, static_cast<const MatchSegDev*>(segs),
+                                                                    nseg, nullptr, 2u);
     return cudaGetLastError();
 }
 
+// k_match with several units per query group, for the pairs' aacc; claim: a
+// zero word that hands out the units after each warp's first (null: every
+// warp takes its share of them).
+cudaError_t launch_match_parts(const FrameDev* frames, const PairDev* pairs, const void* segs, int nseg, int num_sms,
+                               uint32_t* claim, cudaStream_t st) {
+    if (nseg <= 0) return cudaSuccess;
+    k_match<true><<<num_sms * KM_CTAS_PER_SM, KM_THREADS, 0, st>>>(frames, pairs, static_cast<const MatchSegDev*>(segs),
+                                                                   nseg, claim, 2u);
+    return cudaGetLastError();
+}
 cudaError_t launch_bacc_init(const FrameDev* frames, const PairDev* pairs, const SegDev* segs, int nseg,
                              cudaStream_t st) {
     if (nseg <= 0) return cudaSuccess;

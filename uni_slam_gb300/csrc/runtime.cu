@@ -80,11 +80,12 @@ struct uslam_batch {
     FrameDev* d_frames = nullptr;
     PairDev* d_pairs = nullptr;
     uint32_t* d_err = nullptr;
+    char* d_acc = nullptr;  // k_match's accumulators of all pairs
+    size_t acc_bytes = 0;
     char* d_tables = nullptr;
-    // k_match's claim blocks, one per lane (its counters and claim order),
-    // and each lane's group cost buckets
+    // k_match's unit counters, one per lane
     char* d_claim = nullptr;
-    size_t claim_stride = 0, claim_words = 0;
+    static constexpr size_t kClaimStride = 256;
     cudaStream_t stream = nullptr;      // stream in use (own or caller's)
     cudaStream_t own_stream = nullptr;  // created with the batch
     cudaStream_t aux_stream = nullptr;  // k_xsort's branch beside k_blur
@@ -148,12 +149,12 @@ uslam_status build_program(uslam_batch* b, const std::vector<int>& fr, const std
     }
     if (!b->win_tc) {
         // k_match searches both directions from the prev set's queries.  Its
-        // warps claim query groups in segment order, so the costliest groups
-        // go first and the launch's tail is short: a group's windows cover a
-        // fixed share of its frame at about the same feature density, so its
-        // cost grows with the frame's area (larger frames first); within one
-        // size the groups of the first and last level (two pool levels
-        // instead of three) come last (0.594 -> 0.570 ms on the 64-frame step).
+        // warps claim units in segment order, so the costliest go first and
+        // the launch's tail is short: a group's windows cover a fixed share
+        // of its frame at about the same feature density, so its cost grows
+        // with the frame's area (larger frames first); within one size the
+        // groups of the first and last level (two pool levels instead of
+        // three) come last.
         std::vector<int> order;
         for (int l = 1; l + 1 < b->levels; ++l) order.push_back(l);
         order.push_back(0);
@@ -208,24 +209,18 @@ uslam_status build_program(uslam_batch* b, const std::vector<int>& fr, const std
 }
 
 // A lane of launches: a stream, the stream k_xsort forks to, their
-// fork/join events, and the block k_match claims its query groups from (with
-// the group cost buckets its order is built from).
+// fork/join events, and the counter k_match claims its units from.
 struct Lane {
     cudaStream_t st, aux;
     cudaEvent_t fork, join;
     uint32_t* claim;
-    uint8_t* gbucket;
 };
 
 uint32_t* lane_claim(uslam_batch* b, int j) {
-    return reinterpret_cast<uint32_t*>(b->d_claim + static_cast<size_t>(j) * b->claim_stride);
-}
-uint8_t* lane_gbucket(uslam_batch* b, int j) {
-    return reinterpret_cast<uint8_t*>(b->d_claim + static_cast<size_t>(j) * b->claim_stride) +
-           round_up(b->claim_words * sizeof(uint32_t), 256);
+    return reinterpret_cast<uint32_t*>(b->d_claim + static_cast<size_t>(j) * uslam_batch::kClaimStride);
 }
 Lane lane0(uslam_batch* b) {
-    return Lane{b->stream, b->aux_stream, b->ev_fork, b->ev_join, lane_claim(b, 0), lane_gbucket(b, 0)};
+    return Lane{b->stream, b->aux_stream, b->ev_fork, b->ev_join, lane_claim(b, 0)};
 }
 
 // Describe of a program: the gather form k_describe over (frame, level)
@@ -266,7 +261,8 @@ cudaError_t enqueue_frames(uslam_batch* b, const Program& P, const Lane& ln) {
     return describe_stage(b, P, ln.st);
 }
 
-// The pair stages of a program: match and the mutual check / emit.
+// The pair stages of a program: match and the mutual check / emit.  With
+// k_match the accumulators are empty by then (reset_acc).
 cudaError_t enqueue_pairs(uslam_batch* b, const Program& P, const Lane& ln) {
     uslam_ctx* c = b->ctx;
     cudaError_t e = cudaSuccess;
@@ -285,9 +281,7 @@ cudaError_t enqueue_pairs(uslam_batch* b, const Program& P, const Lane& ln) {
             return e;
         return launch_mutual(b->d_frames, b->d_pairs, P.usegs, P.nusegs, b->d_err, ln.st);
     }
-    if ((e = launch_bacc_init(b->d_frames, b->d_pairs, P.usegs, P.nusegs, ln.st)) != cudaSuccess) return e;
-    if ((e = launch_match_dyn(b->d_frames, b->d_pairs, P.msegs, P.nmsegs, c->num_sms, ln.claim, ln.gbucket,
-                              ln.st)) != cudaSuccess)
+    if ((e = launch_match_parts(b->d_frames, b->d_pairs, P.msegs, P.nmsegs, c->num_sms, ln.claim, ln.st)) != cudaSuccess)
         return e;
     return launch_mutual_reset(b->d_frames, b->d_pairs, P.usegs, P.nusegs, b->d_err, ln.claim, ln.st);
 }
@@ -307,8 +301,7 @@ cudaError_t enqueue_split(uslam_batch* b) {
     Lane ln[kLanes];
     for (int j = 0; j < K; ++j)
         ln[j] = j == 0 ? lane0(b)
-                       : Lane{b->lane_st[j], b->lane_aux[j], b->lane_fork[j], b->lane_join[j], lane_claim(b, j),
-                              lane_gbucket(b, j)};
+                       : Lane{b->lane_st[j], b->lane_aux[j], b->lane_fork[j], b->lane_join[j], lane_claim(b, j)};
     cudaError_t e = cudaEventRecord(b->ev_start, b->stream);
     for (int j = 1; j < K && e == cudaSuccess; ++j) e = cudaStreamWaitEvent(ln[j].st, b->ev_start, 0);
     for (int j = 0; j < K && e == cudaSuccess; ++j) {
@@ -324,13 +317,25 @@ cudaError_t enqueue_split(uslam_batch* b) {
     return e;
 }
 
-// Capture what enqueue puts on the batch stream, behind the error word's reset.
+// k_match's accumulators of all pairs to empty (all ones), by their caps.
+cudaError_t reset_acc(uslam_batch* b, cudaStream_t st) {
+    return b->acc_bytes ? cudaMemsetAsync(b->d_acc, 0xff, b->acc_bytes, st) : cudaSuccess;
+}
+
+// Capture what enqueue puts on the batch stream, behind the error word's
+// reset and beside the accumulators', which is on the auxiliary stream before
+// the frames' k_xsort.
 template <typename Enqueue>
 uslam_status capture(uslam_batch* b, cudaGraphExec_t* out, Enqueue enqueue) {
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return b->ctx->cuda_fail(e, "begin capture");
     e = cudaMemsetAsync(b->d_err, 0, sizeof(uint32_t), b->stream);
+    if (e == cudaSuccess && b->acc_bytes) {
+        e = cudaEventRecord(b->ev_fork, b->stream);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(b->aux_stream, b->ev_fork, 0);
+        if (e == cudaSuccess) e = reset_acc(b, b->aux_stream);
+    }
     cudaError_t e2 = e == cudaSuccess ? enqueue() : e;
     e = cudaStreamEndCapture(b->stream, &g);
     if (e2 != cudaSuccess) {
@@ -376,14 +381,8 @@ void free_batch(uslam_batch* b) {
     delete b;
 }
 
-// per_frame_form: the batch serves the one-frame forms (the frontend, feature
-// sets and their matches), where the windowed matcher takes its distances
-// from the tensor cores: for one pair k_match leaves most of the GPU idle and
-// its latency is that of its slowest query group (measured: the one-frame
-// form ran 4,109 frames/s with k_match, 5,497 with k_win_mma).
 uslam_status create_batch(uslam_ctx* ctx, int n_frames, const int* widths, const int* heights, int n_pairs,
-                          const int* pair_prev, const int* pair_curr, bool per_item_programs, uslam_batch** out,
-                          bool per_frame_form = false) {
+                          const int* pair_prev, const int* pair_curr, bool per_item_programs, uslam_batch** out) {
     if (!ctx || !out || n_frames <= 0 || !widths || !heights || n_pairs < 0 || (n_pairs > 0 && (!pair_prev || !pair_curr)))
         return set_err(ctx ? &ctx->err : nullptr, USLAM_INVALID_ARG, "batch_create: bad arguments");
     if (n_frames > 65535) return set_err(&ctx->err, USLAM_INVALID_ARG, "batch_create: more than 65535 frames");
@@ -417,7 +416,7 @@ uslam_status create_batch(uslam_ctx* ctx, int n_frames, const int* widths, const
         const long long c = ctx->cap_override > 0 ? ctx->cap_override : static_cast<long long>(widths[f]) * heights[f] / 250;
         max_cap = static_cast<int>(std::max<long long>(max_cap, c));
     }
-    b->win_tc = (ctx->win_tc || (ctx->matcher == 0 && per_frame_form)) && max_cap <= kWinMaxCap && ctx->max_h < 65535;
+    b->win_tc = ctx->win_tc && max_cap <= kWinMaxCap && ctx->max_h < 65535;
     std::vector<FrameLayout> fl(n_frames);
     for (int f = 0; f < n_frames; ++f) {
         const int W0 = widths[f], H0 = heights[f];
@@ -499,10 +498,11 @@ uslam_status create_batch(uslam_ctx* ctx, int n_frames, const int* widths, const
     b->pairs.resize(n_pairs);
     b->pair_off.resize(n_pairs);
     std::vector<std::pair<size_t, size_t>> dirs(n_pairs);
-    // k_match (matcher 0 without the tensor-core form) searches b -> a into
-    // per-feature accumulators instead of b2a
+    // k_match (matcher 0 without the tensor-core form) searches into
+    // per-feature accumulators, the other matchers write a2b (and b2a)
     const bool sym_match = ctx->matcher == 0 && !b->win_tc;
-    std::vector<size_t> bacc_off(n_pairs, 0);
+    std::vector<size_t> bacc_off(n_pairs, 0), aacc_off(n_pairs, 0);
+    size_t acc_bytes = 0;
     for (int p = 0; p < n_pairs; ++p) {
         const int a = pair_prev[p], c = pair_curr[p];
         if (a < 0 || a >= n_frames || c < 0 || c >= n_frames || a == c) {
@@ -523,12 +523,16 @@ uslam_status create_batch(uslam_ctx* ctx, int n_frames, const int* widths, const
         P.max_dx = 0.1f * static_cast<float>(static_cast<uint32_t>(b->frames[a].W0));
         P.max_dy = 0.1f * static_cast<float>(static_cast<uint32_t>(b->frames[a].H0));
         b->pair_off[p] = take(&out_bytes, round_up(sizeof(uint32_t) * L, 16) + static_cast<size_t>(L) * capa * 16);
-        dirs[p].first = take(&scratch, static_cast<size_t>(L) * capa * 4);
-        dirs[p].second = take(&scratch, static_cast<size_t>(L) * capc * 4);
-        if (sym_match) bacc_off[p] = take(&scratch, static_cast<size_t>(L) * capc * 16);
+        if (!sym_match) {
+            dirs[p].first = take(&scratch, static_cast<size_t>(L) * capa * 4);
+            dirs[p].second = take(&scratch, static_cast<size_t>(L) * capc * 4);
+        }
+        if (sym_match) bacc_off[p] = take(&acc_bytes, static_cast<size_t>(L) * capc * 16);
+        if (sym_match) aacc_off[p] = take(&acc_bytes, static_cast<size_t>(L) * capa * 16);
         P.bf_splits = 1;
         P.bf_ratio = ctx->ratio;
     }
+    const size_t acc_off = take(&scratch, acc_bytes);
     // The brute-force matchers share their work out in equal parts, which cut
     // query blocks (bf_line.h): records for as many parts of a block as
     // equal shares make at least one block a pair, up to a limit (a single
@@ -652,12 +656,15 @@ uslam_status create_batch(uslam_ctx* ctx, int n_frames, const int* widths, const
         PairDev& P = b->pairs[p];
         P.match_count = reinterpret_cast<uint32_t*>(out_base + b->pair_off[p]);
         P.matches = reinterpret_cast<int32_t*>(out_base + b->pair_off[p] + round_up(sizeof(uint32_t) * L, 16));
-        P.a2b = reinterpret_cast<int32_t*>(sc_base + dirs[p].first);
-        P.b2a = reinterpret_cast<int32_t*>(sc_base + dirs[p].second);
-        P.bacc = sym_match ? reinterpret_cast<uint4*>(sc_base + bacc_off[p]) : nullptr;
+        P.a2b = sym_match ? nullptr : reinterpret_cast<int32_t*>(sc_base + dirs[p].first);
+        P.b2a = sym_match ? nullptr : reinterpret_cast<int32_t*>(sc_base + dirs[p].second);
+        P.bacc = sym_match ? reinterpret_cast<uint4*>(sc_base + acc_off + bacc_off[p]) : nullptr;
+        P.aacc = sym_match ? reinterpret_cast<uint4*>(sc_base + acc_off + aacc_off[p]) : nullptr;
         P.bf_part = P.bf_splits > 1 ? reinterpret_cast<uint32_t*>(sc_base + bf_off[p]) : nullptr;
     }
     b->d_err = reinterpret_cast<uint32_t*>(sc_base + err_off);
+    b->d_acc = sc_base + acc_off;
+    b->acc_bytes = acc_bytes;
     b->d_frames = reinterpret_cast<FrameDev*>(sc_base + frames_off);
     b->d_pairs = reinterpret_cast<PairDev*>(sc_base + pairs_off);
     e = cudaMemcpy(b->d_frames, b->frames.data(), sizeof(FrameDev) * n_frames, cudaMemcpyHostToDevice);
@@ -735,23 +742,13 @@ uslam_status create_batch(uslam_ctx* ctx, int n_frames, const int* widths, const
             progs.push_back(&b->pair_prog[p]);
         }
     }
-    // k_match's claim blocks: per lane the counters and an order of up to
-    // max_groups query groups (every program's groups are at most the full
-    // program's), zeroed once here and by k_mutual after every launch
-    {
-        size_t max_groups = 0;
-        for (int p = 0; p < n_pairs; ++p)
-            max_groups += static_cast<size_t>(L) *
-                          (static_cast<size_t>(std::max(b->frames[pair_prev[p]].cap, 1)) / 32 + b->max_bands + 1);
-        b->claim_words = match_claim_words(max_groups);
-        b->claim_stride = round_up(b->claim_words * sizeof(uint32_t), 256) + round_up(std::max<size_t>(max_groups, 1), 256);
-        e = cudaMalloc(&b->d_claim, b->claim_stride * kLanes);
-        if (e == cudaSuccess) e = cudaMemset(b->d_claim, 0, b->claim_stride * kLanes);
-        if (e != cudaSuccess) {
-            free_batch(b);
-            cudaGetLastError();
-            return set_err(&ctx->err, USLAM_OOM, "match claim blocks: allocation refused");
-        }
+    // k_match's unit counters, zeroed once here and by k_mutual after every launch
+    e = cudaMalloc(&b->d_claim, uslam_batch::kClaimStride * kLanes);
+    if (e == cudaSuccess) e = cudaMemset(b->d_claim, 0, uslam_batch::kClaimStride * kLanes);
+    if (e != cudaSuccess) {
+        free_batch(b);
+        cudaGetLastError();
+        return set_err(&ctx->err, USLAM_OOM, "match unit counters: allocation refused");
     }
     size_t tbytes = 0;
     for (Program* P : progs) tbytes += P->host.size();
@@ -1224,16 +1221,14 @@ uslam_status uslam_batch_profile(uslam_batch* b, int iters, float* kernel_ms) {
         if (e == cudaSuccess)
             e = describe_stage(b, P, b->stream);
         mark();
-        if (e == cudaSuccess && c->matcher == 0 && !b->win_tc)
-            e = launch_bacc_init(b->d_frames, b->d_pairs, P.usegs, P.nusegs, b->stream);
+        if (e == cudaSuccess) e = reset_acc(b, b->stream);
         if (e == cudaSuccess)
             e = c->matcher == 1 ? launch_bruteforce(b->d_frames, b->d_pairs, P.psegs, P.npsegs, c->ratio, c->num_sms, b->stream)
                 : c->matcher == 2
                     ? launch_bf_mma(b->d_frames, b->d_pairs, P.psegs, P.npsegs, c->ratio, c->num_sms, b->d_err, b->stream)
                 : b->win_tc ? launch_win_match(b->d_frames, b->d_pairs, P.msegs, P.nmsegs, b->win_umax, P.units,
                                                c->num_sms, b->d_err, b->stream)
-                    : launch_match_dyn(b->d_frames, b->d_pairs, P.msegs, P.nmsegs, c->num_sms,
-                                       lane_claim(b, 0), lane_gbucket(b, 0), b->stream);
+                    : launch_match_parts(b->d_frames, b->d_pairs, P.msegs, P.nmsegs, c->num_sms, lane_claim(b, 0), b->stream);
         mark();
         if (e == cudaSuccess)
             e = c->matcher != 0 ? launch_emit(b->d_frames, b->d_pairs, P.usegs, P.nusegs, b->d_err, b->stream)
@@ -1514,7 +1509,7 @@ uslam_status uslam_frontend_create(uslam_ctx* ctx, int width, int height, uslam_
     const int ws[2] = {width, width}, hs[2] = {height, height};
     const int prev[2] = {1, 0}, curr[2] = {0, 1};  // pair 0: slot1 -> slot0, pair 1: slot0 -> slot1
     uslam_batch* b = nullptr;
-    uslam_status s = create_batch(ctx, 2, ws, hs, 2, prev, curr, true, &b, true);
+    uslam_status s = create_batch(ctx, 2, ws, hs, 2, prev, curr, true, &b);
     if (s != USLAM_OK) return s;
     auto* fe = new uslam_frontend();
     fe->b = b;
@@ -1642,7 +1637,7 @@ extern "C" {
 uslam_status uslam_featset_create(uslam_ctx* ctx, int width, int height, uslam_featset** out) {
     if (!ctx || !out) return USLAM_INVALID_ARG;
     uslam_batch* b = nullptr;
-    uslam_status s = create_batch(ctx, 1, &width, &height, 0, nullptr, nullptr, false, &b, true);
+    uslam_status s = create_batch(ctx, 1, &width, &height, 0, nullptr, nullptr, false, &b);
     if (s != USLAM_OK) return s;
     auto* fs = new uslam_featset();
     fs->ctx = ctx;
@@ -1717,7 +1712,7 @@ uslam_status uslam_match_sets(uslam_ctx* ctx, const uslam_featset* prev, const u
         const int ws[2] = {prev->W, prev->W}, hs[2] = {prev->H, prev->H};
         const int pp = 0, pc = 1;
         uslam_batch* mb = nullptr;
-        uslam_status s = create_batch(ctx, 2, ws, hs, 1, &pp, &pc, true, &mb, true);
+        uslam_status s = create_batch(ctx, 2, ws, hs, 1, &pp, &pc, true, &mb);
         if (s != USLAM_OK) return s;
         it = ctx->match_batches.emplace(key, mb).first;
     }
@@ -1729,6 +1724,7 @@ uslam_status uslam_match_sets(uslam_ctx* ctx, const uslam_featset* prev, const u
     // outputs back made it 671 instead of 386 us for two 637x479 frames
     // detected, read and matched).
     cudaError_t e = launch_take_frames(mb->d_frames, prev->b->d_frames, curr->b->d_frames, mb->d_err, mb->stream);
+    if (e == cudaSuccess) e = reset_acc(mb, mb->stream);
     if (e == cudaSuccess) e = enqueue_program(mb, mb->pair_prog[0]);
     const auto range = pair_out_range(mb, 0);
     if (e == cudaSuccess)

@@ -51,7 +51,6 @@ struct SrvSlot {
     int refs = 0;              // requests queued or in flight that match against it
     int producer_launch = -1;  // in-flight launch that writes its features, or -1
     uint8_t* h_in = nullptr;   // pinned staging of the frame
-    int32_t* a2b = nullptr;    // pair scratch when this slot is the current frame
     uint4* bacc = nullptr;     // k_match's b -> a accumulators when this slot is the current frame
     int32_t* matches = nullptr;
     uint32_t* match_count = nullptr;
@@ -272,7 +271,9 @@ cudaError_t launch_batch(uslam_server* s, const std::vector<uint64_t>& tickets, 
             PairDev P{};
             P.prev = r.ref;
             P.curr = r.slot;
-            P.a2b = sl.a2b;
+            // the a -> b accumulators lie where the matches go: k_mutual has read
+            // an entry before it writes a match there (entry i, match <= i)
+            P.aacc = reinterpret_cast<uint4*>(sl.matches);
             P.bacc = sl.bacc;
             P.matches = sl.matches;
             P.match_count = sl.match_count;
@@ -335,8 +336,8 @@ cudaError_t launch_batch(uslam_server* s, const std::vector<uint64_t>& tickets, 
     if (!pairs.empty()) {
         if ((e = launch_bacc_init(s->d_frames, d_pairs, d_usegs, static_cast<int>(usegs.size()), st)) != cudaSuccess)
             return e;
-        if ((e = launch_match(s->d_frames, d_pairs, d_msegs, static_cast<int>(msegs.size()), c->num_sms, st)) !=
-            cudaSuccess)
+        if ((e = launch_match_parts(s->d_frames, d_pairs, d_msegs, static_cast<int>(msegs.size()), c->num_sms, nullptr,
+                                    st)) != cudaSuccess)
             return e;
         if ((e = launch_mutual(s->d_frames, d_pairs, d_usegs, static_cast<int>(usegs.size()), s->d_err, st)) !=
             cudaSuccess)
@@ -476,7 +477,7 @@ uslam_status uslam_server_create(uslam_ctx* ctx, const uslam_server_params* p, u
     struct SlotLayout {
         size_t bytes, in, counts, lvl[USLAM_MAX_LEVELS], blur[USLAM_MAX_LEVELS], kpmap[USLAM_MAX_LEVELS],
             feats[USLAM_MAX_LEVELS], xorder[USLAM_MAX_LEVELS], colstart[USLAM_MAX_LEVELS], qorder[USLAM_MAX_LEVELS], bands[USLAM_MAX_LEVELS],
-            btile[USLAM_MAX_LEVELS], a2b, bacc, matches, mcount,
+            btile[USLAM_MAX_LEVELS], bacc, matches, mcount,
             tmaps;
     };
     std::vector<SlotLayout> lay(p->n_sizes);
@@ -547,7 +548,6 @@ uslam_status uslam_server_create(uslam_ctx* ctx, const uslam_server_params* p, u
                     C.desc.push_back(bi);
                 }
             }
-        Y.a2b = take(static_cast<size_t>(L) * capa * 4);
         Y.bacc = take(static_cast<size_t>(L) * capa * 16);
         Y.matches = take(static_cast<size_t>(L) * capa * 16);
         Y.mcount = take(sizeof(uint32_t) * L);
@@ -625,7 +625,6 @@ uslam_status uslam_server_create(uslam_ctx* ctx, const uslam_server_params* p, u
             s->frames[g] = F;
             SrvSlot& sl = s->slots[g];
             sl.cls = k;
-            sl.a2b = reinterpret_cast<int32_t*>(base + Y.a2b);
             sl.bacc = reinterpret_cast<uint4*>(base + Y.bacc);
             sl.matches = reinterpret_cast<int32_t*>(base + Y.matches);
             sl.match_count = reinterpret_cast<uint32_t*>(base + Y.mcount);

@@ -109,7 +109,7 @@ struct FrameDev {
 // One frame pair to match: prev = reference set (a), curr = current set (b).
 struct PairDev {
     int prev, curr;         // frame indices in the batch
-    int32_t* a2b;           // [levels * cap_prev]: prev feature -> packed curr feature or -1
+    int32_t* a2b;           // [levels * cap_prev]: prev feature -> packed curr feature or -1 (null with aacc)
     int32_t* b2a;           // [levels * cap_curr] (the tensor-core windowed matcher)
     // k_match's search of each curr feature b (levels * cap_curr entries of
     // 16 bytes): .x = packed (level, index) and .y = distance of its nearest
@@ -117,6 +117,9 @@ struct PairDev {
     // Merged by atomic minima (.x/.y as one 64-bit word); null with the
     // other matchers.
     uint4* bacc;
+    // the same for each prev feature a (levels * cap_prev), where several work
+    // units share a's search; null where one unit has it, which writes a2b
+    uint4* aacc;
     int32_t* matches;       // 4 ints per match (lod_a, idx_a, lod_b, idx_b)
     uint32_t* match_count;  // [levels] matches whose a lies in that level
     int max_matches_per_level;
