@@ -82,19 +82,21 @@ __device__ __forceinline__ int edge_index(float f, int n) {
     return (int)f;
 }
 
-__device__ __forceinline__ int nonzero_bytes(uint32_t v) {
-    return __popc(__vcmpne4(v, 0u)) >> 3;
+// The top bit of each byte that is not 0.
+__device__ __forceinline__ uint32_t nonzero_tops(uint32_t v) {
+    return (((v & 0x7f7f7f7fu) + 0x7f7f7f7fu) | v) & 0x80808080u;
 }
-
+// Bit b of the result: byte b is not 0 (the product gathers the four bits, no
+// two of its terms meet).
+__device__ __forceinline__ uint32_t nonzero_mask(uint32_t v) { return ((nonzero_tops(v) >> 7) * 0x10204080u) >> 28; }
+__device__ __forceinline__ uint32_t nonzero_mask16(const uint4& v) {
+    return nonzero_mask(v.x) | nonzero_mask(v.y) << 4 | nonzero_mask(v.z) << 8 | nonzero_mask(v.w) << 12;
+}
 __device__ __forceinline__ uint32_t nonzero_bytes16(const uint4& v) {
-    return (uint32_t)(nonzero_bytes(v.x) + nonzero_bytes(v.y) + nonzero_bytes(v.z) + nonzero_bytes(v.w));
+    return (uint32_t)__popc(nonzero_tops(v.x) | nonzero_tops(v.y) >> 1 | nonzero_tops(v.z) >> 2 | nonzero_tops(v.w) >> 3);
 }
 
-__device__ __forceinline__ uint32_t warp_sum_u32(uint32_t v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
+__device__ __forceinline__ uint32_t warp_sum_u32(uint32_t v) { return __reduce_add_sync(0xffffffffu, v); }
 
 // FAST response at smem cell (r, c): 1 + longest non-wrapping run of
 // |centre - p_i| > 0.15, kept iff > 9 (detect_corners.wgsl:58-81).
@@ -937,28 +939,28 @@ __device__ __forceinline__ void write_header(uint32_t* feats, uint32_t pos, int 
         make_uint4(__float_as_uint((float)x), __float_as_uint((float)y), s, 0u);
 }
 
-// One lane's 32-pixel row segment of a 32x32 cell (bytes at x >= w zeroed).
-__device__ __forceinline__ void load_cell_row(const uint8_t* kp, int kpitch, int w, int h, int x0, int y,
-                                              uint32_t v[8]) {
-#pragma unroll
-    for (int k = 0; k < 8; ++k) v[k] = 0u;
-    if (y >= h) return;
+// One lane's 32-pixel row segment of a 32x32 cell (the map's padding beyond w is 0).
+__device__ __forceinline__ void load_cell_row(const uint8_t* kp, int kpitch, int w, int h, int x0, int y, uint4 (&v)[2]) {
     const uint8_t* row = kp + (size_t)y * kpitch + x0;
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
-        if (x0 + 16 * j < w) {  // then x0 + 16 j + 16 <= kpitch (a multiple of 16)
-            const uint4 q = *reinterpret_cast<const uint4*>(row + 16 * j);
-            v[4 * j] = q.x;
-            v[4 * j + 1] = q.y;
-            v[4 * j + 2] = q.z;
-            v[4 * j + 3] = q.w;
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        const int rem = w - (x0 + 4 * k);
-        if (rem <= 0) v[k] = 0u;
-        else if (rem < 4) v[k] &= (1u << (8 * rem)) - 1u;
+    for (int j = 0; j < 2; ++j)  // x0 + 16 j + 16 <= kpitch (a multiple of 16)
+        v[j] = y < h && x0 + 16 * j < w ? *reinterpret_cast<const uint4*>(row + 16 * j) : make_uint4(0u, 0u, 0u, 0u);
+}
+
+// The lowest room set bits of mask, which has n.
+__device__ __forceinline__ uint32_t first_bits(uint32_t mask, uint32_t n, uint32_t room) {
+    for (; n > room; --n) mask ^= 1u << (31 - __clz((int)mask));
+    return mask;
+}
+// A lane's keypoints in order: bit b of mask is one at x + b with the strength
+// in byte b of v.  Every lane takes its own next keypoint, so a warp's steps
+// are the most of a lane (2 or 3) instead of all 16 bytes.
+__device__ __forceinline__ void write_headers16(uint32_t* feats, uint32_t mask, const uint4& v, uint32_t pos, int x, int y) {
+    while (mask) {
+        const int b = __ffs((int)mask) - 1;
+        mask &= mask - 1u;
+        const uint32_t s = b < 8 ? __byte_perm(v.x, v.y, b & 7) : __byte_perm(v.z, v.w, b & 7);
+        write_header(feats, pos++, x + b, y, s & 0xffu);
     }
 }
 
@@ -1132,12 +1134,9 @@ k_band_count(const FrameDev* __restrict__ frames, const BandItem* __restrict__ i
     const uint32_t ccap = (uint32_t)F.cell_cap;
     uint32_t r = 0, k = 0;
     for (int cx = warp; cx * 32 < w; cx += KBAND_WARPS) {
-        uint32_t v[8];
+        uint4 v[2];
         load_cell_row(F.kpmap[l], F.kp_pitch[l], w, h, cx * 32, it.band * 32 + lane, v);
-        uint32_t n = 0;
-#pragma unroll
-        for (int q = 0; q < 8; ++q) n += (uint32_t)nonzero_bytes(v[q]);
-        n = warp_sum_u32(n);
+        const uint32_t n = warp_sum_u32(nonzero_bytes16(v[0]) + nonzero_bytes16(v[1]));
         r += n;
         k += n < ccap ? n : ccap;
     }
@@ -1255,22 +1254,14 @@ k_band_write(const FrameDev* __restrict__ frames, const BandItem* __restrict__ i
         for (int x0 = 0; y < h && x0 < w && running < cap; x0 += 512) {
             const int x = x0 + 16 * lane;
             const uint4 v = map16(row, x, w);
-            const uint32_t n = nonzero_bytes16(v);
+            uint32_t mask = nonzero_mask16(v);
+            const uint32_t n = (uint32_t)__popc(mask);
             const uint32_t incl = warp_inclusive_scan(n, lane);
-            uint32_t pos = running + incl - n;
-            const uint32_t words[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                if (words[q] == 0u || pos >= cap) continue;
-                s_note[warp >> 3][(x >> 3) + (q >> 1)] = 1;
-#pragma unroll
-                for (int b = 0; b < 4; ++b) {
-                    const uint32_t sv = (words[q] >> (8 * b)) & 0xffu;
-                    if (sv == 0u) continue;
-                    if (pos < cap) write_header(feats, pos, x + 4 * q + b, y, sv);
-                    ++pos;
-                }
-            }
+            const uint32_t pos = running + incl - n;
+            mask = first_bits(mask, n, pos < cap ? cap - pos : 0u);
+            if (mask & 0x00ffu) s_note[warp >> 3][x >> 3] = 1;
+            if (mask & 0xff00u) s_note[warp >> 3][(x >> 3) + 1] = 1;
+            write_headers16(feats, mask, v, pos, x, y);
             running += __shfl_sync(0xffffffffu, incl, 31);
         }
     } else {
@@ -1282,13 +1273,10 @@ k_band_write(const FrameDev* __restrict__ frames, const BandItem* __restrict__ i
         uint32_t base = prefix;
         for (int c0 = 0; c0 < ncx; c0 += KBAND_WARPS) {
             const int cx = c0 + warp;
-            uint32_t v[8];
-            uint32_t n = 0;
-            if (cx < ncx) {
-                load_cell_row(kp, kpitch, w, h, cx * 32, y, v);
-#pragma unroll
-                for (int q = 0; q < 8; ++q) n += (uint32_t)nonzero_bytes(v[q]);
-            }
+            uint4 v[2] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
+            if (cx < ncx) load_cell_row(kp, kpitch, w, h, cx * 32, y, v);
+            uint32_t mask = nonzero_mask16(v[0]) | nonzero_mask16(v[1]) << 16;
+            const uint32_t n = (uint32_t)__popc(mask);
             const uint32_t incl = warp_inclusive_scan(n, lane);
             const uint32_t tot = __shfl_sync(0xffffffffu, incl, 31);
             if (lane == 0) s_cell[warp] = min(tot, ccap);
@@ -1296,22 +1284,14 @@ k_band_write(const FrameDev* __restrict__ frames, const BandItem* __restrict__ i
             const uint32_t mine = s_cell[lane];
             const uint32_t running = base + warp_sum_u32(lane < warp ? mine : 0u);
             base += warp_sum_u32(mine);
-            uint32_t rank = incl - n;
-            if (cx < ncx) {
+            const uint32_t rank = incl - n, end = running < cap ? min(ccap, cap - running) : 0u;
+            mask = first_bits(mask, n, rank < end ? end - rank : 0u);
 #pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    if (v[q] == 0u || rank >= ccap || running + rank >= cap) continue;
-                    s_note[lane >> 3][4 * cx + (q >> 1)] = 1;
-#pragma unroll
-                    for (int b = 0; b < 4; ++b) {
-                        const uint32_t sv = (v[q] >> (8 * b)) & 0xffu;
-                        if (sv == 0u) continue;
-                        if (rank < ccap && running + rank < cap)
-                            write_header(feats, running + rank, cx * 32 + 4 * q + b, y, sv);
-                        ++rank;
-                    }
-                }
-            }
+            for (int q = 0; q < 4; ++q)
+                if (mask & (0xffu << (8 * q))) s_note[lane >> 3][4 * cx + q] = 1;
+            const uint32_t low = (uint32_t)__popc(mask & 0xffffu);
+            write_headers16(feats, mask & 0xffffu, v[0], running + rank, cx * 32, y);
+            write_headers16(feats, mask >> 16, v[1], running + rank + low, cx * 32 + 16, y);
             __syncthreads();  // s_cell is rewritten
         }
     }
