@@ -101,7 +101,9 @@ __host__ __device__ inline int res_header_words(int L) { return (3 * L + 3) / 4 
 // header, then every kept feature (48 B) level by level, then every match
 // (16 B) level by level -- what uslam_server_result hands out, so the
 // results reach host memory with the launch and a result call reads no
-// device memory.
+// device memory.  kEmitCtas CTAs share a frame: one wrote a frame's 130 KB in 18 us,
+// latency-bound, behind everything else of a launch.
+constexpr int kEmitCtas = 8;
 __global__ void __launch_bounds__(256) k_server_emit(const FrameDev* __restrict__ frames,
                                                       const SrvEmitItem* __restrict__ items, int L) {
     __shared__ uint32_t s_cnt[2][USLAM_MAX_LEVELS];
@@ -120,25 +122,27 @@ __global__ void __launch_bounds__(256) k_server_emit(const FrameDev* __restrict_
             s_off[1][l] = mo;
             fo += k;
             mo += m;
+            if (blockIdx.y > 0) continue;
             it.out[l] = k;
             it.out[L + l] = F.raw[l];
             it.out[2 * L + l] = m;
         }
         s_off[0][L] = fo;
         s_off[1][L] = mo;
-        for (int q = 3 * L; q < hw; ++q) it.out[q] = 0u;
+        for (int q = 3 * L; q < hw && blockIdx.y == 0; ++q) it.out[q] = 0u;
     }
     __syncthreads();
     uint4* fdst = reinterpret_cast<uint4*>(it.out + hw);
     uint4* mdst = fdst + 3u * s_off[0][L];
+    const uint32_t first = blockIdx.y * blockDim.x + threadIdx.x, step = gridDim.y * blockDim.x;
     for (int l = 0; l < L; ++l) {
         const uint4* src = reinterpret_cast<const uint4*>(F.feats[l]);
         uint4* dst = fdst + 3u * s_off[0][l];
-        for (uint32_t i = threadIdx.x; i < 3u * s_cnt[0][l]; i += blockDim.x) dst[i] = src[i];
+        for (uint32_t i = first; i < 3u * s_cnt[0][l]; i += step) dst[i] = src[i];
         if (it.per > 0) {
             const uint4* msrc = reinterpret_cast<const uint4*>(it.matches) + (size_t)l * it.per;
             uint4* md = mdst + s_off[1][l];
-            for (uint32_t i = threadIdx.x; i < s_cnt[1][l]; i += blockDim.x) md[i] = msrc[i];
+            for (uint32_t i = first; i < s_cnt[1][l]; i += step) md[i] = msrc[i];
         }
     }
 }
@@ -344,7 +348,7 @@ cudaError_t launch_batch(uslam_server* s, const std::vector<uint64_t>& tickets, 
             return e;
     }
     // every frame's features and matches to its slot's host result area
-    k_server_emit<<<static_cast<int>(emits.size()), 256, 0, st>>>(s->d_frames, d_emits, lv);
+    k_server_emit<<<dim3(static_cast<unsigned>(emits.size()), kEmitCtas), 256, 0, st>>>(s->d_frames, d_emits, lv);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     // the error word (kernel bounds checks, tile-load wait limits) travels
     // with the launch and is read when the launch completes
