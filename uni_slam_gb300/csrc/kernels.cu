@@ -393,8 +393,9 @@ k_pyramid(const FrameDev* __restrict__ frames, const TileItem* __restrict__ tile
 // the listed ones 32 at a time, so the full circle runs on full warps.  On
 // the 752x480 workload 5 % of the pixels are listed, while nearly every warp
 // ran the circle for one lane or another: 32 frames 0.155 -> 0.100 ms; the cfg
-// profile on 16 frames 0.29 -> 0.144.  Issue-bound still (71 %), 8 CTAs of 32
-// registers per SM.  A persistent form with the next tile's load in flight was
+// profile on 16 frames 0.29 -> 0.144.  Issue-bound still, 8 CTAs of 32 registers
+// per SM; the mask's bits by one lane per 32 pixels, joined to the ballot, took it
+// to 0.084 (eight 3840x2160 frames 482 -> 404 us).  A persistent form with the next tile's load in flight was
 // slower (0.140): the CTAs of a launch already hide each other's loads.
 // The strengths go through shared memory to 16-byte stores, whose nonzero
 // bytes are the band's keypoint counts (without per-cell caps).
@@ -537,29 +538,36 @@ k_detect(const FrameDev* __restrict__ frames, const TileItem* __restrict__ tiles
         }
         __syncwarp();
     } else {
-        // 2. the warp's rows: the cull mask (resources/cull_corners.wgsl; 32
-        //    bits of it per segment), then points 7 and 8, which every
+        // 2. the warp's rows, 32 pixels at a time: the cull mask
+        //    (resources/cull_corners.wgsl; a lane has one segment's bits, none
+        //    outside the level), then points 7 and 8, which every
         //    non-wrapping run of 9 holds, and 4 or 12, one of which it holds
-        const uint32_t* mask = F.mask[l];
-        const int last = (w * h - 1) >> 5;  // (a level holds fewer than 2^31 pixels)
-#pragma unroll
-        for (int rr = 0; rr < ROWS; ++rr) {
-            const int ty = warp * ROWS + rr, y = Y0 + ty;
-            if (y >= h) break;
-#pragma unroll
-            for (int s = 0; s < TW / 32; ++s) {
-                const int tx = 32 * s + lane, x = X0 + tx;
-                const int p0 = y * w + X0 + 32 * s, q0 = p0 >> 5;
-                const uint32_t m = __funnelshift_r(__ldg(mask + min(q0, last)), __ldg(mask + min(q0 + 1, last)), p0 & 31);
-                const int r = ty + HY, c = tx + HX;
-                const float center = sm[r][c];
-                const float d7 = fabsf(center - sm[r + 3][c + 1]), d8 = fabsf(center - sm[r + 3][c]);
-                const float d4 = fabsf(center - sm[r][c + 3]), d12 = fabsf(center - sm[r][c - 3]);
-                const bool pass = (x < w) & ((m >> lane) & 1u) & (fminf(fminf(d7, d8), fmaxf(d4, d12)) > 0.15f);
-                const uint32_t b = __ballot_sync(0xffffffffu, pass);
-                if (pass) list[nlist + __popc(b & below)] = (uint16_t)(ty * TW + tx);
-                nlist += __popc(b);
+        constexpr int SEGS = TW / 32;
+        static_assert(ROWS * SEGS <= 32, "a lane per segment");
+        uint32_t mine = 0u;
+        {
+            const uint32_t* mask = F.mask[l];
+            const int last = (w * h - 1) >> 5;  // (a level holds fewer than 2^31 pixels)
+            const int y = Y0 + warp * ROWS + lane / SEGS, x = X0 + 32 * (lane % SEGS);
+            if (lane < ROWS * SEGS && y < h && x < w) {
+                const int p0 = y * w + x, q0 = p0 >> 5;
+                mine = __funnelshift_r(__ldg(mask + min(q0, last)), __ldg(mask + min(q0 + 1, last)), p0 & 31);
+                if (w - x < 32) mine &= (1u << (w - x)) - 1u;
             }
+        }
+#pragma unroll
+        for (int k = 0; k < ROWS * SEGS; ++k) {
+            const uint32_t m = __shfl_sync(0xffffffffu, mine, k);
+            if (m == 0u) continue;
+            const int ty = warp * ROWS + k / SEGS, tx = 32 * (k % SEGS) + lane;
+            const int r = ty + HY, c = tx + HX;
+            const float center = sm[r][c];
+            const float d7 = fabsf(center - sm[r + 3][c + 1]), d8 = fabsf(center - sm[r + 3][c]);
+            const float d4 = fabsf(center - sm[r][c + 3]), d12 = fabsf(center - sm[r][c - 3]);
+            const uint32_t b = __ballot_sync(0xffffffffu, fminf(fminf(d7, d8), fmaxf(d4, d12)) > 0.15f) & m;
+            if (b == 0u) continue;
+            if ((b >> lane) & 1u) list[nlist + __popc(b & below)] = (uint16_t)(ty * TW + tx);
+            nlist += __popc(b);
         }
         __syncwarp();
         // 3. the listed cells: FAST response (and the rest of the cull)
