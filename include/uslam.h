@@ -81,7 +81,7 @@ typedef struct uslam_params {
      * 2: the same brute-force top-2 with the distances from the tensor cores
      *    (popc(a & b) as an FP8 0/1 dot product, exact): identical results;
      * 3: matcher 0 (the same match lists) with the in-window distances of
-     *    the batch path taken from tensor-core tiles (k_win_mma) where every
+     *    a batch, frame or set taken from tensor-core tiles (k_win_mma) where every
      *    level holds at most 60000 features; slower than matcher 0 on the
      *    752x480 workload, kept as an option. */
     int matcher;
@@ -301,9 +301,9 @@ uslam_status uslam_batch_set_stream(uslam_batch* b, void* cuda_stream);
  * graph and without the fork, with CUDA events between them on the batch
  * stream, and return the mean milliseconds per launch in kernel_ms[0..6]:
  * pyramid (k_pyramid, one launch per tile shape), detect (k_detect, one
- * launch per tile shape), blur-cache border
- * (k_blur_border), compaction (k_band_count + k_band_write + k_xsort),
- * describe (k_describe), match (k_match, k_bruteforce with matcher 1, k_bf_mma with matcher 2) and
+ * launch per tile shape), blur cache (k_blur; it runs after the compaction,
+ * which lists its items), compaction (k_band_count with per-cell caps,
+ * k_band_write, k_xsort), describe (k_describe), match (k_match, k_bruteforce with matcher 1, k_bf_mma with matcher 2) and
  * mutual check / emit (k_mutual).  Synchronous. */
 uslam_status uslam_batch_profile(uslam_batch* b, int iters, float* kernel_ms);
 /* Test hook for the kernels' bounded waits (no reference counterpart): the

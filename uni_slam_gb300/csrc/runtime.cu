@@ -5,14 +5,15 @@
 // frames and frame pairs with every buffer carved out of one arena:
 //   [inputs: LOD0 u8 of every frame][outputs: counts + features of every
 //   frame, counts + matches of every pair][scratch: pyramid, blur cache,
-//   keypoint maps, band counts, the matcher's band lists, match directions,
-//   error word]
+//   keypoint maps, band counts, the matcher's band lists, its accumulators or
+//   match directions, error word]
 // so one H2D copy feeds the whole batch and one D2H copy returns it.  The
-// batch's launch sequence (k_detect per tile shape; k_band_count,
-// k_band_write; k_xsort on a forked branch beside k_blur; k_describe; k_match
-// or k_bruteforce; k_mutual or the emit) is captured once into a CUDA graph.
-// A frontend (uslam_frontend) is a 2-slot batch driven frame by frame with
-// the reference's FeatureSet(0)/(1) rotation.
+// batch's launch sequence (k_pyramid, k_detect per tile shape; k_band_count
+// with per-cell caps, k_band_write; k_xsort on a forked branch beside k_blur;
+// k_describe; k_match, k_bruteforce or k_bf_mma; k_mutual or the emit) is
+// captured once into a CUDA graph.  A frontend (uslam_frontend) is a 2-slot
+// batch driven frame by frame with the reference's FeatureSet(0)/(1)
+// rotation, a graph per slot.
 #include <cuda.h>  // CUtensorMap and its encode enums (types only: the entry point comes through the runtime)
 #include <cuda_runtime.h>
 
@@ -99,7 +100,7 @@ struct uslam_batch {
     cudaEvent_t ev_start = nullptr;
     Program full;
     // the windowed matcher on the tensor cores (k_describe<WIN> / k_win_plan /
-    // k_win_mma; else k_match): matcher 0 with list positions within 16 bits
+    // k_win_mma; else k_match): matcher 3 with list positions within 16 bits
     bool win_tc = false;
     int win_umax = 0;  // unit slots per (pair, direction, level)
     std::vector<Program> frame_prog;  // per frame: detect+describe only
@@ -408,9 +409,8 @@ uslam_status create_batch(uslam_ctx* ctx, int n_frames, const int* widths, const
             btile[USLAM_MAX_LEVELS], counts,
             tmaps, bf8, bfext, bfpop, bfid, wq8, wc8, wcext, wcy, wcid, winv[USLAM_MAX_LEVELS];
     };
-    // the windowed tensor-core matcher (matcher 3, or matcher 0 in the
-    // one-frame forms): every list position and candidate row within 16 bits,
-    // else k_match
+    // the windowed tensor-core matcher (matcher 3): every list position and
+    // candidate row within 16 bits, else k_match
     int max_cap = 1;
     for (int f = 0; f < n_frames; ++f) {
         const long long c = ctx->cap_override > 0 ? ctx->cap_override : static_cast<long long>(widths[f]) * heights[f] / 250;

@@ -1,5 +1,5 @@
 // win_tc.cu — the reference's windowed mutual matcher with the Hamming
-// distances from the tensor cores (tcgen05): the batch path of matcher 0.
+// distances from the tensor cores (tcgen05): matcher 3.
 //
 // FindMatchesInLod (match_features_cpu.cpp:66-150): for every query, the
 // features of the other frame's same level and its two neighbours whose

@@ -11,8 +11,9 @@ from . import capi
 from .capi import FEATURE_DTYPE, MATCH_DTYPE, USlamError, iptr, ptr
 
 
-# stages timed by uslam_batch_profile (the compaction stage is three kernels:
-# k_band_count, k_band_write, k_xsort)
+# stages timed by uslam_batch_profile (the compaction stage is k_band_write and
+# k_xsort, with per-cell caps k_band_count too; k_blur_border is the whole blur
+# cache, evaluated by k_blur, under the name its stage has had)
 KERNELS = ("k_pyramid", "k_detect", "k_blur_border", "compaction", "k_describe", "k_match", "k_mutual")
 
 
