@@ -43,3 +43,29 @@ def test_cfg_profile_bit_exact(brief_pattern):
                 assert len(_mm(b.matches(0))) > 100
             finally:
                 b.close()
+
+
+@pytest.mark.parametrize("kind", ["noise", "steps", "dots"])
+def test_cfg_corner_arithmetic(kind):
+    """Circles of every mask: noise, pixels that differ by the threshold and a
+    step each side of it, and isolated dots (arcs of 16, both polarities)."""
+    pat = np.clip(np.rint(np.random.RandomState(5).normal(0, 6, (256, 4))), -13, 13).astype(np.int32)
+    rs, W, H = np.random.RandomState(17), 163, 121
+    if kind == "noise":
+        f = rs.randint(0, 256, (H, W))
+    elif kind == "steps":
+        f = 100 + rs.choice([-21, -20, -19, 0, 19, 20, 21], (H, W))
+    else:
+        f = np.full((H, W), 120)
+        f[5::9, 4::9] = rs.choice([0, 99, 100, 101, 139, 140, 141, 255], f[5::9, 4::9].shape)
+    f = f.astype(np.uint8)
+    exp = oracle.frame(f, pat, levels=3, cap=4000, detector=1)
+    assert exp[2].sum() > 20
+    with Context(pat, levels=3, max_width=W, max_height=H, cap_per_level=4000, detector=1) as c:
+        b = Batch(c, [(W, H)], [])
+        try:
+            b.process([f])
+            gf, gk, gr = b.features(0)
+            assert np.array_equal(gr, exp[2]) and np.array_equal(gk, exp[1]) and gf.tobytes() == exp[0].tobytes()
+        finally:
+            b.close()

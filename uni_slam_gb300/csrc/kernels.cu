@@ -123,12 +123,19 @@ __device__ __forceinline__ uint32_t fast_response(const float (*sm)[SW], int r, 
     return run;
 }
 
-// Longest run of ones of a 16-bit circle mask, wrapping around (16 if all set).
-__device__ __forceinline__ uint32_t circular_run(uint32_t m) {
+// Longest run of ones of a 16-bit circle mask, wrapping around (16 if all
+// set), where it is at least 9; else 0.
+__device__ __forceinline__ uint32_t circular_run9(uint32_t m) {
     if (m == 0xffffu) return 16u;
-    uint32_t x = m | (m << 16), run = 0;
-    while (x) {
-        x &= x << 1;
+    const uint32_t x = m | (m << 16);
+    uint32_t t = x & (x >> 1);
+    t &= t >> 2;
+    t &= t >> 4;
+    t &= x >> 8;
+    // bit i of t starts a run of 9, so n + 1 adjacent bits of t are a run of 9 + n
+    uint32_t run = t ? 8u : 0u;
+    while (t) {
+        t &= t << 1;
         ++run;
     }
     return run;
@@ -142,28 +149,26 @@ __device__ __forceinline__ uint32_t circular_run(uint32_t m) {
 template <int SW>
 __device__ __forceinline__ float cfg_corner(const float (*sm)[SW], int r, int c, uint32_t* arc) {
     const float center = sm[r][c];
+    // d = p - c; brighter: the sign of T - d, darker (c - p = -d exactly): of
+    // T + d, shifted in from point 15 down
     float d[16];
     uint32_t mb = 0, md = 0;
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        const float p = sm[r + circle_y(i)][c + circle_x(i)];
-        d[i] = p - center;
-        mb |= (d[i] > kCfgThreshold ? 1u : 0u) << i;
-        md |= ((center - p) > kCfgThreshold ? 1u : 0u) << i;
+    for (int i = 15; i >= 0; --i) {
+        d[i] = sm[r + circle_y(i)][c + circle_x(i)] - center;
+        mb = __funnelshift_l(__float_as_uint(kCfgThreshold - d[i]), mb, 1);
+        md = __funnelshift_l(__float_as_uint(kCfgThreshold + d[i]), md, 1);
     }
+    const uint32_t rb = circular_run9(mb), rd = circular_run9(md);
     *arc = 0u;
-    if (__popc(mb) < 9 && __popc(md) < 9) return 0.0f;
-    const uint32_t rb = circular_run(mb), rd = circular_run(md);
-    if (rb < 9u && rd < 9u) return 0.0f;
+    if ((rb | rd) == 0u) return 0.0f;
     const bool bright = rb >= 9u;
     const uint32_t m = bright ? mb : md;
+    const float side = bright ? 1.0f : -1.0f;
     float score = 0.0f;
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        if (!((m >> i) & 1u)) continue;
-        const float dv = bright ? d[i] : (sm[r][c] - sm[r + circle_y(i)][c + circle_x(i)]);
-        score = score + (dv - kCfgThreshold);
-    }
+    for (int i = 0; i < 16; ++i)
+        if ((m >> i) & 1u) score = score + __fmaf_rn(d[i], side, -kCfgThreshold);  // (+-d) - T, rounded once
     *arc = bright ? rb : rd;
     return score;
 }
@@ -393,14 +398,15 @@ k_pyramid(const FrameDev* __restrict__ frames, const TileItem* __restrict__ tile
 // the listed ones 32 at a time, so the full circle runs on full warps.  On
 // the 752x480 workload 5 % of the pixels are listed, while nearly every warp
 // ran the circle for one lane or another: 32 frames 0.155 -> 0.100 ms; the cfg
-// profile on 16 frames 0.29 -> 0.144.  Issue-bound still, 8 CTAs of 32 registers
+// profile on 16 frames 0.29 -> 0.144, and 0.109 with signs for its compares, the run
+// test by shifts and 5 CTAs per SM instead of 4 (6: 0.113).  Issue-bound still, 8 CTAs of 32 registers
 // per SM; the mask's bits by one lane per 32 pixels, joined to the ballot, took it
 // to 0.084 (eight 3840x2160 frames 482 -> 404 us).  A persistent form with the next tile's load in flight was
 // slower (0.140): the CTAs of a launch already hide each other's loads.
 // The strengths go through shared memory to 16-byte stores, whose nonzero
 // bytes are the band's keypoint counts (without per-cell caps).
 template <int TW, int TH, bool CFG>
-__global__ void __launch_bounds__(K1_THREADS, CFG ? 4 : 8)
+__global__ void __launch_bounds__(K1_THREADS, CFG ? 5 : 8)
 k_detect(const FrameDev* __restrict__ frames, const TileItem* __restrict__ tiles, int shape, uint32_t* err) {
     constexpr int HY = CFG ? HY_CFG : uslam::HY;
     constexpr int SW = TW + 2 * HX;                   // staged columns [X0 - HX, X0 + TW + HX)
@@ -493,14 +499,13 @@ k_detect(const FrameDev* __restrict__ frames, const TileItem* __restrict__ tiles
                     if (y >= 3 && y < h - 3 && x >= 3 && x < w - 3) {
                         const int r = sr - 1 + HY, c = sc - 1 + HX;
                         const float center = sm[r][c];
-                        int nb = 0, nd = 0;
-#pragma unroll
-                        for (int k = 0; k < 16; k += 4) {
-                            const float p = sm[r + circle_y(k)][c + circle_x(k)];
-                            nb += p - center > kCfgThreshold ? 1 : 0;
-                            nd += center - p > kCfgThreshold ? 1 : 0;
-                        }
-                        pass = nb >= 2 || nd >= 2;
+                        // two of them beyond the threshold: the second largest or smallest
+                        // is (a rounded difference does not decrease with p)
+                        const float p0 = sm[r + circle_y(0)][c + circle_x(0)], p4 = sm[r + circle_y(4)][c + circle_x(4)];
+                        const float p8 = sm[r + circle_y(8)][c + circle_x(8)], p12 = sm[r + circle_y(12)][c + circle_x(12)];
+                        const float h0 = fmaxf(p0, p4), l0 = fminf(p0, p4), h1 = fmaxf(p8, p12), l1 = fminf(p8, p12);
+                        const float large = fmaxf(fminf(h0, h1), fmaxf(l0, l1)), small = fminf(fmaxf(l0, l1), fminf(h0, h1));
+                        pass = large - center > kCfgThreshold || center - small > kCfgThreshold;
                     }
                 }
                 const uint32_t b = __ballot_sync(0xffffffffu, pass);
