@@ -168,9 +168,8 @@ uslam_status uslam_ransac_score(uslam_ctx* ctx, const double* fmats, int n_hyp, 
         e = cudaMalloc(&ctx->ransac_buf, need);
         if (e == cudaSuccess) ctx->ransac_bytes = need;
     }
-    const bool pinned = need <= PinnedBuf::kMax;
-    if (e == cudaSuccess && pinned) e = ctx->ransac_pin.reserve(need);
     if (e != cudaSuccess) return ctx->cuda_fail(e, "ransac_score: scratch");
+    const bool pinned = ctx->ransac_pin.reserve(need);
     char* base = static_cast<char*>(ctx->ransac_buf);
     double* d_f = reinterpret_cast<double*>(base);
     double2* d_p = reinterpret_cast<double2*>(base + f_b);

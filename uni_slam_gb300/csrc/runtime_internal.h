@@ -273,13 +273,18 @@ struct PinnedBuf {
     static constexpr size_t kMax = size_t(32) << 20;
     char* p = nullptr;
     size_t bytes = 0;
-    cudaError_t reserve(size_t need) {
-        if (need <= bytes) return cudaSuccess;
+    // false: too large, or refused; the call then copies directly
+    bool reserve(size_t need) {
+        if (need <= bytes) return true;
+        if (need > kMax) return false;
         release();
-        const cudaError_t e = cudaHostAlloc(&p, need, cudaHostAllocDefault);
-        if (e == cudaSuccess) bytes = need;
-        else p = nullptr;
-        return e;
+        if (cudaHostAlloc(&p, need, cudaHostAllocDefault) != cudaSuccess) {
+            cudaGetLastError();
+            p = nullptr;
+            return false;
+        }
+        bytes = need;
+        return true;
     }
     void release() {
         if (p) cudaFreeHost(p);
