@@ -13,18 +13,20 @@ pytestmark = pytest.mark.gpu
 PATTERN = np.clip(np.rint(np.random.RandomState(5).normal(0, 6, (256, 4))), -13, 13).astype(np.int32)
 
 
-def _check(frames, levels, cap, least):
+def _check(frames, levels, cap, least, copies=1):
     h, w = frames[0].shape
     exp = [oracle.frame(f, PATTERN, levels=levels, cap=cap) for f in frames]
-    pairs = [(0, 1), (1, 0)]
+    distinct = [(0, 1), (1, 0)]
+    pairs = distinct * copies
+    lists = [oracle.match(exp[p][0], exp[p][1], exp[q][0], exp[q][1], w, h) for p, q in distinct]
     with Context(PATTERN, levels=levels, max_width=w, max_height=h, cap_per_level=cap) as c:
         b = Batch(c, [(w, h)] * 2, pairs)
         try:
             b.process(frames)
-            for k, (p, q) in enumerate(pairs):
+            for k in range(len(pairs)):
                 m = b.matches(k)
                 got = np.stack([m["lod_a"], m["idx_a"], m["lod_b"], m["idx_b"]], 1) if len(m) else np.zeros((0, 4), np.int32)
-                want = oracle.match(exp[p][0], exp[p][1], exp[q][0], exp[q][1], w, h)
+                want = lists[k % 2]
                 assert np.array_equal(got, want), k
                 assert len(want) >= least
         finally:
@@ -45,3 +47,8 @@ def test_caps_at_which_bands_change(cap):
 @pytest.mark.parametrize("cap", [8191, 8192, 8193])
 def test_rounds_of_the_emit(cap):
     _check(synth.warped_pair(2024, 1920, 1080, n_rect=5000, n_check=500, scale_by_area=False), 2, cap, 500)
+
+
+def test_accumulators_emptied_by_kept_features():
+    """Caps far above what is kept (more than 64 MiB of accumulators)."""
+    _check(synth.warped_pair(41, 320, 240), 6, 60000, 100, copies=4)

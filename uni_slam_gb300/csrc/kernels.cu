@@ -15,7 +15,8 @@
 //   k_describe (K2) orientation (one lane per keypoint of a warp's group) +
 //                   256-bit rotated BRIEF (the warp's lanes take 8 tests each)
 //   k_bacc_init     empties the accumulators before a k_match (the caller-
-//                   owned and served forms; batches reset all of theirs at once)
+//                   owned and served forms, and batches of very large caps; others
+//                   reset all of theirs by a memset)
 //   k_match    (K3) windowed top-2 Hamming search of both directions, one
 //                   distance per pair; a warp claims units: 32 x-adjacent
 //                   queries of the previous set in one band against a part of

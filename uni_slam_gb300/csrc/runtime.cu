@@ -38,6 +38,12 @@ namespace {
 
 constexpr int kLanes = 2;  // parts of a split batch graph (3 measured no better)
 
+// k_match's accumulators up to this size are emptied by their caps, by a memset
+// beside the frames' kernels (64 frames of 752x480 have 17 MB, 3 us; a kernel
+// over the kept features took 5 us before each match).  Beyond it the caps may
+// be far above what is kept, and the kernel runs.
+constexpr size_t kAccMemset = size_t{64} << 20;
+
 // Batches of at least this many frames are captured as kLanes parts of their
 // frames on as many streams (see enqueue_split).
 constexpr int kSplitFrames = 16;
@@ -82,7 +88,8 @@ struct uslam_batch {
     PairDev* d_pairs = nullptr;
     uint32_t* d_err = nullptr;
     char* d_acc = nullptr;  // k_match's accumulators of all pairs
-    size_t acc_bytes = 0;
+    size_t acc_bytes = 0;      // bytes of them that reset_acc empties
+    bool acc_by_kept = false;  // k_bacc_init empties the kept features' instead
     char* d_tables = nullptr;
     // k_match's unit counters, one per lane
     char* d_claim = nullptr;
@@ -282,6 +289,7 @@ cudaError_t enqueue_pairs(uslam_batch* b, const Program& P, const Lane& ln) {
             return e;
         return launch_mutual(b->d_frames, b->d_pairs, P.usegs, P.nusegs, b->d_err, ln.st);
     }
+    if (b->acc_by_kept && (e = launch_bacc_init(b->d_frames, b->d_pairs, P.usegs, P.nusegs, ln.st)) != cudaSuccess) return e;
     if ((e = launch_match_parts(b->d_frames, b->d_pairs, P.msegs, P.nmsegs, c->num_sms, ln.claim, ln.st)) != cudaSuccess)
         return e;
     return launch_mutual_reset(b->d_frames, b->d_pairs, P.usegs, P.nusegs, b->d_err, ln.claim, ln.st);
@@ -664,7 +672,8 @@ uslam_status create_batch(uslam_ctx* ctx, int n_frames, const int* widths, const
     }
     b->d_err = reinterpret_cast<uint32_t*>(sc_base + err_off);
     b->d_acc = sc_base + acc_off;
-    b->acc_bytes = acc_bytes;
+    b->acc_by_kept = acc_bytes > kAccMemset;
+    b->acc_bytes = b->acc_by_kept ? 0 : acc_bytes;
     b->d_frames = reinterpret_cast<FrameDev*>(sc_base + frames_off);
     b->d_pairs = reinterpret_cast<PairDev*>(sc_base + pairs_off);
     e = cudaMemcpy(b->d_frames, b->frames.data(), sizeof(FrameDev) * n_frames, cudaMemcpyHostToDevice);
@@ -1222,6 +1231,7 @@ uslam_status uslam_batch_profile(uslam_batch* b, int iters, float* kernel_ms) {
             e = describe_stage(b, P, b->stream);
         mark();
         if (e == cudaSuccess) e = reset_acc(b, b->stream);
+        if (e == cudaSuccess && b->acc_by_kept) e = launch_bacc_init(b->d_frames, b->d_pairs, P.usegs, P.nusegs, b->stream);
         if (e == cudaSuccess)
             e = c->matcher == 1 ? launch_bruteforce(b->d_frames, b->d_pairs, P.psegs, P.npsegs, c->ratio, c->num_sms, b->stream)
                 : c->matcher == 2
