@@ -75,3 +75,33 @@ def test_binary32_decision_equals_binary64(n_hyp, n):
                 counts, masks = c.ransac_score(Fs * scale, p, q, thr, masks=True)
                 ec, em = oracle.sampson_counts(Fs * scale, p, q, thr)
                 assert np.array_equal(counts, ec) and np.array_equal(masks, em), (scale, thr)
+
+
+def test_binary32_decision_far_coordinates():
+    """Coordinates far beyond any frame against matrix entries below
+    binary32's range: what such an entry loses is no small part of its
+    product.  Masks equal the oracle's, for pairs that a bound relative to
+    the terms decides wrongly and for seeded ones over the whole range."""
+    rs = np.random.RandomState(11)
+    pat = np.clip(np.rint(rs.normal(0, 6, (256, 4))), -13, 13).astype(np.int32)
+    cases = [
+        ([5.19847117e-33, 2.86832077e-34, 0, 3.06804363e-47, 0, 1.35253869e-40, 6.74797655e-46, 1, -8.93523470e-09],
+         [3.36596397e+35, 2.21408643e+01, 4.32841209e-12, 1.97015855e+24], 128632.39812623641),
+        ([0, -4.21436813e-47, 0, 5.42532328e-29, 2.07247232e-22, -6.09367600e-20, 1, 2.79263952e-28, 2.31315755e-35],
+         [-3.28058936e+06, 7.43869241e+30, 1.75687029e+35, 1.45843975e+02], 22942.1580560616),
+        ([4.27588295e-38, 1.27277456e-02, -2.13807993e-45, -3.05614648e-46, -1.82482907e-20, -2.96136811e-48, 0, 1, 0],
+         [-1.19746554e+35, -2.46484468e+00, 1.43011554e-10, 1.23084452e+15], 849.8911403708065),
+    ]
+    with Context(pat, levels=6, max_width=752, max_height=480) as c:
+        for f, xy, thr in cases:
+            args = np.array([f]), np.array([xy[:2]]), np.array([xy[2:]]), thr
+            counts, masks = c.ransac_score(*args, masks=True)
+            ec, em = oracle.sampson_counts(*args)
+            assert np.array_equal(counts, ec) and np.array_equal(masks, em), (f, xy)
+        Fs = rs.normal(size=(200, 9)) * 10.0 ** rs.uniform(-48, 0, (200, 9))
+        Fs[np.arange(200), rs.randint(0, 9, 200)] = 1.0
+        xy = rs.normal(size=(500, 4)) * 10.0 ** rs.uniform(-30, 37, (500, 4))
+        for thr in (1e-5, 3.84, 1e5):
+            counts, masks = c.ransac_score(Fs, xy[:, :2], xy[:, 2:], thr, masks=True)
+            ec, em = oracle.sampson_counts(Fs, xy[:, :2], xy[:, 2:], thr)
+            assert np.array_equal(counts, ec) and np.array_equal(masks, em), thr

@@ -55,7 +55,11 @@ struct HypF {
 // and num by at most 10; 2^-20 (16 units) covers both and the rounding of the
 // bounds themselves.  The binary64 evaluation differs from the exact values by
 // 2^-49 of the same sums, far inside what is left.  NaN and infinities compare
-// false and are not certain.
+// false and are not certain.  The bounds are relative, so they miss what a
+// matrix entry or a product below binary32's normal range loses: at most 2^-150
+// each, and 9 (1 + c)^2 2^-150 in num for coordinates up to c.  For c < 1e9
+// (the caller sees to that) this is below 1e-26, against en > 1e-20 and
+// components whose squares add up to lo > 1e-20.
 __device__ __forceinline__ int sampson_certain(const HypF& H, float xp, float yp, float xc, float yc, float thr) {
     constexpr float g = 9.5367431640625e-07f;  // 2^-20
     const float* F = H.f;
@@ -120,10 +124,11 @@ k_sampson(const double* __restrict__ fmats, int n_hyp, const double2* __restrict
         q = curr[i];
     }
     const float xp = (float)p.x, yp = (float)p.y, xc = (float)q.x, yc = (float)q.y, t = (float)thr;
+    const bool usual = fabsf(xp) < 1e9f && fabsf(yp) < 1e9f && fabsf(xc) < 1e9f && fabsf(yc) < 1e9f;
     for (int k = 0; k < nh; ++k) {
         bool in = false;
         if (i < n) {
-            const int c = sampson_certain(s_h[k], xp, yp, xc, yc, t);
+            const int c = usual ? sampson_certain(s_h[k], xp, yp, xc, yc, t) : -1;
             in = c > 0;
             if (c < 0) {
                 double F[9];
