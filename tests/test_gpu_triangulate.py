@@ -182,3 +182,21 @@ def test_close_smallest_eigenvalues(own_ctx, n, seed):
     assert got["cheirality_passes"] == want["in_front"].max()
     assert min(np.abs(got["rotation"] - cands[k][0]).max() + np.abs(got["translation"] - cands[k][1]).max()
                for k in np.flatnonzero(want["in_front"] == want["in_front"].max())) <= 1e-9
+
+
+@pytest.mark.parametrize("n", [20, 80])
+@pytest.mark.parametrize("prev,curr", [(1.0, 1e19), (1.0, 1e20), (1.0, 1e21), (1.0, 1e22), (1e3, 1e21)])
+def test_spreads_beyond_binary32(own_ctx, n, prev, curr):
+    """Current points spread so far that squares of the pose's lengths leave
+    binary32's range.  No 64-bit method can tell the pose of such rows, but
+    they have one: a rotation and a direction of length 1, and as a generic
+    row is in front of both cameras for one of the four candidates, the best
+    of them has points."""
+    cam = np.array([458.0, 457.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0])
+    for seed in range(8):
+        px = np.random.RandomState(seed).normal(0, 300, (n, 4)) * [prev, prev, curr, curr]
+        r = own_ctx.triangulate(px, cam)
+        rot = r["rotation"]
+        assert r["cheirality_passes"] > 0, seed
+        assert np.abs(rot @ rot.T - np.eye(3)).max() <= 1e-9 and abs(np.linalg.det(rot) - 1.0) <= 1e-9, seed
+        assert abs(np.linalg.norm(r["translation"]) - 1.0) <= 1e-9, seed
