@@ -10,6 +10,7 @@ import pytest
 
 from oracle import triangulate as T
 from tri_check import case_opts, check_against_reference
+from tri_order import candidates
 from uni_slam_gb300 import Context, USlamError, synth
 
 pytestmark = pytest.mark.gpu
@@ -200,3 +201,25 @@ def test_spreads_beyond_binary32(own_ctx, n, prev, curr):
         assert r["cheirality_passes"] > 0, seed
         assert np.abs(rot @ rot.T - np.eye(3)).max() <= 1e-9 and abs(np.linalg.det(rot) - 1.0) <= 1e-9, seed
         assert abs(np.linalg.norm(r["translation"]) - 1.0) <= 1e-9, seed
+
+
+@pytest.mark.parametrize("n,seed", [(8, 18), (8, 384), (9, 23), (9, 214), (10, 0), (10, 381), (12, 10), (12, 135), (14, 5),
+                                    (14, 328), (70, 134), (80, 2), (80, 362)])
+def test_tie_goes_to_first_decomposed(own_ctx, n, seed):
+    """Of the candidates that tie for the most points the first in the order
+    of the cyclic decompositions counts.  In these scenes the order in which
+    the faster methods hold the candidates has another one of them first."""
+    px = np.random.RandomState(seed * 20 + n).uniform([20, 20, 20, 20], [700, 440, 700, 440], (n, 4))
+    want = T.triangulate(px, synth.SCENE_CAMERA)
+    top = want["in_front"].max()
+    assert np.count_nonzero(want["in_front"] == top) > 1
+    rays = [T.pixel_to_normalised(v, synth.SCENE_CAMERA, 20, 1e-9) for v in (px[:, :2], px[:, 2:])]
+    plain = T.decompose_essential(T.fit_essential(*rays))  # in_front's order
+    for rot, t in candidates(px, synth.SCENE_CAMERA):
+        k = int(np.argmin([np.abs(rot - a).max() + np.abs(t - b).max() for a, b in plain]))
+        if want["in_front"][k] == top:
+            break
+    got = own_ctx.triangulate(px, synth.SCENE_CAMERA)
+    assert got["cheirality_passes"] == top
+    np.testing.assert_allclose(got["rotation"], rot, rtol=0, atol=1e-9)
+    np.testing.assert_allclose(got["translation"], t, rtol=0, atol=1e-9)
