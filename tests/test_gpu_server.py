@@ -143,3 +143,35 @@ def test_failure_finishes_queued_requests(brief_pattern):
             srv.close()
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("form", [0, 1])
+@pytest.mark.parametrize("w,h,levels,cap,slot", [(752, 480, 6, 0, 11174912), (1920, 1080, 6, 0, 62504960),
+                                                 (640, 480, 6, 5000, 11812096), (64, 64, 4, 333, 287488)])
+def test_slot_bytes_of_a_budget(w, h, levels, cap, slot, form):
+    """A budget of exactly 12 slots of three matcher bands with every array of
+    its own holds 12 (more bands take no slots from it), and the lists that
+    lie in a slot's input frame change no result: 12 frames in flight equal
+    the oracle."""
+    rs = np.random.RandomState(256)
+    pat = np.clip(np.rint(rs.normal(0.0, 6.2, (256, 4))), -13, 13).astype(np.int32)
+    pat[0] = (13, 13, -13, -13)  # a blur margin of 21
+    frames = synth.plane_sequence(17, n=3, w=w, h=h)
+    kw = {"cap": cap} if cap else {}
+    exp = [oracle.frame(f, pat, levels=levels, **kw) for f in frames]
+    with Context(pat, levels=levels, max_width=w, max_height=h, cap_per_level=cap, describe_form=form) as ctx:
+        srv = Server(ctx, [(w, h)], hbm_budget_bytes=12 * slot, max_batch=12)
+        try:
+            assert srv.stats()["slots"] == 12
+            ids = [srv.open_stream(w, h) for _ in range(4)]
+            tickets = [[srv.submit(sid, f) for sid in ids] for f in frames]
+            for i, row in enumerate(tickets):
+                for t in row:
+                    srv.wait(t, 60000)
+                    f, kept, raw, m, _ = srv.result(t)
+                    assert f.tobytes() == exp[i][0].tobytes() and np.array_equal(raw, exp[i][2])
+                    if i:
+                        em = oracle.match(exp[0][0], exp[0][1], exp[i][0], exp[i][1], w, h)
+                        assert np.array_equal(_rows(m), em), i
+        finally:
+            srv.close()

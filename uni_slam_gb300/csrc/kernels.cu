@@ -1731,7 +1731,6 @@ k_describe_tiled(const FrameDev* __restrict__ frames, const BandItem* __restrict
                  const int32_t* __restrict__ pattern, uint32_t* err) {
     extern __shared__ __align__(128) float s_box[];  // [BH][BW] blur-cache box
     __shared__ float4 s_pat[256];
-    __shared__ float s_lut[256];
     __shared__ uint32_t s_list[KDT_THREADS];
     __shared__ uint32_t s_wcount[KDT_WARPS];
     __shared__ uint32_t s_pos[2];
@@ -1776,7 +1775,6 @@ k_describe_tiled(const FrameDev* __restrict__ frames, const BandItem* __restrict
     for (int i = t; i < 256; i += KDT_THREADS) {
         s_pat[i] = make_float4((float)pattern[4 * i], (float)pattern[4 * i + 1], (float)pattern[4 * i + 2],
                                (float)pattern[4 * i + 3]);
-        s_lut[i] = (float)i / 255.0f;
     }
     const uint32_t pos0 = s_pos[0], pos1 = s_pos[1];
     const uint32_t* feats = F.feats[l];
@@ -1791,7 +1789,7 @@ k_describe_tiled(const FrameDev* __restrict__ frames, const BandItem* __restrict
         }
         const uint32_t bal = __ballot_sync(0xffffffffu, sel);
         if (lane == 0) s_wcount[warp] = (uint32_t)__popc(bal);
-        __syncthreads();  // also the pattern and the lookup table of the first round
+        __syncthreads();  // also the pattern of the first round
         uint32_t off = 0, nsel = 0;
         for (int q = 0; q < KDT_WARPS; ++q) {
             off += q < warp ? s_wcount[q] : 0u;
@@ -1818,8 +1816,7 @@ k_describe_tiled(const FrameDev* __restrict__ frames, const BandItem* __restrict
             for (int k = 0; k < 29; ++k) {
                 const int cx = tint_clamp(x + kdx[k], w);
                 const int cy = tint_clamp(y + kdy[k], h);
-                const float v = l == 0 ? s_lut[__ldg(F.img + (size_t)cy * F.img_pitch + cx)]
-                                       : __ldg(lvl + (size_t)cy * (size_t)lp + cx);
+                const float v = __ldg(lvl + (size_t)cy * (size_t)lp + cx);
                 m10 = m10 + (float)kdx[k] * v;
                 m01 = m01 + (float)kdy[k] * v;
             }

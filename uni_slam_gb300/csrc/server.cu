@@ -510,35 +510,62 @@ uslam_status uslam_server_create(uslam_ctx* ctx, const uslam_server_params* p, u
                 return set_err(&ctx->err, USLAM_INVALID_ARG, "server_create: empty pyramid level");
             }
         F.cap = ctx->cap_override > 0 ? ctx->cap_override : static_cast<int>(static_cast<long long>(W0) * H0 / 250);
-        F.nbands = match_bands_for(F.cap, false);
-        s->max_bands = std::max(s->max_bands, F.nbands);
         const size_t capa = static_cast<size_t>(std::max(F.cap, 1));
-        SlotLayout& Y = lay[k];
-        size_t cur = 0;
-        auto take = [&cur](size_t n) {
-            const size_t o = round_up(cur, 256);
-            cur = o + n;
-            return o;
-        };
-        Y.in = take(static_cast<size_t>(H0) * F.img_pitch);
-        Y.counts = take(2 * sizeof(uint32_t) * L);
-        SrvClass C;
-        C.W0 = W0;
-        C.H0 = H0;
         for (int l = 0; l < L; ++l) {
             F.kp_pitch[l] = static_cast<int>(round_up(static_cast<size_t>(F.w[l]), 16));
             F.bl_pitch[l] = lvl_pitch_of(F.w[l] + ctx->margin + 1);  // 16-byte rows (TMA)
             F.lvl_pitch[l] = lvl_pitch_of(F.w[l]);
-            Y.feats[l] = take(capa * 48);
-            Y.lvl[l] = take(static_cast<size_t>(F.h[l]) * F.lvl_pitch[l] * 4);
-            Y.blur[l] = take(static_cast<size_t>(F.h[l] + ctx->margin + 1) * F.bl_pitch[l] * 4);
-            Y.kpmap[l] = take(static_cast<size_t>(F.h[l]) * F.kp_pitch[l]);
-            Y.xorder[l] = take(F.nbands * capa * 4);
-            Y.colstart[l] = take((F.nbands * (static_cast<size_t>(F.w[l]) + 1) + F.nbands + 1) * 4);
-            Y.qorder[l] = take(capa * 4);
-            Y.bands[l] = take(static_cast<size_t>((F.h[l] + 31) / 32) * 8);
-            Y.btile[l] = take(sizeof(uint32_t) * USLAM_BLUR_TILES(F.w[l], F.h[l], F.margin));
         }
+        // A slot with nb matcher bands; its bytes.  Two arrays lie in memory that
+        // the launch is done with or does not use yet: the marks of the blur
+        // tiles (k_pyramid, k_band_write) in the blur cache, which is larger
+        // and not written before them, and (unless own_lists) the candidate lists (k_xsort,
+        // k_match) in the input frame, which k_pyramid alone reads, as many
+        // levels' as fit.
+        SlotLayout& Y = lay[k];
+        auto lay_out = [&](int nb, bool own_lists) {
+            size_t cur = 0, in_used = 0;
+            const size_t in_bytes = static_cast<size_t>(H0) * F.img_pitch, lists = round_up(nb * capa * 4, 16);
+            auto take = [&cur](size_t n) {
+                const size_t o = round_up(cur, 256);
+                cur = o + n;
+                return o;
+            };
+            Y.in = take(in_bytes);
+            Y.counts = take(2 * sizeof(uint32_t) * L);
+            for (int l = 0; l < L; ++l) {
+                Y.feats[l] = take(capa * 48);
+                Y.lvl[l] = take(static_cast<size_t>(F.h[l]) * F.lvl_pitch[l] * 4);
+                Y.blur[l] = Y.btile[l] = take(static_cast<size_t>(F.h[l] + ctx->margin + 1) * F.bl_pitch[l] * 4);
+                Y.kpmap[l] = take(static_cast<size_t>(F.h[l]) * F.kp_pitch[l]);
+                if (!own_lists && in_used + lists <= in_bytes) {
+                    Y.xorder[l] = Y.in + in_used;
+                    in_used += lists;
+                } else {
+                    Y.xorder[l] = take(lists);
+                }
+                Y.colstart[l] = take((nb * (static_cast<size_t>(F.w[l]) + 1) + nb + 1) * 4);
+                Y.qorder[l] = take(capa * 4);
+                Y.bands[l] = take(static_cast<size_t>((F.h[l] + 31) / 32) * 8);
+            }
+            Y.bacc = take(static_cast<size_t>(L) * capa * 16);
+            Y.matches = take(static_cast<size_t>(L) * capa * 16);
+            Y.mcount = take(sizeof(uint32_t) * L);
+            Y.tmaps = take(static_cast<size_t>(L) * USLAM_TMAPS_PER_LEVEL * USLAM_TMAP_BYTES);
+            Y.bytes = round_up(cur, 256);
+            return Y.bytes;
+        };
+        // More bands take memory from the budget's slots: no more of them than
+        // leave a slot within three bands with lists of their own (the full
+        // number for the default caps up to 1920x1080, 12 of 14 at 3840x2160).
+        const size_t most = lay_out(3, true);
+        F.nbands = match_bands_for(F.cap, false);
+        while (F.nbands > 3 && lay_out(F.nbands, false) > most) --F.nbands;
+        lay_out(F.nbands, false);
+        s->max_bands = std::max(s->max_bands, F.nbands);
+        SrvClass C;
+        C.W0 = W0;
+        C.H0 = H0;
         C.shape = ctx->shape_for(W0, H0);
         append_tiles(&C.tiles, 0, F, C.shape);
         for (int l = 0; l < L; ++l)
@@ -552,11 +579,6 @@ uslam_status uslam_server_create(uslam_ctx* ctx, const uslam_server_params* p, u
                     C.desc.push_back(bi);
                 }
             }
-        Y.bacc = take(static_cast<size_t>(L) * capa * 16);
-        Y.matches = take(static_cast<size_t>(L) * capa * 16);
-        Y.mcount = take(sizeof(uint32_t) * L);
-        Y.tmaps = take(static_cast<size_t>(L) * USLAM_TMAPS_PER_LEVEL * USLAM_TMAP_BYTES);
-        Y.bytes = round_up(cur, 256);
         C.tiles_per_frame = static_cast<int>(C.tiles.size());
         C.blur_tiles = blur_tiles_of(F);
         max_blur = std::max(max_blur, C.blur_tiles);
