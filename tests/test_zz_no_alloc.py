@@ -224,3 +224,42 @@ def test_noalloc_rejects_records_outside_level():
         st = call(g, f) if which == 0 else call(f, g)
         assert st == capi.INVALID_ARG and b"inside its level" in err.value, (bad_x, st, err.value)
     assert call(f, f) == capi.OK, err.value.decode()
+
+
+def test_noalloc_largest_sets():
+    """Sets whose lists take all of the fixed scratch (13201 and 13194
+    features in one level, 4 MiB to the byte) are matched; a few features
+    more are refused."""
+    import torch
+
+    import oracle
+
+    lib = capi.load()
+    W, H, L, na, nb = 752, 480, 6, 13201, 13194
+    rs = np.random.RandomState(4)
+    at = np.sort(rs.choice(W * H, na, replace=False))
+    fa = np.zeros(na, oracle.FEATURE_DTYPE)
+    fa["x"], fa["y"], fa["strength"] = at % W, at // W, 12
+    fa["descriptor"] = rs.randint(0, 2**32, size=(na, 8), dtype=np.uint64).astype(np.uint32)
+    fb = fa[:nb].copy()
+    fb["descriptor"][:, 0] ^= rs.randint(0, 2**32, size=nb, dtype=np.uint64).astype(np.uint32)
+    ka, kb = np.array([na, 0, 0, 0, 0, 0], np.int32), np.array([nb, 0, 0, 0, 0, 0], np.int32)
+    da = torch.from_numpy(fa.view(np.uint8).copy()).cuda()
+    db = torch.from_numpy(fb.view(np.uint8).copy()).cuda()
+    out = torch.zeros((L * na * 4,), dtype=torch.int32, device="cuda")
+    counts = torch.zeros(L, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    err = C.create_string_buffer(256)
+
+    def call(a, b, cap):
+        return lib.uslam_match_noalloc(0, W, H, L, C.c_void_p(da.data_ptr()), capi.iptr(a), C.c_void_p(db.data_ptr()),
+                                       capi.iptr(b), C.c_void_p(out.data_ptr()), C.c_void_p(counts.data_ptr()), cap,
+                                       C.c_void_p(torch.cuda.current_stream().cuda_stream), err, len(err))
+
+    assert call(ka, kb, na) == capi.OK, err.value.decode()
+    n = counts.cpu().numpy()
+    got = out.cpu().numpy().reshape(L, na, 4)[0, :n[0]]
+    assert n[1:].sum() == 0 and n[0] > 13000
+    assert np.array_equal(got, oracle.match(fa, ka, fb, kb, W, H))
+    more = np.array([na + 11, 0, 0, 0, 0, 0], np.int32)  # refused on the host, before any device work
+    assert call(more, kb, na + 11) == capi.CAPACITY and b"fixed maximum" in err.value

@@ -56,6 +56,7 @@ struct NoallocTables {
     SegDev usegs[USLAM_MAX_LEVELS];
     SegDev xsegs[2 * USLAM_MAX_LEVELS];
     uint32_t counts[2][2 * USLAM_MAX_LEVELS];  // per frame: kept[levels], raw[levels]
+    uint32_t err;                              // the call's error word
 };
 
 __global__ void k_noalloc_tables(const NoallocTables t, NoallocTables* dst) {
@@ -205,7 +206,7 @@ extern "C" uslam_status uslam_match_noalloc(int device, int width, int height, i
         return fail(err, err_len, USLAM_INVALID_ARG, "match_noalloc: out_cap_per_level below the previous set's largest level");
 
     // scratch layout: [tables][xorder, qorder f0][xorder, qorder f1][colstart f0][colstart f1][a2b][b -> a
-    // accumulators][error]
+    // accumulators]
     // (per level: kBands candidate lists of cap entries, the query order, and per band
     // the column table, then the band offsets)
     size_t cur = align256(sizeof(NoallocTables));
@@ -226,8 +227,6 @@ extern "C" uslam_status uslam_match_noalloc(int device, int width, int height, i
     cur = align256(cur + sizeof(int32_t) * static_cast<size_t>(levels) * cap[0]);
     const size_t bacc_off = cur;
     cur = align256(cur + 16u * static_cast<size_t>(levels) * cap[1]);
-    const size_t err_off = cur;
-    cur += 256;
     if (cur > kNoallocScratchBytes) {
         char msg[160];
         std::snprintf(msg, sizeof msg, "match_noalloc: needs %zu bytes of scratch, the fixed maximum is %zu", cur,
@@ -287,12 +286,11 @@ extern "C" uslam_status uslam_match_noalloc(int device, int width, int height, i
     }
 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    uint32_t* derr = reinterpret_cast<uint32_t*>(base + err_off);
+    uint32_t* derr = &dtab->err;  // zero as the tables arrive
     int max_w = 1;
     for (int l = 0; l < levels; ++l) max_w = std::max(max_w, wl[l]);
     k_noalloc_tables<<<1, 256, 0, st>>>(t, dtab);
     e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaMemsetAsync(derr, 0, sizeof(uint32_t), st);  // the error word must start at zero
     if (e == cudaSuccess && (total[0] > 0 || total[1] > 0)) {
         k_noalloc_validate<<<ds.num_sms, 256, 0, st>>>(dtab, derr);
         e = cudaGetLastError();
