@@ -123,12 +123,14 @@ k_sampson(const double* __restrict__ fmats, int n_hyp, const double2* __restrict
         p = prev[i];
         q = curr[i];
     }
-    const float xp = (float)p.x, yp = (float)p.y, xc = (float)q.x, yc = (float)q.y, t = (float)thr;
-    const bool usual = fabsf(xp) < 1e9f && fabsf(yp) < 1e9f && fabsf(xc) < 1e9f && fabsf(yc) < 1e9f;
+    const float yp = (float)p.y, xc = (float)q.x, yc = (float)q.y, t = (float)thr;
+    float xp = (float)p.x;
+    // far coordinates are not certain: not a number here
+    if (!(fabsf(xp) < 1e9f && fabsf(yp) < 1e9f && fabsf(xc) < 1e9f && fabsf(yc) < 1e9f)) xp = __int_as_float(0x7fc00000);
     for (int k = 0; k < nh; ++k) {
         bool in = false;
         if (i < n) {
-            const int c = usual ? sampson_certain(s_h[k], xp, yp, xc, yc, t) : -1;
+            const int c = sampson_certain(s_h[k], xp, yp, xc, yc, t);
             in = c > 0;
             if (c < 0) {
                 double F[9];
