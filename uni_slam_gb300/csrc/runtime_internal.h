@@ -268,22 +268,25 @@ uslam_status encode_tile_maps(const FrameDev& F, int detector, void* out, ErrTex
 
 // Pinned staging of a call that takes and returns host buffers, grown on
 // demand up to kMax and kept (its owner's lock guards it); a call that needs
-// more copies from and to the caller's memory.
+// more copies from and to the caller's memory.  It at least doubles: a growth
+// takes 0.2 ms, four times a small call, and calls of ever more matches are
+// the rule while a map is built.
 struct PinnedBuf {
-    static constexpr size_t kMax = size_t(32) << 20;
+    static constexpr size_t kMin = size_t(256) << 10, kMax = size_t(32) << 20;
     char* p = nullptr;
     size_t bytes = 0;
     // false: too large, or refused; the call then copies directly
     bool reserve(size_t need) {
         if (need <= bytes) return true;
         if (need > kMax) return false;
+        const size_t grown = std::min(std::max({need, 2 * bytes, kMin}), kMax);
         release();
-        if (cudaHostAlloc(&p, need, cudaHostAllocDefault) != cudaSuccess) {
+        if (cudaHostAlloc(&p, grown, cudaHostAllocDefault) != cudaSuccess) {
             cudaGetLastError();
             p = nullptr;
             return false;
         }
-        bytes = need;
+        bytes = grown;
         return true;
     }
     void release() {
