@@ -21,7 +21,6 @@
 #include <chrono>
 #include <cmath>
 #include <cstring>
-#include <functional>
 #include <map>
 #include <mutex>
 #include <string>
@@ -824,30 +823,45 @@ void build_desc_table(const int32_t* pattern, DescTable* out) {
             if (px[*mx.second] - px[*mx.first] >= py[*my.second] - py[*my.first]) std::sort(a, a + size, by_x);
             else std::sort(a, a + size, by_y);
         }
-    std::vector<int> edges[N][N];  // [cluster][group]: points left
+    // the points of (cluster, group), as linked lists, and the groups a cluster has points of
+    int first[N][N], next[P];
+    uint32_t groups[N] = {};
+    std::fill(&first[0][0], &first[0][0] + N * N, -1);
     for (int i = 0; i < P; ++i) cluster[order[i]] = i / (P / N);
-    for (int i = 0; i < P; ++i) edges[cluster[i]][i / 64 * 2 + (i & 1)].push_back(i);  // point i: test i / 2
-    for (int lane = 0; lane < P / N; ++lane) {
+    for (int i = 0; i < P; ++i) {
+        const int c = cluster[i], g = i / 64 * 2 + (i & 1);  // point i: test i / 2
+        next[i] = first[c][g];
+        first[c][g] = i;
+        groups[c] |= 1u << g;
+    }
+    struct Matching {
+        const uint32_t* groups;
         int of_group[N];
-        std::fill(of_group, of_group + N, -1);
-        for (int c = 0; c < N; ++c) {
-            bool seen[N] = {false};
-            std::function<bool(int)> augment = [&](int u) {
-                for (int g = 0; g < N; ++g) {
-                    if (seen[g] || edges[u][g].empty()) continue;
-                    seen[g] = true;
-                    if (of_group[g] < 0 || augment(of_group[g])) {
-                        of_group[g] = u;
-                        return true;
-                    }
+        uint32_t seen;
+        bool augment(int u) {
+            for (int g = 0; g < N; ++g) {
+                if (!((groups[u] & ~seen) >> g & 1u)) continue;
+                seen |= 1u << g;
+                if (of_group[g] < 0 || augment(of_group[g])) {
+                    of_group[g] = u;
+                    return true;
                 }
-                return false;
-            };
-            augment(c);
+            }
+            return false;
+        }
+    };
+    static_assert(N <= 32, "a word per cluster's groups");
+    for (int lane = 0; lane < P / N; ++lane) {
+        Matching m{groups, {}, 0u};
+        std::fill(m.of_group, m.of_group + N, -1);
+        for (int c = 0; c < N; ++c) {
+            m.seen = 0u;
+            m.augment(c);
         }
         for (int g = 0; g < N; ++g) {
-            const int c = of_group[g], i = edges[c][g].back();
-            edges[c][g].pop_back();
+            const int c = m.of_group[g], i = first[c][g];
+            first[c][g] = next[i];
+            if (next[i] < 0) groups[c] &= ~(1u << g);
             out->pts[c][lane][0] = static_cast<float>(px[i]);
             out->pts[c][lane][1] = static_cast<float>(py[i]);
             const int test = i / 2, shift = (i & 1) * 16;
@@ -1012,20 +1026,20 @@ uslam_status uslam_create(const uslam_params* params, uslam_ctx** out) {
     cudaError_t e = cudaSetDevice(c->device);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, c->device);
     if (e == cudaSuccess) e = init_constants();
-    if (e == cudaSuccess) e = cudaMalloc(&c->d_pattern, 1024 * sizeof(int32_t));
-    if (e == cudaSuccess)
-        e = cudaMemcpy(c->d_pattern, params->brief_pattern, 1024 * sizeof(int32_t), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMalloc(&c->d_desc, sizeof(DescTable));
-    if (e == cudaSuccess) {
-        DescTable table;
-        build_desc_table(params->brief_pattern, &table);
-        e = cudaMemcpy(c->d_desc, &table, sizeof(table), cudaMemcpyHostToDevice);
-    }
+    // the pattern and its table, one allocation and one copy
+    struct {
+        int32_t pattern[1024];
+        DescTable desc;
+    } tables;
+    std::memcpy(tables.pattern, params->brief_pattern, sizeof tables.pattern);
+    build_desc_table(tables.pattern, &tables.desc);
+    if (e == cudaSuccess) e = cudaMalloc(&c->d_pattern, sizeof tables);
+    if (e == cudaSuccess) e = cudaMemcpy(c->d_pattern, &tables, sizeof tables, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) c->d_desc = reinterpret_cast<DescTable*>(c->d_pattern + 1024);
     if (e == cudaSuccess) e = set_describe_smem();
     if (e != cudaSuccess) {
         cudaGetLastError();
         if (c->d_pattern) cudaFree(c->d_pattern);
-        if (c->d_desc) cudaFree(c->d_desc);
         delete c;
         return e == cudaErrorMemoryAllocation ? USLAM_OOM : USLAM_CUDA_ERROR;
     }
@@ -1044,7 +1058,6 @@ void uslam_destroy(uslam_ctx* c) {
     c->ransac_pin.release();
     c->tri_pin.release();
     if (c->d_pattern) cudaFree(c->d_pattern);
-    if (c->d_desc) cudaFree(c->d_desc);
     delete c;
 }
 

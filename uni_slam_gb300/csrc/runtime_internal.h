@@ -334,7 +334,7 @@ struct uslam_ctx {
         return it == tile_shape.end() ? 0 : it->second;
     }
     int32_t* d_pattern = nullptr;
-    DescTable* d_desc = nullptr;  // the same points as k_describe takes them
+    DescTable* d_desc = nullptr;  // the same points as k_describe takes them (behind d_pattern)
     ErrText err;
     std::map<std::pair<int, int>, ResClass> classes;
 
