@@ -794,7 +794,8 @@ uslam_status create_batch(uslam_ctx* ctx, int n_frames, const int* widths, const
         }
         cur += P->host.size();
     }
-    if ((s = capture_graph(b, &b->full)) != USLAM_OK) {
+    // (owners of per-item programs launch those, never the whole)
+    if (!per_item_programs && (s = capture_graph(b, &b->full)) != USLAM_OK) {
         free_batch(b);
         return s;
     }
