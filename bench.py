@@ -363,7 +363,7 @@ def run_reference(a):
     from uni_slam_gb300 import pattern as patmod
     from uni_slam_gb300 import synth
 
-    pat = patmod.load()
+    pat, table = patmod.load_or_stand_in()
     frames = synth.plane_sequence(a.seed, n=a.frames)
     _, kind = _matcher()
     cores = os.cpu_count() or 1
@@ -382,7 +382,7 @@ def run_reference(a):
     line = {
         "impl": "reference", "metric": METRIC, "value": value, "unit": "frames/s", "n_gpus": a.gpus,
         "steps": a.steps, "warmup": a.warmup, "ms_per_step": step_s * 1e3, "higher_is_better": True,
-        "scaling": "weak", "vs_baseline": None, "dtype": "f32+u32", "data": "synthetic (seeded plane trajectory; EuRoC absent)",
+        "scaling": "weak", "vs_baseline": None, "dtype": "f32+u32", "data": f"synthetic (seeded plane trajectory; EuRoC absent; {table})",
         "config": _config(a.frames, a.seed, world),
         "cpu_baseline": {"value": value, "unit": "frames/s", "cores": cores, "kind": kind,
                          "sample": f"the full {a.frames}-frame step on a {cores}-process pool; "
@@ -1147,7 +1147,7 @@ def run_ours(a):
     from uni_slam_gb300 import pattern as patmod
     from uni_slam_gb300 import synth
 
-    pat = patmod.load()
+    pat, table = patmod.load_or_stand_in()
     frames = synth.plane_sequence(a.seed + rank, n=a.frames)
     n = len(frames)
     # the served streams' trajectories, rendered before any GPU work
@@ -1389,7 +1389,7 @@ def run_ours(a):
         line = {
             "metric": METRIC, "value": value, "unit": "frames/s", "n_gpus": world, "steps": a.steps,
             "warmup": a.warmup, "ms_per_step": step_ms_max, "higher_is_better": True, "scaling": "weak",
-            "vs_baseline": None, "dtype": "f32+u32", "data": "synthetic (seeded plane trajectory; EuRoC absent)",
+            "vs_baseline": None, "dtype": "f32+u32", "data": f"synthetic (seeded plane trajectory; EuRoC absent; {table})",
             "config": _config(n, a.seed, world),
             "plain_fps": plain_fps, "batched_over_plain": value / world / plain_fps, "plugin_e2e": plugin,
             "e2e": {"value": n * world / e2e_s, "unit": "frames/s", "h2d_bytes_per_step": h2d,
