@@ -260,8 +260,6 @@ def algorithmic_bytes(kept_per_frame: list[int], matches_per_pair: list[int], fr
     M = sum(kept_per_frame[:-1])  # each pair's reference set is the previous frame
     K = sum(matches_per_pair)
     total = frames * (wh + 4 * (P - wh)) + 48 * N + 32 * (N + M) + 8 * K
-    margin = 21  # blur-cache margin beyond each level edge (pattern radius + 2)
-    border = sum((w + margin + 1) * (h + margin + 1) - w * h for w, h in dims)
     return {
         "pyramid_per_frame": wh + 4 * (P - wh),
         "describe_total": 48 * N,
@@ -269,10 +267,31 @@ def algorithmic_bytes(kept_per_frame: list[int], matches_per_pair: list[int], fr
         "total_per_step": total,
         # per-kernel shares outside the path model, for the roofline of whichever kernel dominates:
         "detect_total": frames * 5 * P,        # f32 level tiles read + u8 keypoint maps written
-        "border_total": frames * 4 * border,   # blur-cache border cells written (f32)
         "compact_total": frames * P + 12 * N,  # keypoint maps read (u8) + feature headers written
         "mutual_total": 16 * K + 8 * M,        # match records written + direction tables read
     }
+
+
+def blur_bytes(features, dims, reach=20):
+    """Level cells read and cache cells written (f32) by k_blur: the 64 x 32
+    tiles of each level that a test of a kept keypoint can read (reach = the
+    pattern's radius + 1; the cells beyond the levels are left out).
+    features: (records, kept per level) of every frame."""
+    import numpy as np
+
+    cells = 0
+    for feats, kept in features:
+        off = np.concatenate([[0], np.cumsum(kept)]).astype(int)
+        for l, (w, h) in enumerate(dims):
+            x, y = (feats[k][off[l]:off[l + 1]].astype(np.int64) for k in ("x", "y"))
+            need = np.zeros(((h + 31) // 32, (w + 63) // 64), bool)
+            for dy in range(-reach, reach + 1, reach):  # (at most a tile's height and width apart)
+                for dx in range(-reach, reach + 1, reach):
+                    need[np.clip(y + dy, 0, h - 1) // 32, np.clip(x + dx, 0, w - 1) // 64] = True
+            tall = np.minimum(32, h - 32 * np.arange(need.shape[0]))
+            wide = np.minimum(64, w - 64 * np.arange(need.shape[1]))
+            cells += int(tall @ need @ wide)
+    return 8 * cells
 
 
 # ------------------------------------------------------------------ CPU side
@@ -1143,7 +1162,7 @@ def run_ours(a):
             dist.barrier()
         torch.cuda.synchronize()
 
-    from uni_slam_gb300 import Batch, Context, Frontend
+    from uni_slam_gb300 import Batch, Context, Frontend, level_dims
     from uni_slam_gb300 import pattern as patmod
     from uni_slam_gb300 import synth
 
@@ -1200,7 +1219,8 @@ def run_ours(a):
     # ---- results of one step (counts for the byte model)
     batch.download()
     batch.sync()
-    kept = [int(batch.features(i)[1].sum()) for i in range(n)]
+    sets = [batch.features(i)[:2] for i in range(n)]
+    kept = [int(k.sum()) for _, k in sets]
     nmatch = [len(batch.matches(p)) for p in range(n - 1)]
     nbytes = algorithmic_bytes(kept, nmatch, n)
     main_lists = [_mm_digest(batch.matches(p)) for p in range(n - 1)]
@@ -1212,7 +1232,7 @@ def run_ours(a):
     kernel_bytes = {
         "k_pyramid": nbytes["pyramid_per_frame"] * n,
         "k_detect": nbytes["detect_total"],
-        "k_blur_border": nbytes["border_total"],
+        "k_blur_border": blur_bytes(sets, level_dims(W, H, LEVELS)),
         "compaction": nbytes["compact_total"],
         "k_describe": nbytes["describe_total"],
         "k_match": nbytes["match_total"],
@@ -1242,6 +1262,8 @@ def run_ours(a):
     # every kernel's own line: its algorithmic bytes / its event-timed launch,
     # its DRAM traffic per launch from the committed captures, its SM side
     pipes = measured_pipes()
+    roofline["stages"] = {"k_blur_border": "k_blur, the blur cache where kept keypoints' tests read it",
+                          "compaction": "k_band_write and k_xsort"}
     roofline["per_kernel"] = {
         k: {"ms": prof[k], "algorithmic_bytes": kernel_bytes[k],
             "achieved": kernel_bytes[k] / (prof[k] / 1e3) / 1e9,

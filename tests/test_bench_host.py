@@ -151,3 +151,24 @@ def test_native_server_client_compiles(tmp_path):
     # wrong argument count: usage and exit code 2, no device touched
     r = subprocess.run([str(exe)], capture_output=True, text=True)
     assert r.returncode == 2 and "usage" in r.stderr
+
+
+def test_blur_bytes_counts_the_tiles_tests_can_read():
+    """The blur stage's byte model against a cell by cell count."""
+    import numpy as np
+
+    from uni_slam_gb300.capi import FEATURE_DTYPE
+
+    dims, reach, rs = [(150, 90), (125, 75), (33, 31)], 20, np.random.RandomState(3)
+    for n in (0, 1, 4, 40):
+        kept = np.array([n, n // 2, n // 3])
+        f = np.zeros(kept.sum(), FEATURE_DTYPE)
+        off = np.concatenate([[0], np.cumsum(kept)])
+        cells = 0
+        for l, (w, h) in enumerate(dims):
+            part = f[off[l]:off[l + 1]]
+            part["x"], part["y"] = rs.randint(0, w, kept[l]), rs.randint(0, h, kept[l])
+            tiles = {(yy // 32, xx // 64) for r in part for yy in range(int(r["y"]) - reach, int(r["y"]) + reach + 1)
+                     for xx in range(int(r["x"]) - reach, int(r["x"]) + reach + 1) if 0 <= yy < h and 0 <= xx < w}
+            cells += sum(min(32, h - 32 * ty) * min(64, w - 64 * tx) for ty, tx in tiles)
+        assert bench.blur_bytes([(f, kept)], dims, reach) == 8 * cells
