@@ -191,18 +191,12 @@ __device__ __forceinline__ float2 mul2_rn(float2 a, float2 b) {
     return d;
 }
 
-// f32(u8) / 255, correctly rounded: u hi + u lo in one fused step with
-// hi + lo = 1/255 to 48 bits (multiplication by a constant held as two words,
-// Brisebarre and Muller 2008); equal to the quotient for all 256 bytes.  Four
-// arithmetic instructions; a 256-entry shared table cost a load with bank
-// conflicts each (k_pyramid on 32 frames of 752x480: 67 us with the table).
-__device__ __forceinline__ float unit_u8(uint32_t byte) {
-    constexpr float hi = 1.0f / 255.0f, lo = (float)(1.0 / 255.0 - (double)hi);
-    const float u = __uint_as_float(0x4B000000u | byte) - 8388608.0f;
-    return __fmaf_rn(u, hi, u * lo);
-}
-
-// Two of them, in packed steps: five instructions instead of eight.
+// f32(u8) / 255 of two bytes, correctly rounded: u hi + u lo in one fused step
+// with hi + lo = 1/255 to 48 bits (multiplication by a constant held as two
+// words, Brisebarre and Muller 2008); equal to the quotient for all 256 bytes.
+// Five packed instructions (u is the byte as the low bits of 2^23 + u, less
+// 2^23); a 256-entry shared table cost a load with bank conflicts each
+// (k_pyramid on 32 frames of 752x480: 67 us with the table).
 __device__ __forceinline__ float2 unit2_u8(uint32_t b0, uint32_t b1) {
     constexpr float hi = 1.0f / 255.0f, lo = (float)(1.0 / 255.0 - (double)hi);
     float2 d;
@@ -212,18 +206,6 @@ __device__ __forceinline__ float2 unit2_u8(uint32_t b0, uint32_t b1) {
         : "=f"(d.x), "=f"(d.y)
         : "f"(__uint_as_float(0x4B000000u | b0)), "f"(__uint_as_float(0x4B000000u | b1)), "f"(-8388608.0f), "f"(hi), "f"(lo));
     return d;
-}
-
-// Left-to-right sum of four packed products, lane by lane, in scalar adds.
-__device__ __forceinline__ float2 sum4(float2 p, float2 q, float2 r, float2 t) {
-    float x = p.x, y = p.y;
-    x = x + q.x;
-    y = y + q.y;
-    x = x + r.x;
-    y = y + r.y;
-    x = x + t.x;
-    y = y + t.y;
-    return make_float2(x, y);
 }
 
 // ------------------------------------------------------ TMA + mbarrier ----
@@ -2745,7 +2727,6 @@ __global__ void __launch_bounds__(128) k_frame_from_f32(const float* __restrict_
 // ------------------------------------------------------------ launch ----
 namespace uslam {
 
-cudaError_t init_constants() { return cudaSuccess; }
 
 template <bool CFG>
 cudaError_t launch_detect_profile(const FrameDev* frames, const TileItem* tiles, int ntiles, int shape, uint32_t* err,

@@ -252,7 +252,7 @@ cudaError_t enqueue_frames(uslam_batch* b, const Program& P, const Lane& ln) {
     cudaError_t e = cudaSuccess;
     if (P.ntiles <= 0) return e;
     if ((e = launch_pyramid_shaped(b->d_frames, P.tiles, P.tile_begin, P.blur.count, ln.st)) != cudaSuccess) return e;
-    if ((e = launch_detect_only_shaped(b->d_frames, P.tiles, P.tile_begin, c->detector, b->d_err, ln.st)) !=
+    if ((e = launch_detect_shaped(b->d_frames, P.tiles, P.tile_begin, c->detector, b->d_err, ln.st)) !=
         cudaSuccess)
         return e;
     if ((e = launch_compact_banded(b->d_frames, P.bands, P.nbands, c->cell_cap, P.blur, ln.st)) != cudaSuccess) return e;
@@ -875,7 +875,6 @@ void build_desc_table(const int32_t* pattern, DescTable* out) {
 uslam_status report_err_word(uslam_batch* b, uint32_t word) {
     if (word != 0u) {
         std::string m = "kernel bounds check tripped:";
-        if (word & USLAM_ERR_SMEM_RANGE) m += " blur tap outside the staged tile;";
         if (word & USLAM_ERR_MATCH_OVERFLOW) m += " match list overflow;";
         if (word & USLAM_ERR_TMA_TIMEOUT) m += " tile load wait limit reached;";
         return set_err(b->err(), USLAM_KERNEL_CHECK, m);
@@ -1026,7 +1025,6 @@ uslam_status uslam_create(const uslam_params* params, uslam_ctx** out) {
     c->margin = static_cast<int>(std::ceil(rmax)) + 2;
     cudaError_t e = cudaSetDevice(c->device);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, c->device);
-    if (e == cudaSuccess) e = init_constants();
     // the pattern and its table, one allocation and one copy
     struct {
         int32_t pattern[1024];

@@ -23,7 +23,6 @@ struct MatchSegDev {
     int dir;
     int level;
 };
-cudaError_t init_constants();
 cudaError_t launch_detect(const FrameDev*, const TileItem*, int, int, int, uint32_t*, cudaStream_t);
 // blur_count: the run's BlurList::count, cleared (null: none)
 cudaError_t launch_pyramid(const FrameDev*, const TileItem*, int, int, uint32_t* blur_count, cudaStream_t);
@@ -211,22 +210,8 @@ inline cudaError_t launch_pyramid_shaped(const FrameDev* frames, const TileItem*
     return cudaSuccess;
 }
 // One k_detect launch per tile shape present (after every pyramid level is written).
-inline cudaError_t launch_detect_only_shaped(const FrameDev* frames, const TileItem* d_tiles, const int* begin,
-                                             int detector, uint32_t* err, cudaStream_t st) {
-    for (int s = 0; s < kNumTileShapes; ++s) {
-        const int n = begin[s + 1] - begin[s];
-        if (n <= 0) continue;
-        const cudaError_t e = launch_detect(frames, d_tiles + begin[s], n, s, detector, err, st);
-        if (e != cudaSuccess) return e;
-    }
-    return cudaSuccess;
-}
-// One k_pyramid launch, then one k_detect launch, per tile shape present
-// (every pyramid level is written before any tile of that shape reads it).
 inline cudaError_t launch_detect_shaped(const FrameDev* frames, const TileItem* d_tiles, const int* begin,
-                                        int detector, uint32_t* err, uint32_t* blur_count, cudaStream_t st) {
-    const cudaError_t e = launch_pyramid_shaped(frames, d_tiles, begin, blur_count, st);
-    if (e != cudaSuccess) return e;
+                                        int detector, uint32_t* err, cudaStream_t st) {
     for (int s = 0; s < kNumTileShapes; ++s) {
         const int n = begin[s + 1] - begin[s];
         if (n <= 0) continue;

@@ -326,7 +326,8 @@ cudaError_t launch_batch(uslam_server* s, const std::vector<uint64_t>& tickets, 
     const auto* d_desc = reinterpret_cast<const BandItem*>(B.d + t_b + f_b + m_b + u_b + p_b + b_b + x_b);
     const BlurList bl{reinterpret_cast<TileItem*>(B.d + B.bytes + 256), reinterpret_cast<uint32_t*>(B.d + B.bytes)};
     const int nf = static_cast<int>(fsegs.size());
-    if ((e = launch_detect_shaped(s->d_frames, d_tiles, shaped.begin, c->detector, s->d_err, bl.count, st)) != cudaSuccess) return e;
+    if ((e = launch_pyramid_shaped(s->d_frames, d_tiles, shaped.begin, bl.count, st)) != cudaSuccess) return e;
+    if ((e = launch_detect_shaped(s->d_frames, d_tiles, shaped.begin, c->detector, s->d_err, st)) != cudaSuccess) return e;
     if ((e = launch_compact_banded(s->d_frames, d_bands, static_cast<int>(bands.size()), c->cell_cap, bl, st)) != cudaSuccess)
         return e;
     if ((e = launch_xsort(s->d_frames, d_fsegs, nf, s->max_w, s->max_bands, st)) != cudaSuccess) return e;

@@ -41,7 +41,6 @@
 #include <vector_types.h>
 
 #define USLAM_MAX_LEVELS 12
-#define USLAM_MAX_BANDS 24  // most horizontal bands of a frame for the matcher's lists (FrameDev::nbands)
 #define USLAM_MAX_MATCH_SEGS 2048  // (pair, level) segments of one k_match launch
 
 // Device copy of one frame's geometry and buffer addresses.
@@ -54,7 +53,7 @@ struct FrameDev {
     int bl_pitch[USLAM_MAX_LEVELS];  // blur cache row pitch (floats): w + margin + 1
     int lvl_pitch[USLAM_MAX_LEVELS]; // pyramid level row pitch (floats): w rounded up to 4
     int margin;                      // blur cache margin M beyond the level
-    int nbands;                      // horizontal bands of the matcher's lists (1 .. USLAM_MAX_BANDS)
+    int nbands;                      // horizontal bands of the matcher's lists
     int cell_cap;                    // > 0: keypoints kept per 32x32 cell (cell order); 0: (y, x) order
     int frame_cap;                   // > 0: features kept per frame, levels filled in order; 0: none
     // polls of the first mbarrier wait of k_detect's tile load and of the
@@ -199,7 +198,6 @@ struct DescTable {
     uint32_t pair[8][32];
 };
 
-#define USLAM_ERR_SMEM_RANGE 1u
 #define USLAM_ERR_MATCH_OVERFLOW 2u
 #define USLAM_ERR_TMA_TIMEOUT 4u  // a tile load did not complete within the wait limit
 
