@@ -176,11 +176,11 @@ __device__ __forceinline__ float cfg_corner(const float (*sm)[SW], int r, int c,
 
 // Packed binary32 products (sm_100 family mul.f32x2): one instruction rounds
 // each lane to nearest even exactly as the scalar mul.rn would, so two
-// independent products cost one issue slot with unchanged bits.  Sums stay
-// scalar: ptxas (CUDA 13.0) contracts mul.rn.f32x2 feeding add.rn.f32x2 into
-// one fused multiply-add (a single rounding) in spite of .rn and
-// --fmad=false, while a packed product feeding a scalar add.rn is kept as two
-// roundings.
+// independent products cost one issue slot with unchanged bits.  Their sums
+// are scalar here and take another form in k_blur (add2): ptxas (CUDA 13.0)
+// contracts mul.rn.f32x2 feeding add.rn.f32x2 into one fused multiply-add (a
+// single rounding) in spite of .rn and --fmad=false, while a packed product
+// feeding a scalar add.rn is kept as two roundings.
 __device__ __forceinline__ float2 mul2_rn(float2 a, float2 b) {
     float2 d;
     asm("{\n\t.reg .b64 pa, pb, pd;\n\t"
@@ -610,9 +610,9 @@ k_detect(const FrameDev* __restrict__ frames, const TileItem* __restrict__ tiles
 // workload (the level caps keep the first features in (y, x) order, so the
 // lower part of most levels holds none), 55 % at 1920x1080 and a few per cent
 // where a frame cap of 20000 is used up by the first level of a 4K frame.
-// 64 frames of 752x480: 0.24 ms here and 0.31 in k_detect, where evaluating
+// 64 frames of 752x480: 0.25 ms here and 0.16 in k_detect, where evaluating
 // every pixel in k_detect and the margins in a kernel of their own took 0.72
-// and 0.20; 8 frames of 3840x2160 with that cap: 0.16 and 0.59 against 1.77
+// and 0.20; 8 frames of 3840x2160 with that cap: 0.16 and 0.40 against 1.77
 // and 0.13.
 constexpr int KBL_THREADS = 128;
 constexpr int KBL_TW = USLAM_BLUR_TW, KBL_TH = USLAM_BLUR_TH;
@@ -2365,7 +2365,7 @@ k_bacc_init(const FrameDev* __restrict__ frames, const PairDev* __restrict__ pai
 // ----------------------------------------------------- brute force ----
 constexpr int KB_THREADS = 64;
 constexpr int KB_CTAS = 512 / KB_THREADS;  // per SM
-constexpr int KB_PAIRS = 2;      // pairs of queries per thread: 512 queries per CTA
+constexpr int KB_PAIRS = 2;      // pairs of queries per thread: 256 queries per CTA
 constexpr int KB_Q = 2 * KB_PAIRS;
 constexpr int KB_TILE = 128;     // train descriptors per shared-memory tile
 static_assert(256 * KB_TILE + KB_TILE - 1 < 0xffff, "distance and tile slot share 16 bits");

@@ -224,12 +224,15 @@ inline cudaError_t launch_detect_shaped(const FrameDev* frames, const TileItem* 
 // Horizontal bands of the matcher's lists for levels of up to cap features.
 // A band's lists hold the rows of its queries and 0.1 H each side, so more
 // bands leave fewer candidates outside the windows, but a group of 32 queries
-// (128 with the tensor cores) then reaches further in x.  Measured with k_match:
-// 64 frames of 752x480 (cap 1443) with 3, 4, 5, 6 and 8 bands 1455, 1427, 1443,
-// 1460, 1519 us a step; the mixed batch (caps 1228, 1443, 3686, 8294, 33177) with
-// 3/4/6/10 bands 4757, 3/4/8/14 4703, 3/6/10/14 4688, 3/6/10/20 4698 us.  On the
-// tensor cores: one 1920x1080 frame with 2, 3, 4, 6, 8, 12 bands 790, 767, 753, 769,
-// 765, 841 us, one 752x480 frame 307, 305, 310, 316 ... us.
+// (128 with the tensor cores) then reaches further in x.  Measured with k_match
+// (two runs of one side differ by 0.5 %): 32 frames of 752x480 (cap 1443) with
+// 3 and 4 bands 721 and 707 us, 64 of them with 4, 5, 6 and 8 1427, 1443, 1460
+// and 1519; 16 frames of 1280x720 (3686) with 3, 4 and 6 1274, 1221 and 1181;
+// one of 1920x1080 (8294) with 3, 6 and 10 597, 566 and 545; the mixed batch
+// with 3 for every cap 5054, with 10 for its 3840x2160 frames (33177) and 6 for
+// 1920x1080 4465, with 14 and 10 4430, with 20 and 10 no better.  On the tensor
+// cores: one 1920x1080 frame with 2, 3, 4, 6, 8, 12 bands 790, 767, 753, 769, 765,
+// 841 us, one 752x480 frame 307, 305, 310, 316 ... us.
 inline int match_bands_for(int cap, bool win_tc) {
     if (win_tc) return cap > 5000 ? 4 : 3;
     return cap > 16000 ? 14 : cap > 5000 ? 10 : cap > 2500 ? 6 : 4;

@@ -21,7 +21,9 @@
 //                                          radius + 2, bl_pitch_l = w_l + M + 1.
 //                                          Evaluated per run in the blur tiles that a test
 //                                          of a kept keypoint can read (k_blur)
-//   btile[l] u32  [USLAM_BLUR_TILES]       1 where the run needs the blur item
+//   btile[l] u32  [USLAM_BLUR_TILES]       1 where the run needs the blur item (k_pyramid
+//                                          clears, k_band_write sets; a served slot keeps
+//                                          them in its blur cache)
 //   kpmap[l] u8   [h_l][kp_pitch_l]        culled FAST strength (0 = no keypoint)
 //   bands[l] u32  [ceil(h_l / 32)][2]      raw and kept keypoint counts per 32-row band
 //   feats[l] Feature[cap]                  gpumodels::Feature records, (y, x) order
@@ -63,7 +65,7 @@ struct FrameDev {
     float* lvl[USLAM_MAX_LEVELS];
     const void* tmaps;  // CUtensorMap [levels][USLAM_TMAPS_PER_LEVEL] (device, 64-byte aligned)
     float* blur[USLAM_MAX_LEVELS];
-    uint32_t* btile[USLAM_MAX_LEVELS];       // blur tiles the run needs (k_band_write sets, k_band_count clears)
+    uint32_t* btile[USLAM_MAX_LEVELS];       // blur items the run needs (k_pyramid clears, k_band_write sets)
     uint8_t* kpmap[USLAM_MAX_LEVELS];
     uint32_t* bands[USLAM_MAX_LEVELS];       // per 32-row band: raw and kept keypoint counts
     const uint32_t* mask[USLAM_MAX_LEVELS];  // combined cull coverage bitmap
