@@ -821,8 +821,9 @@ void build_desc_table(const int32_t* pattern, DescTable* out) {
             const auto by_x = [&](int i, int j) { return px[i] != px[j] ? px[i] < px[j] : i < j; };
             const auto by_y = [&](int i, int j) { return py[i] != py[j] ? py[i] < py[j] : i < j; };
             const auto mx = std::minmax_element(a, a + size, by_x), my = std::minmax_element(a, a + size, by_y);
-            if (px[*mx.second] - px[*mx.first] >= py[*my.second] - py[*my.first]) std::sort(a, a + size, by_x);
-            else std::sort(a, a + size, by_y);
+            int* const half = a + size / 2;
+            if (px[*mx.second] - px[*mx.first] >= py[*my.second] - py[*my.first]) std::nth_element(a, half, a + size, by_x);
+            else std::nth_element(a, half, a + size, by_y);
         }
     // the points of (cluster, group), as linked lists, and the groups a cluster has points of
     int first[N][N], next[P];
